@@ -125,6 +125,41 @@ def test_selective_scan_alone(dtype, sizes):
         assert _rel(kept, last) < 2e-5, cuts
 
 
+@pytest.mark.parametrize("lengths", [(1, 64, 65), (128, 2, 1, 129, 31), (200,)], ids=str)
+@pytest.mark.parametrize("sizes", [(130, 16), (37, 5), (129, 32)], ids=str)
+def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
+    """Requests around the segments' edges side by side, each going on in a second step, against the recurrence in float64; slots
+    that are not theirs by number and the entries around the piece stay as they are. bfloat16 rounds an output to 2^-9 of
+    itself; the float32 state between the segments stays within 2e-5 of the largest entry, as token by token."""
+    from llm_pipeline_b200.ops import kernels
+    monkeypatch.setattr(kernels, "SCAN_SEGMENTS_MIN_TOKENS", 1)
+    inner, states = sizes
+    gen = torch.Generator().manual_seed(inner + states + sum(lengths))
+    dt_bias, skip = torch.randn(inner, generator=gen) * 0.5 - 1.0, torch.randn(inner, generator=gen)
+    A = -torch.exp(torch.rand(inner, states, generator=gen) * 5.0 - 4.5)
+    R, offset, entries = len(lengths), 6, 2 * inner * states
+    state = torch.full((R + 2, offset + entries + 3), 5.0, device=DEV)
+    slots = list(range(R, 0, -1))
+    state[slots] = 0.0
+    rows = [tuple(torch.randn(2 * n, width, generator=gen) for width in (inner, inner, inner, 3 + 2 * states)) for n in lengths]
+    want, last = [], []
+    for x, raw, z, bc in rows:
+        dt = torch.nn.functional.softplus(raw.double() + dt_bias.double())
+        y, S = plain.scan(x.double(), dt, A.double(), bc[:, 3:3 + states].double(), bc[:, 3 + states:].double(), skip.double())
+        want.append(y * plain.silu(z.double()))
+        last.append(S)
+    for step in range(2):
+        x, raw, z, bc = (torch.cat([r[k][step * n:(step + 1) * n] for r, n in zip(rows, lengths)]).to(DEV) for k in range(4))
+        out = torch.empty(x.shape, device=DEV, dtype=torch.bfloat16)
+        kernels.selective_scan(x, raw, dt_bias.to(DEV), bc[:, 3:3 + states], bc[:, 3 + states:], A.to(DEV), skip.to(DEV), z, state, offset,
+                               _i32([0] + list(itertools.accumulate(lengths))), _i32(slots),
+                               _i32([p for n in lengths for p in range(step * n, (step + 1) * n)]), out, max(lengths))
+        assert _rel(out, torch.cat([w[step * n:(step + 1) * n] for w, n in zip(want, lengths)])) < 4e-3, step
+    for slot, n, S in zip(slots, lengths, last):
+        assert _rel(state[slot, offset:offset + entries].view(2, inner, states)[(2 * n - 1) & 1], S) < 2e-5
+    assert (state[[0, R + 1]] == 5.0).all() and (state[slots, :offset] == 0.0).all() and (state[slots, offset + entries:] == 0.0).all()
+
+
 def _window_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap, size, keep, plant=None, rows=None, gate=True):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine output, plain output) for
     the token rows ``rows`` (all by default), each launched as the portion it is."""
