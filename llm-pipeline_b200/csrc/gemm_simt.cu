@@ -4,62 +4,114 @@
 // row's result does not depend on how many other rows are in the call.
 #include "common.cuh"
 
-#define GT_BM 64
-#define GT_BN 64
-#define GT_BK 16
+namespace {
 
-template <typename TI, typename TO>
-__global__ void __launch_bounds__(256)
+// Four consecutive entries of a row from k on; entries from K on are 0. VEC: 4-entry pieces are aligned and K is a multiple of 4.
+template <bool VEC> __device__ __forceinline__ float4 gt_load4(const float* row, int k, int K) {
+    if (VEC) return k < K ? *reinterpret_cast<const float4*>(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(k < K ? row[k] : 0.f, k + 1 < K ? row[k + 1] : 0.f, k + 2 < K ? row[k + 2] : 0.f, k + 3 < K ? row[k + 3] : 0.f);
+}
+template <bool VEC> __device__ __forceinline__ float4 gt_load4(const bf16* row, int k, int K) {
+    if (VEC) {
+        if (k >= K) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint2 raw = *reinterpret_cast<const uint2*>(row + k);
+        const __nv_bfloat162* v = reinterpret_cast<const __nv_bfloat162*>(&raw);
+        return make_float4(__low2float(v[0]), __high2float(v[0]), __low2float(v[1]), __high2float(v[1]));
+    }
+    return make_float4(k < K ? to_float(row[k]) : 0.f, k + 1 < K ? to_float(row[k + 1]) : 0.f, k + 2 < K ? to_float(row[k + 2]) : 0.f,
+                       k + 3 < K ? to_float(row[k + 3]) : 0.f);
+}
+
+// A block makes BM x BN outputs with TM x TN of them a thread. BK entries of K at a time lie in shared memory as rows padded by 4
+// (a quarter-warp's 16-byte reads of consecutive rows meet no bank twice), in two buffers, one barrier for each; those of the next
+// AHEAD are on their way in registers. A thread reads 4 entries of K of its TM + TN rows as 16-byte words for 4 TM TN multiply-adds.
+template <typename TI, typename TO, int BM, int BN, int BK, int TM, int TN, int AHEAD, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* __restrict__ bias, int bias_bf16,
-               TO* __restrict__ C, int M, int N, int K, long lda, long ldw, long ldc, long batch_a = 0, long batch_w = 0,
-               long batch_c = 0) {
+               TO* __restrict__ C, int M, int N, int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c) {
+    constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY, QUADS = BK / 4, LD = BK + 4;
+    constexpr int LA = BM * QUADS / THREADS, LW = BN * QUADS / THREADS;      // 4-entry pieces of each operand a thread brings
+    static_assert(LA * THREADS == BM * QUADS && LW * THREADS == BN * QUADS, "the pieces of a tile are shared out evenly");
     // blockIdx.z counts the products of a batch: each has its own A, W and C, the given strides apart
     A += (size_t)blockIdx.z * batch_a;
     W += (size_t)blockIdx.z * batch_w;
     C += (size_t)blockIdx.z * batch_c;
-    __shared__ float As[GT_BK][GT_BM + 4];
-    __shared__ float Ws[GT_BK][GT_BN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * GT_BM, n0 = blockIdx.x * GT_BN;
-    float acc[4][4];
+    __shared__ __align__(16) float As[2][BM * LD], Ws[2][BN * LD];
+    const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float acc[TM][TN] = {};
+    float4 ra[AHEAD][LA], rw[AHEAD][LW];
+    auto fetch = [&](int k0, float4 (&pa)[LA], float4 (&pw)[LW]) {           // past the end of K: zeros, without a read
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-    for (int k0 = 0; k0 < K; k0 += GT_BK) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = tid + 256 * r;
-            const int row = e >> 4, col = e & 15;
-            const int k = k0 + col;
-            const int m = m0 + row, n = n0 + row;
-            As[col][row] = (m < M && k < K) ? to_float(A[(size_t)m * lda + k]) : 0.f;
-            Ws[col][row] = (n < N && k < K) ? to_float(W[(size_t)n * ldw + k]) : 0.f;
+        for (int r = 0; r < LA; ++r) {
+            const int e = tid + r * THREADS, m = m0 + e / QUADS;
+            pa[r] = m < M ? gt_load4<VEC>(A + (size_t)m * lda, k0 + e % QUADS * 4, K) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        __syncthreads();
 #pragma unroll
-        for (int k = 0; k < GT_BK; ++k) {
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int r = 0; r < LW; ++r) {
+            const int e = tid + r * THREADS, n = n0 + e / QUADS;
+            pw[r] = n < N ? gt_load4<VEC>(W + (size_t)n * ldw, k0 + e % QUADS * 4, K) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        __syncthreads();
+    };
+    auto keep = [&](int buffer, const float4 (&pa)[LA], const float4 (&pw)[LW]) {
+#pragma unroll
+        for (int r = 0; r < LA; ++r) {
+            const int e = tid + r * THREADS;
+            *reinterpret_cast<float4*>(&As[buffer][e / QUADS * LD + e % QUADS * 4]) = pa[r];
+        }
+#pragma unroll
+        for (int r = 0; r < LW; ++r) {
+            const int e = tid + r * THREADS;
+            *reinterpret_cast<float4*>(&Ws[buffer][e / QUADS * LD + e % QUADS * 4]) = pw[r];
+        }
+    };
+    auto multiply = [&](int buffer) {
+#pragma unroll
+        for (int q = 0; q < QUADS; ++q) {
+            float4 a[TM], w[TN];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(&As[buffer][(ty + i * TY) * LD + q * 4]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(&Ws[buffer][(tx + j * TX) * LD + q * 4]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
+        }
+    };
+#pragma unroll
+    for (int d = 0; d < AHEAD; ++d) fetch(d * BK, ra[d], rw[d]);
+    const int steps = (K + BK - 1) / BK;
+    for (int i0 = 0; i0 < steps; i0 += AHEAD) {
+#pragma unroll
+        for (int d = 0; d < AHEAD; ++d) {
+            const int i = i0 + d;
+            if (i >= steps) break;
+            keep(i & 1, ra[d], rw[d]);                         // everyone left this buffer a barrier ago
+            __syncthreads();
+            fetch((i + AHEAD) * BK, ra[d], rw[d]);
+            multiply(i & 1);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty + i * TY;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx + j * TX;
             if (n >= N) continue;
             float v = acc[i][j];
             if (bias) v += load_as_float(bias, bias_bf16, n);
@@ -68,24 +120,59 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
     }
 }
 
+// Shared memory delivers a thread's words at 128 bytes a clock and SM whether lanes ask for the same or not, so a tile's speed is
+// its multiply-adds per word read: 8 x 8 outputs a thread make 42 TFLOP/s (700 x 6,144 x 2,048; 4 x 4 made 31, and 4-byte reads
+// of a single buffer 21), but their blocks of two warps need three an SM. Fewer blocks, smaller tiles, so that every SM has
+// one; and where even the smallest leave SMs idle, more threads a tile for the latency. 203 rows, microseconds before and now:
+// 4,096 x 1,024 114 -> 77, 1,024 x 2,048 148 -> 53, 96 x 2,048 148 -> 35; 1 row, 1,024 x 1,024 74 -> 18; 2,048 rows, 4,096 x
+// 4,096 2,951 -> 1,708. An output's sum runs in ascending k whatever the tile: the same bits.
+template <typename TI, typename TO, bool VEC>
+void launch_nt(const TI* A, const TI* W, const void* bias, int bias_bf16, TO* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
+               long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
+    constexpr long SMS = 148;
+    auto blocks = [&](int bm, int bn) { return (long)((N + bn - 1) / bn) * ((M + bm - 1) / bm) * batch; };
+#define LLMP_NT(BM, BN, BK, TM, TN, AHEAD)                                                                                              \
+    gemm_nt_kernel<TI, TO, BM, BN, BK, TM, TN, AHEAD, VEC><<<dim3((N + BN - 1) / BN, (M + BM - 1) / BM, batch), (BM / TM) * (BN / TN), 0, stream>>>( \
+        A, W, bias, bias_bf16, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c)
+    if (blocks(64, 64) >= 3 * SMS) LLMP_NT(64, 64, 32, 8, 8, 1);
+    else if (blocks(64, 64) >= SMS) LLMP_NT(64, 64, 16, 8, 4, 1);
+    else if (blocks(32, 32) >= SMS) LLMP_NT(32, 32, 32, 4, 4, 1);
+    else LLMP_NT(32, 32, 32, 2, 2, 2);
+#undef LLMP_NT
+}
+
+template <typename TI, typename TO>
+void launch_nt_types(const void* A, const void* W, const void* bias, int bias_bf16, void* C, int batch, int M, int N, int K, long lda, long ldw,
+                     long ldc, long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
+    const size_t piece = 4 * sizeof(TI);
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && batch_a % 4 == 0 && batch_w % 4 == 0 && ((size_t)A | (size_t)W) % piece == 0;
+    if (vec) launch_nt<TI, TO, true>((const TI*)A, (const TI*)W, bias, bias_bf16, (TO*)C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream);
+    else launch_nt<TI, TO, false>((const TI*)A, (const TI*)W, bias, bias_bf16, (TO*)C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream);
+}
+
+// false: no such combination of types
+bool launch_nt_any(const void* A, const void* W, const void* bias, int bias_bf16, void* C, int in_dtype, int out_dtype, int batch, int M, int N,
+                   int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
+#define LLMP_NT_TYPES(TI, TO) launch_nt_types<TI, TO>(A, W, bias, bias_bf16, C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream)
+    if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32) LLMP_NT_TYPES(float, float);
+    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16) LLMP_NT_TYPES(bf16, bf16);
+    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_F32) LLMP_NT_TYPES(bf16, float);
+    else return false;
+#undef LLMP_NT_TYPES
+    return true;
+}
+
+}  // namespace
+
+#define GT_MAX_ROWS (65535 * 32)      // rows of the smallest tile that a grid can hold
+
 // in_dtype: type of A and W.  out_dtype: type of C (float32, or the input type).
 LLMP_API int llmp_gemm_simt(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int in_dtype,
                             int out_dtype, int M, int N, int K, long lda, long ldw, long ldc, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     LLMP_REQUIRE(K > 0, "gemm: bad K %d", K);
-    LLMP_REQUIRE((M + GT_BM - 1) / GT_BM <= 65535, "gemm: too many rows %d", M);
-    dim3 grid((N + GT_BN - 1) / GT_BN, (M + GT_BM - 1) / GT_BM);
-    const int bb = bias_dtype == LLMP_BF16;
-    if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32)
-        gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)A, (const float*)W, bias, bb, (float*)C,
-                                                               M, N, K, lda, ldw, ldc);
-    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16)
-        gemm_nt_kernel<bf16, bf16><<<grid, 256, 0, stream>>>((const bf16*)A, (const bf16*)W, bias, bb, (bf16*)C, M, N,
-                                                             K, lda, ldw, ldc);
-    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_F32)
-        gemm_nt_kernel<bf16, float><<<grid, 256, 0, stream>>>((const bf16*)A, (const bf16*)W, bias, bb, (float*)C, M,
-                                                              N, K, lda, ldw, ldc);
-    else {
+    LLMP_REQUIRE(M <= GT_MAX_ROWS, "gemm: too many rows %d", M);
+    if (!launch_nt_any(A, W, bias, bias_dtype == LLMP_BF16, C, in_dtype, out_dtype, 1, M, N, K, lda, ldw, ldc, 0, 0, 0, stream)) {
         llmp_set_error("gemm: unsupported type combination in=%d out=%d", in_dtype, out_dtype);
         return 1;
     }
@@ -163,7 +250,7 @@ LLMP_API int llmp_gemm_simt_batched(const void* A, const void* W, void* C, int i
                                     cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     LLMP_REQUIRE(K > 0, "batched gemm: bad K %d", K);
-    LLMP_REQUIRE((M + GT_BM - 1) / GT_BM <= 65535 && batch <= 65535, "batched gemm: too many rows %d or products %d", M, batch);
+    LLMP_REQUIRE(M <= GT_MAX_ROWS && batch <= 65535, "batched gemm: too many rows %d or products %d", M, batch);
     if (M <= GR_MAX_ROWS && (N + 7) / 8 <= 65535) {
         dim3 rows_grid((N + 7) / 8, batch);
         const size_t esize = in_dtype == LLMP_F32 ? 4 : 2;
@@ -186,17 +273,7 @@ LLMP_API int llmp_gemm_simt_batched(const void* A, const void* W, void* C, int i
 #undef LLMP_ROWS
         return llmp_check_launch("gemm_simt_batched (rows)");
     }
-    dim3 grid((N + GT_BN - 1) / GT_BN, (M + GT_BM - 1) / GT_BM, batch);
-    if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32)
-        gemm_nt_kernel<float, float><<<grid, 256, 0, stream>>>((const float*)A, (const float*)W, nullptr, 0, (float*)C, M, N, K,
-                                                               lda, ldw, ldc, batch_a, batch_w, batch_c);
-    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16)
-        gemm_nt_kernel<bf16, bf16><<<grid, 256, 0, stream>>>((const bf16*)A, (const bf16*)W, nullptr, 0, (bf16*)C, M, N, K, lda,
-                                                             ldw, ldc, batch_a, batch_w, batch_c);
-    else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_F32)
-        gemm_nt_kernel<bf16, float><<<grid, 256, 0, stream>>>((const bf16*)A, (const bf16*)W, nullptr, 0, (float*)C, M, N, K,
-                                                              lda, ldw, ldc, batch_a, batch_w, batch_c);
-    else {
+    if (!launch_nt_any(A, W, nullptr, 0, C, in_dtype, out_dtype, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream)) {
         llmp_set_error("batched gemm: unsupported type combination in=%d out=%d", in_dtype, out_dtype);
         return 1;
     }

@@ -147,6 +147,25 @@ def test_gemm_simt(dtype, M, N, Kd):
     assert torch.equal(single[0], out[M - 1])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("M,N,Kd", [(33, 31, 7), (65, 1000, 64), (203, 1025, 130), (129, 4097, 36), (513, 5000, 33)])
+def test_gemm_simt_gives_one_sum_whatever_the_tile(dtype, M, N, Kd):
+    """Around the tiles' edges, for K that is and is not a multiple of 4, in each of the four tile sizes: every row has the bits it
+    has alone (one row takes the smallest tile), and is within K 2^-24 of the sum of the products' sizes (2^-8 more where the
+    result is bfloat16) of the float64 product."""
+    gen = torch.Generator().manual_seed(M + N + Kd)
+    a, w = (torch.randn(n, Kd + 4, generator=gen).to(dtype).to(DEV)[:, :Kd] for n in (M, N))
+    out = torch.empty(M, N, dtype=dtype, device=DEV)
+    K().gemm_simt(a, w, out)
+    want, sizes = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+    assert ((out.double() - want).abs() <= bound).all()
+    for m in {0, M // 2, M - 1}:
+        single = torch.empty(1, N, dtype=dtype, device=DEV)
+        K().gemm_simt(a[m:m + 1], w, single)
+        assert torch.equal(single[0], out[m]), m
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
 @pytest.mark.parametrize("M,N,Kd", [(1, 130, 64), (8, 4096, 4096), (7, 100, 1048), (16, 6144, 520), (13, 331, 264),
                                      (9, 20000, 1032), (3, 17000, 256), (5, 20, 8)])
