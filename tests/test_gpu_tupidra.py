@@ -129,7 +129,7 @@ def test_selective_scan_alone(dtype, sizes):
 @pytest.mark.parametrize("sizes", [(130, 16), (37, 5), (129, 32)], ids=str)
 def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
     """Requests around the segments' edges side by side, each going on in a second step, against the recurrence in float64; slots
-    that are not theirs by number and the entries around the piece stay as they are. bfloat16 rounds an output to 2^-9 of
+    that are not theirs by number and the entries around the piece stay as they are. bfloat16 rounds an output to 2^-8 of
     itself; the float32 state between the segments stays within 2e-5 of the largest entry, as token by token."""
     from llm_pipeline_b200.ops import kernels
     monkeypatch.setattr(kernels, "SCAN_SEGMENTS_MIN_TOKENS", 1)
