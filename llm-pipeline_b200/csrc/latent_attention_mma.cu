@@ -329,12 +329,12 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
 }
 
 // Adds the segments of a row: out = sum_s 2^(m_s - m) o_s / sum_s 2^(m_s - m) l_s over the segments that hold keys the
-// row sees, in ascending order. grid (tokens, heads).
+// row sees, in ascending order. grid (tokens from `first` on, heads).
 __global__ void latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int* __restrict__ positions,
-                                    bf16* __restrict__ out, long o_t, long o_h, int N, int H, int rank, int seg_keys,
-                                    const float* __restrict__ sink) {
-    const int n = blockIdx.x, h = blockIdx.y;
-    const int segs = positions[n] / seg_keys + 1;
+                                    bf16* __restrict__ out, long o_t, long o_h, int N, int H, int rank, int seg_keys, int segments,
+                                    int first, const float* __restrict__ sink) {
+    const int n = first + blockIdx.x, h = blockIdx.y;
+    const int segs = min(positions[n] / seg_keys + 1, segments);      // (a row whose request is not in the tiles may be at any position)
     const float sk = sink ? sink[h] * 1.4426950408889634f : -INFINITY;
     float m = sk;
     for (int s = 0; s < segs; ++s) m = fmaxf(m, part_ml[(((size_t)s * N + n) * H + h) * 2]);
@@ -361,12 +361,12 @@ LLMP_API int llmp_latent_mma_supports(int rank, int rot, int page_size) {
     return rank > 0 && rank % 16 == 0 && rot >= 0 && rot % 16 == 0 && page_size > 0 && smem <= 200 * 1024;
 }
 
-// scratch: float32, segments * N * H * (rank + 2) entries when seg_keys > 0 (segments = ceil(longest context / seg_keys)).
+// first_row, end_row: where the rows of the tiles' requests lie. scratch: float32, segments * N * H * (rank + 2) entries when seg_keys > 0 (segments = ceil(longest context / seg_keys)).
 LLMP_API int llmp_latent_attention_mma(const void* q_lat, long ql_t, long ql_h, const void* q_rot, long qr_t, long qr_h,
                                        const void* pages, const int* tables, int table_stride, const int* q_start, const int* ctx_len,
                                        const int* positions, const int* tile_req, const int* tile_tok0, int num_tiles, void* out,
                                        long o_t, long o_h, int N, int H, int rank, int rot, int page_size, float scale, int seg_keys,
-                                       int segments, float* scratch, const float* sink, cudaStream_t stream) {
+                                       int segments, float* scratch, int first_row, int end_row, const float* sink, cudaStream_t stream) {
     if (N <= 0 || num_tiles <= 0) return 0;
     LLMP_REQUIRE(llmp_latent_mma_supports(rank, rot, page_size), "latent_attention_mma: sizes rank=%d rot=%d are not served", rank, rot);
     LLMP_REQUIRE(ql_t % 8 == 0 && ql_h % 8 == 0 && qr_t % 8 == 0 && qr_h % 8 == 0 && o_t % 2 == 0 && o_h % 2 == 0 &&
@@ -374,6 +374,7 @@ LLMP_API int llmp_latent_attention_mma(const void* q_lat, long ql_t, long ql_h, 
                  "latent_attention_mma: query rows must be 16-byte aligned");
     LLMP_REQUIRE(seg_keys == 0 || (seg_keys % LM_KEYS == 0 && segments > 0 && segments <= 65535 && scratch != nullptr),
                  "latent_attention_mma: segments of %d keys", seg_keys);
+    LLMP_REQUIRE(0 <= first_row && first_row < end_row && end_row <= N, "latent_attention_mma: rows %d to %d of %d", first_row, end_row, N);
     LatentMmaParams p;
     p.q_lat = (const bf16*)q_lat; p.ql_t = ql_t; p.ql_h = ql_h;
     p.q_rot = (const bf16*)q_rot; p.qr_t = qr_t; p.qr_h = qr_h;
@@ -405,6 +406,7 @@ LLMP_API int llmp_latent_attention_mma(const void* q_lat, long ql_t, long ql_h, 
         latent_attention_mma_kernel<256><<<grid, LM_THREADS, smem, stream>>>(p);
     }
     if (seg_keys > 0)
-        latent_merge_kernel<<<dim3(N, H), 128, 0, stream>>>(p.part_o, p.part_ml, positions, (bf16*)out, o_t, o_h, N, H, rank, seg_keys, sink);
+        latent_merge_kernel<<<dim3(end_row - first_row, H), 128, 0, stream>>>(p.part_o, p.part_ml, positions, (bf16*)out, o_t, o_h, N, H, rank, seg_keys,
+                                                                              segments, first_row, sink);
     return llmp_check_launch("latent_attention_mma");
 }

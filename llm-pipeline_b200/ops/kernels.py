@@ -67,7 +67,9 @@ _SIGNATURES = {
     "llmp_latent_kv_post": [_P, _I, _L, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _P, _P, _I, _P],
     "llmp_latent_attention": [_P, _L, _L, _P, _L, _L, _P, _I, _P, _I, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _F, _P, _P],
     "llmp_latent_attention_mma": [_P, _L, _L, _P, _L, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _L, _L, _I, _I, _I, _I, _I, _F, _I,
-                                  _I, _P, _P, _P],
+                                  _I, _P, _I, _I, _P, _P],
+    "llmp_latent_gather": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P],
+    "llmp_latent_prompt_attention": [_P, _L, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _L, _L, _I, _I, _I, _I, _I, _F, _P, _P, _P],
     "llmp_latent_rows_post": [_P, _L, _P, _L, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _I, _P, _I, _L, _P, _P, _I, _P],
     "llmp_capped_qkv_post": [_P, _L, _P, _I, _F, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "llmp_capped_rows_post": [_P, _L, _P, _P, _F, _P, _P, _I, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
@@ -1112,11 +1114,13 @@ def latent_mma_tokens_per_tile(num_heads: int) -> int:
 
 def latent_attention_mma(q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor, q_start: torch.Tensor,
                          ctx_len: torch.Tensor, positions: torch.Tensor, tile_req: torch.Tensor, tile_tok0: torch.Tensor,
-                         out: torch.Tensor, scale: float, segments: int = 0, sink: Optional[torch.Tensor] = None) -> torch.Tensor:
+                         out: torch.Tensor, scale: float, segments: int = 0, sink: Optional[torch.Tensor] = None,
+                         rows: Optional[Sequence[int]] = None) -> torch.Tensor:
     """``latent_attention`` on the tensor cores for bfloat16. ``tile_req``/``tile_tok0``: the work list (request and
     first token of every tile of ``latent_mma_tokens_per_tile`` tokens). ``segments`` > 0: the keys are cut into that many
     segments of ``LATENT_SEGMENT_KEYS``, each with blocks of its own, and a second kernel adds them up (for steps of few
-    rows over long contexts; ``segments`` must cover the longest context)."""
+    rows over long contexts; ``segments`` must cover the longest context). A work list of some of the step's requests needs
+    ``rows`` = (first, end), between which their rows lie; what the other rows of ``out`` there hold afterwards means nothing."""
     N, H, rank = q_lat.shape
     rot = q_rot.shape[2]
     _sink(sink, H)
@@ -1134,7 +1138,54 @@ def latent_attention_mma(q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch.
     _call("llmp_latent_attention_mma", _ptr(q_lat), q_lat.stride(0), q_lat.stride(1), _ptr(q_rot), q_rot.stride(0), q_rot.stride(1),
           _ptr(pages), _ptr(tables), tables.shape[1], _ptr(q_start), _ptr(ctx_len), _ptr(positions), _ptr(tile_req), _ptr(tile_tok0),
           tile_req.numel(), _ptr(out), out.stride(0), out.stride(1), N, H, rank, rot, pages.shape[1], float(scale),
-          LATENT_SEGMENT_KEYS if segments > 0 else 0, int(segments), _ptr(scratch), _ptr(sink), _stream())
+          LATENT_SEGMENT_KEYS if segments > 0 else 0, int(segments), _ptr(scratch), *(rows or (0, N)), _ptr(sink), _stream())
+    return out
+
+
+LATENT_PROMPT_TOKENS = 128           # new tokens of a tile of the kernel with formed keys and values
+
+
+def latent_prompt_keys(dim: int, rot: int, vdim: int, rank: int) -> int:
+    """Keys of a key tile of ``latent_prompt_attention`` for heads of these sizes, the unit a request's gathered rows are padded
+    to; 0: the kernel does not serve them."""
+    fn = library().llmp_latent_prompt_keys
+    fn.argtypes = [_I, _I, _I, _I]
+    fn.restype = _I
+    return int(fn(dim, rot, vdim, rank))
+
+
+def latent_gather(pages: torch.Tensor, tables: torch.Tensor, ctx_len: torch.Tensor, block_req: torch.Tensor, block_key0: torch.Tensor,
+                  keys: int, rows: torch.Tensor) -> torch.Tensor:
+    """The cached rows of requests as one matrix (csrc/latent_prompt_tc.cu): rows b ``keys`` .. of ``rows`` [blocks keys, row] are the
+    keys from ``block_key0[b]`` on of request ``block_req[b]``, zeros past its ``ctx_len``."""
+    for t, name in ((tables, "tables"), (ctx_len, "ctx_len"), (block_req, "block_req"), (block_key0, "block_key0")):
+        _i32(t, name)
+    _need(pages.dtype == rows.dtype == torch.bfloat16 and pages.is_contiguous() and rows.is_contiguous() and pages.shape[2] == rows.shape[1],
+          "latent_gather takes contiguous bfloat16 rows")
+    _need(block_req.numel() == block_key0.numel() and rows.shape[0] == block_req.numel() * keys, "latent_gather: shapes do not match")
+    _call("llmp_latent_gather", _ptr(pages), _ptr(tables), tables.shape[1], _ptr(ctx_len), _ptr(block_req), _ptr(block_key0), block_req.numel(),
+          int(keys), pages.shape[1], rows.shape[1], _ptr(rows), _stream())
+    return rows
+
+
+def latent_prompt_attention(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tensor, q_start: torch.Tensor, ctx_len: torch.Tensor,
+                            tile_req: torch.Tensor, tile_tok0: torch.Tensor, tile_base: torch.Tensor, out: torch.Tensor, dim: int, rank: int,
+                            scale: float, sink: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Causal latent attention of long prompt portions with formed keys and values (csrc/latent_prompt_tc.cu): ``q`` [tokens, heads,
+    dim + rot], ``rows`` what ``latent_gather`` gave ([gathered rows, rank + rot]), ``kv`` [gathered rows, heads dim | heads vdim], the
+    keys and values of its latents. Tiles are ``LATENT_PROMPT_TOKENS`` new tokens of request ``tile_req`` from ``tile_tok0`` on, whose
+    keys begin at gathered row ``tile_base``; ``out`` [tokens, heads, vdim]: the rows of other requests are left alone."""
+    N, H, width = q.shape
+    rot, vdim = width - dim, out.shape[2]
+    _sink(sink, H)
+    _need(all(t.dtype == torch.bfloat16 for t in (q, kv, rows, out)), "latent_prompt_attention takes bfloat16")
+    _need(q.stride(2) == 1 and out.stride(2) == 1 and out.shape[:2] == (N, H) and kv.is_contiguous() and rows.is_contiguous() and
+          kv.shape == (rows.shape[0], H * (dim + vdim)) and rows.shape[1] == rank + rot, "latent_prompt_attention: shapes do not match")
+    for t, name in ((q_start, "q_start"), (ctx_len, "ctx_len"), (tile_req, "tile_req"), (tile_tok0, "tile_tok0"), (tile_base, "tile_base")):
+        _i32(t, name)
+    _call("llmp_latent_prompt_attention", _ptr(q), q.stride(0), q.stride(1), _ptr(kv), _ptr(rows), rows.shape[0], _ptr(q_start), _ptr(ctx_len),
+          _ptr(tile_req), _ptr(tile_tok0), _ptr(tile_base), tile_req.numel(), _ptr(out), out.stride(0), out.stride(1), H, int(dim), int(rot),
+          int(vdim), int(rank), float(scale), _ptr(sink), error_flag().data_ptr(), _stream())
     return out
 
 

@@ -17,6 +17,9 @@ kv_rank + rot_dim entries and the rows' first kv_rank entries as values, in prom
 are one batched product over the heads before and after the attention kernel. Scores, softmax, norm and angles are
 float32. ``rot_dims`` (<= rot_dim) entries of the rotated parts take the rotation, the rest pass unchanged.
 
+Long prompt portions in bfloat16 take the other order (``_formed_plan``): k_h and v_h of the request's rows are formed by one product
+and attended over as they are, which costs a (query, key, head) dim + rot + vdim multiply-adds instead of 2 kv_rank + rot.
+
 Options that other designs of this family use (all off by default): the queries through a normed latent of their own
 (``q_rank``: ``c_q = rms_norm(Wdq h) * w_q``, ``q = Wuq c_q``), a learned sink per head in the softmax's denominator, a
 sigmoid gate ``sigmoid(Wg h)`` on the heads' outputs before ``Wo``, the interleaved pairing of rotated entries, and a
@@ -65,7 +68,8 @@ class LatentAttention(Mixer):
         self.split = bool(self.q_rank or self.gate or not self.own_rows or self.interleaved)
         self.q_size = self.num_heads * (self.dim + self.rot_dim)
         self.w_in = self.w_uk_t = self.w_uv = self.w_o = self.c_norm = None
-        self.w_dq = self.q_norm = self.w_uq = self.w_rest = self.sinks = None
+        self.w_dq = self.q_norm = self.w_uq = self.w_rest = self.sinks = self.w_ukv = None
+        self.formed_keys = 0          # keys of a key tile of the kernel with formed keys and values; 0: it does not take this mixer
 
     def cache_spec(self) -> Optional[TokenPagesSpec]:
         return TokenPagesSpec((self.kv_rank + self.rot_dim,), None) if self.own_rows else None
@@ -97,6 +101,11 @@ class LatentAttention(Mixer):
         self.w_uk_t = get(f"{p}.uk", "matrix").view(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = get(f"{p}.uv", "matrix").view(H, self.vdim, self.kv_rank).contiguous()
         self.w_o = get(f"{p}.o", "matrix").contiguous()
+        formed = self.dim + self.rot_dim + self.vdim < 2 * self.kv_rank + self.rot_dim
+        self.formed_keys = (kernels.latent_prompt_keys(self.dim, self.rot_dim, self.vdim, self.kv_rank)
+                            if formed and self.w_o.is_cuda and self.w_o.dtype == torch.bfloat16 else 0)
+        if self.formed_keys:
+            self.w_ukv = torch.cat([get(f"{p}.uk", "matrix"), get(f"{p}.uv", "matrix")], dim=0).contiguous()
         if self.own_rows:
             self.c_norm = get(f"{p}.dkv.norm", "vector").contiguous()
         if self.sink:
@@ -118,13 +127,96 @@ class LatentAttention(Mixer):
     SEGMENTS_BELOW_BLOCKS_PER_SM = 2.0
     SEGMENTS_MIN_CONTEXT = 2 * kernels.LATENT_SEGMENT_KEYS
 
-    def attend(self, ctx, q_lat, q_rot, out, cache: LayerCache) -> None:
+    # New tokens of a request from which its keys and values are formed (one request of 128 tokens: 102 us a layer against 115, of
+    # 2,048 136 against 695; the host launches as many kernels either way). Requests of fewer tokens beside it join while their
+    # keys are no more than FORMED_JOIN_KEYS together, whose forming costs the device less than the second path's launches cost
+    # the host (70 us: requests of 130 and 62 tokens 172 us apart, 117 over the latents). Above that the second path has to be worth
+    # it: FORMED_MIN_GAIN_US by the rates of the two kernels at 2,048 tokens (in TFLOP/s: 120 over latents, 350 formed, 600 forming).
+    # The formed keys and values of a step take at most FORMED_MAX_BYTES; beyond, its requests attend over the latents.
+    FORMED_MIN_TOKENS = 128
+    FORMED_JOIN_KEYS = 4096
+    FORMED_MIN_GAIN_US = 100.0
+    FORMED_MAX_BYTES = 512 << 20
+
+    def _formed_requests(self, ctx):
+        """The requests of the step whose keys and values are formed."""
+        taken = [r for r, n in enumerate(ctx.q_lens) if n >= self.FORMED_MIN_TOKENS]
+        others = sum(s + n for s, n in zip(ctx.starts, ctx.q_lens) if n < self.FORMED_MIN_TOKENS)
+        if others <= self.FORMED_JOIN_KEYS:
+            return list(range(len(ctx.q_lens)))
+        pairs = sum(ctx.q_lens[r] * (ctx.starts[r] + (ctx.q_lens[r] + 1) / 2) for r in taken)
+        gain = pairs * ((2 * self.kv_rank + self.rot_dim) / 120 - (self.dim + self.rot_dim + self.vdim) / 350)
+        gain -= sum(ctx.starts[r] for r in taken) * (self.dim + self.vdim) * self.kv_rank / 600
+        return taken if 2e-6 * self.num_heads * gain > self.FORMED_MIN_GAIN_US else []
+
+    def _formed_plan(self, ctx):
+        """Which requests of the step attend over formed keys and values: None, or (their blocks of keys: request, first key; their
+        tiles: request, first token, first gathered row; the rows of the other requests as (first, end) runs; the tiles of the
+        others for ``latent_attention_mma``, their longest context). Made once per step and kept in ``ctx.memo``."""
+        if not self.formed_keys or ctx.max_q_len < self.FORMED_MIN_TOKENS:
+            return None
+        keys, per_tile = self.formed_keys, kernels.latent_mma_tokens_per_tile(self.num_heads)
+        width = self.num_heads * (self.dim + self.vdim)
+        key = ("latent_attention_formed", keys, per_tile, width)
+        if key in ctx.memo:
+            return ctx.memo[key]
+        taken = self._formed_requests(ctx)
+        base, total, blocks = {}, 0, []
+        for r in taken:
+            base[r] = total
+            count = -(-(ctx.starts[r] + ctx.q_lens[r]) // keys)
+            blocks += [(r, t * keys) for t in range(count)]
+            total += count * keys
+        plan = None
+        if 0 < total * width * 2 <= self.FORMED_MAX_BYTES:
+            # in the order of the keys a tile sees: the kernels start the last tile first
+            tiles = sorted((ctx.starts[r] + min(t + kernels.LATENT_PROMPT_TOKENS, ctx.q_lens[r]), r, t)
+                           for r in taken for t in range(0, ctx.q_lens[r], kernels.LATENT_PROMPT_TOKENS))
+            rest = [(ctx.starts[r] + min(t + per_tile, n), r, t) for r, n in enumerate(ctx.q_lens) if r not in base for t in range(0, n, per_tile)]
+            runs, at = [], 0
+            for r, n in enumerate(ctx.q_lens):
+                if r not in base:
+                    if runs and runs[-1][1] == at:
+                        runs[-1] = (runs[-1][0], at + n)
+                    else:
+                        runs.append((at, at + n))
+                at += n
+            rest.sort()
+            host = torch.tensor([r for r, _k in blocks] + [k for _r, k in blocks] + [r for _c, r, _t in tiles] + [t for _c, _r, t in tiles] +
+                                [base[r] for _c, r, _t in tiles] + [r for _c, r, _t in rest] + [t for _c, _r, t in rest], dtype=torch.int32)
+            dev = torch.split(host.pin_memory().to(ctx.device, non_blocking=True), [len(blocks)] * 2 + [len(tiles)] * 3 + [len(rest)] * 2)
+            plan = (dev[:2], dev[2:5], runs, dev[5:], max((c for c, _r, _t in rest), default=0))
+        ctx.memo[key] = plan
+        return plan
+
+    def _formed(self, ctx, plan, q, values, cache: LayerCache) -> None:
+        """The values of the requests whose keys and values are formed."""
+        (block_req, block_key0), tiles, *_others = plan
+        rows = torch.empty((block_req.numel() * self.formed_keys, self.kv_rank + self.rot_dim), dtype=q.dtype, device=q.device)
+        kernels.latent_gather(cache.pages, ctx.block_tables[cache.group], ctx.ctx_len, block_req, block_key0, self.formed_keys, rows)
+        kv = linear(rows[:, :self.kv_rank], self.w_ukv)
+        kernels.latent_prompt_attention(q, kv, rows, ctx.q_start, ctx.ctx_len, *tiles, values, self.dim, self.kv_rank, self.scale, sink=self.sinks)
+
+    def attend(self, ctx, q_lat, q_rot, out, cache: LayerCache, some=None) -> None:
         """Attention of the step's rows over the cache: the tensor-core kernel for bfloat16 where it serves the sizes,
-        else the general kernel (float32, sizes that are no multiples of 16)."""
+        else the general kernel (float32, sizes that are no multiples of 16). ``some``: the tiles of the requests to take,
+        their longest context and the rows between which theirs lie; None: all requests."""
         tables = ctx.block_tables[cache.group]
         if not kernels.latent_mma_supports(q_lat.dtype, self.kv_rank, self.rot_dim, cache.pages.shape[1]) or self.dim % 8 or self.rot_dim % 8:
             kernels.latent_attention(q_lat, q_rot, cache.pages, tables, ctx.token_request, ctx.positions, out, self.scale, sink=self.sinks)
             return
+        if some is not None:
+            tiles, longest, rows = some
+        else:
+            tiles, longest, rows = self._tiles(ctx), ctx.decode_ctx_bound or ctx.max_ctx_len, None
+        blocks = tiles[0].numel() * -(-self.num_heads // 16) * -(-self.kv_rank // 128)
+        segments = 0
+        if blocks < self.SEGMENTS_BELOW_BLOCKS_PER_SM * kernels.sm_count() and longest >= self.SEGMENTS_MIN_CONTEXT:
+            segments = -(-longest // kernels.LATENT_SEGMENT_KEYS)
+        kernels.latent_attention_mma(q_lat, q_rot, cache.pages, tables, ctx.q_start, ctx.ctx_len, ctx.positions, tiles[0], tiles[1],
+                                     out, self.scale, segments, sink=self.sinks, rows=rows)
+
+    def _tiles(self, ctx):
         per_tile = kernels.latent_mma_tokens_per_tile(self.num_heads)
         key = ("latent_attention_tiles", per_tile)
         tiles = ctx.memo.get(key)
@@ -139,13 +231,7 @@ class LatentAttention(Mixer):
                 dev = host.to(ctx.device, non_blocking=True)
                 tiles = (dev[0].contiguous(), dev[1].contiguous())
             ctx.memo[key] = tiles
-        longest = ctx.decode_ctx_bound or ctx.max_ctx_len
-        blocks = tiles[0].numel() * -(-self.num_heads // 16) * -(-self.kv_rank // 128)
-        segments = 0
-        if blocks < self.SEGMENTS_BELOW_BLOCKS_PER_SM * kernels.sm_count() and longest >= self.SEGMENTS_MIN_CONTEXT:
-            segments = -(-longest // kernels.LATENT_SEGMENT_KEYS)
-        kernels.latent_attention_mma(q_lat, q_rot, cache.pages, tables, ctx.q_start, ctx.ctx_len, ctx.positions, tiles[0], tiles[1],
-                                     out, self.scale, segments, sink=self.sinks)
+        return tiles
 
     def forward(self, x, ctx, cache: LayerCache):
         if cache.pages is None or cache.group is None:
@@ -178,12 +264,21 @@ class LatentAttention(Mixer):
                                      self.rot_dims, self.interleaved, q, ctx.slot_mapping[cache.group] if writes else None,
                                      cache.pages if writes else None)
             q = q.view(N, H, self.dim + rot)
-        q_lat = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
-        batched_linear(q[:, :, :self.dim].transpose(0, 1), self.w_uk_t, q_lat.transpose(0, 1))
-        mixed = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
-        self.attend(ctx, q_lat, q[:, :, self.dim:], mixed, cache)
         values = torch.empty((N, H, self.vdim), dtype=x.dtype, device=x.device)
-        batched_linear(mixed.transpose(0, 1), self.w_uv, values.transpose(0, 1))
+        plan = self._formed_plan(ctx)
+        runs, some = [(0, N)], None
+        if plan is not None:
+            self._formed(ctx, plan, q, values, cache)
+            runs = plan[2]
+            some = (*plan[3:], (runs[0][0], runs[-1][1])) if runs else None
+        if runs:
+            q_lat = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
+            for first, end in runs:
+                batched_linear(q[first:end, :, :self.dim].transpose(0, 1), self.w_uk_t, q_lat[first:end].transpose(0, 1))
+            mixed = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
+            self.attend(ctx, q_lat, q[:, :, self.dim:], mixed, cache, some)
+            for first, end in runs:
+                batched_linear(mixed[first:end].transpose(0, 1), self.w_uv, values[first:end].transpose(0, 1))
         values = values.view(N, H * self.vdim)
         if gate is not None:
             kernels.sigmoid_gate(values, gate)

@@ -1,0 +1,111 @@
+"""Latent attention of long prompt portions, whose keys and values are formed: the kernels against float64, and steps in which
+such portions stand beside decoded tokens and short portions that attend over the latents."""
+
+import pytest
+import torch
+
+import helpers as H
+import zupilorn_cases as Z
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _i32(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("sink", [False, True], ids=["", "sink"])
+@pytest.mark.parametrize("dim,rot,rank", [(128, 64, 128), (128, 16, 64), (64, 32, 64)], ids=str)
+@pytest.mark.parametrize("lengths", [((0, 1), (0, 97)), ((95, 128), (1, 129), (0, 33)), ((300, 200),)], ids=str)
+def test_formed_keys_and_values(dim, rot, rank, lengths, sink):
+    """Requests of (cached, new) tokens around the tiles' edges over shuffled pages, pages of others filled with NaN. Against
+    float64 over the same formed keys and values, the probabilities and the result are rounded to bfloat16 (8 bits: 2^-8 each at
+    most) and the scores' sums and exponentials are float32: within 2^-7 (1 + 1/8) of the weighted sum of the values' sizes."""
+    from llm_pipeline_b200.ops import kernels
+    heads, page, gen = 3, 16, torch.Generator().manual_seed(dim + rot + len(lengths))
+    R, dk = len(lengths), rank + rot
+    ctx = [s + n for s, n in lengths]
+    N = sum(n for _s, n in lengths)
+    need = [-(-c // page) for c in ctx]
+    order = torch.randperm(sum(need) + 3, generator=gen).tolist()
+    pages = torch.full((sum(need) + 3, page, dk), float("nan"))
+    tables = torch.full((R, max(need)), -1, dtype=torch.int32)
+    latents = [torch.randn(c, dk, generator=gen).to(torch.bfloat16).float() for c in ctx]
+    for r, c in enumerate(ctx):
+        for i in range(need[r]):
+            tables[r, i] = order.pop()
+            part = latents[r][i * page:(i + 1) * page]
+            pages[tables[r, i], :part.shape[0]] = part
+    q = torch.randn(N, heads, dim + rot, generator=gen).to(torch.bfloat16)
+    w = (torch.randn(heads * 2 * dim, rank, generator=gen) * rank ** -0.5).to(torch.bfloat16)
+    sinks = torch.randn(heads, generator=gen) if sink else None
+    keys = kernels.latent_prompt_keys(dim, rot, dim, rank)
+    blocks = [(r, t) for r in range(R) for t in range(0, ctx[r], keys)]
+    base = [next(i for i, b in enumerate(blocks) if b[0] == r) * keys for r in range(R)]
+    rows = torch.empty(len(blocks) * keys, dk, dtype=torch.bfloat16, device=DEV)
+    ctx_len = _i32(ctx)
+    kernels.latent_gather(pages.to(DEV, torch.bfloat16), tables.to(DEV), ctx_len, _i32([r for r, _t in blocks]), _i32([t for _r, t in blocks]), keys, rows)
+    for r in range(R):
+        padded = rows[base[r]:base[r] + -(-ctx[r] // keys) * keys].float().cpu()
+        assert torch.equal(padded[:ctx[r]], latents[r]) and (padded[ctx[r]:] == 0).all()
+    kv = (rows[:, :rank].float() @ w.to(DEV).float().T).to(torch.bfloat16)
+    out = torch.full((N, heads, dim), 7.0, dtype=torch.bfloat16, device=DEV)
+    tiles = [(r, t) for r, (_s, n) in enumerate(lengths) for t in range(0, n, kernels.LATENT_PROMPT_TOKENS)]
+    starts = [0]
+    for _s, n in lengths:
+        starts.append(starts[-1] + n)
+    scale = (dim + rot) ** -0.5 * 3.0
+    kernels.latent_prompt_attention(q.to(DEV), kv, rows, _i32(starts), ctx_len, _i32([r for r, _t in tiles]), _i32([t for _r, t in tiles]),
+                                    _i32([base[r] for r, _t in tiles]), out, dim, rank, scale, sink=sinks.to(DEV) if sink else None)
+    torch.cuda.synchronize()
+    kernels.check_error_flag()
+    kv, got = kv.double().cpu(), out.double().cpu()
+    for r, (s, n) in enumerate(lengths):
+        mine = kv[base[r]:base[r] + ctx[r]].view(ctx[r], 2 * heads, dim)
+        k, v = mine[:, :heads], mine[:, heads:]
+        qr = q[starts[r]:starts[r + 1]].double()
+        score = (torch.einsum("nhd,thd->hnt", qr[..., :dim], k) + torch.einsum("nhd,td->hnt", qr[..., dim:], latents[r][:, rank:].double())) * scale
+        score = score.masked_fill(torch.arange(ctx[r]) > s + torch.arange(n)[:, None], float("-inf"))
+        if sink:
+            score = torch.cat([score, sinks.double()[:, None, None].expand(heads, n, 1)], dim=2)
+        p = torch.softmax(score, dim=2)[:, :, :ctx[r]]
+        want, sizes = torch.einsum("hnt,thd->nhd", p, v), torch.einsum("hnt,thd->nhd", p, v.abs())
+        assert ((got[starts[r]:starts[r + 1]] - want).abs() <= 1.125 * 2.0 ** -7 * sizes).all(), r
+
+
+def test_formed_portions_beside_decoded_tokens_and_short_portions(tmp_path, monkeypatch):
+    """Whole models in bfloat16 with portions of 40 tokens and more formed, cut and mixed so that steps hold both kinds (and ones
+    that join), over contexts of several key segments; and a bound on the formed rows' memory that sends every request to the latents."""
+    from llm_pipeline_b200.ops import kernels
+    from llm_pipeline_b200.parts.latent_attention import LatentAttention
+    for name, value in (("FORMED_MIN_TOKENS", 40), ("FORMED_JOIN_KEYS", 30), ("FORMED_MIN_GAIN_US", 0.0)):
+        monkeypatch.setattr(LatentAttention, name, value)
+    cfg = Z.config([Z.latent_layer(3, 64, 32, 64, 128, None), Z.latent_layer(3, 64, 32, 64, 128, None)], width=96, vocab=61)
+    W = Z.weights_for(cfg, 21)
+    folder = Z.write_model(str(tmp_path), cfg, W)
+    seg = kernels.LATENT_SEGMENT_KEYS
+    requests = {f"r{i}": H.random_tokens(61, n, 40 + i) for i, n in enumerate([2 * seg + 60, 130, 2 * seg + 90, 3])}
+    want = Z.oracle(cfg, W, requests)
+    runner = H.make_runner(folder, torch.bfloat16, page_size=16, num_pages=100, max_request_tokens=3 * seg, max_requests=4)
+    calls = {"formed": 0, "both": 0}
+    formed, attend = kernels.latent_prompt_attention, kernels.latent_attention_mma
+
+    def counting(*args, **kwargs):
+        calls["formed"] += 1
+        return formed(*args, **kwargs)
+
+    def beside(*args, **kwargs):
+        calls["both"] += kwargs.get("rows") is not None
+        return attend(*args, **kwargs)
+
+    monkeypatch.setattr(kernels, "latent_prompt_attention", counting)
+    monkeypatch.setattr(kernels, "latent_attention_mma", beside)
+    Z.assert_matches(H.replay(runner, H.cut_whole(requests)), want, torch.bfloat16, "whole")
+    Z.assert_matches(H.replay(runner, H.cut_portions(requests, (39, 70, 3, 128, 129, 41))), want, torch.bfloat16, "portions")
+    Z.assert_matches(H.replay(runner, H.cut_mixed(requests, (60, 2, 131, 90, 7), max_live=4, decode_tail=30)), want, torch.bfloat16, "mixed")
+    assert calls["formed"] and calls["both"]
+    monkeypatch.setattr(LatentAttention, "FORMED_MAX_BYTES", 1)
+    calls["formed"] = 0
+    Z.assert_matches(H.replay(runner, H.cut_whole(requests)), want, torch.bfloat16, "nothing formed")
+    assert calls["formed"] == 0
