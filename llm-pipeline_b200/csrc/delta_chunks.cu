@@ -1,0 +1,465 @@
+// The gated delta rule of delta_rule.cu for the many tokens of a prompt portion (bfloat16 path), in chunks of 16 tokens.
+//
+//   S <- diag(g_t) S;   u_t = beta_t (v_t - S^T k_t);   S <- S + k_t u_t^T;   o_t = S^T q_t
+// Token by token that is a chain of dependent passes over the state, 0.3 us each whatever its size. Within a chunk, with G_t the
+// product of the chunk's decays up to t (per channel) and S the state before the chunk, the u are the solution of a triangular
+// system that does not depend on S but for its right-hand side:
+//   A[t, j] = sum_c k_t k_j G_t / G_j (j < t),   T = (I + diag(beta) A)^-1 diag(beta),   U = T V - (T (G k)) S
+//   o_t = (G_t q_t)^T S + sum_(j <= t) B[t, j] u_j,   B[t, j] = sum_c q_t k_j G_t / G_j
+//   S' = diag(G_16) S + sum_j (G_16 / G_j k_j) u_j^T
+// Two launches:
+//   1. every (chunk, head) side by side: unit vectors, decays and beta from the projections (the work of delta_prep), A, B, T, and
+//      what the chain needs of a chunk: W = T (G k), Q = G q, K = G_16 / G k, B, Y = T V, G_16;
+//   2. the chain: a block per (request, head, 16 value columns) walks the request's chunks with the state in registers: four
+//      products of 16 tokens a chunk on the tensor cores instead of 16 passes.
+// Everything is float32; ratios of decays are exponentials of differences of their logarithms (never above one, so nothing
+// overflows however fast a channel forgets). Where a float32 number enters a product it is split into two bfloat16 halves, and of
+// the four products of halves the three larger are summed in float32 (16 bits of each factor). The operands of launch 2 lie in
+// scratch in the order of its fragments, the two halves beside each other, and are copied as they are.
+#include "tcgen05.cuh"
+
+namespace {
+
+constexpr int DC_TOKENS = 16;             // tokens of a chunk
+constexpr int DC_PREP_THREADS = 128;
+constexpr int DC_CHAIN_THREADS = 128;     // of the chain: four quarters of the channels
+constexpr int DC_STAGES = 4;              // records of its ring
+constexpr float DC_LOG2_E = 1.4426950408889634f;
+
+struct DeltaChunkArgs {
+    const float* q; long q_t; const float* k; long k_t; const float* v; long v_t;     // as the convolution left them
+    const float* decay; long decay_t; const float* beta; long beta_t;                 // pre-activations
+    const float* a_log; const float* dt_bias;                                         // [H], [H d]
+    float* state; long state_slot; long state_half;                                   // copy: [H][d][dv]
+    const int* q_start; const int* slots; const int* positions;
+    float* o; long o_t;
+    unsigned char* scratch;               // [chunks][H] records
+    int* error_flag;
+    int requests, H, G, dv;
+};
+
+// Bytes of a record, whose parts are, in order: W, Q, K (64 a channel each), B (1024), Y (64 a column), G (4 a channel).
+__host__ __device__ constexpr int dc_record(int d, int dv) { return 3 * d * 64 + 1024 + dv * 64 + d * 4; }
+
+__device__ __forceinline__ float dc_ex2(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float dc_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
+
+__device__ __forceinline__ void dc_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two floats as a pair of bfloat16, and what that leaves of them as another pair.
+__device__ __forceinline__ void dc_split(float u, float v, unsigned& hi, unsigned& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(u, v);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(u - __low2float(h), v - __high2float(h));
+    hi = *reinterpret_cast<const unsigned*>(&h);
+    lo = *reinterpret_cast<const unsigned*>(&l);
+}
+__device__ __forceinline__ float4 dc_add4(const float4& a, const float4& b, const float4& c, const float4& d) {
+    return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
+}
+
+__device__ __forceinline__ void dc_bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(tc_smem_u32(dst)), "l"(src), "r"(bytes), "r"(tc_smem_u32(bar)) : "memory");
+}
+
+// Chunk number `at` of the step (in the order of the requests), by a warp; false: there is none.
+__device__ __forceinline__ bool find_chunk(const int* q_start, int requests, int at, int& row0, int& count) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int base = 0; base < requests; base += 32) {
+        const int r = base + lane;
+        const int first = r < requests ? q_start[r] : 0, last = r < requests ? q_start[r + 1] : 0;
+        const int own = (max(last - first, 0) + DC_TOKENS - 1) / DC_TOKENS;
+        int upto = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        const unsigned reach = __ballot_sync(0xffffffffu, before + upto > at);
+        if (reach) {
+            const int src = __ffs(reach) - 1;
+            const int index = at - before - (__shfl_sync(0xffffffffu, upto, src) - __shfl_sync(0xffffffffu, own, src));
+            row0 = __shfl_sync(0xffffffffu, first, src) + index * DC_TOKENS;
+            count = min(DC_TOKENS, __shfl_sync(0xffffffffu, last, src) - row0);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
+// ---- 1 -----------------------------------------------------------------------------------------------------------------
+// A thread owns a channel (its 16 tokens of decays, keys, queries) or a value column, but for the unit vectors (a warp per row) and
+// the sums A, B (a thread per pair of tokens, 4 channels at a time). The record is put together in shared memory, in two parts that
+// take turns there.
+template <int D>
+__global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const DeltaChunkArgs a) {
+    extern __shared__ __align__(16) unsigned char dc_raw[];
+    constexpr int LD = D + 4;
+    float* ks = reinterpret_cast<float*>(dc_raw);              // [16][LD]
+    float* qs = ks + DC_TOKENS * LD;
+    float* Ls = qs + DC_TOKENS * LD;                           // log2 of the decays' products
+    unsigned char* rec = reinterpret_cast<unsigned char*>(Ls + DC_TOKENS * LD);
+    __shared__ __align__(16) float As[DC_TOKENS][DC_TOKENS], Ts[DC_TOKENS][DC_TOKENS];
+    __shared__ float Bs[DC_TOKENS][DC_TOKENS + 1], beta[DC_TOKENS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, kh = h / (a.H / a.G), dv = a.dv;
+    pdl_wait();
+    pdl_trigger();
+    int row0, cnt;
+    if (!find_chunk(a.q_start, a.requests, blockIdx.x, row0, cnt)) return;
+    unsigned char* rec_q = rec, *rec_k = rec + D * 64, *rec_b = rec + 2 * D * 64;          // first Q, K, B and G,
+    float* rec_g = reinterpret_cast<float*>(rec_b + 1024);
+    unsigned char* rec_w = rec, *rec_y = rec + D * 64;                                      // then W and Y in their place
+    unsigned char* to = a.scratch + ((size_t)blockIdx.x * a.H + h) * dc_record(D, dv);
+    auto copy = [&](int at, int bytes, const void* from) {
+        for (int i = tid; i < bytes / 16; i += DC_PREP_THREADS) reinterpret_cast<uint4*>(to + at)[i] = reinterpret_cast<const uint4*>(from)[i];
+    };
+
+    // every load first: a thread's decays and values (of its first channel and column), then the rows of k and q
+    const int ch = tid % D, col = tid >= D ? tid - D : tid + DC_PREP_THREADS - D;
+    float raw[DC_TOKENS], value[DC_TOKENS];
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) raw[t] = t < cnt ? a.decay[(size_t)(row0 + t) * a.decay_t + (size_t)h * D + ch] : 0.f;
+#pragma unroll
+    for (int t = 0; t < DC_TOKENS; ++t) value[t] = col < dv && t < cnt ? a.v[(size_t)(row0 + t) * a.v_t + (size_t)h * dv + col] : 0.f;
+    constexpr int ROWS = DC_PREP_THREADS / D;                  // rows the block's threads read at once
+#pragma unroll
+    for (int i = 0; i < DC_TOKENS / ROWS; ++i) {
+        const int t = i * ROWS + tid / D;
+        ks[t * LD + ch] = t < cnt ? a.k[(size_t)(row0 + t) * a.k_t + (size_t)kh * D + ch] : 0.f;
+        qs[t * LD + ch] = t < cnt ? a.q[(size_t)(row0 + t) * a.q_t + (size_t)kh * D + ch] : 0.f;
+    }
+    if (tid < D) {
+        const float rate = -expf(a.a_log[h]), bias = a.dt_bias[(size_t)h * D + ch];
+        float sum = 0.f;
+#pragma unroll
+        for (int t = 0; t < DC_TOKENS; ++t) {
+            float l = rate * dc_softplus(raw[t] + bias) * DC_LOG2_E;
+            if (l < -1e4f) l = -1e4f;                          // a decay of zero; differences of the sums stay numbers
+            if (t < cnt) sum += l;
+            Ls[t * LD + ch] = sum;
+        }
+    }
+    if (tid < DC_TOKENS) beta[tid] = tid < cnt ? 1.f / (1.f + expf(-a.beta[(size_t)(row0 + tid) * a.beta_t + h])) : 0.f;
+    As[tid / 16][tid % 16] = 0.f;
+    As[8 + tid / 16][tid % 16] = 0.f;
+    __syncthreads();
+    {   // unit vectors, and B's diagonal
+        const float q_scale = 1.f / sqrtf((float)D);
+#pragma unroll
+        for (int i = 0; i < DC_TOKENS / 4; ++i) {
+            const int t = warp * (DC_TOKENS / 4) + i;
+            float kk = 0.f, qq = 0.f, kq = 0.f;
+#pragma unroll
+            for (int c = 0; c < D; c += 32) {
+                const float kv = ks[t * LD + c + lane], qv = qs[t * LD + c + lane];
+                kk = fmaf(kv, kv, kk);
+                qq = fmaf(qv, qv, qq);
+                kq = fmaf(kv, qv, kq);
+            }
+            kk = warp_sum(kk);
+            qq = warp_sum(qq);
+            kq = warp_sum(kq);
+            const float kf = 1.f / sqrtf(kk + 1e-6f), qf = q_scale / sqrtf(qq + 1e-6f);
+#pragma unroll
+            for (int c = 0; c < D; c += 32) {
+                ks[t * LD + c + lane] *= kf;
+                qs[t * LD + c + lane] *= qf;
+            }
+            if (lane < DC_TOKENS) Bs[t][lane] = lane == t ? kq * kf * qf : 0.f;
+        }
+    }
+    __syncthreads();
+    if (tid < DC_TOKENS * (DC_TOKENS - 1) / 2) {
+        int t = 1, j = tid;
+        while (j >= t) j -= t++;
+        const float4* kt = reinterpret_cast<const float4*>(ks + t * LD), *kj = reinterpret_cast<const float4*>(ks + j * LD);
+        const float4* qt = reinterpret_cast<const float4*>(qs + t * LD);
+        const float4* lt = reinterpret_cast<const float4*>(Ls + t * LD), *lj = reinterpret_cast<const float4*>(Ls + j * LD);
+        float s0 = 0.f, s1 = 0.f, b0 = 0.f, b1 = 0.f;
+#pragma unroll 4
+        for (int c = 0; c < D / 4; ++c) {
+            const float4 l = lt[c], m = lj[c], kv = kj[c], x = kt[c], y = qt[c];
+            const float e0 = kv.x * dc_ex2(l.x - m.x), e1 = kv.y * dc_ex2(l.y - m.y), e2 = kv.z * dc_ex2(l.z - m.z), e3 = kv.w * dc_ex2(l.w - m.w);
+            s0 = fmaf(x.x, e0, s0); s1 = fmaf(x.y, e1, s1); s0 = fmaf(x.z, e2, s0); s1 = fmaf(x.w, e3, s1);
+            b0 = fmaf(y.x, e0, b0); b1 = fmaf(y.y, e1, b1); b0 = fmaf(y.z, e2, b0); b1 = fmaf(y.w, e3, b1);
+        }
+        As[t][j] = s0 + s1;
+        Bs[t][j] = b0 + b1;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        if (lane < DC_TOKENS) {                                // column `lane` of T by forward substitution
+            float x[DC_TOKENS];
+#pragma unroll
+            for (int t = 0; t < DC_TOKENS; ++t) {
+                float s = t == lane ? 1.f : 0.f, s2 = 0.f;
+#pragma unroll
+                for (int i = 0; i < t; ++i) {
+                    if (i & 1) s2 = fmaf(-As[t][i], x[i], s2);
+                    else s = fmaf(-As[t][i], x[i], s);
+                }
+                x[t] = beta[t] * (s + s2);
+                Ts[t][lane] = x[t];
+            }
+        }
+    } else {                                                   // meanwhile the others: B, and Q, K, G, which need neither A nor T
+        if (warp >= 2) {                                       // j along k, t along n (above the diagonal B is zero)
+            const int n = warp - 2, t = n * 8 + (lane >> 2), j = (lane & 3) * 2;
+            uint4 w;
+            dc_split(Bs[t][j], Bs[t][j + 1], w.x, w.z);
+            dc_split(Bs[t][j + 8], Bs[t][j + 9], w.y, w.w);
+            *reinterpret_cast<uint4*>(rec_b + n * 512 + lane * 16) = w;
+        }
+        for (int c = tid - 32; c < D; c += DC_PREP_THREADS - 32) {
+            const float last = Ls[(DC_TOKENS - 1) * LD + c];
+            rec_g[c] = dc_ex2(last);
+            float kb[DC_TOKENS];
+#pragma unroll
+            for (int t = 0; t < DC_TOKENS; ++t) {
+                const float L = Ls[t * LD + c];
+                kb[t] = ks[t * LD + c] * dc_ex2(last - L);
+                // B operand with channels along k and tokens along n
+                const float x = qs[t * LD + c] * dc_ex2(L);
+                const bf16 hi = __float2bfloat16_rn(x), lo = __float2bfloat16_rn(x - __bfloat162float(hi));
+                bf16* at = reinterpret_cast<bf16*>(rec_q + ((c >> 4) * 2 + (t >> 3)) * 512 + ((t & 7) * 4 + ((c & 7) >> 1)) * 16 + ((c >> 3) & 1) * 4) + (c & 1);
+                at[0] = hi;
+                at[4] = lo;
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {                      // B operand with tokens along k and channels along n
+                uint4 w;
+                dc_split(kb[2 * p], kb[2 * p + 1], w.x, w.z);
+                dc_split(kb[8 + 2 * p], kb[9 + 2 * p], w.y, w.w);
+                *reinterpret_cast<uint4*>(rec_k + (c >> 3) * 512 + ((c & 7) * 4 + p) * 16) = w;
+            }
+        }
+    }
+    __syncthreads();
+    copy(D * 64, 2 * D * 64 + 1024, rec_q);
+    copy(3 * D * 64 + 1024 + dv * 64, D * 4, rec_g);
+    __syncthreads();
+    for (int i = tid; i < D + dv; i += DC_PREP_THREADS) {      // W, Y: rows of T times a channel's keys or a column's values
+        const bool key = i < D;
+        const int c = key ? i : i - D;
+        float x[DC_TOKENS];
+        if (key) {
+#pragma unroll
+            for (int t = 0; t < DC_TOKENS; ++t) x[t] = ks[t * LD + c] * dc_ex2(Ls[t * LD + c]);
+        } else {
+#pragma unroll
+            for (int t = 0; t < DC_TOKENS; ++t) {
+                if (c == col) x[t] = value[t];
+                else x[t] = t < cnt ? a.v[(size_t)(row0 + t) * a.v_t + (size_t)h * dv + c] : 0.f;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < DC_TOKENS; t += 2) {
+            float y[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+                for (int j = 0; j <= t + u; ++j) {
+                    if (j & 1) s1 = fmaf(Ts[t + u][j], x[j], s1);
+                    else s0 = fmaf(Ts[t + u][j], x[j], s0);
+                }
+                y[u] = s0 + s1;
+            }
+            if (key) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int tt = t + u;
+                    const bf16 hi = __float2bfloat16_rn(y[u]), lo = __float2bfloat16_rn(y[u] - __bfloat162float(hi));
+                    bf16* at = reinterpret_cast<bf16*>(rec_w + ((c >> 4) * 2 + (tt >> 3)) * 512 + ((tt & 7) * 4 + ((c & 7) >> 1)) * 16 + ((c >> 3) & 1) * 4) + (c & 1);
+                    at[0] = hi;
+                    at[4] = lo;
+                }
+            } else {                                           // accumulator with columns along m and tokens along n
+                *reinterpret_cast<float2*>(rec_y + ((c >> 4) * 2 + (t >> 3)) * 512 + ((c & 7) * 4 + ((t & 7) >> 1)) * 16 + ((c >> 3) & 1) * 8) =
+                    make_float2(y[0], y[1]);
+            }
+        }
+    }
+    __syncthreads();
+    copy(0, D * 64, rec_w);
+    copy(3 * D * 64 + 1024, dv * 64, rec_y);
+}
+
+// ---- 2 -----------------------------------------------------------------------------------------------------------------
+// The state is held transposed, S^T with columns along m and channels along n: its accumulators are then, as they lie, the A
+// operand of the products with W and Q, and U^T that of the products with K and B. A block has 16 value columns, a warp a quarter of
+// the channels. The quarters' shares of U^T and of the outputs meet in shared memory (two buffers, one barrier a chunk), where every
+// warp adds all of U^T and its part of the outputs. The records come through a ring of DC_STAGES by bulk copies; a stage is
+// free once every warp is in the chunk after it.
+template <int KS>
+__global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const DeltaChunkArgs a) {
+    constexpr int D = 64 * KS, MAIN = 3 * D * 64 + 1024, STAGE = MAIN + 1024 + D * 4;
+    extern __shared__ __align__(128) unsigned char dc_ring[];
+    __shared__ __align__(16) float4 shares[2][4][4][32];       // [buffer][quarter][U, U, o, o][lane]
+    __shared__ __align__(8) uint64_t full[DC_STAGES];
+    const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int h = blockIdx.x, r = blockIdx.z, dv = a.dv;
+    if (tid == 0) {
+        for (int i = 0; i < DC_STAGES; ++i) mbar_init(&full[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    const int begin = a.q_start[r], tokens = a.q_start[r + 1] - begin;
+    if (tokens <= 0) return;
+    const int chunks = (tokens + DC_TOKENS - 1) / DC_TOKENS;
+    int first = 0;
+    for (int i = lane; i < r; i += 32) first += (max(a.q_start[i + 1] - a.q_start[i], 0) + DC_TOKENS - 1) / DC_TOKENS;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+    const int bytes = dc_record(D, dv);
+    const size_t stride = (size_t)a.H * bytes;
+    const unsigned char* rec = a.scratch + ((size_t)first * a.H + h) * bytes;
+    auto issue = [&](int s) {                                  // thread 0
+        const unsigned char* at = rec + (size_t)s * stride;
+        unsigned char* to = dc_ring + (s % DC_STAGES) * STAGE;
+        uint64_t* bar = &full[s % DC_STAGES];
+        mbar_expect_tx(bar, STAGE);
+        dc_bulk_copy(to, at, MAIN, bar);
+        dc_bulk_copy(to + MAIN, at + MAIN + blockIdx.y * 1024, 1024, bar);
+        dc_bulk_copy(to + MAIN + 1024, at + MAIN + dv * 64, D * 4, bar);
+    };
+    if (tid == 0)
+        for (int s = 0; s < min(chunks, DC_STAGES); ++s) issue(s);
+    const int col0 = blockIdx.y * 16, c0 = part * 16 * KS;
+    const int p0 = a.positions[begin];
+    float* slot = a.state + (size_t)a.slots[r] * a.state_slot + (size_t)h * D * dv;
+    const float* rd = slot + ((p0 + 1) & 1) * a.state_half;
+    float* wr = slot + ((p0 + tokens - 1) & 1) * a.state_half;
+    float S[2 * KS][4];
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n) {
+        const float* at = rd + (size_t)(c0 + n * 8 + 2 * t4) * dv + col0 + g;
+        S[n][0] = at[0];
+        S[n][1] = at[dv];
+        S[n][2] = at[8];
+        S[n][3] = at[dv + 8];
+    }
+    __syncthreads();                                           // the barriers are set up
+    float* out = a.o + (size_t)begin * a.o_t + (size_t)h * dv + col0 + g;
+    for (int s = 0; s < chunks; ++s) {
+        const unsigned char* st = dc_ring + (s % DC_STAGES) * STAGE;
+        const uint4* frags = reinterpret_cast<const uint4*>(st) + lane;
+        mbar_wait(&full[s % DC_STAGES], (uint32_t)(s / DC_STAGES) & 1u, a.error_flag);
+        float u[2][4] = {}, o[2][4] = {};
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            unsigned hi[4], lo[4];
+            dc_split(S[2 * k][0], S[2 * k][1], hi[0], lo[0]);
+            dc_split(S[2 * k][2], S[2 * k][3], hi[1], lo[1]);
+            dc_split(S[2 * k + 1][0], S[2 * k + 1][1], hi[2], lo[2]);
+            dc_split(S[2 * k + 1][2], S[2 * k + 1][3], hi[3], lo[3]);
+            const int at = (part * KS + k) * 2;
+            const uint4 w0 = frags[at * 32], w1 = frags[(at + 1) * 32], q0 = frags[(4 * D / 32 + at) * 32], q1 = frags[(4 * D / 32 + at + 1) * 32];
+            dc_mma(u[0], hi, w0.x, w0.y); dc_mma(u[1], hi, w1.x, w1.y); dc_mma(o[0], hi, q0.x, q0.y); dc_mma(o[1], hi, q1.x, q1.y);
+            dc_mma(u[0], lo, w0.x, w0.y); dc_mma(u[1], lo, w1.x, w1.y); dc_mma(o[0], lo, q0.x, q0.y); dc_mma(o[1], lo, q1.x, q1.y);
+            dc_mma(u[0], hi, w0.z, w0.w); dc_mma(u[1], hi, w1.z, w1.w); dc_mma(o[0], hi, q0.z, q0.w); dc_mma(o[1], hi, q1.z, q1.w);
+        }
+        float4 (*meet)[4][32] = shares[s & 1];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            meet[part][n][lane] = make_float4(u[n][0], u[n][1], u[n][2], u[n][3]);
+            meet[part][2 + n][lane] = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
+        }
+        __syncthreads();
+        if (tid == 0 && s > 0 && s - 1 + DC_STAGES < chunks) issue(s - 1 + DC_STAGES);
+        unsigned hi[4], lo[4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            const float4 sum = dc_add4(meet[0][n][lane], meet[1][n][lane], meet[2][n][lane], meet[3][n][lane]);
+            const float4 y = *reinterpret_cast<const float4*>(st + MAIN + (n * 32 + lane) * 16);
+            dc_split(y.x - sum.x, y.y - sum.y, hi[2 * n], lo[2 * n]);
+            dc_split(y.z - sum.z, y.w - sum.w, hi[2 * n + 1], lo[2 * n + 1]);
+        }
+        const float2* decay = reinterpret_cast<const float2*>(st + MAIN + 1024) + (c0 >> 1) + t4;
+        uint4 kf[2 * KS];
+#pragma unroll
+        for (int n = 0; n < 2 * KS; ++n) {
+            const float2 d = decay[n * 4];
+            kf[n] = frags[(8 * D / 32 + part * 2 * KS + n) * 32];
+            S[n][0] *= d.x; S[n][1] *= d.y; S[n][2] *= d.x; S[n][3] *= d.y;
+        }
+        // a quarter stores the outputs of a half of the tokens and of 8 of the columns
+        const int half = part & 1, upper = part >> 1;
+        const float4 sum = dc_add4(meet[0][2 + half][lane], meet[1][2 + half][lane], meet[2][2 + half][lane], meet[3][2 + half][lane]);
+        float y[4] = {sum.x, sum.y, sum.z, sum.w};
+        const uint4 bf = frags[(12 * D / 32 + half) * 32];
+#pragma unroll
+        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], hi, kf[n].x, kf[n].y);
+        dc_mma(y, hi, bf.x, bf.y);
+#pragma unroll
+        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], lo, kf[n].x, kf[n].y);
+        dc_mma(y, lo, bf.x, bf.y);
+#pragma unroll
+        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], hi, kf[n].z, kf[n].w);
+        dc_mma(y, hi, bf.z, bf.w);
+        const int t = s * DC_TOKENS + half * 8 + 2 * t4;
+        float* to = out + (size_t)t * a.o_t + upper * 8;
+        if (t < tokens) to[0] = upper ? y[2] : y[0];
+        if (t + 1 < tokens) to[a.o_t] = upper ? y[3] : y[1];
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * KS; ++n) {
+        float* at = wr + (size_t)(c0 + n * 8 + 2 * t4) * dv + col0 + g;
+        at[0] = S[n][0];
+        at[dv] = S[n][1];
+        at[8] = S[n][2];
+        at[dv + 8] = S[n][3];
+    }
+}
+
+template <int KS> void launch_chunks(const DeltaChunkArgs& a, int chunks, cudaStream_t stream) {
+    constexpr int D = 64 * KS;
+    const int part1 = 2 * D * 64 + 1024 + D * 4, part2 = D * 64 + a.dv * 64;
+    const size_t smem = (size_t)3 * DC_TOKENS * (D + 4) * sizeof(float) + (part1 > part2 ? part1 : part2);
+    LLMP_ALLOW_SMEM(delta_chunks_kernel<D>, smem);
+    llmp_launch_dependent(delta_chunks_kernel<D>, dim3(chunks, a.H), dim3(DC_PREP_THREADS), smem, stream, a);
+    const size_t ring = (size_t)DC_STAGES * (3 * D * 64 + 1024 + 1024 + D * 4);
+    LLMP_ALLOW_SMEM(delta_chain_kernel<KS>, ring);
+    llmp_launch_dependent(delta_chain_kernel<KS>, dim3(a.H, a.dv / 16, a.requests), dim3(DC_CHAIN_THREADS), ring, stream, a);
+}
+
+}  // namespace
+
+// Bytes of scratch for `rows` tokens of R requests; 0: these sizes are not served.
+LLMP_API long llmp_delta_chunks_scratch(int rows, int R, int H, int d, int dv) {
+    if (rows <= 0 || R <= 0 || H <= 0 || (d != 64 && d != 128) || dv < 16 || dv % 16 || dv > 512) return 0;
+    return ((long)(rows - 1) / DC_TOKENS + R) * H * dc_record(d, dv);
+}
+
+// q, k, v: the convolved rows; decay, beta: pre-activations (delta_prep and delta_scan in one).
+LLMP_API int llmp_delta_chunks(const float* q, long q_t, const float* k, long k_t, const float* v, long v_t, const float* decay, long decay_t,
+                               const float* beta, long beta_t, const float* a_log, const float* dt_bias, float* state, long state_slot,
+                               long state_half, const int* q_start, const int* slots, const int* positions, float* o, long o_t, void* scratch,
+                               long scratch_bytes, int rows, int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
+    if (R <= 0 || rows <= 0) return 0;
+    LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && H <= 65535 && R <= 65535, "delta_chunks: bad sizes heads=%d qk_heads=%d requests=%d", H, G, R);
+    LLMP_REQUIRE(error_flag != nullptr, "delta_chunks: an error flag in device memory is required");
+    const long need = llmp_delta_chunks_scratch(rows, R, H, d, dv);
+    LLMP_REQUIRE(need > 0, "delta_chunks: heads of %d x %d are not served", d, dv);
+    LLMP_REQUIRE(scratch != nullptr && scratch_bytes >= need && (size_t)scratch % 16 == 0, "delta_chunks: %ld bytes of scratch are needed", need);
+    DeltaChunkArgs a;
+    a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.v = v; a.v_t = v_t; a.decay = decay; a.decay_t = decay_t; a.beta = beta; a.beta_t = beta_t;
+    a.a_log = a_log; a.dt_bias = dt_bias; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
+    a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.scratch = (unsigned char*)scratch; a.requests = R; a.H = H; a.G = G; a.dv = dv;
+    a.error_flag = error_flag;
+    const int chunks = (rows - 1) / DC_TOKENS + R;
+    if (d == 64) launch_chunks<1>(a, chunks, stream);
+    else launch_chunks<2>(a, chunks, stream);
+    return llmp_check_launch("delta_chunks");
+}

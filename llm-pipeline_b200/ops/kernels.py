@@ -104,6 +104,7 @@ _SIGNATURES = {
     "llmp_gated_group_norm": [_P, _L, _P, _L, _P, _P, _I, _L, _I, _I, _I, _I, _F, _P],
     "llmp_delta_prep": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _P],
     "llmp_delta_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _P],
+    "llmp_delta_chunks": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
     "llmp_sig_qkv_post": [_P, _L, _P, _I, _P, _P, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "llmp_sigmoid_attention": [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "llmp_sigmoid_attention_mma": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
@@ -1617,6 +1618,42 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     _call("llmp_delta_scan", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0),
           _ptr(beta), beta.stride(0), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
           slots.numel(), heads, qk_heads, dim, vdim, _stream())
+    return out
+
+
+DELTA_CHUNKS_MIN_TOKENS = 32
+DELTA_CHUNKS_MAX_BYTES = 512 << 20
+
+
+def delta_chunks_scratch(dtype: torch.dtype, rows: int, requests: int, max_q_len: int, heads: int, dim: int, vdim: int) -> int:
+    """Bytes of scratch that ``delta_chunks`` takes for a step, or 0 where ``delta_prep`` and ``delta_scan`` serve it: float32, short
+    portions, sizes without an instance, and steps whose chunks would take more than ``DELTA_CHUNKS_MAX_BYTES``."""
+    if dtype != torch.bfloat16 or max_q_len < DELTA_CHUNKS_MIN_TOKENS:
+        return 0
+    fn = library().llmp_delta_chunks_scratch
+    fn.argtypes, fn.restype = [_I, _I, _I, _I, _I], _L
+    need = int(fn(rows, requests, heads, dim, vdim))
+    return need if need <= DELTA_CHUNKS_MAX_BYTES else 0
+
+
+def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, a_log: torch.Tensor,
+                 dt_bias: torch.Tensor, state: torch.Tensor, state_offset: int, q_start: torch.Tensor, slots: torch.Tensor,
+                 positions: torch.Tensor, out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, scratch: int) -> torch.Tensor:
+    """``delta_prep`` and ``delta_scan`` for steps with long portions, in chunks on the tensor cores (csrc/delta_chunks.cu): the same
+    rows before ``delta_prep``, which stay as they are. ``scratch``: what ``delta_chunks_scratch`` gave."""
+    H, G, d, dv = int(heads), int(qk_heads), int(dim), int(vdim)
+    N = q.shape[0]
+    for t, name, width in ((q, "q", G * d), (k, "k", G * d), (v, "v", H * dv), (decay, "decay", H * d), (beta, "beta", H), (out, "out", H * dv)):
+        _need(t.dtype == torch.float32 and t.stride(1) == 1 and t.shape == (N, width), f"delta_chunks: {name} must be float32 rows of {width} entries")
+    _need(a_log.dtype == dt_bias.dtype == torch.float32 and a_log.numel() == H and dt_bias.numel() == H * d and a_log.is_contiguous() and
+          dt_bias.is_contiguous(), "delta_chunks takes float32 vectors of one entry per head, and per head and channel")
+    for t, name in ((q_start, "q_start"), (slots, "slots"), (positions, "positions")):
+        _i32(t, name)
+    ptr, slot_stride, half = _state_views(state, state_offset, H * d * dv, "delta_chunks")
+    room = torch.empty(scratch, dtype=torch.uint8, device=q.device)
+    _call("llmp_delta_chunks", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0), _ptr(beta),
+          beta.stride(0), _ptr(a_log), _ptr(dt_bias), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
+          _ptr(room), scratch, N, slots.numel(), H, G, d, dv, error_flag().data_ptr(), _stream())
     return out
 
 

@@ -13,7 +13,8 @@ query/key head i // (H / G))::
 
 The six products that read h are one product against [Wq; Wk; Wv; Wb; Wa1; Wg1] with a float32 result; the inner sizes of
 the two-step projections are whatever the tensors have. Convolutions, unit norms, step sizes, decays, state and read-out
-are float32 (``csrc/short_conv.cu``, ``csrc/delta_rule.cu``); the gated rows are rounded once to the compute type for the
+are float32 (``csrc/short_conv.cu``, ``csrc/delta_rule.cu``; long portions in bfloat16 in chunks on the tensor cores with split
+factors, ``csrc/delta_chunks.cu``); the gated rows are rounded once to the compute type for the
 output product.
 
 State of a request: one float32 vector ``[conv piece | state piece]``, each piece two copies that take turns by the parity
@@ -114,10 +115,15 @@ class GatedDeltaRule(Mixer):
         kernels.short_conv(proj[:, :C], self.conv_w, None, cache.state, 0, ctx.q_start, ctx.slots, ctx.positions, ctx.token_request,
                            mixed, ctx.max_q_len, silu=True)
         q, k, v = mixed[:, :self.qk_size], mixed[:, self.qk_size:2 * self.qk_size], mixed[:, 2 * self.qk_size:]
-        kernels.delta_prep(q, k, decay, beta, self.a_log, self.dt_bias, H, self.qk_heads, self.dim)
         o = torch.empty((N, self.v_size), dtype=torch.float32, device=x.device)
-        kernels.delta_scan(q, k, v, decay, beta, cache.state, self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, o,
-                           H, self.qk_heads, self.dim, self.vdim)
+        scratch = kernels.delta_chunks_scratch(x.dtype, N, ctx.num_requests, ctx.max_q_len, H, self.dim, self.vdim)
+        if scratch:
+            kernels.delta_chunks(q, k, v, decay, beta, self.a_log, self.dt_bias, cache.state, self.conv_entries, ctx.q_start, ctx.slots,
+                                 ctx.positions, o, H, self.qk_heads, self.dim, self.vdim, scratch)
+        else:
+            kernels.delta_prep(q, k, decay, beta, self.a_log, self.dt_bias, H, self.qk_heads, self.dim)
+            kernels.delta_scan(q, k, v, decay, beta, cache.state, self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, o,
+                               H, self.qk_heads, self.dim, self.vdim)
         normed = torch.empty((N, self.v_size), dtype=x.dtype, device=x.device)
         kernels.gated_group_norm(o, gate, self.norm_w, normed, self.vdim, self.eps, gate_first=False)
         return linear(normed, self.w_out, out_dtype=torch.float32), None
