@@ -14,8 +14,12 @@
 //      products of 16 tokens a chunk on the tensor cores instead of 16 passes.
 // Everything is float32; ratios of decays are exponentials of differences of their logarithms (never above one, so nothing
 // overflows however fast a channel forgets). Where a float32 number enters a product it is split into two bfloat16 halves, and of
-// the four products of halves the three larger are summed in float32 (16 bits of each factor). The operands of launch 2 lie in
-// scratch in the order of its fragments, the two halves beside each other, and are copied as they are.
+// the four products of halves the three larger are summed in float32 (16 bits of each factor): outputs and state are 5e-6 from
+// 64 bits of the same rows (token by token 2e-7), a layer's rows 1.8e-3 either way, which is what its bfloat16 products leave.
+// The operands of launch 2 lie in scratch in the order of its fragments, the two halves beside each other, and are copied as they
+// are. 2,048 tokens of 16 heads of 128 x 128: 191 us, prepared and walked token by token 660. Launch 1 (91 us with cold caches) is
+// issue-bound at 44 % with 14 warps an SM; launch 2 (99) is the chain's latency, 0.77 us a chunk, of which the products are a
+// fifth. On the way: 32 columns a block with fragments loaded from global memory 143 us, two barriers a chunk 114.
 #include "tcgen05.cuh"
 
 namespace {

@@ -1621,6 +1621,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     return out
 
 
+# From two chunks of 16 tokens on for some request: one call instead of two (a layer of 32 tokens: 162 us either way, the host's time;
+# 300 + 147 tokens 232 -> 169). Single tokens and the shortest portions read and write the state once either way, and scratch
+# would only be in their way. The chunks' operands take 34 KB each at heads of 128 x 128.
 DELTA_CHUNKS_MIN_TOKENS = 32
 DELTA_CHUNKS_MAX_BYTES = 512 << 20
 

@@ -185,6 +185,55 @@ def test_gated_delta_rule_alone(sizes):
         assert (o.cpu().double() - want.view(n, -1)).abs().max() < 1e-4, cuts
 
 
+@pytest.mark.parametrize("lengths", [((16, 1), (33,)), ((5, 17), (64, 15), (1, 1)), ((100, 31),)], ids=str)
+@pytest.mark.parametrize("sizes", [(4, 2, 64, 48, 0.0), (2, 2, 128, 128, -3.0), (3, 1, 128, 16, 6.0)], ids=str)
+def test_gated_delta_rule_in_chunks(sizes, lengths):
+    """Requests around the chunks' edges side by side, going on in a second step, in slots that are not theirs by number, with decays
+    near one, mixed and near zero, against the rule written out in float64. Factors of 16 bits (2^-17 of each at most) in three
+    products a token one after another: within 2^-14 of the largest entry. Other slots and what lies beside the state stay."""
+    from llm_pipeline_b200.ops import kernels
+    heads, qk_heads, dim, vdim, shift = sizes
+    gen = torch.Generator().manual_seed(sum(sum(n) for n in lengths) + dim + vdim)
+    dev, R, offset, piece = "cuda", len(lengths), 4, heads * dim * vdim
+    a_log, dt_bias = torch.rand(heads, generator=gen) * 2 - 1, torch.randn(heads * dim, generator=gen) + shift
+    widths = (qk_heads * dim, qk_heads * dim, heads * vdim, heads * dim, heads)
+    rows = [[torch.randn(sum(n), w, generator=gen) for w in widths] for n in lengths]
+    state = torch.full((R + 2, offset + 2 * piece + 4), 5.0, device=dev)
+    slots = list(range(R, 0, -1))
+    state[slots] = 0.0
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)   # noqa: E731
+    got = [[] for _ in lengths]
+    for step in range(2):
+        mine = [r for r in range(R) if len(lengths[r]) > step]
+        at = [sum(lengths[r][:step]) for r in mine]
+        count = [lengths[r][step] for r in mine]
+        x = [torch.cat([rows[r][k][a:a + n] for r, a, n in zip(mine, at, count)]).to(dev) for k in range(5)]
+        o, starts = torch.empty(sum(count), heads * vdim, device=dev), [sum(count[:k]) for k in range(len(mine) + 1)]
+        need = kernels.delta_chunks_scratch(torch.bfloat16, sum(count), len(mine), kernels.DELTA_CHUNKS_MIN_TOKENS, heads, dim, vdim)
+        kernels.delta_chunks(*x, a_log.to(dev), dt_bias.to(dev), state, offset, i32(starts), i32([slots[r] for r in mine]),
+                             i32([p for a, n in zip(at, count) for p in range(a, a + n)]), o, heads, qk_heads, dim, vdim, need)
+        for r, a, n in zip(mine, starts, count):
+            got[r].append(o[a:a + n].double().cpu())
+    kernels.check_error_flag()
+    for r, (q, k, v, pre, beta) in enumerate(rows):
+        n = q.shape[0]
+        q, k = (y.double().view(n, qk_heads, dim) for y in (q, k))
+        q, k = (y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6) for y in (q, k))
+        decay = torch.exp(-torch.exp(a_log.double())[None, :, None] * plain.softplus(pre.double() + dt_bias.double()).view(n, heads, dim))
+        beta, want, S = torch.sigmoid(beta.double()), torch.zeros(n, heads, vdim, dtype=torch.float64), torch.zeros(heads, dim, vdim, dtype=torch.float64)
+        own = torch.arange(heads) // (heads // qk_heads)
+        for t in range(n):
+            S = decay[t][:, :, None] * S
+            u = beta[t][:, None] * (v[t].double().view(heads, vdim) - torch.einsum("hdv,hd->hv", S, k[t, own]))
+            S = S + k[t, own][:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t, own]) * dim ** -0.5
+        want = want.view(n, -1)
+        assert (torch.cat(got[r]) - want).abs().max() <= 2.0 ** -14 * want.abs().max(), r
+        kept = state[slots[r], offset + ((n - 1) & 1) * piece:][:piece].double().cpu().view(heads, dim, vdim)
+        assert (kept - S).abs().max() <= 2.0 ** -14 * S.abs().max(), r
+    assert (state[[0, R + 1]] == 5.0).all() and (state[slots, :offset] == 0.0).all() and (state[slots, offset + 2 * piece:] == 0.0).all()
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
     from llm_pipeline_b200.ops import kernels
