@@ -4,14 +4,17 @@
 // A block takes a tile of up to 16 consecutive new tokens of one request and one range of keys, with a warp per
 // query head. Keys are walked in tiles of 32 aligned to key 0. For a key tile
 //   1. warp g multiplies its head's 16 queries with the 32 keys of its key/value head, caps the scores, takes the
-//      sigmoid (float32) and leaves the 16 x 32 weights in shared memory, in the layout of the accumulator registers;
-//   2. warp h adds the weights of all heads with the coefficients of row h of the mixing matrix (float32; every lane
-//      reads the entries that it holds itself in the accumulator layout, so the reads are dense);
-//   3. warp h rounds its mixed weights to bfloat16 and multiplies them with the 32 values of its key/value head.
+//      sigmoid (float32) and leaves the halves of the 16 x 32 weights in shared memory, the pairs in the order of its registers;
+//   2. the weights of all heads are mixed by the matrix of the heads as a product of its own: 16 heads out, 16 heads in, a column
+//      for each of the 512 (token, key) pairs, dealt out over the warps. Both factors are split into two bfloat16 halves and
+//      the three larger products of halves summed in float32, which leaves the mixed weights 16 bits;
+//   3. they are rounded to bfloat16, and warp h multiplies those of its head with the 32 values of its key/value head.
 // Nothing is normalised over keys, so the output registers simply add up over key tiles and key ranges: with more
 // than one range the blocks leave float32 partial sums that a second kernel adds in the order of the ranges.
 // The keys of the next tile are copied (cp.async) while the weights are mixed and multiplied with the values, the
 // values of the next tile while the next scores are made.
+// With every warp adding up all heads' float32 weights on the CUDA cores, a key tile moved 512 KB through shared memory for the
+// mix alone, 4,096 clocks of an SM; as a product it moves 100 KB.
 #include "common.cuh"
 
 namespace {
@@ -31,6 +34,7 @@ struct SigMmaArgs {
     float* partial;
     int H, G, page_size, segments, segment_keys;
     float scale, cap;
+    bool late_keys;             // the mixed weights lie where the keys do
 };
 
 __device__ __forceinline__ void sm_cp_async_16(void* smem_dst, const void* gmem_src, bool valid) {
@@ -62,12 +66,27 @@ __device__ __forceinline__ unsigned sm_pack(float lo, float hi) {
     return *reinterpret_cast<const unsigned*>(&v);
 }
 
-// sigmoid(cap tanh(s / cap) + b) with tanh(x) = 1 - 2 / (1 + e^(2x)); the exponentials' relative error is about 2^-21,
-// which leaves the weight's absolute error near 1e-7.
-__device__ __forceinline__ float sm_weight(float s, float cap, float inv_cap, float b) {
-    if (cap > 0.f) s = cap * (1.f - __fdividef(2.f, 1.f + __expf(2.f * s * inv_cap)));
-    return __fdividef(1.f, 1.f + __expf(-(s + b)));
+// Two floats as a pair of bfloat16, and what that leaves of them as another pair.
+__device__ __forceinline__ void sm_split(float u, float v, unsigned& hi, unsigned& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(u, v);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(u - __low2float(h), v - __high2float(h));
+    hi = *reinterpret_cast<const unsigned*>(&h);
+    lo = *reinterpret_cast<const unsigned*>(&l);
 }
+
+// cap tanh(s / cap). SMALL: |s / cap| <= SM_SMALL, where five terms of tanh's series leave 2.4e-7 of the result and no work for
+// the special-function unit; else tanh(x) = 1 - 2 / (1 + e^(2x)) with exponentials whose relative error is about 2^-21.
+constexpr float SM_SMALL = 0.35f;
+template <bool SMALL> __device__ __forceinline__ float sm_cap(float s, float cap, float inv_cap) {
+    if (!SMALL) return cap * (1.f - __fdividef(2.f, 1.f + __expf(2.f * s * inv_cap)));
+    const float x = s * inv_cap, y = x * x;
+    return s * fmaf(y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), 1.f);
+}
+__device__ __forceinline__ float sm_sigmoid(float s) { return __fdividef(1.f, 1.f + __expf(-s)); }
+
+constexpr int SM_PAIRS = SM_ROWS * SM_KEYS + 8;        // entries of a head's (token, key) pairs in shared memory: conflict-free ldmatrix
+constexpr int SM_PS = SM_KEYS + 8;                     // of a token's mixed weights
+constexpr int SM_PH = SM_ROWS * SM_PS + 8;             // of a head's: eight heads' rows meet no bank twice
 
 // D16: dim / 16, DV16: vdim / 16. One warp per query head.
 template <int D16, int DV16>
@@ -79,8 +98,10 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     bf16* Qs = reinterpret_cast<bf16*>(sm_smem);                    // [H][16][KS]
     bf16* Ks = Qs + (size_t)H * SM_ROWS * KS;                       // [G][32][KS]
     bf16* Vs = Ks + (size_t)G * SM_KEYS * KS;                       // [G][32][VS]
-    float4* Ws = reinterpret_cast<float4*>(Vs + (size_t)G * SM_KEYS * VS);   // [H][4][32 lanes] of 4 floats
-    float* tk = reinterpret_cast<float*>(Ws + (size_t)H * 4 * 32);  // [H][H]
+    const int wrows = min(SM_MAX_HEADS, H + 1);
+    bf16* Wh = Vs + (size_t)G * SM_KEYS * VS;                       // [wrows][SM_PAIRS]: the weights' halves; row H, if any, is zero
+    bf16* Wl = Wh + wrows * SM_PAIRS;
+    bf16* Ps = a.late_keys ? Ks : Wl + wrows * SM_PAIRS;            // [H][16][SM_PS] with SM_PH entries a head: the mixed weights
     __shared__ long long key_off[SM_KEYS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
     const int gr = lane >> 2, t = lane & 3;
@@ -107,7 +128,13 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
         const bool ok = row < ntok;
         sm_cp_async_16(Qs + ((size_t)h * SM_ROWS + row) * KS + c, ok ? a.q + (size_t)(first + row) * a.q_t + (size_t)h * D + c : a.q, ok);
     }
-    for (int i = tid; i < H * H; i += nthreads) tk[i] = a.talk[i];
+    for (int i = tid; i < (wrows - H) * SM_PAIRS; i += nthreads) Wh[H * SM_PAIRS + i] = Wl[H * SM_PAIRS + i] = __float2bfloat16_rn(0.f);
+    unsigned th[4], tl[4];                                          // the mixing matrix as an A operand: heads out along m, heads in along k
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int ho = gr + 8 * (i & 1), hi = 2 * t + 8 * (i >> 1);
+        sm_split(ho < H && hi < H ? a.talk[ho * H + hi] : 0.f, ho < H && hi + 1 < H ? a.talk[ho * H + hi + 1] : 0.f, th[i], tl[i]);
+    }
     auto issue_keys = [&](int j0) {
         if (j0 <= hi) {
             if (tid < SM_KEYS) {
@@ -175,38 +202,70 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
                 sm_mma(s[nb + 1], qa, kf[2], kf[3]);
             }
         }
+        float top = 0.f;
 #pragma unroll
-        for (int nb = 0; nb < 4; ++nb) {
-            float w[4];
+        for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int j = j0 + nb * 8 + 2 * t + (c & 1);
-                w[c] = j <= row_pos[c >> 1] ? sm_weight(s[nb][c] * a.scale, a.cap, inv_cap, bias) : 0.f;
+                s[nb][c] *= a.scale;
+                top = fmaxf(top, fabsf(s[nb][c]));                  // a NaN is one either way
             }
-            Ws[((size_t)h * 4 + nb) * 32 + lane] = make_float4(w[0], w[1], w[2], w[3]);
+        if (a.cap > 0.f) {
+            if (__all_sync(0xffffffffu, top <= SM_SMALL * a.cap)) {
+#pragma unroll
+                for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_cap<true>(s[nb][c], a.cap, inv_cap);
+            } else {
+#pragma unroll
+                for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_cap<false>(s[nb][c], a.cap, inv_cap);
+            }
+        }
+        // the pairs of token gr + 8 hr and keys nb 8 .. of the tile are columns (2 nb + hr) 64 + 8 gr ..: a warp writes 128 bytes
+        {
+            unsigned* wh = reinterpret_cast<unsigned*>(Wh + h * SM_PAIRS) + lane;
+            unsigned* wl = reinterpret_cast<unsigned*>(Wl + h * SM_PAIRS) + lane;
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                for (int hr = 0; hr < 2; ++hr) {
+                    const int j = j0 + nb * 8 + 2 * t;
+                    const float w0 = j <= row_pos[hr] ? sm_sigmoid(s[nb][2 * hr] + bias) : 0.f;
+                    const float w1 = j + 1 <= row_pos[hr] ? sm_sigmoid(s[nb][2 * hr + 1] + bias) : 0.f;
+                    sm_split(w0, w1, wh[(2 * nb + hr) * 32], wl[(2 * nb + hr) * 32]);
+                }
         }
         __syncthreads();                                            // all weights are in place, the keys are free
-        issue_keys(j0 + SM_KEYS);
+        if (!a.late_keys) issue_keys(j0 + SM_KEYS);
+        // 32 times 16 columns over the warps: the mixed weights of all heads for two tokens and 8 keys each
+        for (int pair = warp; pair < 32; pair += H) {
+            unsigned bh[4], bl[4];
+            const int at = min(((lane >> 3) & 1) * 8 + (lane & 7), wrows - 1);      // heads past H: the zero row
+            sm_ldmatrix_x4_trans(bh, Wh + at * SM_PAIRS + pair * 16 + (lane >> 4) * 8);
+            sm_ldmatrix_x4_trans(bl, Wl + at * SM_PAIRS + pair * 16 + (lane >> 4) * 8);
+            float m[2][4] = {};
 #pragma unroll
-        for (int nb = 0; nb < 4; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
-        for (int g = 0; g < H; ++g) {
-            const float c = tk[h * H + g];
+            for (int n = 0; n < 2; ++n) sm_mma(m[n], th, bh[2 * n], bh[2 * n + 1]);
 #pragma unroll
-            for (int nb = 0; nb < 4; ++nb) {
-                const float4 w = Ws[((size_t)g * 4 + nb) * 32 + lane];
-                s[nb][0] = fmaf(c, w.x, s[nb][0]); s[nb][1] = fmaf(c, w.y, s[nb][1]);
-                s[nb][2] = fmaf(c, w.z, s[nb][2]); s[nb][3] = fmaf(c, w.w, s[nb][3]);
+            for (int n = 0; n < 2; ++n) sm_mma(m[n], tl, bh[2 * n], bh[2 * n + 1]);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) sm_mma(m[n], th, bl[2 * n], bl[2 * n + 1]);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int q = pair * 2 + n, token = (q & 7) + 8 * ((q >> 3) & 1), key = (q >> 4) * 8 + 2 * t;
+                if (gr < H) *reinterpret_cast<unsigned*>(Ps + gr * SM_PH + token * SM_PS + key) = sm_pack(m[n][0], m[n][1]);
+                if (gr + 8 < H) *reinterpret_cast<unsigned*>(Ps + (gr + 8) * SM_PH + token * SM_PS + key) = sm_pack(m[n][2], m[n][3]);
             }
         }
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");     // this tile's values are here
+        if (!a.late_keys) asm volatile("cp.async.wait_group 1;\n" ::: "memory");     // this tile's values are here
+        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
             unsigned pa[4];
-            pa[0] = sm_pack(s[2 * kk][0], s[2 * kk][1]);
-            pa[1] = sm_pack(s[2 * kk][2], s[2 * kk][3]);
-            pa[2] = sm_pack(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-            pa[3] = sm_pack(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+            sm_ldmatrix_x4(pa, Ps + h * SM_PH + (lane & 15) * SM_PS + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
             for (int nb2 = 0; nb2 < DV16; ++nb2) {
                 unsigned v[4];
@@ -216,6 +275,7 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
             }
         }
         __syncthreads();                                            // the values and the weights are free
+        if (a.late_keys) issue_keys(j0 + SM_KEYS);
         issue_values(j0 + SM_KEYS);
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -236,9 +296,16 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     }
 }
 
-size_t sm_smem_bytes(int H, int G, int d, int dv) {
-    return sizeof(bf16) * ((size_t)H * SM_ROWS * (d + 8) + (size_t)G * SM_KEYS * (d + 8) + (size_t)G * SM_KEYS * (dv + 8)) +
-           sizeof(float) * ((size_t)H * 16 * 32 + (size_t)H * H);
+// Shared memory with the mixed weights in a place of their own or (`late_keys`) in that of the keys, whose copies then wait for the
+// values' product: for sizes that would not fit otherwise.
+size_t sm_smem_bytes(int H, int G, int d, int dv, bool late_keys) {
+    const size_t keys = (size_t)G * SM_KEYS * (d + 8), mixed = (size_t)H * SM_PH;
+    return sizeof(bf16) * ((size_t)H * SM_ROWS * (d + 8) + keys + (size_t)G * SM_KEYS * (dv + 8) + 2 * (size_t)(H < SM_MAX_HEADS ? H + 1 : H) * SM_PAIRS +
+                           (late_keys ? 0 : mixed));
+}
+constexpr size_t SM_MOST_BYTES = 226 * 1024;
+bool sm_late_keys(int H, int G, int d, int dv) {
+    return sm_smem_bytes(H, G, d, dv, false) > SM_MOST_BYTES && (size_t)G * SM_KEYS * (d + 8) >= (size_t)H * SM_PH;
 }
 
 }  // namespace
@@ -264,7 +331,7 @@ LLMP_API int llmp_sigmoid_attention_mma_supports(int H, int G, int d, int dv) {
     if (H <= 0 || G <= 0 || H % G || H > SM_MAX_HEADS) return 0;
     auto instance = [](int x) { return x == 16 || x == 32 || x == 64 || x == 96 || x == 128; };
     if (!instance(d) || !instance(dv)) return 0;
-    return sm_smem_bytes(H, G, d, dv) <= 220 * 1024 ? 1 : 0;
+    return sm_smem_bytes(H, G, d, dv, sm_late_keys(H, G, d, dv)) <= SM_MOST_BYTES ? 1 : 0;
 }
 
 LLMP_API int llmp_sigmoid_attention_mma(const void* q, long q_t, const void* pages, const int* tables, int width, const int* q_start,
@@ -284,7 +351,8 @@ LLMP_API int llmp_sigmoid_attention_mma(const void* q, long q_t, const void* pag
     a.ctx_len = ctx_len; a.tile_req = tile_req; a.tile_tok0 = tile_tok0; a.num_tiles = num_tiles; a.talk = talk; a.pb = pb;
     a.out = (bf16*)out; a.out_t = out_t; a.partial = partial; a.H = H; a.G = G; a.page_size = page_size; a.segments = segments;
     a.segment_keys = segments > 1 ? segment_keys : 0; a.scale = scale; a.cap = cap;
-    const size_t smem = sm_smem_bytes(H, G, d, dv);
+    a.late_keys = sm_late_keys(H, G, d, dv);
+    const size_t smem = sm_smem_bytes(H, G, d, dv, a.late_keys);
     dim3 grid(num_tiles, segments);
 #define LLMP_SM_CASE(A, B)                                                                   \
     if (d == 16 * A && dv == 16 * B) {                                                       \
