@@ -14,7 +14,11 @@
 // The keys of the next tile are copied (cp.async) while the weights are mixed and multiplied with the values, the
 // values of the next tile while the next scores are made.
 // With every warp adding up all heads' float32 weights on the CUDA cores, a key tile moved 512 KB through shared memory for the
-// mix alone, 4,096 clocks of an SM; as a product it moves 100 KB.
+// mix alone, 4,096 clocks of an SM; as a product it moves 100 KB. 2,048 tokens of 16 heads of 128: 285 us before, 197 with the
+// product, 168 with tanh as a series where the scores are far below the cap, exponentials and reciprocals without their range
+// checks, masks only where a row's end is near, and a tile's places found a tile ahead. What is left is the latency of four
+// phases between barriers at four warps a scheduler (issue slots 42 %, tensor pipe 28 %). Shorter key ranges (512, 256 keys) lose
+// to their partial sums: 205, 222 us against 197.
 #include "common.cuh"
 
 namespace {
@@ -74,15 +78,27 @@ __device__ __forceinline__ void sm_split(float u, float v, unsigned& hi, unsigne
     lo = *reinterpret_cast<const unsigned*>(&l);
 }
 
-// cap tanh(s / cap). SMALL: |s / cap| <= SM_SMALL, where five terms of tanh's series leave 2.4e-7 of the result and no work for
-// the special-function unit; else tanh(x) = 1 - 2 / (1 + e^(2x)) with exponentials whose relative error is about 2^-21.
-constexpr float SM_SMALL = 0.35f;
-template <bool SMALL> __device__ __forceinline__ float sm_cap(float s, float cap, float inv_cap) {
-    if (!SMALL) return cap * (1.f - __fdividef(2.f, 1.f + __expf(2.f * s * inv_cap)));
-    const float x = s * inv_cap, y = x * x;
-    return s * fmaf(y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), 1.f);
+__device__ __forceinline__ float sm_ex2(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+    return r;
 }
-__device__ __forceinline__ float sm_sigmoid(float s) { return __fdividef(1.f, 1.f + __expf(-s)); }
+__device__ __forceinline__ float sm_rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+    return r;
+}
+constexpr float SM_LOG2_E = 1.4426950408889634f;
+// tanh(x). SMALL: |x| <= SM_SMALL, where five terms of its series leave 2.4e-7 of the result and no work for the special-function
+// unit; else 1 - 2 / (1 + e^(2x)) with an exponential whose relative error is about 2^-21.
+constexpr float SM_SMALL = 0.35f;
+template <bool SMALL> __device__ __forceinline__ float sm_tanh(float x) {
+    if (!SMALL) return fmaf(-2.f, sm_rcp(1.f + sm_ex2(2.f * SM_LOG2_E * x)), 1.f);
+    const float y = x * x;
+    return x * fmaf(y, fmaf(y, fmaf(y, fmaf(y, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), 1.f);
+}
+// The sigmoid of a number given times -log2(e); the exponential's and the reciprocal's errors leave the weight's near 1e-7.
+__device__ __forceinline__ float sm_sigmoid(float minus_log2) { return sm_rcp(1.f + sm_ex2(minus_log2)); }
 
 constexpr int SM_PAIRS = SM_ROWS * SM_KEYS + 8;        // entries of a head's (token, key) pairs in shared memory: conflict-free ldmatrix
 constexpr int SM_PS = SM_KEYS + 8;                     // of a token's mixed weights
@@ -102,7 +118,7 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     bf16* Wh = Vs + (size_t)G * SM_KEYS * VS;                       // [wrows][SM_PAIRS]: the weights' halves; row H, if any, is zero
     bf16* Wl = Wh + wrows * SM_PAIRS;
     bf16* Ps = a.late_keys ? Ks : Wl + wrows * SM_PAIRS;            // [H][16][SM_PS] with SM_PH entries a head: the mixed weights
-    __shared__ long long key_off[SM_KEYS];
+    __shared__ long long key_off[2][SM_KEYS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
     const int gr = lane >> 2, t = lane & 3;
     const int tile = a.num_tiles - 1 - (int)blockIdx.x;             // the tiles that see most keys start first
@@ -135,50 +151,49 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
         const int ho = gr + 8 * (i & 1), hi = 2 * t + 8 * (i >> 1);
         sm_split(ho < H && hi < H ? a.talk[ho * H + hi] : 0.f, ho < H && hi + 1 < H ? a.talk[ho * H + hi + 1] : 0.f, th[i], tl[i]);
     }
-    auto issue_keys = [&](int j0) {
+    // Where the keys of a tile lie among the pages (-1: nowhere), found a tile ahead by the first warp; a barrier lies between.
+    auto find_keys = [&](int j0) {
+        if (tid < SM_KEYS) {
+            const int j = j0 + tid;
+            long long off = -1;
+            if (j <= hi) {
+                const int page = table[j / a.page_size];
+                if (page >= 0) off = (long long)(((size_t)page * G) * a.page_size + (j % a.page_size)) * rs;
+            }
+            key_off[(j0 / SM_KEYS) & 1][tid] = off;
+        }
+    };
+    // A thread copies piece `tid % pieces` of every (threads / pieces)-th row of the tile's [key/value head][key].
+    const size_t head_step = (size_t)a.page_size * rs;
+    auto copy_rows = [&](int j0, bf16* dst, int stride, int pieces, int from) {
         if (j0 <= hi) {
-            if (tid < SM_KEYS) {
-                const int j = j0 + tid;
-                long long off = -1;
-                if (j <= hi) {
-                    const int page = table[j / a.page_size];
-                    if (page >= 0) off = (long long)(((size_t)page * G) * a.page_size + (j % a.page_size)) * rs;
+            const int step = nthreads / pieces, c = tid % pieces * 8, row0 = tid / pieces;
+            const long long* offs = key_off[(j0 / SM_KEYS) & 1];
+            if (row0 < step)
+                for (int row = row0; row < G * SM_KEYS; row += step) {
+                    const long long off = offs[row % SM_KEYS];
+                    sm_cp_async_16(dst + (size_t)row * stride + c, off >= 0 ? a.pages + off + (row / SM_KEYS) * head_step + from + c : a.pages, off >= 0);
                 }
-                key_off[tid] = off;
-            }
-            __syncthreads();
-            for (int e = tid; e < G * SM_KEYS * QV; e += nthreads) {
-                const int c = (e % QV) * 8, key = (e / QV) % SM_KEYS, kv = e / (QV * SM_KEYS);
-                const long long off = key_off[key];
-                const bool ok = off >= 0;
-                sm_cp_async_16(Ks + ((size_t)kv * SM_KEYS + key) * KS + c, ok ? a.pages + off + (size_t)kv * a.page_size * rs + c : a.pages, ok);
-            }
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    auto issue_values = [&](int j0) {        // after issue_keys of the same tile: its offsets are still in place
-        if (j0 <= hi) {
-            for (int e = tid; e < G * SM_KEYS * VV; e += nthreads) {
-                const int c = (e % VV) * 8, key = (e / VV) % SM_KEYS, kv = e / (VV * SM_KEYS);
-                const long long off = key_off[key];
-                const bool ok = off >= 0;
-                sm_cp_async_16(Vs + ((size_t)kv * SM_KEYS + key) * VS + c, ok ? a.pages + off + (size_t)kv * a.page_size * rs + D + c : a.pages, ok);
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
+    auto issue_keys = [&](int j0) { copy_rows(j0, Ks, KS, QV, 0); };
+    auto issue_values = [&](int j0) { copy_rows(j0, Vs, VS, VV, D); };
 
     const int h = warp;                                             // this warp's head, in all three steps
     const int kvh = h / hpg;
     int row_pos[2];
     row_pos[0] = gr < ntok ? pos0 + tok0 + gr : -1;
     row_pos[1] = gr + 8 < ntok ? pos0 + tok0 + gr + 8 : -1;
-    const float bias = a.pb[h], inv_cap = a.cap > 0.f ? 1.f / a.cap : 0.f;
+    // a weight is sm_sigmoid(x slope + shift), with x the score or, under a cap, tanh(score to_cap)
+    const float to_cap = a.cap > 0.f ? a.scale / a.cap : 0.f, slope = -SM_LOG2_E * (a.cap > 0.f ? a.cap : a.scale), shift = -SM_LOG2_E * a.pb[h];
     float o[2 * DV16][4];
 #pragma unroll
     for (int i = 0; i < 2 * DV16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
 
     const int tile_lo = (lo / SM_KEYS) * SM_KEYS;                   // lo is a multiple of the key tile anyway
+    find_keys(tile_lo);
+    __syncthreads();
     issue_keys(tile_lo);                                            // group: the queries and the first keys
     issue_values(tile_lo);
     const bf16* Qw = Qs + ((size_t)h * SM_ROWS + (lane & 15)) * KS + (lane >> 4) * 8;
@@ -187,6 +202,7 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     for (int j0 = tile_lo; j0 <= hi; j0 += SM_KEYS) {
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");     // this tile's keys are here
         __syncthreads();
+        find_keys(j0 + SM_KEYS);                                    // (nobody reads the other half any more)
         float s[4][4];
 #pragma unroll
         for (int nb = 0; nb < 4; ++nb) s[nb][0] = s[nb][1] = s[nb][2] = s[nb][3] = 0.f;
@@ -202,26 +218,37 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
                 sm_mma(s[nb + 1], qa, kf[2], kf[3]);
             }
         }
-        float top = 0.f;
-#pragma unroll
-        for (int nb = 0; nb < 4; ++nb)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                s[nb][c] *= a.scale;
-                top = fmaxf(top, fabsf(s[nb][c]));                  // a NaN is one either way
-            }
         if (a.cap > 0.f) {
-            if (__all_sync(0xffffffffu, top <= SM_SMALL * a.cap)) {
+            float top = 0.f;                                        // a NaN is one either way
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    s[nb][c] *= to_cap;
+                    top = fmaxf(top, fabsf(s[nb][c]));
+                }
+            if (__all_sync(0xffffffffu, top <= SM_SMALL)) {
 #pragma unroll
                 for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_cap<true>(s[nb][c], a.cap, inv_cap);
+                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_tanh<true>(s[nb][c]);
             } else {
 #pragma unroll
                 for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_cap<false>(s[nb][c], a.cap, inv_cap);
+                    for (int c = 0; c < 4; ++c) s[nb][c] = sm_tanh<false>(s[nb][c]);
             }
+        }
+#pragma unroll
+        for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) s[nb][c] = sm_sigmoid(fmaf(s[nb][c], slope, shift));
+        if (ntok < SM_ROWS || j0 + SM_KEYS - 1 > pos0 + tok0) {     // some row does not see all of these keys
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (j0 + nb * 8 + 2 * t + (c & 1) > row_pos[c >> 1]) s[nb][c] = 0.f;
         }
         // the pairs of token gr + 8 hr and keys nb 8 .. of the tile are columns (2 nb + hr) 64 + 8 gr ..: a warp writes 128 bytes
         {
@@ -230,12 +257,7 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
 #pragma unroll
             for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
-                for (int hr = 0; hr < 2; ++hr) {
-                    const int j = j0 + nb * 8 + 2 * t;
-                    const float w0 = j <= row_pos[hr] ? sm_sigmoid(s[nb][2 * hr] + bias) : 0.f;
-                    const float w1 = j + 1 <= row_pos[hr] ? sm_sigmoid(s[nb][2 * hr + 1] + bias) : 0.f;
-                    sm_split(w0, w1, wh[(2 * nb + hr) * 32], wl[(2 * nb + hr) * 32]);
-                }
+                for (int hr = 0; hr < 2; ++hr) sm_split(s[nb][2 * hr], s[nb][2 * hr + 1], wh[(2 * nb + hr) * 32], wl[(2 * nb + hr) * 32]);
         }
         __syncthreads();                                            // all weights are in place, the keys are free
         if (!a.late_keys) issue_keys(j0 + SM_KEYS);
@@ -312,15 +334,22 @@ bool sm_late_keys(int H, int G, int d, int dv) {
 
 namespace {
 
-// out[n, c] = sum over the key ranges that hold a visible key of partial[n, range, c], in their order.
-__global__ void sigmoid_mma_ranges_kernel(const float* __restrict__ partial, const int* __restrict__ positions, bf16* __restrict__ out,
-                                          long out_t, int W, int segments, int segment_keys) {
+// out[n, c] = sum over the key ranges that hold a visible key of partial[n, range, c], in their order; four columns a thread (value
+// sizes are multiples of 16).
+__global__ void __launch_bounds__(256) sigmoid_mma_ranges_kernel(const float* __restrict__ partial, const int* __restrict__ positions,
+                                                                 bf16* __restrict__ out, long out_t, int W, int segments, int segment_keys) {
     const int n = blockIdx.x;
     const int used = min(segments, positions[n] / segment_keys + 1);
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        float s = 0.f;
-        for (int k = 0; k < used; ++k) s += partial[((size_t)n * segments + k) * W + c];
-        out[(size_t)n * out_t + c] = from_float<bf16>(s);
+    for (int c = threadIdx.x * 4; c < W; c += blockDim.x * 4) {
+        const float* at = partial + (size_t)n * segments * W + c;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < used; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(at + (size_t)k * W);
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        unsigned* o = reinterpret_cast<unsigned*>(out + (size_t)n * out_t + c);
+        o[0] = sm_pack(s.x, s.y);
+        o[1] = sm_pack(s.z, s.w);
     }
 }
 

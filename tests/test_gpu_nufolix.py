@@ -301,6 +301,18 @@ def test_sigmoid_attention_alone(dtype, sizes):
         assert err < (1e-5 if dtype == torch.float32 else 1e-2), (name, float(err))
 
 
+@pytest.mark.parametrize("sizes", [(16, 16, 64, 64, 30.0), (16, 2, 128, 128, 1.5), (15, 3, 96, 32, 30.0), (9, 9, 128, 128, 0.0), (1, 1, 16, 16, 4.0)],
+                         ids=str)
+def test_sigmoid_attention_mixes_heads_as_a_product(sizes):
+    """Head counts up to and below the mixing product's 16, with the mixed weights in a place of their own and where the keys lie (16
+    key/value heads of 64), caps that scores stay far below and ones they reach, in one key range and in several. The mixed
+    weights and the result are rounded to bfloat16 (2^-8 each at most): within 2^-7 of the largest result."""
+    heads, kv_heads, dim, vdim, cap = sizes
+    results, want = _sigmoid_attention_case(torch.bfloat16, heads, kv_heads, dim, vdim, 333, page=16, seed=heads + dim, cap=cap, segments=(1, 2), bias=-3.0)
+    for name, got in results.items():
+        assert (got.double() - want).abs().max() <= 2.0 ** -7 * want.abs().max(), name
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_one_far_key_holds_all_the_weight(dtype):
     """Every query has a score of about -12 with every key but one, which lies 1 to 1,100 tokens back and gets +12: across
