@@ -204,6 +204,8 @@ gemm_rows_kernel(const TI* __restrict__ A, const TI* __restrict__ W, TO* __restr
                  long ldc, long batch_a, long batch_w, long batch_c) {
     const int lane = threadIdx.x & 31;
     const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (n >= N) return;
     A += (size_t)blockIdx.y * batch_a;
     C += (size_t)blockIdx.y * batch_c;
@@ -258,10 +260,8 @@ LLMP_API int llmp_gemm_simt_batched(const void* A, const void* W, void* C, int i
                          ((size_t)A | (size_t)W) % 16 == 0 && esize > 0;
 #define LLMP_ROWS(TI, TO)                                                                                                         \
     do {                                                                                                                          \
-        if (vec) gemm_rows_kernel<TI, TO, true><<<rows_grid, 256, 0, stream>>>((const TI*)A, (const TI*)W, (TO*)C, M, N, K, lda, ldw,   \
-                                                                               ldc, batch_a, batch_w, batch_c);                  \
-        else gemm_rows_kernel<TI, TO, false><<<rows_grid, 256, 0, stream>>>((const TI*)A, (const TI*)W, (TO*)C, M, N, K, lda, ldw, ldc, \
-                                                                            batch_a, batch_w, batch_c);                          \
+        llmp_launch_dependent(vec ? gemm_rows_kernel<TI, TO, true> : gemm_rows_kernel<TI, TO, false>, rows_grid, dim3(256), 0, stream,  \
+                              (const TI*)A, (const TI*)W, (TO*)C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);            \
     } while (0)
         if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32) LLMP_ROWS(float, float);
         else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16) LLMP_ROWS(bf16, bf16);

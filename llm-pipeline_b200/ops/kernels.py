@@ -68,6 +68,7 @@ _SIGNATURES = {
     "llmp_latent_attention": [_P, _L, _L, _P, _L, _L, _P, _I, _P, _I, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _F, _P, _P],
     "llmp_latent_attention_mma": [_P, _L, _L, _P, _L, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _L, _L, _I, _I, _I, _I, _I, _F, _I,
                                   _I, _P, _I, _I, _P, _P],
+    "llmp_latent_decode": [_P, _L, _L, _P, _L, _L, _P, _P, _I, _P, _P, _L, _L, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P],
     "llmp_latent_gather": [_P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P],
     "llmp_latent_prompt_attention": [_P, _L, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _L, _L, _I, _I, _I, _I, _I, _F, _P, _P, _P],
     "llmp_latent_rows_post": [_P, _L, _P, _L, _I, _I, _I, _I, _P, _I, _F, _P, _P, _I, _I, _P, _I, _L, _P, _P, _I, _P],
@@ -1140,6 +1141,48 @@ def latent_attention_mma(q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch.
           _ptr(pages), _ptr(tables), tables.shape[1], _ptr(q_start), _ptr(ctx_len), _ptr(positions), _ptr(tile_req), _ptr(tile_tok0),
           tile_req.numel(), _ptr(out), out.stride(0), out.stride(1), N, H, rank, rot, pages.shape[1], float(scale),
           LATENT_SEGMENT_KEYS if segments > 0 else 0, int(segments), _ptr(scratch), *(rows or (0, N)), _ptr(sink), _stream())
+    return out
+
+
+LATENT_DECODE_KEYS = 128             # keys that latent_decode takes at a time; its ranges are multiples
+
+
+def latent_decode_supports(rank: int, rot: int, page_size: int) -> bool:
+    """Whether the kernel for single tokens serves these sizes (bfloat16; latents of 128, 256, 384 or 512)."""
+    fn = library().llmp_latent_decode_supports
+    fn.argtypes = [_I, _I, _I]
+    fn.restype = _I
+    return bool(fn(rank, rot, page_size))
+
+
+def latent_decode_ranges(tokens: int, num_heads: int, rank: int, longest: int, sms: int):
+    """(ranges, keys of a range) for ``tokens`` single tokens whose longest context is ``longest``: as many ranges of 128 keys as
+    give every place on the SMs a block (two an SM up to latents of 256, whose keys take half as much shared memory), longer
+    ones beyond, so that the sums left for the second kernel stay few."""
+    places = sms * (2 if rank <= 256 else 1)
+    blocks = tokens * -(-num_heads // 16) * -(-longest // LATENT_DECODE_KEYS)
+    keys = LATENT_DECODE_KEYS * max(1, -(-blocks // places))
+    return -(-longest // keys), keys
+
+
+def latent_decode(q_lat: torch.Tensor, q_rot: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor, ctx_len: torch.Tensor,
+                  out: torch.Tensor, scale: float, longest: int, sink: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``latent_attention_mma`` for a step of single tokens (csrc/latent_decode.cu): row n is request n's. ``longest``: the most keys a
+    request may see."""
+    N, H, rank = q_lat.shape
+    rot = q_rot.shape[2]
+    _sink(sink, H)
+    _need(q_lat.dtype == q_rot.dtype == pages.dtype == out.dtype == torch.bfloat16, "latent_decode takes bfloat16")
+    _need(q_rot.shape[:2] == (N, H) and out.shape == (N, H, rank) and q_lat.stride(2) == 1 and out.stride(2) == 1 and
+          (rot == 0 or q_rot.stride(2) == 1) and ctx_len.numel() == N == tables.shape[0], "latent_decode: shapes do not match")
+    _need(pages.is_contiguous() and pages.dim() == 3 and pages.shape[2] == rank + rot, "latent pages have the wrong layout")
+    for t, name in ((tables, "tables"), (ctx_len, "ctx_len")):
+        _i32(t, name)
+    ranges, keys = latent_decode_ranges(N, H, rank, longest, sm_count())
+    scratch = torch.empty(ranges * N * H * (rank + 2), dtype=torch.float32, device=q_lat.device) if ranges > 1 else None
+    _call("llmp_latent_decode", _ptr(q_lat), q_lat.stride(0), q_lat.stride(1), _ptr(q_rot), q_rot.stride(0), q_rot.stride(1), _ptr(pages),
+          _ptr(tables), tables.shape[1], _ptr(ctx_len), _ptr(out), out.stride(0), out.stride(1), N, H, rank, rot, pages.shape[1], float(scale),
+          keys, ranges, _ptr(scratch), _ptr(sink), _stream())
     return out
 
 

@@ -205,6 +205,10 @@ class LatentAttention(Mixer):
         if not kernels.latent_mma_supports(q_lat.dtype, self.kv_rank, self.rot_dim, cache.pages.shape[1]) or self.dim % 8 or self.rot_dim % 8:
             kernels.latent_attention(q_lat, q_rot, cache.pages, tables, ctx.token_request, ctx.positions, out, self.scale, sink=self.sinks)
             return
+        if ctx.max_q_len == 1 and kernels.latent_decode_supports(self.kv_rank, self.rot_dim, cache.pages.shape[1]):
+            kernels.latent_decode(q_lat, q_rot, cache.pages, tables, ctx.ctx_len, out, self.scale, ctx.decode_ctx_bound or ctx.max_ctx_len,
+                                  sink=self.sinks)
+            return
         if some is not None:
             tiles, longest, rows = some
         else:
