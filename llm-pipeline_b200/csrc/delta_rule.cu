@@ -26,6 +26,8 @@ struct PrepArgs {
 };
 
 __global__ void delta_prep_kernel(const PrepArgs a) {
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const float q_scale = 1.f / sqrtf((float)a.d);
@@ -96,6 +98,8 @@ __global__ void __launch_bounds__(DS_THREADS + 32 * DS_COPY_WARPS) delta_scan_ke
     constexpr int COLS = DS_THREADS / R;                 // columns of a block
     constexpr int ROW = 3 * DP + COLS + 4;               // k, q, decay (padded), the block's columns of v, beta
     const int r = blockIdx.x, h = blockIdx.y;
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int begin = a.q_start[r], end = a.q_start[r + 1];
     if (end <= begin) return;
     const int d = a.d, dv = a.dv;
@@ -202,7 +206,7 @@ LLMP_API int llmp_delta_prep(float* q, long q_t, float* k, long k_t, float* deca
     PrepArgs a;
     a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.decay = decay; a.decay_t = decay_t; a.beta = beta; a.beta_t = beta_t;
     a.a_log = a_log; a.dt_bias = dt_bias; a.H = H; a.G = G; a.d = d;
-    delta_prep_kernel<<<tokens, 256, 0, stream>>>(a);
+    llmp_launch_dependent(delta_prep_kernel, dim3(tokens), dim3(256), 0, stream, a);
     return llmp_check_launch("delta_prep");
 }
 
@@ -241,7 +245,7 @@ LLMP_API int llmp_delta_scan(const float* q, long q_t, const float* k, long k_t,
 #define LLMP_DELTA(NT, RW)                                                                          \
     if (nt == NT && rows == RW) {                                                                   \
         LLMP_ALLOW_SMEM((delta_scan_kernel<NT, RW>), smem);                                         \
-        delta_scan_kernel<NT, RW><<<grid, DS_THREADS + 32 * DS_COPY_WARPS, smem, stream>>>(a, stage_tokens, vec);   \
+        llmp_launch_dependent(delta_scan_kernel<NT, RW>, grid, dim3(DS_THREADS + 32 * DS_COPY_WARPS), smem, stream, a, stage_tokens, vec); \
     } else
     LLMP_DELTA(1, 1) LLMP_DELTA(2, 1) LLMP_DELTA(4, 1) LLMP_DELTA(8, 1) LLMP_DELTA(16, 1) LLMP_DELTA(16, 2) LLMP_DELTA(16, 4)
     LLMP_DELTA(16, 8) LLMP_DELTA(16, 16) LLMP_DELTA(16, 32) LLMP_DELTA(32, 32)

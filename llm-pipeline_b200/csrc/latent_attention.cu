@@ -18,6 +18,8 @@ __global__ void latent_kv_post_kernel(T* __restrict__ qd, long ld, int H, int d,
                                       int nw_bf16, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                       int rot_dims, const int* __restrict__ slots, T* __restrict__ pages) {
     __shared__ float scratch[32];
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int n = blockIdx.x;
     T* q = qd + (size_t)n * ld;
     const T* dkv = q + (size_t)H * (d + r);
@@ -62,10 +64,10 @@ LLMP_API int llmp_latent_kv_post(void* qd, int dtype, long ld, int H, int d, int
                  "latent_kv_post: bad sizes heads=%d dim=%d rot=%d rank=%d rotated=%d", H, d, r, rank, rot_dims);
     LLMP_REQUIRE(rot_dims == 0 || (cos_t && sin_t), "latent_kv_post: a rotation needs its tables");
     if (dtype == LLMP_F32)
-        latent_kv_post_kernel<float><<<N, 128, 0, stream>>>((float*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
+        llmp_launch_dependent(latent_kv_post_kernel<float>, dim3(N), dim3(128), 0, stream, (float*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
                                                             sin_t, rot_dims, slots, (float*)pages);
     else
-        latent_kv_post_kernel<bf16><<<N, 128, 0, stream>>>((bf16*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
+        llmp_launch_dependent(latent_kv_post_kernel<bf16>, dim3(N), dim3(128), 0, stream, (bf16*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
                                                            sin_t, rot_dims, slots, (bf16*)pages);
     return llmp_check_launch("latent_kv_post");
 }

@@ -29,6 +29,8 @@ __global__ void sig_qkv_post_kernel(const float* __restrict__ qkv, long qkv_t, c
                                     const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                                     T* __restrict__ q_out, long q_out_t, const int* __restrict__ slots, T* __restrict__ pages,
                                     int page_size, int H, int G, int d, int dv) {
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int n = blockIdx.x;
     const float* row = qkv + (size_t)n * qkv_t;
     const int half = rot / 2;
@@ -189,10 +191,10 @@ LLMP_API int llmp_sig_qkv_post(const float* qkv, long qkv_t, const void* bias, i
     LLMP_REQUIRE(!rot || (cos_t && sin_t), "sig_qkv_post: a rotation needs its tables");
     LLMP_REQUIRE(!pages || (slots && page_size > 0), "sig_qkv_post: pages need slots and a page size");
     if (dtype == LLMP_BF16)
-        sig_qkv_post_kernel<bf16><<<N, 256, 0, stream>>>(qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), cos_t, sin_t, rot, (bf16*)q_out,
+        llmp_launch_dependent(sig_qkv_post_kernel<bf16>, dim3(N), dim3(256), 0, stream, qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), cos_t, sin_t, rot, (bf16*)q_out,
                                                          q_out_t, slots, (bf16*)pages, page_size, H, G, d, dv);
     else
-        sig_qkv_post_kernel<float><<<N, 256, 0, stream>>>(qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), cos_t, sin_t, rot, (float*)q_out,
+        llmp_launch_dependent(sig_qkv_post_kernel<float>, dim3(N), dim3(256), 0, stream, qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), cos_t, sin_t, rot, (float*)q_out,
                                                           q_out_t, slots, (float*)pages, page_size, H, G, d, dv);
     return llmp_check_launch("sig_qkv_post");
 }

@@ -123,6 +123,8 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     const int gr = lane >> 2, t = lane & 3;
     const int tile = a.num_tiles - 1 - (int)blockIdx.x;             // the tiles that see most keys start first
     const int seg = blockIdx.y;
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int r = a.tile_req[tile], tok0 = a.tile_tok0[tile];
     const int q_begin = a.q_start[r];
     const int q_len = a.q_start[r + 1] - q_begin;
@@ -338,6 +340,8 @@ namespace {
 // sizes are multiples of 16).
 __global__ void __launch_bounds__(256) sigmoid_mma_ranges_kernel(const float* __restrict__ partial, const int* __restrict__ positions,
                                                                  bf16* __restrict__ out, long out_t, int W, int segments, int segment_keys) {
+    pdl_wait();                                    // what the kernels before wrote is complete
+    pdl_trigger();
     const int n = blockIdx.x;
     const int used = min(segments, positions[n] / segment_keys + 1);
     for (int c = threadIdx.x * 4; c < W; c += blockDim.x * 4) {
@@ -386,7 +390,7 @@ LLMP_API int llmp_sigmoid_attention_mma(const void* q, long q_t, const void* pag
 #define LLMP_SM_CASE(A, B)                                                                   \
     if (d == 16 * A && dv == 16 * B) {                                                       \
         LLMP_ALLOW_SMEM((sigmoid_attention_mma_kernel<A, B>), smem);                         \
-        sigmoid_attention_mma_kernel<A, B><<<grid, H * 32, smem, stream>>>(a);               \
+        llmp_launch_dependent(sigmoid_attention_mma_kernel<A, B>, grid, dim3(H * 32), smem, stream, a); \
     } else
 #define LLMP_SM_ROW(A) LLMP_SM_CASE(A, 1) LLMP_SM_CASE(A, 2) LLMP_SM_CASE(A, 4) LLMP_SM_CASE(A, 6) LLMP_SM_CASE(A, 8)
     LLMP_SM_ROW(1) LLMP_SM_ROW(2) LLMP_SM_ROW(4) LLMP_SM_ROW(6) LLMP_SM_ROW(8)
@@ -397,6 +401,7 @@ LLMP_API int llmp_sigmoid_attention_mma(const void* q, long q_t, const void* pag
 #undef LLMP_SM_ROW
 #undef LLMP_SM_CASE
     if (segments > 1)
-        sigmoid_mma_ranges_kernel<<<N, 256, 0, stream>>>(partial, positions, (bf16*)out, out_t, H * dv, segments, segment_keys);
+        llmp_launch_dependent(sigmoid_mma_ranges_kernel, dim3(N), dim3(256), 0, stream, (const float*)partial, positions, (bf16*)out, out_t, H * dv, segments,
+                              segment_keys);
     return llmp_check_launch("sigmoid_attention_mma");
 }
