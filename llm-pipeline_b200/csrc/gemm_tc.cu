@@ -370,42 +370,36 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         }
     } else {
         const int quarter = warp & 3;
+        float* stage_rows = reinterpret_cast<float*>(tiles + (size_t)STAGES * STAGE_BYTES) + quarter * TC_STAGE_FLOATS;
+        const bool whole_lines = (size_t)Y % 16 == 0 && ldy * sizeof(TO) % 16 == 0;
         int n = 0;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++n) {
             const int acc = n & 1;
             if (!mbar_wait(&acc_full[acc], (n >> 1) & 1, error_flag)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const int a0 = (tile % m_tiles) * TC_BM, b0 = (tile / m_tiles) * BN;
-            const int arow = a0 + quarter * 32 + lane;
-#pragma unroll 4
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                float v[16];
-                tmem_ld_16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + c0), v);
-                if (arow < rows_a) {
-                    TO* dst = Y + (size_t)arow * ldy + b0 + c0;
-                    if (b0 + c0 + 16 <= rows_b && ((size_t)dst % 16) == 0) {
-                        if (sizeof(TO) == 4) {
+            const int row0 = a0 + quarter * 32;
+#pragma unroll 2
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                if (b0 + c0 >= rows_b) break;
+                const uint32_t from = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + c0);
+                float v[32];
+                {
+                    float part[16];
+                    tmem_ld_16(from, part);
 #pragma unroll
-                            for (int j = 0; j < 16; j += 4)
-                                *reinterpret_cast<float4*>(reinterpret_cast<float*>(dst) + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                        } else {
+                    for (int j = 0; j < 16; ++j) v[j] = part[j];
+                    tmem_ld_16(from + 16, part);
 #pragma unroll
-                            for (int j = 0; j < 16; j += 8) {
-                                uint4 pack;
-                                __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]), h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-                                __nv_bfloat162 h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]), h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-                                pack.x = *reinterpret_cast<unsigned*>(&h0);
-                                pack.y = *reinterpret_cast<unsigned*>(&h1);
-                                pack.z = *reinterpret_cast<unsigned*>(&h2);
-                                pack.w = *reinterpret_cast<unsigned*>(&h3);
-                                *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dst) + j) = pack;
-                            }
-                        }
-                    } else {
+                    for (int j = 0; j < 16; ++j) v[16 + j] = part[j];
+                }
+                if (whole_lines && b0 + c0 + 32 <= rows_b) {
+                    tc_store_rows(v, stage_rows, lane, [&](int r) -> TO* { return row0 + r < rows_a ? Y + (size_t)(row0 + r) * ldy + b0 + c0 : nullptr; }, (TO*)nullptr);
+                } else if (row0 + lane < rows_a) {
+                    TO* dst = Y + (size_t)(row0 + lane) * ldy + b0 + c0;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (b0 + c0 + j < rows_b) dst[j] = from_float<TO>(v[j]);
-                    }
+                    for (int j = 0; j < 32; ++j)
+                        if (b0 + c0 + j < rows_b) dst[j] = from_float<TO>(v[j]);
                 }
             }
             // this warp has read its part of the accumulator: one arrival per warp frees it for the MMA thread
@@ -562,7 +556,7 @@ static int launch_tc_persistent(const void* A, long rows_a, long lda, const void
                                 long ldy, int* error_flag, cudaStream_t stream) {
     CUtensorMap map_a, map_b;
     if (llmp_matrix_tensor_map(A, rows_a, K, lda, TC_BM, &map_a) || llmp_matrix_tensor_map(B, rows_b, K, ldb, BN, &map_b)) return 1;
-    constexpr size_t smem = (size_t)STAGES * (TC_BM * 128 + BN * 128) + 1024;
+    constexpr size_t smem = (size_t)STAGES * (TC_BM * 128 + BN * 128) + 1024 + 4 * TC_STAGE_FLOATS * sizeof(float);
     auto kernel = gemm_tc_persistent_kernel<BN, STAGES, TO>;
     LLMP_ALLOW_SMEM(kernel, smem);
     static int sms = 0;
@@ -584,7 +578,11 @@ static int dispatch_tc(const void* X, const void* W, TO* Y, int M, int N, int K,
     if (M <= 16) return launch_tc_splitk<16, 10, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 32) return launch_tc_splitk<32, 9, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 64) return launch_tc_splitk<64, 8, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
-    // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs
+    // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs, and 128 x 32 where even
+    // those leave SMs without one: 2,048 rows, 160 columns, K 4,096 26.2 us -> 22.2; 96 columns, K 2,048 15.8 -> 12.6. (Sharing K among
+    // the blocks of a cluster, 64 rows by 128 columns each, lost: 31 and 25 us.)
+    if (N < 256 && (long)((M + TC_BM - 1) / TC_BM) * ((N + 31) / 32) <= 148)
+        return launch_tc_persistent<32, 8, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     if (N >= 256) return launch_tc_persistent<256, 4, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     return launch_tc_persistent<128, 6, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
 }

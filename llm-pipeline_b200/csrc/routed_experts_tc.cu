@@ -191,6 +191,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         }
     } else {
         const int quarter = warp & 3;
+        float* stage_rows = reinterpret_cast<float*>(tiles + (size_t)MT_STAGES * STAGE_BYTES) + quarter * TC_STAGE_FLOATS;
         int n = 0;
         for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++n) {
             const int acc = n & 1;
@@ -202,36 +203,39 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const uint32_t t0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * MT_COLS);
             const int cols = min(OUT_COLS, a.cols - c0);
-#pragma unroll 4
-            for (int c = 0; c < cols; c += 16) {
-                float v[16];
-                tmem_ld_16(t0 + (uint32_t)c, v);
-                if (GATED) {
-                    float u[16];
-                    tmem_ld_16(t0 + (uint32_t)(OUT_COLS + c), u);
+#pragma unroll 1
+            for (int c = 0; c < cols; c += 32) {
+                float v[32];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = expert_act(v[j], u[j], w, a.limit, a.form);
-                } else if (FIRST) {
+                for (int half = 0; half < 32; half += 16) {
+                    float x[16];
+                    tmem_ld_16(t0 + (uint32_t)(c + half), x);
+                    if (GATED) {
+                        float u[16];
+                        tmem_ld_16(t0 + (uint32_t)(OUT_COLS + c + half), u);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = expert_act(0.f, v[j], w, a.limit, EXPERT_FORM_UNGATED);
-                }
-                if (pair < 0) continue;
-                if (FIRST) {
-                    bf16* dst = a.y + (size_t)row * a.cols + c0 + c;
+                        for (int j = 0; j < 16; ++j) v[half + j] = expert_act(x[j], u[j], w, a.limit, a.form);
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 8) {            // the widths are multiples of 8
-                        if (c + j < cols) {
-                            const __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]), h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-                            const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]), h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-                            *reinterpret_cast<uint4*>(dst + j) = make_uint4(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1),
-                                                                           *reinterpret_cast<const unsigned*>(&h2), *reinterpret_cast<const unsigned*>(&h3));
-                        }
+                        for (int j = 0; j < 16; ++j) v[half + j] = FIRST ? expert_act(0.f, x[j], w, a.limit, EXPERT_FORM_UNGATED) : x[j];
                     }
-                } else {
-                    float* dst = a.out + (size_t)pair * a.cols + c0 + c;
+                }
+                if (c + 32 <= cols) {
+                    auto pair_of = [&](int r) { return __shfl_sync(0xffffffffu, pair, r); };
+                    if (FIRST)
+                        tc_store_rows(v, stage_rows, lane, [&](int r) -> bf16* {
+                            return pair_of(r) >= 0 ? a.y + (size_t)(row - lane + r) * a.cols + c0 + c : nullptr; }, (bf16*)nullptr);
+                    else
+                        tc_store_rows(v, stage_rows, lane, [&](int r) -> float* {
+                            const int p = pair_of(r);
+                            return p >= 0 ? a.out + (size_t)p * a.cols + c0 + c : nullptr; }, (float*)nullptr);
+                } else if (pair >= 0) {                          // the last columns of a width that is no multiple of 32 (it is one of 8)
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4)
-                        if (c + j < cols) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    for (int j = 0; j < 32; ++j)
+                        if (c + j < cols) {
+                            if (FIRST) a.y[(size_t)row * a.cols + c0 + c + j] = __float2bfloat16_rn(v[j]);
+                            else a.out[(size_t)pair * a.cols + c0 + c + j] = v[j];
+                        }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -277,7 +281,7 @@ int launch_moe_tc(const bf16* A, long rows_a, const bf16* B, long rows_b, const 
     CUtensorMap map_a, map_b;
     if (llmp_matrix_tensor_map(A, rows_a, a.K, a.K, MT_ROWS, &map_a) ||
         llmp_matrix_tensor_map(B, rows_b, a.K, a.K, GATED ? MT_COLS / 2 : MT_COLS, &map_b)) return 1;
-    constexpr size_t smem = (size_t)MT_STAGES * (MT_ROWS + MT_COLS) * 128 + 1024;
+    constexpr size_t smem = (size_t)MT_STAGES * (MT_ROWS + MT_COLS) * 128 + 1024 + 4 * TC_STAGE_FLOATS * sizeof(float);
     LLMP_ALLOW_SMEM((moe_tc_kernel<FIRST, GATED>), smem);
     const int out_cols = GATED ? MT_COLS / 2 : MT_COLS;
     const long tiles = tiles_max * ((a.cols + out_cols - 1) / out_cols);
