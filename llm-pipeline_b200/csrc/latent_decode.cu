@@ -3,7 +3,9 @@
 // A decoded token's rows are its heads: 16 of them are one m16 tile, which the tile of 64 rows there fills a quarter of, two of eight
 // warps at work. Here a block takes up to 16 heads of one token and one range of keys, 128 keys at a time, whose rows come in
 // two halves of 64 by 16-byte cp.async, all asked for at once. Scores: a warp makes those of 8 keys of each half over the whole row.
-// Softmax: the warps' maxima and sums meet in shared memory, the probabilities go there as bfloat16. Values: a warp makes an
+// Softmax: the warps' maxima and sums meet in shared memory, the probabilities go there as two bfloat16 halves. (One half was 0.6 %
+// further from 64 bits than latent_attention_mma on average, whose smaller key tiles leave more probabilities at exactly 1; with two
+// 2.8 % nearer, at no cost: the products share the values' fragments.) Values: a warp makes an
 // eighth of the latent's columns over all 128 keys, which lie in shared memory already. A range of more keys goes on with a
 // running softmax. With several ranges the blocks leave unnormalised sums, and a second kernel adds a row's in ascending order.
 // 8 requests of 2,048 keys, 16 heads, latents of 512 + 64: 37 us there (ranges of 256 keys), 22 here (as single launches; a layer of
@@ -66,7 +68,8 @@ __global__ void __launch_bounds__(LD_THREADS, 1) latent_decode_kernel(const Late
     const int dk = RANK + a.rot, stride = dk + 8, pieces = dk / 8;
     bf16* Qs = reinterpret_cast<bf16*>(ld_raw);                  // [16][stride]
     bf16* Ks = Qs + LD_ROWS * stride;                            // [128][stride]: keys, and in their first columns values
-    bf16* Ps = Ks + (size_t)LD_KEYS * stride;                    // [16][LD_PS]
+    bf16* Ps = Ks + (size_t)LD_KEYS * stride;                    // [16][LD_PS]: probabilities, then what their rounding left
+    bf16* Pl = Ps + LD_ROWS * LD_PS;
     __shared__ float row_max[8][LD_ROWS], row_sum[8][LD_ROWS];
     __shared__ long long key_off[LD_KEYS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -157,7 +160,10 @@ __global__ void __launch_bounds__(LD_THREADS, 1) latent_decode_kernel(const Late
             for (int half = 0; half < 2; ++half) {
                 const float p0 = ld_ex2(s[half][2 * r] - base), p1 = ld_ex2(s[half][2 * r + 1] - base);
                 sum += p0 + p1;
-                *reinterpret_cast<unsigned*>(Ps + (g + 8 * r) * LD_PS + half * LD_HALF + warp * 8 + 2 * t) = ld_pack(p0, p1);
+                const unsigned hi2 = ld_pack(p0, p1);
+                const int at = (g + 8 * r) * LD_PS + half * LD_HALF + warp * 8 + 2 * t;
+                *reinterpret_cast<unsigned*>(Ps + at) = hi2;
+                *reinterpret_cast<unsigned*>(Pl + at) = ld_pack(p0 - __uint_as_float(hi2 << 16), p1 - __uint_as_float(hi2 & 0xffff0000u));
             }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -177,8 +183,9 @@ __global__ void __launch_bounds__(LD_THREADS, 1) latent_decode_kernel(const Late
         }
         const int steps = min(LD_KEYS, hi - j0 + 16) / 16;       // 16 keys each; rows past the range are zeros
         for (int k = 0; k < steps; ++k) {
-            unsigned pa[4];
+            unsigned pa[4], pl[4];
             ld_x4(pa, Ps + (lane & 15) * LD_PS + k * 16 + (lane >> 4) * 8);
+            ld_x4(pl, Pl + (lane & 15) * LD_PS + k * 16 + (lane >> 4) * 8);
             const bf16* Vw = Ks + (size_t)(k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * stride + warp * NT * 8 + (lane >> 4) * 8;
 #pragma unroll
             for (int i = 0; i < NT; i += 2) {
@@ -186,6 +193,8 @@ __global__ void __launch_bounds__(LD_THREADS, 1) latent_decode_kernel(const Late
                 ld_x4_trans(v, Vw + i * 8);
                 ld_mma(o[i], pa, v[0], v[1]);
                 ld_mma(o[i + 1], pa, v[2], v[3]);
+                ld_mma(o[i], pl, v[0], v[1]);
+                ld_mma(o[i + 1], pl, v[2], v[3]);
             }
         }
     }
@@ -254,7 +263,7 @@ __global__ void __launch_bounds__(128) latent_decode_merge_kernel(const LatentDe
     }
 }
 
-size_t ld_smem(int rank, int rot) { return sizeof(bf16) * ((size_t)(LD_ROWS + LD_KEYS) * (rank + rot + 8) + LD_ROWS * LD_PS); }
+size_t ld_smem(int rank, int rot) { return sizeof(bf16) * ((size_t)(LD_ROWS + LD_KEYS) * (rank + rot + 8) + 2 * LD_ROWS * LD_PS); }
 
 template <int C128> void launch_decode(const LatentDecodeArgs& a, int ranges, cudaStream_t stream) {
     const size_t smem = ld_smem(C128 * 128, a.rot);

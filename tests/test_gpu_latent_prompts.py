@@ -109,3 +109,43 @@ def test_formed_portions_beside_decoded_tokens_and_short_portions(tmp_path, monk
     calls["formed"] = 0
     Z.assert_matches(H.replay(runner, H.cut_whole(requests)), want, torch.bfloat16, "nothing formed")
     assert calls["formed"] == 0
+
+
+@pytest.mark.parametrize("sink", [False, True], ids=["", "sink"])
+@pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (3, 128, 16), (17, 256, 32), (33, 384, 64)], ids=str)
+@pytest.mark.parametrize("ctx", [(1, 127, 128, 129), (64, 65, 4096), (777,)], ids=str)
+def test_single_tokens(ctx, heads, rank, rot, sink):
+    """Contexts around the edges of 128 keys and their halves beside long ones (ranges that end before others begin), heads of one
+    tile and more, in one step, for a bound above every context too. Against float64 over the same rows, the probabilities and the
+    result are rounded to bfloat16 (8 bits: 2^-8 each at most) and the scores' sums and exponentials are float32: within
+    2^-7 (1 + 1/8) of the weighted sum of the values' sizes. Pages of others and rows past a context are NaN."""
+    from llm_pipeline_b200.ops import kernels
+    page, gen = 16, torch.Generator().manual_seed(sum(ctx) + heads + rank)
+    assert kernels.latent_decode_supports(rank, rot, page)
+    need = [-(-c // page) for c in ctx]
+    order = torch.randperm(sum(need) + 3, generator=gen).tolist()
+    pages = torch.full((sum(need) + 3, page, rank + rot), float("nan"))
+    tables = torch.full((len(ctx), max(need)), -1, dtype=torch.int32)
+    rows = [torch.randn(c, rank + rot, generator=gen).to(torch.bfloat16).float() for c in ctx]
+    for r in range(len(ctx)):
+        for i in range(need[r]):
+            tables[r, i] = order.pop()
+            part = rows[r][i * page:(i + 1) * page]
+            pages[tables[r, i], :part.shape[0]] = part
+    q = torch.randn(len(ctx), heads, rank + rot, generator=gen).to(torch.bfloat16)
+    sinks = torch.randn(heads, generator=gen) if sink else None
+    on = q.to(DEV)
+    scale = (rank + rot) ** -0.5 * 3.0
+    for longest in (max(ctx), max(ctx) + 1000):
+        out = torch.full((len(ctx), heads, rank), 7.0, dtype=torch.bfloat16, device=DEV)
+        kernels.latent_decode(on[..., :rank], on[..., rank:], pages.to(DEV, torch.bfloat16), tables.to(DEV), _i32(ctx), out, scale, longest,
+                              sink=sinks.to(DEV) if sink else None)
+        torch.cuda.synchronize()
+        kernels.check_error_flag()
+        for r in range(len(ctx)):
+            score = (q[r].double() @ rows[r].double().T) * scale
+            if sink:
+                score = torch.cat([score, sinks.double()[:, None]], dim=1)
+            p = torch.softmax(score, dim=1)[:, :ctx[r]]
+            v = rows[r][:, :rank].double()
+            assert ((out[r].double().cpu() - p @ v).abs() <= 2.0 ** -7 * (1 + 1 / 8) * (p @ v.abs())).all(), (r, longest)
