@@ -152,7 +152,7 @@ __global__ void short_conv_parallel_kernel(const ConvArgs a, const int N) {
 
 // The same with four channels a thread in 16-byte accesses, for K = 2, 3 or 4 taps. A tile of one request, which most are, is walked
 // CONV_AHEAD tokens at a time: their inputs are all asked for before the first of them is used or anything stored, and nothing looks
-// at the requests between (2,048 tokens of 6,144 channels: 49 us with a look and a load per token, 41 so; what is left is mostly the
+// at the requests between (2,048 tokens of 6,144 channels: 49 us with a look and a load per token, 41 to 44 so; what is left is mostly the
 // exact exponential and division of SiLU).
 constexpr int CONV_AHEAD = 4;
 

@@ -130,8 +130,9 @@ class LatentAttention(Mixer):
     # New tokens of a request from which its keys and values are formed (one request of 128 tokens: 102 us a layer against 115, of
     # 2,048 136 against 695; the host launches as many kernels either way). Requests of fewer tokens beside it join while their
     # keys are no more than FORMED_JOIN_KEYS together, whose forming costs the device less than the second path's launches cost
-    # the host (requests of 130 and 62 tokens: 106 us a layer joined, 174 on two paths, 125 over the latents). Above that the second path has to be worth
-    # it: FORMED_MIN_GAIN_US by the rates of the two kernels at 2,048 tokens (in TFLOP/s: 120 over latents, 350 formed, 600 forming).
+    # the host (requests of 130 and 62 tokens: 106 us a layer joined, 174 on two paths, 125 over the latents). Above that the
+    # second path has to be worth it: FORMED_MIN_GAIN_US by the rates of the two kernels at 2,048 tokens (in TFLOP/s: 120 over
+    # latents, 350 formed, 600 forming).
     # The formed keys and values of a step take at most FORMED_MAX_BYTES; beyond, its requests attend over the latents.
     FORMED_MIN_TOKENS = 128
     FORMED_JOIN_KEYS = 4096
