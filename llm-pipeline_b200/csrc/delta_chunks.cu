@@ -12,8 +12,9 @@
 //      what the chain needs of a chunk: W = T (G k), Q = G q, K = G_16 / G k, B, Y = T V, G_16;
 //   2. the chain: a block per (request, head, 16 value columns) walks the request's chunks with the state in registers: four
 //      products of 16 tokens a chunk on the tensor cores instead of 16 passes.
-// Everything is float32; ratios of decays are exponentials of differences of their logarithms (never above one, so nothing
-// overflows however fast a channel forgets). Where a float32 number enters a product it is split into two bfloat16 halves, and of
+// Everything is float32; ratios of decays are products of the decays between (never above one, so nothing overflows however fast a
+// channel forgets; exponentials of differences of summed logarithms lose a slow decay's bits to a fast one before it: 5e-3 of the
+// state after a reset). Where a float32 number enters a product it is split into two bfloat16 halves, and of
 // the four products of halves the three larger are summed in float32 (16 bits of each factor): outputs and state are 5e-6 from
 // 64 bits of the same rows (token by token 2e-7), a layer's rows 1.8e-3 either way, which is what its bfloat16 products leave.
 // The operands of launch 2 lie in scratch in the order of its fragments, the two halves beside each other, and are copied as they
@@ -28,7 +29,6 @@ constexpr int DC_TOKENS = 16;             // tokens of a chunk
 constexpr int DC_PREP_THREADS = 128;
 constexpr int DC_CHAIN_THREADS = 128;     // of the chain: four quarters of the channels
 constexpr int DC_STAGES = 4;              // records of its ring
-constexpr float DC_LOG2_E = 1.4426950408889634f;
 
 struct DeltaChunkArgs {
     const float* q; long q_t; const float* k; long k_t; const float* v; long v_t;     // as the convolution left them
@@ -45,11 +45,6 @@ struct DeltaChunkArgs {
 // Bytes of a record, whose parts are, in order: W, Q, K (64 a channel each), B (1024), Y (64 a column), G (4 a channel).
 __host__ __device__ constexpr int dc_record(int d, int dv) { return 3 * d * 64 + 1024 + dv * 64 + d * 4; }
 
-__device__ __forceinline__ float dc_ex2(float v) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
-    return r;
-}
 __device__ __forceinline__ float dc_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
 __device__ __forceinline__ void dc_mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
@@ -62,6 +57,22 @@ __device__ __forceinline__ void dc_split(float u, float v, unsigned& hi, unsigne
     const __nv_bfloat162 l = __floats2bfloat162_rn(u - __low2float(h), v - __high2float(h));
     hi = *reinterpret_cast<const unsigned*>(&h);
     lo = *reinterpret_cast<const unsigned*>(&l);
+}
+__device__ __forceinline__ float dc_dot(const float4& a, const float4& b, float s) {
+    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s))));
+}
+// The sums over 16 neighbouring lanes of v[0] .. v[15]: lane i of them gets that of v[i].
+__device__ __forceinline__ float dc_sum16(float (&v)[16], int lane) {
+#pragma unroll
+    for (int half = 8; half > 0; half >>= 1) {
+        const bool upper = lane & half;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float give = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    return v[0];
 }
 __device__ __forceinline__ float4 dc_add4(const float4& a, const float4& b, const float4& c, const float4& d) {
     return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
@@ -101,7 +112,8 @@ __device__ __forceinline__ bool find_chunk(const int* q_start, int requests, int
 
 // ---- 1 -----------------------------------------------------------------------------------------------------------------
 // A thread owns a channel (its 16 tokens of decays, keys, queries) or a value column, but for the unit vectors (a warp per row) and
-// the sums A, B (a thread per pair of tokens, 4 channels at a time). The record is put together in shared memory, in two parts that
+// the sums A, B: 16 lanes take columns j and 14 - j one after the other, which are 16 pairs of tokens whichever j, with the key
+// of column j decaying in their registers as the rows go down. The record is put together in shared memory, in two parts that
 // take turns there.
 template <int D>
 __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const DeltaChunkArgs a) {
@@ -109,8 +121,8 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
     constexpr int LD = D + 4;
     float* ks = reinterpret_cast<float*>(dc_raw);              // [16][LD]
     float* qs = ks + DC_TOKENS * LD;
-    float* Ls = qs + DC_TOKENS * LD;                           // log2 of the decays' products
-    unsigned char* rec = reinterpret_cast<unsigned char*>(Ls + DC_TOKENS * LD);
+    float* gs = qs + DC_TOKENS * LD;                           // decays
+    unsigned char* rec = reinterpret_cast<unsigned char*>(gs + DC_TOKENS * LD);
     __shared__ __align__(16) float As[DC_TOKENS][DC_TOKENS], Ts[DC_TOKENS][DC_TOKENS];
     __shared__ float Bs[DC_TOKENS][DC_TOKENS + 1], beta[DC_TOKENS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -143,14 +155,8 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
     }
     if (tid < D) {
         const float rate = -expf(a.a_log[h]), bias = a.dt_bias[(size_t)h * D + ch];
-        float sum = 0.f;
 #pragma unroll
-        for (int t = 0; t < DC_TOKENS; ++t) {
-            float l = rate * dc_softplus(raw[t] + bias) * DC_LOG2_E;
-            if (l < -1e4f) l = -1e4f;                          // a decay of zero; differences of the sums stay numbers
-            if (t < cnt) sum += l;
-            Ls[t * LD + ch] = sum;
-        }
+        for (int t = 0; t < DC_TOKENS; ++t) gs[t * LD + ch] = t < cnt ? expf(rate * dc_softplus(raw[t] + bias)) : 1.f;
     }
     if (tid < DC_TOKENS) beta[tid] = tid < cnt ? 1.f / (1.f + expf(-a.beta[(size_t)(row0 + tid) * a.beta_t + h])) : 0.f;
     As[tid / 16][tid % 16] = 0.f;
@@ -182,22 +188,36 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
         }
     }
     __syncthreads();
-    if (tid < DC_TOKENS * (DC_TOKENS - 1) / 2) {
-        int t = 1, j = tid;
-        while (j >= t) j -= t++;
-        const float4* kt = reinterpret_cast<const float4*>(ks + t * LD), *kj = reinterpret_cast<const float4*>(ks + j * LD);
-        const float4* qt = reinterpret_cast<const float4*>(qs + t * LD);
-        const float4* lt = reinterpret_cast<const float4*>(Ls + t * LD), *lj = reinterpret_cast<const float4*>(Ls + j * LD);
-        float s0 = 0.f, s1 = 0.f, b0 = 0.f, b1 = 0.f;
-#pragma unroll 4
-        for (int c = 0; c < D / 4; ++c) {
-            const float4 l = lt[c], m = lj[c], kv = kj[c], x = kt[c], y = qt[c];
-            const float e0 = kv.x * dc_ex2(l.x - m.x), e1 = kv.y * dc_ex2(l.y - m.y), e2 = kv.z * dc_ex2(l.z - m.z), e3 = kv.w * dc_ex2(l.w - m.w);
-            s0 = fmaf(x.x, e0, s0); s1 = fmaf(x.y, e1, s1); s0 = fmaf(x.z, e2, s0); s1 = fmaf(x.w, e3, s1);
-            b0 = fmaf(y.x, e0, b0); b1 = fmaf(y.y, e1, b1); b0 = fmaf(y.z, e2, b0); b1 = fmaf(y.w, e3, b1);
+    {   // A and B below their diagonals
+        constexpr int F4 = D / 64;                             // 16-byte pieces of a row a lane takes
+        const int m = tid >> 4, at = (tid & 15) * 4, turn = DC_TOKENS - 1 - m;
+        float sa[DC_TOKENS], sb[DC_TOKENS];
+        float4 p[F4];
+        auto row = [&](const float* from, int t, int i) { return *reinterpret_cast<const float4*>(from + t * LD + i * 64 + at); };
+#pragma unroll
+        for (int i = 0; i < F4; ++i) p[i] = row(ks, m, i);
+#pragma unroll
+        for (int s = 0; s < DC_TOKENS; ++s) {                  // column m down to the last row, then column 14 - m
+            const int t = s < turn ? m + 1 + s : s;
+            if (s >= DC_TOKENS / 2 && s == turn) {
+#pragma unroll
+                for (int i = 0; i < F4; ++i) p[i] = row(ks, turn - 1, i);
+            }
+            sa[s] = sb[s] = 0.f;
+#pragma unroll
+            for (int i = 0; i < F4; ++i) {
+                const float4 g = row(gs, t, i);
+                p[i] = make_float4(p[i].x * g.x, p[i].y * g.y, p[i].z * g.z, p[i].w * g.w);
+                sa[s] = dc_dot(row(ks, t, i), p[i], sa[s]);
+                sb[s] = dc_dot(row(qs, t, i), p[i], sb[s]);
+            }
         }
-        As[t][j] = s0 + s1;
-        Bs[t][j] = b0 + b1;
+        const float va = dc_sum16(sa, lane), vb = dc_sum16(sb, lane);
+        const int s = tid & 15, t = s < turn ? m + 1 + s : s, j = s < turn ? m : turn - 1;
+        if (m < 7 || s < turn) {                               // (column 7 is its own partner)
+            As[t][j] = va;
+            Bs[t][j] = vb;
+        }
     }
     __syncthreads();
     if (tid < 32) {
@@ -224,20 +244,25 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
             *reinterpret_cast<uint4*>(rec_b + n * 512 + lane * 16) = w;
         }
         for (int c = tid - 32; c < D; c += DC_PREP_THREADS - 32) {
-            const float last = Ls[(DC_TOKENS - 1) * LD + c];
-            rec_g[c] = dc_ex2(last);
-            float kb[DC_TOKENS];
+            float g[DC_TOKENS], kb[DC_TOKENS], upto = 1.f, after = 1.f;
+#pragma unroll
+            for (int t = 0; t < DC_TOKENS; ++t) g[t] = gs[t * LD + c];
+#pragma unroll
+            for (int t = DC_TOKENS - 1; t >= 0; --t) {
+                kb[t] = ks[t * LD + c] * after;
+                after *= g[t];
+            }
 #pragma unroll
             for (int t = 0; t < DC_TOKENS; ++t) {
-                const float L = Ls[t * LD + c];
-                kb[t] = ks[t * LD + c] * dc_ex2(last - L);
+                upto *= g[t];
                 // B operand with channels along k and tokens along n
-                const float x = qs[t * LD + c] * dc_ex2(L);
+                const float x = qs[t * LD + c] * upto;
                 const bf16 hi = __float2bfloat16_rn(x), lo = __float2bfloat16_rn(x - __bfloat162float(hi));
                 bf16* at = reinterpret_cast<bf16*>(rec_q + ((c >> 4) * 2 + (t >> 3)) * 512 + ((t & 7) * 4 + ((c & 7) >> 1)) * 16 + ((c >> 3) & 1) * 4) + (c & 1);
                 at[0] = hi;
                 at[4] = lo;
             }
+            rec_g[c] = upto;
 #pragma unroll
             for (int p = 0; p < 4; ++p) {                      // B operand with tokens along k and channels along n
                 uint4 w;
@@ -256,8 +281,12 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
         const int c = key ? i : i - D;
         float x[DC_TOKENS];
         if (key) {
+            float upto = 1.f;
 #pragma unroll
-            for (int t = 0; t < DC_TOKENS; ++t) x[t] = ks[t * LD + c] * dc_ex2(Ls[t * LD + c]);
+            for (int t = 0; t < DC_TOKENS; ++t) {
+                upto *= gs[t * LD + c];
+                x[t] = ks[t * LD + c] * upto;
+            }
         } else {
 #pragma unroll
             for (int t = 0; t < DC_TOKENS; ++t) {

@@ -234,6 +234,61 @@ def test_gated_delta_rule_in_chunks(sizes, lengths):
     assert (state[[0, R + 1]] == 5.0).all() and (state[slots, :offset] == 0.0).all() and (state[slots, offset + 2 * piece:] == 0.0).all()
 
 
+def _delta_rule_alone(rows, a_log, dt_bias, heads, qk_heads, dim, vdim):
+    """(outputs, last state) of the rule written out in float64 for one request's rows before ``delta_prep``."""
+    q, k, v, pre, beta = rows
+    n = q.shape[0]
+    q, k = (y.double().view(n, qk_heads, dim) for y in (q, k))
+    q, k = (y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6) for y in (q, k))
+    decay = torch.exp(-torch.exp(a_log.double())[None, :, None] * plain.softplus(pre.double() + dt_bias.double()).view(n, heads, dim))
+    beta, want, S = torch.sigmoid(beta.double()), torch.zeros(n, heads, vdim, dtype=torch.float64), torch.zeros(heads, dim, vdim, dtype=torch.float64)
+    own = torch.arange(heads) // (heads // qk_heads)
+    for t in range(n):
+        S = decay[t][:, :, None] * S
+        u = beta[t][:, None] * (v[t].double().view(heads, vdim) - torch.einsum("hdv,hd->hv", S, k[t, own]))
+        S = S + k[t, own][:, :, None] * u[:, None, :]
+        want[t] = torch.einsum("hdv,hd->hv", S, q[t, own]) * dim ** -0.5
+    return want.view(n, -1), S
+
+
+def _delta_rule_rows(gen, n, heads, qk_heads, dim, vdim):
+    return [torch.randn(n, w, generator=gen) for w in (qk_heads * dim, qk_heads * dim, heads * vdim, heads * dim, heads)]
+
+
+def _delta_rule_by(form, rows, a_log, dt_bias, heads, qk_heads, dim, vdim):
+    """(outputs, last state) of one request's rows from ``delta_chunks`` or from ``delta_prep`` and ``delta_scan``."""
+    from llm_pipeline_b200.ops import kernels
+    dev, n, piece = "cuda", rows[0].shape[0], heads * dim * vdim
+    x, o, state = [y.to(dev) for y in rows], torch.empty(n, heads * vdim, device=dev), torch.zeros(1, 2 * piece, device=dev)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)   # noqa: E731
+    at = (i32([0, n]), i32([0]), i32(list(range(n))))
+    if form == "chunks":
+        need = kernels.delta_chunks_scratch(torch.bfloat16, n, 1, max(n, kernels.DELTA_CHUNKS_MIN_TOKENS), heads, dim, vdim)
+        kernels.delta_chunks(*x, a_log.to(dev), dt_bias.to(dev), state, 0, *at, o, heads, qk_heads, dim, vdim, need)
+    else:
+        q, k, v, decay, beta = x
+        kernels.delta_prep(q, k, decay, beta, a_log.to(dev), dt_bias.to(dev), heads, qk_heads, dim)
+        kernels.delta_scan(q, k, v, decay, beta, state, 0, *at, o, heads, qk_heads, dim, vdim)
+    kernels.check_error_flag()
+    return o.double().cpu(), state[0, ((n - 1) & 1) * piece:][:piece].double().cpu().view(heads, dim, vdim)
+
+
+@pytest.mark.parametrize("fast", [2.0, 25.0, 1e5], ids=["e-40", "e-500", "zero"])
+@pytest.mark.parametrize("sizes", [(2, 2, 64, 48), (2, 1, 128, 16)], ids=str)
+def test_gated_delta_rule_in_chunks_holds_after_a_reset(sizes, fast):
+    """Channels that forget at once at a third of the tokens and hardly at all at the others, within the same chunks: what is held keeps
+    its bits whatever was forgotten before. Within 2^-14 of the largest entry, as for decays of one kind."""
+    heads, qk_heads, dim, vdim = sizes
+    gen = torch.Generator().manual_seed(dim + int(fast))
+    a_log, dt_bias = torch.full((heads,), 3.0), torch.zeros(heads * dim)
+    rows = _delta_rule_rows(gen, 90, heads, qk_heads, dim, vdim)
+    rows[3] = torch.where(torch.rand(rows[3].shape, generator=gen) < 0.3, torch.full_like(rows[3], fast), rows[3] * 0.5 - 8.0)
+    got, kept = _delta_rule_by("chunks", rows, a_log, dt_bias, *sizes)
+    want, S = _delta_rule_alone(rows, a_log, dt_bias, *sizes)
+    assert (got - want).abs().max() <= 2.0 ** -14 * want.abs().max()
+    assert (kept - S).abs().max() <= 2.0 ** -14 * S.abs().max()
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
     from llm_pipeline_b200.ops import kernels
