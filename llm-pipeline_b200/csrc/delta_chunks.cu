@@ -14,13 +14,13 @@
 //      products of 16 tokens a chunk on the tensor cores instead of 16 passes.
 // Everything is float32; ratios of decays are products of the decays between (never above one, so nothing overflows however fast a
 // channel forgets; exponentials of differences of summed logarithms lose a slow decay's bits to a fast one before it: 5e-3 of the
-// state after a reset). Where a float32 number enters a product it is split into two bfloat16 halves, and of
-// the four products of halves the three larger are summed in float32 (16 bits of each factor): outputs and state are 5e-6 from
-// 64 bits of the same rows (token by token 2e-7), a layer's rows 1.8e-3 either way, which is what its bfloat16 products leave.
-// The operands of launch 2 lie in scratch in the order of its fragments, the two halves beside each other, and are copied as they
-// are. 2,048 tokens of 16 heads of 128 x 128: 191 us, prepared and walked token by token 660. Launch 1 (91 us with cold caches) is
-// issue-bound at 44 % with 14 warps an SM; launch 2 (99) is the chain's latency, 0.77 us a chunk, of which the products are a
-// fifth. On the way: 32 columns a block with fragments loaded from global memory 143 us, two barriers a chunk 114.
+// state after a reset). Where a float32 number enters a product it is split into three bfloat16 pieces, which hold all of
+// its 24 bits, and of the nine products of pieces the six larger are summed in float32, the largest apart: outputs and state are
+// as far from 64 bits as token by token (1.5e-7 to 3e-7 at decays from fast to slow, and after resets; with two pieces and three
+// products 5e-6, at 42 us less). The operands of launch 2 lie in scratch in the order of its fragments, pieces beside each other,
+// and are copied as they are. A layer of 2,048 tokens and 16 heads of 128 x 128 takes 375 us, 806 token by token. Launch 2 is its
+// chain's latency. On the way: 32 columns a block with fragments loaded from global memory,
+// two barriers a chunk (each slower by 15 to 45 %).
 #include "tcgen05.cuh"
 
 namespace {
@@ -42,8 +42,8 @@ struct DeltaChunkArgs {
     int requests, H, G, dv;
 };
 
-// Bytes of a record, whose parts are, in order: W, Q, K (64 a channel each), B (1024), Y (64 a column), G (4 a channel).
-__host__ __device__ constexpr int dc_record(int d, int dv) { return 3 * d * 64 + 1024 + dv * 64 + d * 4; }
+// Bytes of a record, whose parts are, in order: W, Q, K (96 a channel each), B (1536), Y (64 a column), G (4 a channel).
+__host__ __device__ constexpr int dc_record(int d, int dv) { return 3 * d * 96 + 1536 + dv * 64 + d * 4; }
 
 __device__ __forceinline__ float dc_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
@@ -51,12 +51,49 @@ __device__ __forceinline__ void dc_mma(float (&d)[4], const unsigned (&a)[4], un
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two floats as a pair of bfloat16, and what that leaves of them as another pair.
-__device__ __forceinline__ void dc_split(float u, float v, unsigned& hi, unsigned& lo) {
+// A float as three bfloat16 numbers that add up to it.
+__device__ __forceinline__ void dc_split(float u, bf16& hi, bf16& mid, bf16& lo) {
+    hi = __float2bfloat16_rn(u);
+    const float rest = u - __bfloat162float(hi);
+    mid = __float2bfloat16_rn(rest);
+    lo = __float2bfloat16_rn(rest - __bfloat162float(mid));
+}
+// Two floats as three such pairs.
+__device__ __forceinline__ void dc_split(float u, float v, unsigned& hi, unsigned& mid, unsigned& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(u, v);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(u - __low2float(h), v - __high2float(h));
+    const float ru = u - __low2float(h), rv = v - __high2float(h);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(ru, rv);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(ru - __low2float(m), rv - __high2float(m));
     hi = *reinterpret_cast<const unsigned*>(&h);
+    mid = *reinterpret_cast<const unsigned*>(&m);
     lo = *reinterpret_cast<const unsigned*>(&l);
+}
+// A fragment of a record (a k16 x n8 operand, split): the larger two pieces of a lane's two words beside each other, then all
+// lanes' smallest.
+constexpr int DC_FRAGMENT = 768;
+struct DcFragment { unsigned piece[3][2]; };
+__device__ __forceinline__ DcFragment dc_fragment(const unsigned char* at, int lane) {
+    const uint4 a = *reinterpret_cast<const uint4*>(at + lane * 16);
+    const uint2 b = *reinterpret_cast<const uint2*>(at + 512 + lane * 8);
+    return {{{a.x, a.y}, {a.z, a.w}, {b.x, b.y}}};
+}
+__device__ __forceinline__ void dc_put(unsigned char* at, int lane, const unsigned (&b0)[3], const unsigned (&b1)[3]) {
+    *reinterpret_cast<uint4*>(at + lane * 16) = make_uint4(b0[0], b1[0], b0[1], b1[1]);
+    *reinterpret_cast<uint2*>(at + 512 + lane * 8) = make_uint2(b0[2], b1[2]);
+}
+// one entry of a fragment: of a lane's word `word` the half `half`
+__device__ __forceinline__ void dc_put(unsigned char* at, int lane, int word, int half, float x) {
+    bf16* pair = reinterpret_cast<bf16*>(at + lane * 16 + word * 4) + half;
+    dc_split(x, pair[0], pair[4], reinterpret_cast<bf16*>(at + 512 + lane * 8 + word * 4)[half]);
+}
+// Products of split factors with T operands: of the nine products of pieces the six larger ones, the largest apart from the others,
+// so that neither loses bits to the other's rounding.
+template <int T> __device__ __forceinline__ void dc_products(float (&big)[T][4], float (&small)[T][4], const unsigned (&a)[3][4], const DcFragment (&b)[T]) {
+    constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int n = 0; n < T; ++n) dc_mma(i == 5 ? big[n] : small[n], a[PA[i]], b[n].piece[PB[i]][0], b[n].piece[PB[i]][1]);
 }
 __device__ __forceinline__ float dc_dot(const float4& a, const float4& b, float s) {
     return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s))));
@@ -131,9 +168,9 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
     pdl_trigger();
     int row0, cnt;
     if (!find_chunk(a.q_start, a.requests, blockIdx.x, row0, cnt)) return;
-    unsigned char* rec_q = rec, *rec_k = rec + D * 64, *rec_b = rec + 2 * D * 64;          // first Q, K, B and G,
-    float* rec_g = reinterpret_cast<float*>(rec_b + 1024);
-    unsigned char* rec_w = rec, *rec_y = rec + D * 64;                                      // then W and Y in their place
+    unsigned char* rec_q = rec, *rec_k = rec + D * 96, *rec_b = rec + 2 * D * 96;          // first Q, K, B and G,
+    float* rec_g = reinterpret_cast<float*>(rec_b + 1536);
+    unsigned char* rec_w = rec, *rec_y = rec + D * 96;                                      // then W and Y in their place
     unsigned char* to = a.scratch + ((size_t)blockIdx.x * a.H + h) * dc_record(D, dv);
     auto copy = [&](int at, int bytes, const void* from) {
         for (int i = tid; i < bytes / 16; i += DC_PREP_THREADS) reinterpret_cast<uint4*>(to + at)[i] = reinterpret_cast<const uint4*>(from)[i];
@@ -238,10 +275,10 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
     } else {                                                   // meanwhile the others: B, and Q, K, G, which need neither A nor T
         if (warp >= 2) {                                       // j along k, t along n (above the diagonal B is zero)
             const int n = warp - 2, t = n * 8 + (lane >> 2), j = (lane & 3) * 2;
-            uint4 w;
-            dc_split(Bs[t][j], Bs[t][j + 1], w.x, w.z);
-            dc_split(Bs[t][j + 8], Bs[t][j + 9], w.y, w.w);
-            *reinterpret_cast<uint4*>(rec_b + n * 512 + lane * 16) = w;
+            unsigned b0[3], b1[3];
+            dc_split(Bs[t][j], Bs[t][j + 1], b0[0], b0[1], b0[2]);
+            dc_split(Bs[t][j + 8], Bs[t][j + 9], b1[0], b1[1], b1[2]);
+            dc_put(rec_b + n * DC_FRAGMENT, lane, b0, b1);
         }
         for (int c = tid - 32; c < D; c += DC_PREP_THREADS - 32) {
             float g[DC_TOKENS], kb[DC_TOKENS], upto = 1.f, after = 1.f;
@@ -256,25 +293,21 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
             for (int t = 0; t < DC_TOKENS; ++t) {
                 upto *= g[t];
                 // B operand with channels along k and tokens along n
-                const float x = qs[t * LD + c] * upto;
-                const bf16 hi = __float2bfloat16_rn(x), lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-                bf16* at = reinterpret_cast<bf16*>(rec_q + ((c >> 4) * 2 + (t >> 3)) * 512 + ((t & 7) * 4 + ((c & 7) >> 1)) * 16 + ((c >> 3) & 1) * 4) + (c & 1);
-                at[0] = hi;
-                at[4] = lo;
+                dc_put(rec_q + ((c >> 4) * 2 + (t >> 3)) * DC_FRAGMENT, (t & 7) * 4 + ((c & 7) >> 1), (c >> 3) & 1, c & 1, qs[t * LD + c] * upto);
             }
             rec_g[c] = upto;
 #pragma unroll
             for (int p = 0; p < 4; ++p) {                      // B operand with tokens along k and channels along n
-                uint4 w;
-                dc_split(kb[2 * p], kb[2 * p + 1], w.x, w.z);
-                dc_split(kb[8 + 2 * p], kb[9 + 2 * p], w.y, w.w);
-                *reinterpret_cast<uint4*>(rec_k + (c >> 3) * 512 + ((c & 7) * 4 + p) * 16) = w;
+                unsigned b0[3], b1[3];
+                dc_split(kb[2 * p], kb[2 * p + 1], b0[0], b0[1], b0[2]);
+                dc_split(kb[8 + 2 * p], kb[9 + 2 * p], b1[0], b1[1], b1[2]);
+                dc_put(rec_k + (c >> 3) * DC_FRAGMENT, (c & 7) * 4 + p, b0, b1);
             }
         }
     }
     __syncthreads();
-    copy(D * 64, 2 * D * 64 + 1024, rec_q);
-    copy(3 * D * 64 + 1024 + dv * 64, D * 4, rec_g);
+    copy(D * 96, 2 * D * 96 + 1536, rec_q);
+    copy(3 * D * 96 + 1536 + dv * 64, D * 4, rec_g);
     __syncthreads();
     for (int i = tid; i < D + dv; i += DC_PREP_THREADS) {      // W, Y: rows of T times a channel's keys or a column's values
         const bool key = i < D;
@@ -309,13 +342,8 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
             }
             if (key) {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int tt = t + u;
-                    const bf16 hi = __float2bfloat16_rn(y[u]), lo = __float2bfloat16_rn(y[u] - __bfloat162float(hi));
-                    bf16* at = reinterpret_cast<bf16*>(rec_w + ((c >> 4) * 2 + (tt >> 3)) * 512 + ((tt & 7) * 4 + ((c & 7) >> 1)) * 16 + ((c >> 3) & 1) * 4) + (c & 1);
-                    at[0] = hi;
-                    at[4] = lo;
-                }
+                for (int u = 0; u < 2; ++u)
+                    dc_put(rec_w + ((c >> 4) * 2 + (t >> 3)) * DC_FRAGMENT, ((t + u) & 7) * 4 + ((c & 7) >> 1), (c >> 3) & 1, c & 1, y[u]);
             } else {                                           // accumulator with columns along m and tokens along n
                 *reinterpret_cast<float2*>(rec_y + ((c >> 4) * 2 + (t >> 3)) * 512 + ((c & 7) * 4 + ((t & 7) >> 1)) * 16 + ((c >> 3) & 1) * 8) =
                     make_float2(y[0], y[1]);
@@ -323,8 +351,8 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
         }
     }
     __syncthreads();
-    copy(0, D * 64, rec_w);
-    copy(3 * D * 64 + 1024, dv * 64, rec_y);
+    copy(0, D * 96, rec_w);
+    copy(3 * D * 96 + 1536, dv * 64, rec_y);
 }
 
 // ---- 2 -----------------------------------------------------------------------------------------------------------------
@@ -335,7 +363,7 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
 // free once every warp is in the chunk after it.
 template <int KS>
 __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const DeltaChunkArgs a) {
-    constexpr int D = 64 * KS, MAIN = 3 * D * 64 + 1024, STAGE = MAIN + 1024 + D * 4;
+    constexpr int D = 64 * KS, MAIN = 3 * D * 96 + 1536, STAGE = MAIN + 1024 + D * 4;
     extern __shared__ __align__(128) unsigned char dc_ring[];
     __shared__ __align__(16) float4 shares[2][4][4][32];       // [buffer][quarter][U, U, o, o][lane]
     __shared__ __align__(8) uint64_t full[DC_STAGES];
@@ -387,60 +415,51 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
     float* out = a.o + (size_t)begin * a.o_t + (size_t)h * dv + col0 + g;
     for (int s = 0; s < chunks; ++s) {
         const unsigned char* st = dc_ring + (s % DC_STAGES) * STAGE;
-        const uint4* frags = reinterpret_cast<const uint4*>(st) + lane;
+        auto fragment = [&](int i) { return dc_fragment(st + i * DC_FRAGMENT, lane); };
         mbar_wait(&full[s % DC_STAGES], (uint32_t)(s / DC_STAGES) & 1u, a.error_flag);
-        float u[2][4] = {}, o[2][4] = {};
+        float uo[4][4] = {}, rest[4][4] = {};                  // U of tokens 0 .. 7, of 8 .. 15, o likewise
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            unsigned hi[4], lo[4];
-            dc_split(S[2 * k][0], S[2 * k][1], hi[0], lo[0]);
-            dc_split(S[2 * k][2], S[2 * k][3], hi[1], lo[1]);
-            dc_split(S[2 * k + 1][0], S[2 * k + 1][1], hi[2], lo[2]);
-            dc_split(S[2 * k + 1][2], S[2 * k + 1][3], hi[3], lo[3]);
+            unsigned sp[3][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dc_split(S[2 * k + (i >> 1)][(i & 1) * 2], S[2 * k + (i >> 1)][(i & 1) * 2 + 1], sp[0][i], sp[1][i], sp[2][i]);
             const int at = (part * KS + k) * 2;
-            const uint4 w0 = frags[at * 32], w1 = frags[(at + 1) * 32], q0 = frags[(4 * D / 32 + at) * 32], q1 = frags[(4 * D / 32 + at + 1) * 32];
-            dc_mma(u[0], hi, w0.x, w0.y); dc_mma(u[1], hi, w1.x, w1.y); dc_mma(o[0], hi, q0.x, q0.y); dc_mma(o[1], hi, q1.x, q1.y);
-            dc_mma(u[0], lo, w0.x, w0.y); dc_mma(u[1], lo, w1.x, w1.y); dc_mma(o[0], lo, q0.x, q0.y); dc_mma(o[1], lo, q1.x, q1.y);
-            dc_mma(u[0], hi, w0.z, w0.w); dc_mma(u[1], hi, w1.z, w1.w); dc_mma(o[0], hi, q0.z, q0.w); dc_mma(o[1], hi, q1.z, q1.w);
+            const DcFragment wq[4] = {fragment(at), fragment(at + 1), fragment(D / 8 + at), fragment(D / 8 + at + 1)};
+            dc_products(uo, rest, sp, wq);
         }
         float4 (*meet)[4][32] = shares[s & 1];
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            meet[part][n][lane] = make_float4(u[n][0], u[n][1], u[n][2], u[n][3]);
-            meet[part][2 + n][lane] = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
-        }
+        for (int n = 0; n < 4; ++n)
+            meet[part][n][lane] = make_float4(uo[n][0] + rest[n][0], uo[n][1] + rest[n][1], uo[n][2] + rest[n][2], uo[n][3] + rest[n][3]);
         __syncthreads();
         if (tid == 0 && s > 0 && s - 1 + DC_STAGES < chunks) issue(s - 1 + DC_STAGES);
-        unsigned hi[4], lo[4];
+        unsigned up[3][4];
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const float4 sum = dc_add4(meet[0][n][lane], meet[1][n][lane], meet[2][n][lane], meet[3][n][lane]);
             const float4 y = *reinterpret_cast<const float4*>(st + MAIN + (n * 32 + lane) * 16);
-            dc_split(y.x - sum.x, y.y - sum.y, hi[2 * n], lo[2 * n]);
-            dc_split(y.z - sum.z, y.w - sum.w, hi[2 * n + 1], lo[2 * n + 1]);
+            dc_split(y.x - sum.x, y.y - sum.y, up[0][2 * n], up[1][2 * n], up[2][2 * n]);
+            dc_split(y.z - sum.z, y.w - sum.w, up[0][2 * n + 1], up[1][2 * n + 1], up[2][2 * n + 1]);
         }
         const float2* decay = reinterpret_cast<const float2*>(st + MAIN + 1024) + (c0 >> 1) + t4;
-        uint4 kf[2 * KS];
+        // a quarter stores the outputs of a half of the tokens and of 8 of the columns
+        const int half = part & 1, upper = part >> 1;
+        DcFragment kb[2 * KS + 1];                             // K of the quarter's channels, and B
+#pragma unroll
+        for (int n = 0; n < 2 * KS; ++n) kb[n] = fragment(2 * D / 8 + part * 2 * KS + n);
+        kb[2 * KS] = fragment(3 * D / 8 + half);
+        float big[2 * KS + 1][4] = {}, small[2 * KS + 1][4] = {};
+        dc_products(big, small, up, kb);
 #pragma unroll
         for (int n = 0; n < 2 * KS; ++n) {
             const float2 d = decay[n * 4];
-            kf[n] = frags[(8 * D / 32 + part * 2 * KS + n) * 32];
-            S[n][0] *= d.x; S[n][1] *= d.y; S[n][2] *= d.x; S[n][3] *= d.y;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) S[n][i] = fmaf(S[n][i], i & 1 ? d.y : d.x, big[n][i] + small[n][i]);
         }
-        // a quarter stores the outputs of a half of the tokens and of 8 of the columns
-        const int half = part & 1, upper = part >> 1;
         const float4 sum = dc_add4(meet[0][2 + half][lane], meet[1][2 + half][lane], meet[2][2 + half][lane], meet[3][2 + half][lane]);
         float y[4] = {sum.x, sum.y, sum.z, sum.w};
-        const uint4 bf = frags[(12 * D / 32 + half) * 32];
 #pragma unroll
-        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], hi, kf[n].x, kf[n].y);
-        dc_mma(y, hi, bf.x, bf.y);
-#pragma unroll
-        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], lo, kf[n].x, kf[n].y);
-        dc_mma(y, lo, bf.x, bf.y);
-#pragma unroll
-        for (int n = 0; n < 2 * KS; ++n) dc_mma(S[n], hi, kf[n].z, kf[n].w);
-        dc_mma(y, hi, bf.z, bf.w);
+        for (int i = 0; i < 4; ++i) y[i] += big[2 * KS][i] + small[2 * KS][i];
         const int t = s * DC_TOKENS + half * 8 + 2 * t4;
         float* to = out + (size_t)t * a.o_t + upper * 8;
         if (t < tokens) to[0] = upper ? y[2] : y[0];
@@ -458,11 +477,11 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
 
 template <int KS> void launch_chunks(const DeltaChunkArgs& a, int chunks, cudaStream_t stream) {
     constexpr int D = 64 * KS;
-    const int part1 = 2 * D * 64 + 1024 + D * 4, part2 = D * 64 + a.dv * 64;
+    const int part1 = 2 * D * 96 + 1536 + D * 4, part2 = D * 96 + a.dv * 64;
     const size_t smem = (size_t)3 * DC_TOKENS * (D + 4) * sizeof(float) + (part1 > part2 ? part1 : part2);
     LLMP_ALLOW_SMEM(delta_chunks_kernel<D>, smem);
     llmp_launch_dependent(delta_chunks_kernel<D>, dim3(chunks, a.H), dim3(DC_PREP_THREADS), smem, stream, a);
-    const size_t ring = (size_t)DC_STAGES * (3 * D * 64 + 1024 + 1024 + D * 4);
+    const size_t ring = (size_t)DC_STAGES * (3 * D * 96 + 1536 + 1024 + D * 4);
     LLMP_ALLOW_SMEM(delta_chain_kernel<KS>, ring);
     llmp_launch_dependent(delta_chain_kernel<KS>, dim3(a.H, a.dv / 16, a.requests), dim3(DC_CHAIN_THREADS), ring, stream, a);
 }

@@ -13,8 +13,8 @@ query/key head i // (H / G))::
 
 The six products that read h are one product against [Wq; Wk; Wv; Wb; Wa1; Wg1] with a float32 result; the inner sizes of
 the two-step projections are whatever the tensors have. Convolutions, unit norms, step sizes, decays, state and read-out
-are float32 (``csrc/short_conv.cu``, ``csrc/delta_rule.cu``; long portions in bfloat16 in chunks on the tensor cores with split
-factors, ``csrc/delta_chunks.cu``); the gated rows are rounded once to the compute type for the
+are float32 (``csrc/short_conv.cu``, ``csrc/delta_rule.cu``; long portions in bfloat16 in chunks on the tensor cores with factors of
+three bfloat16 pieces, ``csrc/delta_chunks.cu``); the gated rows are rounded once to the compute type for the
 output product.
 
 State of a request: one float32 vector ``[conv piece | state piece]``, each piece two copies that take turns by the parity

@@ -289,6 +289,22 @@ def test_gated_delta_rule_in_chunks_holds_after_a_reset(sizes, fast):
     assert (kept - S).abs().max() <= 2.0 ** -14 * S.abs().max()
 
 
+@pytest.mark.parametrize("shift", [-4.0, 1.0, 25.0], ids=["slow", "mixed", "resets"])
+@pytest.mark.parametrize("sizes,n", [((2, 1, 128, 32), 203), ((2, 2, 64, 16), 700)], ids=str)
+def test_gated_delta_rule_in_chunks_is_as_near_as_token_by_token(sizes, n, shift):
+    """Outputs and carried state as far from float64 as the walk leaves them: both round to float32's 24 bits, in another order, so
+    their errors are alike (2-norm; at most twice). Factors of 16 bits would be twenty times further off."""
+    heads, qk_heads, dim, vdim = sizes
+    gen = torch.Generator().manual_seed(n + dim)
+    a_log, dt_bias = torch.full((heads,), min(shift, 3.0)), torch.zeros(heads * dim)
+    rows = _delta_rule_rows(gen, n, *sizes)
+    if shift > 3.0:
+        rows[3] = torch.where(torch.rand(rows[3].shape, generator=gen) < 0.2, torch.full_like(rows[3], shift), rows[3] * 0.5 - 8.0)
+    want = _delta_rule_alone(rows, a_log, dt_bias, *sizes)
+    by = {form: [float((x - y).norm() / y.norm()) for x, y in zip(_delta_rule_by(form, rows, a_log, dt_bias, *sizes), want)] for form in ("chunks", "walk")}
+    assert all(c <= 2.0 * w for c, w in zip(by["chunks"], by["walk"])), by
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
     from llm_pipeline_b200.ops import kernels
