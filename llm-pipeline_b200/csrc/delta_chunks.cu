@@ -433,13 +433,17 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
             meet[part][n][lane] = make_float4(uo[n][0] + rest[n][0], uo[n][1] + rest[n][1], uo[n][2] + rest[n][2], uo[n][3] + rest[n][3]);
         __syncthreads();
         if (tid == 0 && s > 0 && s - 1 + DC_STAGES < chunks) issue(s - 1 + DC_STAGES);
+        float u[2][4], none = 0.f;                             // U^T; `none`: 0, or a NaN if an entry is no finite number
         unsigned up[3][4];
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             const float4 sum = dc_add4(meet[0][n][lane], meet[1][n][lane], meet[2][n][lane], meet[3][n][lane]);
             const float4 y = *reinterpret_cast<const float4*>(st + MAIN + (n * 32 + lane) * 16);
-            dc_split(y.x - sum.x, y.y - sum.y, up[0][2 * n], up[1][2 * n], up[2][2 * n]);
-            dc_split(y.z - sum.z, y.w - sum.w, up[0][2 * n + 1], up[1][2 * n + 1], up[2][2 * n + 1]);
+            u[n][0] = y.x - sum.x; u[n][1] = y.y - sum.y; u[n][2] = y.z - sum.z; u[n][3] = y.w - sum.w;
+            dc_split(u[n][0], u[n][1], up[0][2 * n], up[1][2 * n], up[2][2 * n]);
+            dc_split(u[n][2], u[n][3], up[0][2 * n + 1], up[1][2 * n + 1], up[2][2 * n + 1]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) none = fmaf(u[n][i], 0.f, none);
         }
         const float2* decay = reinterpret_cast<const float2*>(st + MAIN + 1024) + (c0 >> 1) + t4;
         // a quarter stores the outputs of a half of the tokens and of 8 of the columns
@@ -458,8 +462,31 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
         }
         const float4 sum = dc_add4(meet[0][2 + half][lane], meet[1][2 + half][lane], meet[2][2 + half][lane], meet[3][2 + half][lane]);
         float y[4] = {sum.x, sum.y, sum.z, sum.w};
+        if (__any_sync(0xffffffffu, none != none)) {           // a zero of B above its diagonal times what is no number would be none
+            float v[2][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) y[i] += big[2 * KS][i] + small[2 * KS][i];
+            for (int n = 0; n < 2; ++n) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[n][i] = fabsf(u[n][i]) < INFINITY ? u[n][i] : 0.f;
+                dc_split(v[n][0], v[n][1], up[0][2 * n], up[1][2 * n], up[2][2 * n]);
+                dc_split(v[n][2], v[n][3], up[0][2 * n + 1], up[1][2 * n + 1], up[2][2 * n + 1]);
+            }
+            float b[1][4] = {}, r[1][4] = {};
+            const DcFragment only[1] = {kb[2 * KS]};
+            dc_products(b, r, up, only);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                y[i] += b[0][i] + r[0][i];
+#pragma unroll
+                for (int j = 0; j < DC_TOKENS; ++j) {          // and such entries of tokens up to the output's own, in column g + 8 (i / 2)
+                    const float uj = __shfl_sync(0xffffffffu, u[j >> 3][(i & 2) + (j & 1)], g * 4 + ((j & 7) >> 1));
+                    if (j <= half * 8 + 2 * t4 + (i & 1) && !(fabsf(uj) < INFINITY)) y[i] += uj;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) y[i] += big[2 * KS][i] + small[2 * KS][i];
+        }
         const int t = s * DC_TOKENS + half * 8 + 2 * t4;
         float* to = out + (size_t)t * a.o_t + upper * 8;
         if (t < tokens) to[0] = upper ? y[2] : y[0];

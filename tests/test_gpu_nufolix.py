@@ -305,6 +305,23 @@ def test_gated_delta_rule_in_chunks_is_as_near_as_token_by_token(sizes, n, shift
     assert all(c <= 2.0 * w for c, w in zip(by["chunks"], by["walk"])), by
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")], ids=str)
+@pytest.mark.parametrize("what,t", [(2, 21), (2, 37), (1, 21)], ids=["v21", "v37", "k21"])
+def test_gated_delta_rule_in_chunks_is_causal_for_what_is_no_number(what, t, bad):
+    """A value or key that is no finite number reaches the tokens behind it and, a value, its own column only: all others have the
+    bits they have without it."""
+    sizes, gen = (2, 1, 64, 32), torch.Generator().manual_seed(t)
+    rows = _delta_rule_rows(gen, 45, *sizes)
+    a_log, dt_bias = torch.zeros(2), torch.zeros(128)
+    want, _S = _delta_rule_by("chunks", rows, a_log, dt_bias, *sizes)
+    rows[what][t, 5] = bad
+    got, _S = _delta_rule_by("chunks", rows, a_log, dt_bias, *sizes)
+    assert torch.equal(got[:t], want[:t]) and not torch.isfinite(got[t:, 5]).any()
+    if what == 2:
+        others = [c for c in range(64) if c != 5]
+        assert torch.equal(got[:, others], want[:, others])
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
     from llm_pipeline_b200.ops import kernels
