@@ -39,6 +39,7 @@ struct DeltaChunkArgs {
     float* o; long o_t;
     unsigned char* scratch;               // [chunks][H] records
     int* error_flag;
+    const int* list;                      // the requests to take, in order; null: all
     int requests, H, G, dv;
 };
 
@@ -120,13 +121,14 @@ __device__ __forceinline__ void dc_bulk_copy(void* dst, const void* src, uint32_
                  ::"r"(tc_smem_u32(dst)), "l"(src), "r"(bytes), "r"(tc_smem_u32(bar)) : "memory");
 }
 
-// Chunk number `at` of the step (in the order of the requests), by a warp; false: there is none.
-__device__ __forceinline__ bool find_chunk(const int* q_start, int requests, int at, int& row0, int& count) {
+// Chunk number `at` of the requests that are taken (in their order), by a warp; false: there is none.
+__device__ __forceinline__ bool find_chunk(const int* q_start, const int* list, int requests, int at, int& row0, int& count) {
     const int lane = threadIdx.x & 31;
     int before = 0;
     for (int base = 0; base < requests; base += 32) {
-        const int r = base + lane;
-        const int first = r < requests ? q_start[r] : 0, last = r < requests ? q_start[r + 1] : 0;
+        const bool have = base + lane < requests;
+        const int r = have && list ? list[base + lane] : base + lane;
+        const int first = have ? q_start[r] : 0, last = have ? q_start[r + 1] : 0;
         const int own = (max(last - first, 0) + DC_TOKENS - 1) / DC_TOKENS;
         int upto = own;
 #pragma unroll
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(DC_PREP_THREADS, 4) delta_chunks_kernel(const 
     pdl_wait();
     pdl_trigger();
     int row0, cnt;
-    if (!find_chunk(a.q_start, a.requests, blockIdx.x, row0, cnt)) return;
+    if (!find_chunk(a.q_start, a.list, a.requests, blockIdx.x, row0, cnt)) return;
     unsigned char* rec_q = rec, *rec_k = rec + D * 96, *rec_b = rec + 2 * D * 96;          // first Q, K, B and G,
     float* rec_g = reinterpret_cast<float*>(rec_b + 1536);
     unsigned char* rec_w = rec, *rec_y = rec + D * 96;                                      // then W and Y in their place
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
     __shared__ __align__(8) uint64_t full[DC_STAGES];
     const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
-    const int h = blockIdx.x, r = blockIdx.z, dv = a.dv;
+    const int h = blockIdx.x, r = a.list ? a.list[blockIdx.z] : blockIdx.z, dv = a.dv;
     if (tid == 0) {
         for (int i = 0; i < DC_STAGES; ++i) mbar_init(&full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -380,7 +382,10 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS) delta_chain_kernel(const Del
     if (tokens <= 0) return;
     const int chunks = (tokens + DC_TOKENS - 1) / DC_TOKENS;
     int first = 0;
-    for (int i = lane; i < r; i += 32) first += (max(a.q_start[i + 1] - a.q_start[i], 0) + DC_TOKENS - 1) / DC_TOKENS;
+    for (int i = lane; i < blockIdx.z; i += 32) {
+        const int other = a.list ? a.list[i] : i;
+        first += (max(a.q_start[other + 1] - a.q_start[other], 0) + DC_TOKENS - 1) / DC_TOKENS;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
     const int bytes = dc_record(D, dv);
@@ -515,30 +520,48 @@ template <int KS> void launch_chunks(const DeltaChunkArgs& a, int chunks, cudaSt
 
 }  // namespace
 
+// delta_rule.cu
+LLMP_API int llmp_delta_prep(float* q, long q_t, float* k, long k_t, float* decay, long decay_t, float* beta, long beta_t, const float* a_log,
+                             const float* dt_bias, const int* token_request, const int* q_start, int max_tokens, int tokens, int H, int G, int d,
+                             cudaStream_t stream);
+LLMP_API int llmp_delta_scan(const float* q, long q_t, const float* k, long k_t, const float* v, long v_t, const float* decay, long decay_t,
+                             const float* beta, long beta_t, float* state, long state_slot, long state_half, const int* q_start, const int* slots,
+                             const int* positions, float* o, long o_t, int max_tokens, int R, int H, int G, int d, int dv, cudaStream_t stream);
+
 // Bytes of scratch for `rows` tokens of R requests; 0: these sizes are not served.
 LLMP_API long llmp_delta_chunks_scratch(int rows, int R, int H, int d, int dv) {
     if (rows <= 0 || R <= 0 || H <= 0 || (d != 64 && d != 128) || dv < 16 || dv % 16 || dv > 512) return 0;
     return ((long)(rows - 1) / DC_TOKENS + R) * H * dc_record(d, dv);
 }
 
-// q, k, v: the convolved rows; decay, beta: pre-activations (delta_prep and delta_scan in one).
-LLMP_API int llmp_delta_chunks(const float* q, long q_t, const float* k, long k_t, const float* v, long v_t, const float* decay, long decay_t,
-                               const float* beta, long beta_t, const float* a_log, const float* dt_bias, float* state, long state_slot,
+// q, k, v: the convolved rows; decay, beta: pre-activations (delta_prep and delta_scan in one). list: `count` of the R requests, in
+// ascending order, which have `rows` of the step's tokens together; the others, which have up to max_tokens each, go token by token
+// (their rows are prepared in place). null: all requests in chunks.
+LLMP_API int llmp_delta_chunks(float* q, long q_t, float* k, long k_t, const float* v, long v_t, float* decay, long decay_t,
+                               float* beta, long beta_t, const float* a_log, const float* dt_bias, float* state, long state_slot,
                                long state_half, const int* q_start, const int* slots, const int* positions, float* o, long o_t, void* scratch,
-                               long scratch_bytes, int rows, int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
-    if (R <= 0 || rows <= 0) return 0;
+                               long scratch_bytes, const int* list, int count, int rows, const int* token_request, int max_tokens, int tokens, int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
+    if (R <= 0 || tokens <= 0) return 0;
+    LLMP_REQUIRE(rows > 0 && rows <= tokens && count > 0 && count <= R && (list ? token_request != nullptr : count == R && rows == tokens),
+                 "delta_chunks: %d of %d requests, %d of %d tokens", count, R, rows, tokens);
     LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && H <= 65535 && R <= 65535, "delta_chunks: bad sizes heads=%d qk_heads=%d requests=%d", H, G, R);
     LLMP_REQUIRE(error_flag != nullptr, "delta_chunks: an error flag in device memory is required");
-    const long need = llmp_delta_chunks_scratch(rows, R, H, d, dv);
+    const long need = llmp_delta_chunks_scratch(rows, count, H, d, dv);
     LLMP_REQUIRE(need > 0, "delta_chunks: heads of %d x %d are not served", d, dv);
     LLMP_REQUIRE(scratch != nullptr && scratch_bytes >= need && (size_t)scratch % 16 == 0, "delta_chunks: %ld bytes of scratch are needed", need);
     DeltaChunkArgs a;
     a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.v = v; a.v_t = v_t; a.decay = decay; a.decay_t = decay_t; a.beta = beta; a.beta_t = beta_t;
     a.a_log = a_log; a.dt_bias = dt_bias; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
-    a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.scratch = (unsigned char*)scratch; a.requests = R; a.H = H; a.G = G; a.dv = dv;
+    a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.scratch = (unsigned char*)scratch; a.list = list; a.requests = count; a.H = H; a.G = G; a.dv = dv;
     a.error_flag = error_flag;
-    const int chunks = (rows - 1) / DC_TOKENS + R;
+    const int chunks = (rows - 1) / DC_TOKENS + count;
     if (d == 64) launch_chunks<1>(a, chunks, stream);
     else launch_chunks<2>(a, chunks, stream);
+    if (list) {
+        const int failed = llmp_delta_prep(q, q_t, k, k_t, decay, decay_t, beta, beta_t, a_log, dt_bias, token_request, q_start, max_tokens, tokens, H, G, d, stream);
+        if (failed) return failed;
+        return llmp_delta_scan(q, q_t, k, k_t, v, v_t, decay, decay_t, beta, beta_t, state, state_slot, state_half, q_start, slots, positions, o, o_t,
+                               max_tokens, R, H, G, d, dv, stream);
+    }
     return llmp_check_launch("delta_chunks");
 }

@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from typing import Optional, Sequence
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -103,9 +103,10 @@ _SIGNATURES = {
     "llmp_chunked_scan": [_P, _P, _P, _L, _P, _L, _P, _P, _P, _P, _P, _L, _L, _P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _P],
     "llmp_stream_step": [_P, _L, _L, _P, _P, _I, _P, _F, _F, _P, _I, _P, _F, _F, _P, _P, _P, _P, _P, _I, _F, _P, _I, _P, _I, _I, _I, _P],
     "llmp_gated_group_norm": [_P, _L, _P, _L, _P, _P, _I, _L, _I, _I, _I, _I, _F, _P],
-    "llmp_delta_prep": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _I, _I, _I, _I, _P],
-    "llmp_delta_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _P],
-    "llmp_delta_chunks": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
+    "llmp_delta_prep": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
+    "llmp_delta_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
+    "llmp_delta_chunks": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I,
+                          _I, _P, _P],
     "llmp_sig_qkv_post": [_P, _L, _P, _I, _P, _P, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "llmp_sigmoid_attention": [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "llmp_sigmoid_attention_mma": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
@@ -1642,7 +1643,7 @@ def delta_prep(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, beta: torc
     _need(a_log.dtype == torch.float32 and a_log.numel() == heads and a_log.is_contiguous() and dt_bias.dtype == torch.float32 and
           dt_bias.numel() == heads * dim and dt_bias.is_contiguous(), "delta_prep takes float32 A_log [heads] and dt_bias [heads dim]")
     _call("llmp_delta_prep", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(decay), decay.stride(0), _ptr(beta), beta.stride(0),
-          _ptr(a_log), _ptr(dt_bias), N, heads, qk_heads, dim, _stream())
+          _ptr(a_log), _ptr(dt_bias), None, None, 0, N, heads, qk_heads, dim, _stream())
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,
@@ -1660,20 +1661,23 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     ptr, slot_stride, half = _state_views(state, state_offset, heads * dim * vdim, "delta_scan")
     _call("llmp_delta_scan", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0),
           _ptr(beta), beta.stride(0), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
-          slots.numel(), heads, qk_heads, dim, vdim, _stream())
+          (1 << 31) - 1, slots.numel(), heads, qk_heads, dim, vdim, _stream())
     return out
 
 
-# From two chunks of 16 tokens on for some request: one call instead of two (a layer of 32 tokens: 162 us either way, the host's time;
-# 300 + 147 tokens 232 -> 169). Single tokens and the shortest portions read and write the state once either way, and scratch
-# would only be in their way. The chunks' operands take 47 KB each at heads of 128 x 128 (of 16 heads, 15,600 tokens in 704 MB).
-DELTA_CHUNKS_MIN_TOKENS = 32
+# A request's tokens in a step from which it goes in chunks. Up to there the walk (0.3 us a token) hides behind the host's launches, or
+# beside the walks of the step's other requests: 64 decoded tokens with a portion of 64, of 96, of 128, of 300: walked 222, 240, 255,
+# 356 us a layer, the portion in chunks 238, 242, 246, 282 (the two launches more cost the host 3); all of them in chunks 281, 286,
+# 289, 333, since a block of the chain fills an SM for a token's sake. The chunks' operands take 47 KB each at heads of 128 x 128 (of 16
+# heads, 15,600 tokens in 704 MB).
+DELTA_CHUNKS_MIN_TOKENS = 96
 DELTA_CHUNKS_MAX_BYTES = 704 << 20
 
 
 def delta_chunks_scratch(dtype: torch.dtype, rows: int, requests: int, max_q_len: int, heads: int, dim: int, vdim: int) -> int:
-    """Bytes of scratch that ``delta_chunks`` takes for a step, or 0 where ``delta_prep`` and ``delta_scan`` serve it: float32, short
-    portions, sizes without an instance, and steps whose chunks would take more than ``DELTA_CHUNKS_MAX_BYTES``."""
+    """Bytes of scratch that ``delta_chunks`` takes for ``rows`` tokens of ``requests`` requests, or 0 where ``delta_prep`` and
+    ``delta_scan`` serve the step: float32, short portions, sizes without an instance, and chunks that would take more than
+    ``DELTA_CHUNKS_MAX_BYTES``."""
     if dtype != torch.bfloat16 or max_q_len < DELTA_CHUNKS_MIN_TOKENS:
         return 0
     fn = library().llmp_delta_chunks_scratch
@@ -1684,9 +1688,13 @@ def delta_chunks_scratch(dtype: torch.dtype, rows: int, requests: int, max_q_len
 
 def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, a_log: torch.Tensor,
                  dt_bias: torch.Tensor, state: torch.Tensor, state_offset: int, q_start: torch.Tensor, slots: torch.Tensor,
-                 positions: torch.Tensor, out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, scratch: int) -> torch.Tensor:
-    """``delta_prep`` and ``delta_scan`` for steps with long portions, in chunks on the tensor cores (csrc/delta_chunks.cu): the same
-    rows before ``delta_prep``, which stay as they are. ``scratch``: what ``delta_chunks_scratch`` gave."""
+                 positions: torch.Tensor, out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, scratch: int,
+                 long: Optional[Tuple[torch.Tensor, int]] = None, token_request: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``delta_prep`` and ``delta_scan`` in chunks on the tensor cores (csrc/delta_chunks.cu): the same rows before ``delta_prep``,
+    which stay as they are. ``long``: which of the step's requests (int32 on the device, ascending: those of at least
+    ``DELTA_CHUNKS_MIN_TOKENS`` tokens) and their tokens together; the others, whose rows ``token_request`` tells, are prepared in place
+    and walked token by token in the same call. None: all requests in chunks. ``scratch``: what ``delta_chunks_scratch`` gave for the
+    tokens and the number of the requests in chunks."""
     H, G, d, dv = int(heads), int(qk_heads), int(dim), int(vdim)
     N = q.shape[0]
     for t, name, width in ((q, "q", G * d), (k, "k", G * d), (v, "v", H * dv), (decay, "decay", H * d), (beta, "beta", H), (out, "out", H * dv)):
@@ -1695,11 +1703,18 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch
           dt_bias.is_contiguous(), "delta_chunks takes float32 vectors of one entry per head, and per head and channel")
     for t, name in ((q_start, "q_start"), (slots, "slots"), (positions, "positions")):
         _i32(t, name)
+    R = slots.numel()
+    if long is not None:
+        _i32(long[0], "long requests")
+        _i32(token_request, "token_request")
+        _need(0 < long[0].numel() < R and 0 < long[1] <= N == token_request.numel(), "delta_chunks: some of the step's requests and tokens")
     ptr, slot_stride, half = _state_views(state, state_offset, H * d * dv, "delta_chunks")
     room = torch.empty(scratch, dtype=torch.uint8, device=q.device)
     _call("llmp_delta_chunks", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0), _ptr(beta),
           beta.stride(0), _ptr(a_log), _ptr(dt_bias), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
-          _ptr(room), scratch, N, slots.numel(), H, G, d, dv, error_flag().data_ptr(), _stream())
+          _ptr(room), scratch, *((None, R, N, None, 0) if long is None else (_ptr(long[0]), long[0].numel(), long[1], _ptr(token_request),
+                                                                             DELTA_CHUNKS_MIN_TOKENS - 1)),
+          N, R, H, G, d, dv, error_flag().data_ptr(), _stream())
     return out
 
 

@@ -34,6 +34,22 @@ from .base import LayerCache, Mixer, TensorGetter
 from .registry import register_mixer
 
 
+def _long_requests(ctx):
+    """(the step's requests whose portions go in chunks, as ``kernels.delta_chunks`` wants them; their tokens; their number). Which form a
+    request takes follows from its own tokens. Made once per step; nothing of it in a step of short portions."""
+    least = kernels.DELTA_CHUNKS_MIN_TOKENS
+    if ctx.max_q_len < least:
+        return None, 0, 0
+    plan = ctx.memo.get(("delta_rule", least))
+    if plan is None:
+        taken = [r for r, n in enumerate(ctx.q_lens) if n >= least]
+        rows, some = sum(ctx.q_lens[r] for r in taken), None
+        if len(taken) < len(ctx.q_lens):
+            some = (torch.tensor(taken, dtype=torch.int32).pin_memory().to(ctx.device, non_blocking=True), rows)
+        plan = ctx.memo[("delta_rule", least)] = (some, rows, len(taken))
+    return plan
+
+
 @register_mixer("gated_delta_rule")
 class GatedDeltaRule(Mixer):
     graph_safe = True
@@ -116,10 +132,11 @@ class GatedDeltaRule(Mixer):
                            mixed, ctx.max_q_len, silu=True)
         q, k, v = mixed[:, :self.qk_size], mixed[:, self.qk_size:2 * self.qk_size], mixed[:, 2 * self.qk_size:]
         o = torch.empty((N, self.v_size), dtype=torch.float32, device=x.device)
-        scratch = kernels.delta_chunks_scratch(x.dtype, N, ctx.num_requests, ctx.max_q_len, H, self.dim, self.vdim)
+        some, rows, count = _long_requests(ctx)
+        scratch = kernels.delta_chunks_scratch(x.dtype, rows, count, ctx.max_q_len, H, self.dim, self.vdim) if count else 0
         if scratch:
             kernels.delta_chunks(q, k, v, decay, beta, self.a_log, self.dt_bias, cache.state, self.conv_entries, ctx.q_start, ctx.slots,
-                                 ctx.positions, o, H, self.qk_heads, self.dim, self.vdim, scratch)
+                                 ctx.positions, o, H, self.qk_heads, self.dim, self.vdim, scratch, some, ctx.token_request)
         else:
             kernels.delta_prep(q, k, decay, beta, self.a_log, self.dt_bias, H, self.qk_heads, self.dim)
             kernels.delta_scan(q, k, v, decay, beta, cache.state, self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, o,

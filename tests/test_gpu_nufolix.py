@@ -322,6 +322,52 @@ def test_gated_delta_rule_in_chunks_is_causal_for_what_is_no_number(what, t, bad
         assert torch.equal(got[:, others], want[:, others])
 
 
+@pytest.mark.parametrize("sizes", [(2, 1, 64, 16), (1, 1, 128, 48)], ids=str)
+def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
+    """Forty portions in chunks and as many short ones token by token in one step, more than a warp looks at in one go, in an order
+    that mixes them: every request's outputs and state have the bits they have alone, and other rows and slots stay."""
+    from llm_pipeline_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNKS_MIN_TOKENS", 17)
+    heads, qk_heads, dim, vdim = sizes
+    gen, dev, piece = torch.Generator().manual_seed(dim), "cuda", heads * dim * vdim
+    lengths = [(1, 17, 16, 40, 3, 33, 2, 18)[i % 8] for i in range(80)]
+    starts = [sum(lengths[:r]) for r in range(81)]
+    a_log, dt_bias = torch.rand(heads, generator=gen).to(dev), torch.randn(heads * dim, generator=gen).to(dev)
+    rows = [x.to(dev) for x in _delta_rule_rows(gen, starts[-1], *sizes)]
+    state = torch.randn(81, 2 * piece, generator=gen).to(dev)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)   # noqa: E731
+
+    def step(requests):
+        own = [lengths[r] for r in requests]
+        x = [torch.cat([y[starts[r]:starts[r + 1]] for r in requests]) for y in rows]
+        o, left = torch.full((sum(own), heads * vdim), 7.0, device=dev), state.clone()
+        where = (i32([sum(own[:k]) for k in range(len(own) + 1)]), i32([80 - r for r in requests]), i32([5 + p for n in own for p in range(n)]))
+        q, k, v, decay, beta = x
+        taken = [k for k, n in enumerate(own) if n >= 17]
+        if not taken:
+            kernels.delta_prep(q, k, decay, beta, a_log, dt_bias, heads, qk_heads, dim)
+            kernels.delta_scan(q, k, v, decay, beta, left, 0, *where, o, heads, qk_heads, dim, vdim)
+            return o, left
+        count = sum(own[k] for k in taken)
+        long = None if len(taken) == len(own) else (i32(taken), count)
+        need = kernels.delta_chunks_scratch(torch.bfloat16, count, len(taken), max(own), heads, dim, vdim)
+        kernels.delta_chunks(q, k, v, decay, beta, a_log, dt_bias, left, 0, *where, o, heads, qk_heads, dim, vdim, need, long,
+                             i32([k for k, n in enumerate(own) for _ in range(n)]))
+        return o, left
+
+    o, left = step(list(range(80)))
+    long_only, _left = step([r for r in range(80) if lengths[r] >= 17])
+    at = 0
+    for r in range(80):
+        alone, mine = step([r])
+        assert torch.equal(o[starts[r]:starts[r + 1]], alone) and torch.equal(left[80 - r], mine[80 - r]), r
+        if lengths[r] >= 17:
+            assert torch.equal(long_only[at:at + lengths[r]], alone), r
+            at += lengths[r]
+    assert torch.equal(left[0], state[0])
+    kernels.check_error_flag()
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
     from llm_pipeline_b200.ops import kernels
@@ -503,6 +549,29 @@ def test_prefill_decoding_portions_and_batches(tmp_path, name, dtype):
     N.assert_matches(got, want, dtype, f"{name}: mixed batches", share)
     assert runner.cache.num_live == 0                                   # seven requests went through four slots
     assert runner.cache.pages_reused > 0 or all(layer["type"] != "parallel" for layer in cfg["layers"])
+
+
+def test_delta_rule_portions_in_chunks_beside_single_tokens(tmp_path, monkeypatch):
+    """A whole model in bfloat16 whose portions of 16 tokens and more go in chunks, in steps that hold decoded tokens and shorter
+    portions as well: the state passes from one form to the other and back."""
+    from llm_pipeline_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNKS_MIN_TOKENS", 16)
+    cfg = N.config([N.parallel(N.left(2, 1, 64, 32, rot_dims=32), N.right(2, 1, 64, 32, conv=4))] * 2, width=40, vocab=71)
+    W = N.weights_for(cfg, 11)
+    folder = N.write_model(str(tmp_path), cfg, W)
+    requests = requests_for(cfg, [150, 40, 97, 3, 66], 50)
+    want = N.oracle(cfg, W, requests)
+    runner = H.make_runner(folder, torch.bfloat16, page_size=8, num_pages=64, max_request_tokens=160, max_requests=4)
+    mixed, chunks = [], kernels.delta_chunks
+
+    def counting(*args):
+        mixed.append(args[18] is not None)
+        return chunks(*args)
+
+    monkeypatch.setattr(kernels, "delta_chunks", counting)
+    N.assert_matches(H.replay(runner, H.cut_portions(requests, (33, 2, 16, 15))), want, torch.bfloat16, "portions", 0.99)
+    N.assert_matches(H.replay(runner, H.cut_mixed(requests, (33, 2, 16, 15), max_live=4, decode_tail=20)), want, torch.bfloat16, "mixed", 0.99)
+    assert any(mixed) and not all(mixed)
 
 
 def test_the_same_logits_alone_and_in_a_batch(tmp_path):
