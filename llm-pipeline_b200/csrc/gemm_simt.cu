@@ -4,6 +4,8 @@
 // row's result does not depend on how many other rows are in the call.
 #include "common.cuh"
 
+int llmp_sm_count();
+
 namespace {
 
 // Four consecutive entries of a row from k on; entries from K on are 0. VEC: 4-entry pieces are aligned and K is a multiple of 4.
@@ -129,14 +131,14 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
 template <typename TI, typename TO, bool VEC>
 void launch_nt(const TI* A, const TI* W, const void* bias, int bias_bf16, TO* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
                long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
-    constexpr long SMS = 148;
+    const long sms = llmp_sm_count();
     auto blocks = [&](int bm, int bn) { return (long)((N + bn - 1) / bn) * ((M + bm - 1) / bm) * batch; };
 #define LLMP_NT(BM, BN, BK, TM, TN, AHEAD)                                                                                              \
     gemm_nt_kernel<TI, TO, BM, BN, BK, TM, TN, AHEAD, VEC><<<dim3((N + BN - 1) / BN, (M + BM - 1) / BM, batch), (BM / TM) * (BN / TN), 0, stream>>>( \
         A, W, bias, bias_bf16, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c)
-    if (blocks(64, 64) >= 3 * SMS) LLMP_NT(64, 64, 32, 8, 8, 1);
-    else if (blocks(64, 64) >= SMS) LLMP_NT(64, 64, 16, 8, 4, 1);
-    else if (blocks(32, 32) >= SMS) LLMP_NT(32, 32, 32, 4, 4, 1);
+    if (blocks(64, 64) >= 3 * sms) LLMP_NT(64, 64, 32, 8, 8, 1);
+    else if (blocks(64, 64) >= sms) LLMP_NT(64, 64, 16, 8, 4, 1);
+    else if (blocks(32, 32) >= sms) LLMP_NT(32, 32, 32, 4, 4, 1);
     else LLMP_NT(32, 32, 32, 2, 2, 2);
 #undef LLMP_NT
 }
@@ -164,7 +166,7 @@ bool launch_nt_any(const void* A, const void* W, const void* bias, int bias_bf16
 
 }  // namespace
 
-#define GT_MAX_ROWS (65535 * 32)      // rows of the smallest tile that a grid can hold
+#define GT_MAX_ROWS (65535 * 64)      // what a grid can hold of the tiles of 64 rows, which so many rows take whatever N is
 
 // in_dtype: type of A and W.  out_dtype: type of C (float32, or the input type).
 LLMP_API int llmp_gemm_simt(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int in_dtype,

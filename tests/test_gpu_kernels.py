@@ -166,6 +166,23 @@ def test_gemm_simt_gives_one_sum_whatever_the_tile(dtype, M, N, Kd):
         assert torch.equal(single[0], out[m]), m
 
 
+def test_gemm_simt_takes_as_many_rows_as_its_largest_tiles_hold():
+    """More rows than a grid of the smallest tiles could hold: the last rows, and one of each grid row, have the bits they have alone;
+    a row too many is an error."""
+    M = 65535 * 32 + 33
+    gen = torch.Generator().manual_seed(1)
+    a, w = (torch.randn(n, 4, generator=gen).to(DEV) for n in (M, 3))
+    out = torch.empty(M, 3, device=DEV)
+    K().gemm_simt(a, w, out)
+    rows = torch.cat([torch.arange(0, M, 64), torch.arange(M - 64, M)]).to(DEV)
+    alone = torch.empty(rows.numel(), 3, device=DEV)
+    K().gemm_simt(a[rows].contiguous(), w, alone)
+    assert torch.equal(out[rows], alone)
+    assert ((out.double() - a.double() @ w.double().T).abs() <= 4 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)).all()
+    with pytest.raises(Exception, match="too many rows"):
+        K().gemm_simt(a[:1].expand(65535 * 64 + 1, 4), w, out[:1].expand(65535 * 64 + 1, 3))
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
 @pytest.mark.parametrize("M,N,Kd", [(1, 130, 64), (8, 4096, 4096), (7, 100, 1048), (16, 6144, 520), (13, 331, 264),
                                      (9, 20000, 1032), (3, 17000, 256), (5, 20, 8)])
