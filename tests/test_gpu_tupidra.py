@@ -160,6 +160,42 @@ def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
     assert (state[[0, R + 1]] == 5.0).all() and (state[slots, :offset] == 0.0).all() and (state[slots, offset + entries:] == 0.0).all()
 
 
+@pytest.mark.parametrize("sizes", [(130, 16), (37, 5)], ids=str)
+def test_selective_scan_in_company(sizes, monkeypatch):
+    """Eighty requests in segments in one step, more than a warp looks at in one go: each has the bits it has alone in segments, and
+    what it has alone token by token but for roundings: an output differs by bfloat16's 2^-8 of itself where its rounding flips,
+    the float32 state by 2e-5 of the largest entry, within which both forms are from float64."""
+    from llm_pipeline_b200.ops import kernels
+    monkeypatch.setattr(kernels, "SCAN_SEGMENTS_MIN_TOKENS", 0)
+    inner, states = sizes
+    gen = torch.Generator().manual_seed(inner)
+    lengths = [(1, 65, 64, 130, 2, 1, 33, 66)[i % 8] for i in range(80)]
+    starts = [0] + list(itertools.accumulate(lengths))
+    dt_bias, skip = (torch.randn(inner, generator=gen).to(DEV) for _ in range(2))
+    A = -torch.exp(torch.rand(inner, states, generator=gen) * 5.0 - 4.5).to(DEV)
+    x, raw, z, bc = (torch.randn(starts[-1], width, generator=gen).to(DEV) for width in (inner, inner, inner, 2 * states))
+    state = torch.randn(81, 2 * inner * states, generator=gen).to(DEV)
+
+    def step(requests, longest):
+        own = [lengths[r] for r in requests]
+        part = [torch.cat([y[starts[r]:starts[r + 1]] for r in requests]) for y in (x, raw, z, bc)]
+        out, left = torch.empty(sum(own), inner, device=DEV, dtype=torch.bfloat16), state.clone()
+        kernels.selective_scan(part[0], part[1], dt_bias, part[3][:, :states], part[3][:, states:], A, skip, part[2], left, 0,
+                               _i32([0] + list(itertools.accumulate(own))), _i32([80 - r for r in requests]),
+                               _i32([7 + p for n in own for p in range(n)]), out, longest)
+        return out, left
+
+    out, left = step(list(range(80)), max(lengths))
+    for r in range(80):
+        mine = out[starts[r]:starts[r + 1]]
+        alone, kept = step([r], lengths[r])
+        assert torch.equal(mine, alone) and torch.equal(left[80 - r], kept[80 - r]), r
+        walked, kept = step([r], 0)
+        assert _rel(left[80 - r], kept[80 - r].double().cpu()) < 4e-5 and ((mine.float() - walked.float()).abs() <= 2.0 ** -7 * walked.float().abs() + 4e-5 *
+                                                           walked.float().abs().max()).all(), r
+    assert torch.equal(left[0], state[0])
+
+
 def _window_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap, size, keep, plant=None, rows=None, gate=True):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine output, plain output) for
     the token rows ``rows`` (all by default), each launched as the portion it is."""
