@@ -4,10 +4,10 @@
 // A block takes a tile of up to 16 consecutive new tokens of one request and one range of keys, with a warp per
 // query head. Keys are walked in tiles of 32 aligned to key 0. For a key tile
 //   1. warp g multiplies its head's 16 queries with the 32 keys of its key/value head, caps the scores, takes the
-//      sigmoid (float32) and leaves the halves of the 16 x 32 weights in shared memory, the pairs in the order of its registers;
+//      sigmoid (float32) and leaves the 16 x 32 weights in shared memory, the pairs in the order of its registers;
 //   2. the weights of all heads are mixed by the matrix of the heads as a product of its own: 16 heads out, 16 heads in, a column
-//      for each of the 512 (token, key) pairs, dealt out over the warps. Both factors are split into two bfloat16 halves and
-//      the three larger products of halves summed in float32, which leaves the mixed weights 16 bits;
+//      for each of the 512 (token, key) pairs, dealt out over the warps. Both factors are split into three bfloat16 pieces, which
+//      hold all 24 bits, and the six larger products of pieces summed in float32: rows of the matrix may cancel;
 //   3. they are rounded to bfloat16, and warp h multiplies those of its head with the 32 values of its key/value head.
 // Nothing is normalised over keys, so the output registers simply add up over key tiles and key ranges: with more
 // than one range the blocks leave float32 partial sums that a second kernel adds in the order of the ranges.
@@ -16,7 +16,8 @@
 // With every warp adding up all heads' float32 weights on the CUDA cores, a key tile moved 512 KB through shared memory for the
 // mix alone, 4,096 clocks of an SM; as a product it moves 100 KB. 2,048 tokens of 16 heads of 128: 285 us before, 197 with the
 // product, 168 with tanh as a series where the scores are far below the cap, exponentials and reciprocals without their range
-// checks, masks only where a row's end is near, and a tile's places found a tile ahead. What is left is the latency of four
+// checks, masks only where a row's end is near, and a tile's places found a tile ahead (three pieces instead of two: a layer 230
+// -> 240). What is left is the latency of four
 // phases between barriers at four warps a scheduler (issue slots 42 %, tensor pipe 28 %). Shorter key ranges (512, 256 keys) lose
 // to their partial sums: 205, 222 us against 197.
 #include "common.cuh"
@@ -70,11 +71,14 @@ __device__ __forceinline__ unsigned sm_pack(float lo, float hi) {
     return *reinterpret_cast<const unsigned*>(&v);
 }
 
-// Two floats as a pair of bfloat16, and what that leaves of them as another pair.
-__device__ __forceinline__ void sm_split(float u, float v, unsigned& hi, unsigned& lo) {
+// Two floats as three pairs of bfloat16 that add up to them.
+__device__ __forceinline__ void sm_split(float u, float v, unsigned& hi, unsigned& mid, unsigned& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(u, v);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(u - __low2float(h), v - __high2float(h));
+    const float ru = u - __low2float(h), rv = v - __high2float(h);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(ru, rv);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(ru - __low2float(m), rv - __high2float(m));
     hi = *reinterpret_cast<const unsigned*>(&h);
+    mid = *reinterpret_cast<const unsigned*>(&m);
     lo = *reinterpret_cast<const unsigned*>(&l);
 }
 
@@ -100,7 +104,7 @@ template <bool SMALL> __device__ __forceinline__ float sm_tanh(float x) {
 // The sigmoid of a number given times -log2(e); the exponential's and the reciprocal's errors leave the weight's near 1e-7.
 __device__ __forceinline__ float sm_sigmoid(float minus_log2) { return sm_rcp(1.f + sm_ex2(minus_log2)); }
 
-constexpr int SM_PAIRS = SM_ROWS * SM_KEYS + 8;        // entries of a head's (token, key) pairs in shared memory: conflict-free ldmatrix
+constexpr int SM_PAIRS = SM_ROWS * SM_KEYS + 4;        // a head's weights in shared memory: neighbouring heads' lie 4 banks apart
 constexpr int SM_PS = SM_KEYS + 8;                     // of a token's mixed weights
 constexpr int SM_PH = SM_ROWS * SM_PS + 8;             // of a head's: eight heads' rows meet no bank twice
 
@@ -115,9 +119,8 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
     bf16* Ks = Qs + (size_t)H * SM_ROWS * KS;                       // [G][32][KS]
     bf16* Vs = Ks + (size_t)G * SM_KEYS * KS;                       // [G][32][VS]
     const int wrows = min(SM_MAX_HEADS, H + 1);
-    bf16* Wh = Vs + (size_t)G * SM_KEYS * VS;                       // [wrows][SM_PAIRS]: the weights' halves; row H, if any, is zero
-    bf16* Wl = Wh + wrows * SM_PAIRS;
-    bf16* Ps = a.late_keys ? Ks : Wl + wrows * SM_PAIRS;            // [H][16][SM_PS] with SM_PH entries a head: the mixed weights
+    float* Ws = reinterpret_cast<float*>(Vs + (size_t)G * SM_KEYS * VS);    // [wrows][SM_PAIRS]: the weights; row H, if any, is zero
+    bf16* Ps = a.late_keys ? Ks : reinterpret_cast<bf16*>(Ws + wrows * SM_PAIRS);   // [H][16][SM_PS] with SM_PH entries a head: the mixed weights
     __shared__ long long key_off[2][SM_KEYS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
     const int gr = lane >> 2, t = lane & 3;
@@ -146,12 +149,12 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
         const bool ok = row < ntok;
         sm_cp_async_16(Qs + ((size_t)h * SM_ROWS + row) * KS + c, ok ? a.q + (size_t)(first + row) * a.q_t + (size_t)h * D + c : a.q, ok);
     }
-    for (int i = tid; i < (wrows - H) * SM_PAIRS; i += nthreads) Wh[H * SM_PAIRS + i] = Wl[H * SM_PAIRS + i] = __float2bfloat16_rn(0.f);
-    unsigned th[4], tl[4];                                          // the mixing matrix as an A operand: heads out along m, heads in along k
+    for (int i = tid; i < (wrows - H) * SM_PAIRS; i += nthreads) Ws[H * SM_PAIRS + i] = 0.f;
+    unsigned mix[3][4];                                             // the mixing matrix as an A operand: heads out along m, heads in along k
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int ho = gr + 8 * (i & 1), hi = 2 * t + 8 * (i >> 1);
-        sm_split(ho < H && hi < H ? a.talk[ho * H + hi] : 0.f, ho < H && hi + 1 < H ? a.talk[ho * H + hi + 1] : 0.f, th[i], tl[i]);
+        sm_split(ho < H && hi < H ? a.talk[ho * H + hi] : 0.f, ho < H && hi + 1 < H ? a.talk[ho * H + hi + 1] : 0.f, mix[0][i], mix[1][i], mix[2][i]);
     }
     // Where the keys of a tile lie among the pages (-1: nowhere), found a tile ahead by the first warp; a barrier lies between.
     auto find_keys = [&](int j0) {
@@ -254,28 +257,30 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
         }
         // the pairs of token gr + 8 hr and keys nb 8 .. of the tile are columns (2 nb + hr) 64 + 8 gr ..: a warp writes 128 bytes
         {
-            unsigned* wh = reinterpret_cast<unsigned*>(Wh + h * SM_PAIRS) + lane;
-            unsigned* wl = reinterpret_cast<unsigned*>(Wl + h * SM_PAIRS) + lane;
+            float2* w = reinterpret_cast<float2*>(Ws + h * SM_PAIRS) + lane;
 #pragma unroll
             for (int nb = 0; nb < 4; ++nb)
 #pragma unroll
-                for (int hr = 0; hr < 2; ++hr) sm_split(s[nb][2 * hr], s[nb][2 * hr + 1], wh[(2 * nb + hr) * 32], wl[(2 * nb + hr) * 32]);
+                for (int hr = 0; hr < 2; ++hr) w[(2 * nb + hr) * 32] = make_float2(s[nb][2 * hr], s[nb][2 * hr + 1]);
         }
         __syncthreads();                                            // all weights are in place, the keys are free
         if (!a.late_keys) issue_keys(j0 + SM_KEYS);
         // 32 times 16 columns over the warps: the mixed weights of all heads for two tokens and 8 keys each
         for (int pair = warp; pair < 32; pair += H) {
-            unsigned bh[4], bl[4];
-            const int at = min(((lane >> 3) & 1) * 8 + (lane & 7), wrows - 1);      // heads past H: the zero row
-            sm_ldmatrix_x4_trans(bh, Wh + at * SM_PAIRS + pair * 16 + (lane >> 4) * 8);
-            sm_ldmatrix_x4_trans(bl, Wl + at * SM_PAIRS + pair * 16 + (lane >> 4) * 8);
+            unsigned b[2][3][2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {                           // this lane's heads in: 2 t, 2 t + 1 and eight further
+                const float* w0 = Ws + min(2 * t + 8 * k, wrows - 1) * SM_PAIRS + pair * 16 + gr;      // heads past H: the zero row
+                const float* w1 = Ws + min(2 * t + 8 * k + 1, wrows - 1) * SM_PAIRS + pair * 16 + gr;
+#pragma unroll
+                for (int n = 0; n < 2; ++n) sm_split(w0[8 * n], w1[8 * n], b[n][0][k], b[n][1][k], b[n][2][k]);
+            }
             float m[2][4] = {};
+            constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};      // the smaller products first
 #pragma unroll
-            for (int n = 0; n < 2; ++n) sm_mma(m[n], th, bh[2 * n], bh[2 * n + 1]);
+            for (int i = 0; i < 6; ++i)
 #pragma unroll
-            for (int n = 0; n < 2; ++n) sm_mma(m[n], tl, bh[2 * n], bh[2 * n + 1]);
-#pragma unroll
-            for (int n = 0; n < 2; ++n) sm_mma(m[n], th, bl[2 * n], bl[2 * n + 1]);
+                for (int n = 0; n < 2; ++n) sm_mma(m[n], mix[PA[i]], b[n][PB[i]][0], b[n][PB[i]][1]);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
                 const int q = pair * 2 + n, token = (q & 7) + 8 * ((q >> 3) & 1), key = (q >> 4) * 8 + 2 * t;
@@ -324,8 +329,8 @@ __global__ void __launch_bounds__(SM_MAX_HEADS * 32, 1) sigmoid_attention_mma_ke
 // values' product: for sizes that would not fit otherwise.
 size_t sm_smem_bytes(int H, int G, int d, int dv, bool late_keys) {
     const size_t keys = (size_t)G * SM_KEYS * (d + 8), mixed = (size_t)H * SM_PH;
-    return sizeof(bf16) * ((size_t)H * SM_ROWS * (d + 8) + keys + (size_t)G * SM_KEYS * (dv + 8) + 2 * (size_t)(H < SM_MAX_HEADS ? H + 1 : H) * SM_PAIRS +
-                           (late_keys ? 0 : mixed));
+    return sizeof(bf16) * ((size_t)H * SM_ROWS * (d + 8) + keys + (size_t)G * SM_KEYS * (dv + 8) + (late_keys ? 0 : mixed)) +
+           sizeof(float) * (size_t)(H < SM_MAX_HEADS ? H + 1 : H) * SM_PAIRS;
 }
 constexpr size_t SM_MOST_BYTES = 226 * 1024;
 bool sm_late_keys(int H, int G, int d, int dv) {

@@ -368,8 +368,10 @@ def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
     kernels.check_error_flag()
 
 
-def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0):
-    """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output)."""
+def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0,
+                            mixed=None):
+    """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output). ``mixed``
+    changes the mixing matrix and the heads' biases in place."""
     from llm_pipeline_b200.ops import kernels
     gen = torch.Generator().manual_seed(seed)
     dev = "cuda"
@@ -379,6 +381,8 @@ def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, ca
     pb = torch.randn(heads, generator=gen) * 0.5 + bias
     if plant is not None:
         plant(q, k, v)
+    if mixed is not None:
+        mixed(talk, pb)
     q, k, v = (t.to(torch.bfloat16).float() for t in (q, k, v))
     scale = 1.0 / math.sqrt(dim)
     kv_of = torch.arange(heads) // (heads // kv_heads)
@@ -445,6 +449,29 @@ def test_sigmoid_attention_mixes_heads_as_a_product(sizes):
     results, want = _sigmoid_attention_case(torch.bfloat16, heads, kv_heads, dim, vdim, 333, page=16, seed=heads + dim, cap=cap, segments=(1, 2), bias=-3.0)
     for name, got in results.items():
         assert (got.double() - want).abs().max() <= 2.0 ** -7 * want.abs().max(), name
+
+
+@pytest.mark.parametrize("heads,cap", [(4, 0.0), (16, 30.0)])
+def test_sigmoid_attention_mixes_heads_that_cancel(heads, cap):
+    """Heads 0 and 1 differ by a unit in the last place of one small query entry and enter heads 0 and 2 with large coefficients of
+    opposite sign: what is left is a few 2^-16 of the products' sizes, so the mix has to hold float32's bits before it is rounded.
+    The mixed weights and the result are rounded to bfloat16 (2^-8 each at most): within 2^-7 in the 2-norm of a head."""
+    def plant(q, k, v):
+        q[:, 0, 0] *= 0.125
+        q[:, 0] = q[:, 0].to(torch.bfloat16).float()
+        q[:, 1] = q[:, 0]
+        q[:, 1, 0] *= 1.0 + 2.0 ** -6
+
+    def mixed(talk, pb):
+        talk *= 0.1
+        talk[0, :2], talk[2, :2] = torch.tensor([1024.0, -1024.0]), torch.tensor([-700.0, 700.0])
+        pb.fill_(-1.0)
+
+    results, want = _sigmoid_attention_case(torch.bfloat16, heads, heads // 2, 64, 32, 333, page=16, seed=heads, cap=cap, plant=plant, mixed=mixed)
+    want = want.view(333, heads, 32)
+    for name, got in results.items():
+        off = (got.double().view(want.shape) - want).norm(dim=(0, 2)) / want.norm(dim=(0, 2))
+        assert (off <= 2.0 ** -7).all(), (name, off)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
