@@ -295,7 +295,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                           TO* __restrict__ Y, int rows_a, int rows_b, int K, long ldy, int* __restrict__ error_flag) {
     extern __shared__ unsigned char tc_raw[];
     constexpr uint32_t A_BYTES = TC_BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
-    constexpr uint32_t COLS = 2 * BN;                          // two accumulators (BN = 128 or 256: a power of two)
+    constexpr uint32_t COLS = 2 * BN;                          // two accumulators (BN = 32, 128 or 256: a power of two)
     __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     const uint32_t raw_addr = tc_smem_u32(tc_raw);
@@ -396,10 +396,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 if (whole_lines && b0 + c0 + 32 <= rows_b) {
                     tc_store_rows(v, stage_rows, lane, [&](int r) -> TO* { return row0 + r < rows_a ? Y + (size_t)(row0 + r) * ldy + b0 + c0 : nullptr; }, (TO*)nullptr);
                 } else if (row0 + lane < rows_a) {
-                    TO* dst = Y + (size_t)(row0 + lane) * ldy + b0 + c0;
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (b0 + c0 + j < rows_b) dst[j] = from_float<TO>(v[j]);
+                    tc_store_own_row(v, Y + (size_t)(row0 + lane) * ldy + b0 + c0, rows_b - b0 - c0);
                 }
             }
             // this warp has read its part of the accumulator: one arrival per warp frees it for the MMA thread
@@ -559,13 +556,7 @@ static int launch_tc_persistent(const void* A, long rows_a, long lda, const void
     constexpr size_t smem = (size_t)STAGES * (TC_BM * 128 + BN * 128) + 1024 + 4 * TC_STAGE_FLOATS * sizeof(float);
     auto kernel = gemm_tc_persistent_kernel<BN, STAGES, TO>;
     LLMP_ALLOW_SMEM(kernel, smem);
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
+    const int sms = llmp_sm_count();
     const long tiles = ((rows_a + TC_BM - 1) / TC_BM) * ((rows_b + BN - 1) / BN);
     const int grid = (int)(tiles < sms ? tiles : sms);
     kernel<<<grid, TC_THREADS, smem, stream>>>(map_a, map_b, Y, (int)rows_a, (int)rows_b, K, ldy, error_flag);
@@ -578,10 +569,10 @@ static int dispatch_tc(const void* X, const void* W, TO* Y, int M, int N, int K,
     if (M <= 16) return launch_tc_splitk<16, 10, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 32) return launch_tc_splitk<32, 9, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 64) return launch_tc_splitk<64, 8, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
-    // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs, and 128 x 32 where even
-    // those leave SMs without one: 2,048 rows, 160 columns, K 4,096 26.2 us -> 22.2; 96 columns, K 2,048 15.8 -> 12.6. (Sharing K among
+    // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs, and 128 x 32 where the SMs
+    // take even those in one go: 2,048 rows, 160 columns, K 4,096 26.2 us -> 22.2; 96 columns, K 2,048 15.8 -> 12.6. (Sharing K among
     // the blocks of a cluster, 64 rows by 128 columns each, lost: 31 and 25 us.)
-    if (N < 256 && (long)((M + TC_BM - 1) / TC_BM) * ((N + 31) / 32) <= 148)
+    if (N < 256 && (long)((M + TC_BM - 1) / TC_BM) * ((N + 31) / 32) <= llmp_sm_count())
         return launch_tc_persistent<32, 8, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     if (N >= 256) return launch_tc_persistent<256, 4, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     return launch_tc_persistent<128, 6, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);

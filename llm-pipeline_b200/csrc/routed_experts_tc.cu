@@ -230,12 +230,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                             const int p = pair_of(r);
                             return p >= 0 ? a.out + (size_t)p * a.cols + c0 + c : nullptr; }, (float*)nullptr);
                 } else if (pair >= 0) {                          // the last columns of a width that is no multiple of 32 (it is one of 8)
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (c + j < cols) {
-                            if (FIRST) a.y[(size_t)row * a.cols + c0 + c + j] = __float2bfloat16_rn(v[j]);
-                            else a.out[(size_t)pair * a.cols + c0 + c + j] = v[j];
-                        }
+                    if (FIRST) tc_store_own_row(v, a.y + (size_t)row * a.cols + c0 + c, cols - c);
+                    else tc_store_own_row(v, a.out + (size_t)pair * a.cols + c0 + c, cols - c);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");

@@ -125,6 +125,32 @@ template <typename RowPtr> __device__ __forceinline__ void tc_store_rows(const f
     __syncwarp();
 }
 
+// The same without turning: a lane stores the first `cols` (up to 32) of its own row, 16 bytes at a time where those are whole and
+// aligned. For rows that are not 16-byte aligned and for what a width leaves of 32 columns.
+template <typename TO> __device__ __forceinline__ void tc_store_own_row(const float (&v)[32], TO* dst, int cols) {
+    constexpr int PIECE = 16 / sizeof(TO);
+#pragma unroll
+    for (int j = 0; j < 32; j += PIECE) {
+        if (j + PIECE <= cols && (size_t)(dst + j) % 16 == 0) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if constexpr (sizeof(TO) == 4) {
+                    w[k] = __float_as_uint(v[j + k]);
+                } else {
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(v[j + 2 * k], v[j + 2 * k + 1]);
+                    w[k] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+            }
+            *reinterpret_cast<uint4*>(dst + j) = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < PIECE; ++k)
+                if (j + k < cols) dst[j + k] = from_float<TO>(v[j + k]);
+        }
+    }
+}
+
 // ---- thread-block clusters: rank, barrier, a float32 store into another block's shared memory ----
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;

@@ -224,6 +224,25 @@ def test_gemm_tcgen05(out_dtype, M, N, Kd):
         assert torch.equal(single[0], out[M - 1])
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
+@pytest.mark.parametrize("stride,offset", [(0, 0), (1, 0), (4, 0), (8, 3)], ids=["whole", "odd", "half", "off"])
+@pytest.mark.parametrize("M,N,Kd", [(2500, 250, 72), (2500, 200, 64), (300, 200, 72), (300, 24, 72), (200, 264, 128), (129, 300, 64)])
+def test_gemm_tcgen05_stores(out_dtype, M, N, Kd, stride, offset):
+    """Tiles of 128, 32 and 256 columns, several side by side, whole lines followed by a partial group of columns, into rows that are
+    16-byte aligned, here and there or nowhere: float32 sums of K products within K 2^-24 of the products' sizes (bfloat16: 2^-8 of
+    the result more), and what lies around them stays."""
+    x, w = rnd(M, Kd, dtype=torch.bfloat16, seed=15), rnd(N, Kd, dtype=torch.bfloat16, seed=16)
+    width = -(-N // 8) * 8 + 8 + stride
+    room = torch.full((M, width), 7.0, dtype=out_dtype, device=DEV)
+    K().gemm_tc(x, w, room[:, offset:offset + N])
+    torch.cuda.synchronize()
+    K().check_error_flag()
+    want, sizes = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0)
+    assert ((room[:, offset:offset + N].double() - want).abs() <= bound).all()
+    assert (room[:, :offset] == 7.0).all() and (room[:, offset + N:] == 7.0).all()
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,Kd", [(1, 130, 64), (8, 4096, 4096), (5, 6144, 1024), (16, 1000, 192), (9, 331, 128),
                                     (3, 24576, 512), (8, 40000, 256), (2, 7, 64), (17, 4096, 256), (32, 5120, 512),
