@@ -105,7 +105,8 @@ class LatentAttention(Mixer):
         self.formed_keys = (kernels.latent_prompt_keys(self.dim, self.rot_dim, self.vdim, self.kv_rank)
                             if formed and self.w_o.is_cuda and self.w_o.dtype == torch.bfloat16 else 0)
         if self.formed_keys:
-            self.w_ukv = torch.cat([get(f"{p}.uk", "matrix"), get(f"{p}.uv", "matrix")], dim=0).contiguous()
+            self.w_ukv = torch.cat([get(f"{p}.uk", "matrix"), self.w_uv.view(H * self.vdim, self.kv_rank)], dim=0)
+            self.w_uv = self.w_ukv[H * self.dim:].view(H, self.vdim, self.kv_rank)      # held once
         if self.own_rows:
             self.c_norm = get(f"{p}.dkv.norm", "vector").contiguous()
         if self.sink:

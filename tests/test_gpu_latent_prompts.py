@@ -111,6 +111,24 @@ def test_formed_portions_beside_decoded_tokens_and_short_portions(tmp_path, monk
     assert calls["formed"] == 0
 
 
+def _mixer(heads, rank, seed=1):
+    from llm_pipeline_b200.parts import lookup
+    part = lookup("mixer", "latent_attention")("p", hidden_size=64, num_heads=heads, dim=64, rot_dim=32, vdim=64, kv_rank=rank,
+                                               scale=96 ** -0.5, norm_eps=1e-5)
+    gen = torch.Generator().manual_seed(seed)
+    weights = {name: torch.randn(spec.shape, generator=gen).to(DEV, torch.bfloat16) for name, spec in part.param_specs().items()}
+    part.load(lambda name, role: weights[name])
+    return part, weights
+
+
+def test_the_maps_of_the_values_are_held_once():
+    part, weights = _mixer(4, 128)
+    assert part.formed_keys
+    assert torch.equal(part.w_ukv, torch.cat([weights["p.uk"], weights["p.uv"]]))
+    assert torch.equal(part.w_uv, weights["p.uv"].view(4, 64, 128)) and part.w_uv.is_contiguous()
+    assert part.w_uv.untyped_storage().data_ptr() == part.w_ukv.untyped_storage().data_ptr()
+
+
 @pytest.mark.parametrize("sink", [False, True], ids=["", "sink"])
 @pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (3, 128, 16), (17, 256, 32), (33, 384, 64)], ids=str)
 @pytest.mark.parametrize("ctx", [(1, 127, 128, 129), (64, 65, 4096), (777,)], ids=str)
