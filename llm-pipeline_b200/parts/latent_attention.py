@@ -159,7 +159,8 @@ class LatentAttention(Mixer):
             return None
         keys, per_tile = self.formed_keys, kernels.latent_mma_tokens_per_tile(self.num_heads)
         width = self.num_heads * (self.dim + self.vdim)
-        key = ("latent_attention_formed", keys, per_tile, width)
+        # (all sizes that the choice of requests and the tiles follow from)
+        key = ("latent_attention_formed", keys, per_tile, self.num_heads, self.kv_rank, self.dim, self.rot_dim, self.vdim)
         if key in ctx.memo:
             return ctx.memo[key]
         taken = self._formed_requests(ctx)

@@ -129,6 +129,24 @@ def test_the_maps_of_the_values_are_held_once():
     assert part.w_uv.untyped_storage().data_ptr() == part.w_ukv.untyped_storage().data_ptr()
 
 
+def test_layers_of_other_sizes_choose_for_themselves():
+    """A portion worth a second path beside a long context in a layer of large latents and not in one of small: each layer of a step
+    chooses by its own sizes, whichever comes first."""
+    from llm_pipeline_b200.engine.context import StepContext
+    large, small = _mixer(16, 1024)[0], _mixer(16, 128)[0]
+
+    def context():
+        ctx = StepContext(torch.device(DEV), torch.bfloat16)
+        ctx.q_lens, ctx.starts, ctx.max_q_len = [1100, 100], [0, 5000], 1100
+        return ctx
+
+    alone = [part._formed_plan(context()) is not None for part in (large, small)]
+    assert alone == [True, False]
+    for order in ((large, small), (small, large)):
+        ctx = context()
+        assert [part._formed_plan(ctx) is not None for part in order] == [part is large for part in order]
+
+
 @pytest.mark.parametrize("sink", [False, True], ids=["", "sink"])
 @pytest.mark.parametrize("heads,rank,rot", [(16, 512, 64), (3, 128, 16), (17, 256, 32), (33, 384, 64)], ids=str)
 @pytest.mark.parametrize("ctx", [(1, 127, 128, 129), (64, 65, 4096), (777,)], ids=str)
