@@ -42,6 +42,15 @@ from .base import LayerCache, Mixer, TensorGetter
 from .registry import register_mixer
 
 
+def _by_run(runs, rows, weights, out) -> None:
+    """Per head ``out`` = ``rows`` x ``weights``^T, both [tokens, heads, ..], for the runs of rows (first, end); None: for all of them."""
+    if runs is None:
+        batched_linear(rows.transpose(0, 1), weights, out.transpose(0, 1))
+        return
+    for first, end in runs:
+        batched_linear(rows[first:end].transpose(0, 1), weights, out[first:end].transpose(0, 1))
+
+
 @register_mixer("latent_attention")
 class LatentAttention(Mixer):
     graph_safe = True      # a step only writes this step's cache rows: repeating it changes nothing
@@ -273,19 +282,17 @@ class LatentAttention(Mixer):
             q = q.view(N, H, self.dim + rot)
         values = torch.empty((N, H, self.vdim), dtype=x.dtype, device=x.device)
         plan = self._formed_plan(ctx)
-        runs, some = [(0, N)], None
+        runs, some = None, None                              # None: all rows (and no views of them, a microsecond of the host's each)
         if plan is not None:
             self._formed(ctx, plan, q, values, cache)
             runs = plan[2]
             some = (*plan[3:], (runs[0][0], runs[-1][1])) if runs else None
-        if runs:
+        if runs is None or runs:
             q_lat = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
-            for first, end in runs:
-                batched_linear(q[first:end, :, :self.dim].transpose(0, 1), self.w_uk_t, q_lat[first:end].transpose(0, 1))
+            _by_run(runs, q[:, :, :self.dim], self.w_uk_t, q_lat)
             mixed = torch.empty((N, H, rank), dtype=x.dtype, device=x.device)
             self.attend(ctx, q_lat, q[:, :, self.dim:], mixed, cache, some)
-            for first, end in runs:
-                batched_linear(mixed[first:end].transpose(0, 1), self.w_uv, values[first:end].transpose(0, 1))
+            _by_run(runs, mixed, self.w_uv, values)
         values = values.view(N, H * self.vdim)
         if gate is not None:
             kernels.sigmoid_gate(values, gate)
