@@ -11,8 +11,9 @@
 // out has the compute type. Between steps a request keeps S in its state slot, as two copies [inner][states] that take
 // turns by the parity of the last position written, so a step of one token never overwrites what it read.
 //
-// Two forms. Where some request brings more than one token, the output is bfloat16 and a channel has up to 32 state entries:
-// segments of SEG_TOKENS tokens side by side (below, at `SegArgs`). Else, token by token: a block is one warp and takes 32 / L
+// Two forms. Steps whose longest portion is long (the caller's rule: above 288 tokens), where the output is bfloat16 and a channel has
+// up to 32 state entries: segments of SEG_TOKENS tokens side by side, for all requests of the step (below, at `SegArgs`). Else,
+// token by token: a block is one warp and takes 32 / L
 // channels of one request: L lanes share a channel and hold NS state entries each (entry n = k L + lane, so the lanes read
 // neighbouring words), the sum over n ends with log2(L) shuffles. The request's tokens are walked in chunks of 8 with the next
 // chunks on their way while this one is worked on: the B and C rows of three chunks by asynchronous copies into a ring of
@@ -21,7 +22,7 @@
 // it, the lanes taking a chunk's tokens in turn, so it costs a chunk one pass and not eight; the walk gets a token's step size
 // from its lane by a shuffle. The chain itself is one multiply-add per token and entry. Where the output is bfloat16 they use
 // the special-function unit's exponential and logarithm. L and NS follow from `states` alone, so a row's operations do not
-// depend on the step.
+// depend on the step as long as its form does not; between the forms rows and state differ at rounding level.
 #include "common.cuh"
 
 namespace {
@@ -222,7 +223,7 @@ void launch_scan(const ScanArgs& a, int out_dtype, int R, cudaStream_t stream) {
 // Token by token, a prompt was one chain of 2,048 steps with 110 instructions a token and warp of two channels, most of them
 // spent on what 16 lanes share. Here a thread holds a whole channel, so a token's step size, gate and sum over the entries
 // cost once and the entries' multiply-adds go two at a time; the bound is then the special-function unit (an exponential per
-// token and entry, in 1 and in 3: busy for 71 and 59 % of these launches). 2,048 tokens of 4,096 channels with 16 entries: 641 us
+// token and entry, in 1 and in 3: busy for 72 and 59 % of these launches). 2,048 tokens of 4,096 channels with 16 entries: 641 us
 // token by token, 126 so (51, 18 and 68 with cold caches). Tried: three pairs of eight exponentials as polynomials on the
 // multiply-add pipe (137 us), segments of 96 tokens (128), loads two tokens ahead (133), seven blocks an SM (126).
 constexpr int SEG_TOKENS = 64;
