@@ -541,7 +541,8 @@ LLMP_API long llmp_delta_chunks_scratch(int rows, int R, int H, int d, int dv) {
 LLMP_API int llmp_delta_chunks(float* q, long q_t, float* k, long k_t, const float* v, long v_t, float* decay, long decay_t,
                                float* beta, long beta_t, const float* a_log, const float* dt_bias, float* state, long state_slot,
                                long state_half, const int* q_start, const int* slots, const int* positions, float* o, long o_t, void* scratch,
-                               long scratch_bytes, const int* list, int count, int rows, const int* token_request, int max_tokens, int tokens, int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
+                               long scratch_bytes, const int* list, int count, int rows, const int* token_request, int max_tokens, int tokens,
+                               int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
     if (R <= 0 || tokens <= 0) return 0;
     LLMP_REQUIRE(rows > 0 && rows <= tokens && count > 0 && count <= R && (list ? token_request != nullptr : count == R && rows == tokens),
                  "delta_chunks: %d of %d requests, %d of %d tokens", count, R, rows, tokens);
@@ -553,13 +554,14 @@ LLMP_API int llmp_delta_chunks(float* q, long q_t, float* k, long k_t, const flo
     DeltaChunkArgs a;
     a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.v = v; a.v_t = v_t; a.decay = decay; a.decay_t = decay_t; a.beta = beta; a.beta_t = beta_t;
     a.a_log = a_log; a.dt_bias = dt_bias; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
-    a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.scratch = (unsigned char*)scratch; a.list = list; a.requests = count; a.H = H; a.G = G; a.dv = dv;
-    a.error_flag = error_flag;
+    a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.scratch = (unsigned char*)scratch; a.list = list; a.requests = count;
+    a.H = H; a.G = G; a.dv = dv; a.error_flag = error_flag;
     const int chunks = (rows - 1) / DC_TOKENS + count;
     if (d == 64) launch_chunks<1>(a, chunks, stream);
     else launch_chunks<2>(a, chunks, stream);
     if (list) {
-        const int failed = llmp_delta_prep(q, q_t, k, k_t, decay, decay_t, beta, beta_t, a_log, dt_bias, token_request, q_start, max_tokens, tokens, H, G, d, stream);
+        const int failed = llmp_delta_prep(q, q_t, k, k_t, decay, decay_t, beta, beta_t, a_log, dt_bias, token_request, q_start, max_tokens, tokens,
+                                           H, G, d, stream);
         if (failed) return failed;
         return llmp_delta_scan(q, q_t, k, k_t, v, v_t, decay, decay_t, beta, beta_t, state, state_slot, state_half, q_start, slots, positions, o, o_t,
                                max_tokens, R, H, G, d, dv, stream);

@@ -17,8 +17,8 @@
 // mix alone, 4,096 clocks of an SM; as a product it moves 100 KB. 2,048 tokens of 16 heads of 128: 285 us before, 197 with the
 // product, 168 with tanh as a series where the scores are far below the cap, exponentials and reciprocals without their range
 // checks, masks only where a row's end is near, and a tile's places found a tile ahead (three pieces instead of two: a layer 230
-// -> 240). What is left is the latency of four phases between barriers at four warps a scheduler (issue slots 44 %, tensor pipe 30 %). Shorter key ranges (512, 256 keys) lose
-// to their partial sums: 205, 222 us against 197.
+// -> 240). What is left is the latency of four phases between barriers at four warps a scheduler (issue slots 44 %, tensor
+// pipe 30 %). Shorter key ranges (512, 256 keys) lose to their partial sums: 205, 222 us against 197.
 #include "common.cuh"
 
 namespace {

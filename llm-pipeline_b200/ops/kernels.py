@@ -1669,8 +1669,8 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
 # beside the walks of the step's other requests, while the two launches more for both forms cost the host 5 to 9 us. 8 decoded tokens with
 # a portion of 128, of 200, of 300: walked 165, 190, 260 us a layer, the portion in chunks 174, 177, 179 (a layer of half the size
 # 165, 170, 183 and 174, 173, 173). 64 decoded tokens with a portion of 64, of 128, of 300: walked 222, 255, 356, the portion in
-# chunks 238, 246, 282; all of them in chunks 281, 289, 333, since a block of the chain fills an SM for a token's sake. The chunks' operands take 47 KB each at heads of 128 x 128 (of 16
-# heads, 15,600 tokens in 704 MB).
+# chunks 238, 246, 282; all of them in chunks 281, 289, 333, since a block of the chain fills an SM for a token's sake.
+# The chunks' operands take 47 KB each at heads of 128 x 128 (of 16 heads, 15,600 tokens in 704 MB).
 DELTA_CHUNKS_MIN_TOKENS = 160
 DELTA_CHUNKS_MAX_BYTES = 704 << 20
 

@@ -6,19 +6,21 @@ With h the mixer's input, H heads, per head ``dim`` unrotated and ``rot_dim`` ro
     q = Wq h                                  per head [dim | rot_dim]; the rot_dim part is rotated by the position
     [l | k_r] = Wdkv h                        kv_rank + rot_dim entries
     c = rms_norm(l) * w_c                     the latent; k_r is rotated by the position and shared by all heads
-    k_h = Wuk_h c,  v_h = Wuv_h c             never formed: see below
+    k_h = Wuk_h c,  v_h = Wuv_h c             formed for long prompt portions only: see below
     score_h(i, j) = (q_h,plain(i) . k_h(j) + q_h,rot(i) . k_r(j)) * scale,  j <= i,  softmax over j
     out = Wo concat_h(sum_j p_h(i, j) v_h(j))
 
 Only ``[c | k_r]`` is cached (``TokenPagesSpec``: one row of kv_rank + rot_dim entries per token). Both up-projections
 are linear, so they move to the query's side: ``q_h,plain . (Wuk_h c) = (Wuk_h^T q_h,plain) . c`` and
 ``sum_j p_j (Wuv_h c_j) = Wuv_h (sum_j p_j c_j)``. Every head then attends over the same cached rows, with a query of
-kv_rank + rot_dim entries and the rows' first kv_rank entries as values, in prompts and in decoding alike; the two maps
-are one batched product over the heads before and after the attention kernel. Scores, softmax, norm and angles are
+kv_rank + rot_dim entries and the rows' first kv_rank entries as values; the two maps are one batched product over the
+heads before and after the attention kernel. Scores, softmax, norm and angles are
 float32. ``rot_dims`` (<= rot_dim) entries of the rotated parts take the rotation, the rest pass unchanged.
 
 Long prompt portions in bfloat16 take the other order (``_formed_plan``): k_h and v_h of the request's rows are formed by one product
-and attended over as they are, which costs a (query, key, head) dim + rot + vdim multiply-adds instead of 2 kv_rank + rot.
+and attended over as they are, which costs a (query, key, head) dim + rot + vdim multiply-adds instead of 2 kv_rank + rot. Which
+requests do, and into how many ranges a decoded token's keys are cut, follows from the whole step, so that a row can differ at
+rounding level between steps.
 
 Options that other designs of this family use (all off by default): the queries through a normed latent of their own
 (``q_rank``: ``c_q = rms_norm(Wdq h) * w_q``, ``q = Wuq c_q``), a learned sink per head in the softmax's denominator, a

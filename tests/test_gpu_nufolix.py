@@ -189,8 +189,8 @@ def test_gated_delta_rule_alone(sizes):
 @pytest.mark.parametrize("sizes", [(4, 2, 64, 48, 0.0), (2, 2, 128, 128, -3.0), (3, 1, 128, 16, 6.0)], ids=str)
 def test_gated_delta_rule_in_chunks(sizes, lengths):
     """Requests around the chunks' edges side by side, going on in a second step, in slots that are not theirs by number, with decays
-    near one, mixed and near zero, against the rule written out in float64. Factors of 16 bits (2^-17 of each at most) in three
-    products a token one after another: within 2^-14 of the largest entry. Other slots and what lies beside the state stay."""
+    near one, mixed and near zero, against the rule written out in float64: within 2^-14 of the largest entry (how near the form is
+    beyond that is measured against the walk below). Other slots and what lies beside the state stay."""
     from llm_pipeline_b200.ops import kernels
     heads, qk_heads, dim, vdim, shift = sizes
     gen = torch.Generator().manual_seed(sum(sum(n) for n in lengths) + dim + vdim)
