@@ -11,26 +11,28 @@
 // out has the compute type. Between steps a request keeps S in its state slot, as two copies [inner][states] that take
 // turns by the parity of the last position written, so a step of one token never overwrites what it read.
 //
-// Two forms. Steps whose longest portion is long (the caller's rule: above 288 tokens), where the output is bfloat16 and a channel has
-// up to 32 state entries: segments of SEG_TOKENS tokens side by side, for all requests of the step (below, at `SegArgs`). Else,
-// token by token: a block is one warp and takes 32 / L
-// channels of one request: L lanes share a channel and hold NS state entries each (entry n = k L + lane, so the lanes read
-// neighbouring words), the sum over n ends with log2(L) shuffles. The request's tokens are walked in chunks of 8 with the next
-// chunks on their way while this one is worked on: the B and C rows of three chunks by asynchronous copies into a ring of
-// stages in shared memory, x, step sizes and gates of the next chunk as loads into registers that nothing reads before the
-// chunk's turn. What a token needs once (its loads, the softplus, the gate, the store) is done by one lane of the channel for
-// it, the lanes taking a chunk's tokens in turn, so it costs a chunk one pass and not eight; the walk gets a token's step size
-// from its lane by a shuffle. The chain itself is one multiply-add per token and entry. Where the output is bfloat16 they use
-// the special-function unit's exponential and logarithm. L and NS follow from `states` alone, so a row's operations do not
-// depend on the step as long as its form does not; between the forms rows and state differ at rounding level.
+// G lanes share a channel and hold E neighbouring state entries each; the lanes' sums are added in one fixed order. G and E follow
+// from `states` alone and the first two forms do the same operations in the same order, so a row and the state after it have the same
+// bits in any company.
+//   step: requests of a single token. A thread loads its entries, takes the step and stores them: the state is read and written once
+//         (8 requests of 4,096 channels with 16 entries 3.5 us; 17.9 as a walk).
+//   walk: a block takes a request and the channels of its walking warps, token by token. A walk needs each exponential once (segments
+//         twice), so the special-function unit would be done with 2,048 tokens of 4,096 channels in 37 us; what keeps a walk from that
+//         is that a scheduler has one or two warps of it, which wait for every instruction's result. So whatever the chain does not
+//         need is other warps' work (copies into a ring, step sizes and gates of the stages to come, the sums over a channel's lanes and
+//         the outputs of the stage behind; they meet the walkers at one barrier a stage), and a walker's turn of SS_RUN tokens mixes
+//         three: the chain over one run, the decays of the next, the loads of the one after. Microseconds, before and after: 2,048
+//         tokens of 4,096 channels 117 (segments) and 94, of 2,048 channels 84 and 54; 100 tokens 33 and 9; 203 in float64 68 and 31;
+//         64 single tokens beside 300 102 and 57. On the way: all of it in one warp 209 and 149, sums by shuffles among the walkers 155
+//         and 106, stages of 16 tokens 109 and 84, two warps for step sizes and gates 104 and 74.
+//   segments: few channels and many tokens in bfloat16 (below).
 #include "common.cuh"
 
 namespace {
 
-constexpr int SS_THREADS = 32;
-constexpr int SS_CHUNK = 8;
-constexpr int SS_AHEAD = 3;                // chunks whose inputs are under way beside the one at work
-constexpr int SS_STAGES = SS_AHEAD + 1;
+constexpr int SS_RUN = 4;                  // tokens of a turn of the walk
+// threads of a block that walk; then come a warp that copies, four for step sizes and gates, two for the outputs
+template <int G> constexpr int SS_WALKERS = G < 8 ? 64 : 128;
 
 struct ScanArgs {
     const float* x; long x_t;
@@ -43,189 +45,469 @@ struct ScanArgs {
     float* state; long state_slot; long state_half;
     const int* q_start; const int* slots; const int* positions;
     void* out; long out_t;
-    int inner, states, L;
+    int inner, states;
+    int singles;                          // 1: the walk leaves requests of one token to the step kernel
 };
 
-// the recurrence's arithmetic in the accumulator's type: exact library functions for float64 (the true 32-bit path), the
-// special-function unit for float32 (the bfloat16 path, whose products carry 8 bits)
-__device__ __forceinline__ double ss_exp(double v) { return exp(v); }
-__device__ __forceinline__ float ss_exp(float v) { return __expf(v); }
+// The arithmetic in the accumulator's type: exact library functions for float64 (the true 32-bit path), the special-function
+// unit for float32 (the bfloat16 path, whose products carry 8 bits). Decays: 2 to the power of the step size times A log2(e) there.
 __device__ __forceinline__ double ss_softplus(double v) { return v > 20.0 ? v : log1p(exp(v)); }
 __device__ __forceinline__ float ss_softplus(float v) { return v > 15.f ? v : __logf(1.f + __expf(v)); }
+__device__ __forceinline__ float ss_gate(float z, double) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float ss_gate(float z, float) { return __fdividef(z, 1.f + __expf(-z)); }
+constexpr float LOG2_E = 1.4426950408889634f;
+__device__ __forceinline__ double ss_rate(float a, double) { return (double)a; }
+__device__ __forceinline__ float ss_rate(float a, float) { return a * LOG2_E; }
 
-__device__ __forceinline__ void ss_cp_async_4(float* smem_dst, const float* gmem_src) {
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(gmem_src) : "memory");
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ float ex2(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
+    return r;
 }
 
-template <typename T, typename ACC, int L, int NS>
-__global__ void __launch_bounds__(SS_THREADS) selective_scan_kernel(const ScanArgs a) {
-    extern __shared__ float bc_s[];                            // the ring: SS_STAGES stages of a chunk's inputs
-    pdl_wait();                                    // what the kernels before wrote is complete
-    pdl_trigger();
-    constexpr int OWN = (SS_CHUNK + L - 1) / L;                // tokens of a chunk that a lane looks after
-    const int r = blockIdx.x;
-    const int Nst = a.states;
-    constexpr int per_block = SS_THREADS / L;
-    const int c = blockIdx.y * per_block + threadIdx.x / L;
-    const int l = threadIdx.x % L;
+// A token's decays of a lane's E entries and what it adds to them; then S <- decay S + add, and the lane's share of sum S C.
+template <int E>
+__device__ __forceinline__ void ss_decays(const float (&A)[E], float dt, float dx, const float* b, float (&decay)[E], float (&add)[E]) {
+    const float2 dt2 = make_float2(dt, dt), dx2 = make_float2(dx, dx);
+#pragma unroll
+    for (int e = 0; e < E; e += 2) {
+        const float2 p = mul2(dt2, make_float2(A[e], A[e + 1])), q = mul2(dx2, make_float2(b[e], b[e + 1]));
+        decay[e] = ex2(p.x); decay[e + 1] = ex2(p.y);
+        add[e] = q.x; add[e + 1] = q.y;
+    }
+}
+template <int E>
+__device__ __forceinline__ float ss_advance(float (&S)[E], const float (&decay)[E], const float (&add)[E], const float* c) {
+    float2 y = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < E; e += 2) {
+        const float2 s = fma2(make_float2(decay[e], decay[e + 1]), make_float2(S[e], S[e + 1]), make_float2(add[e], add[e + 1]));
+        S[e] = s.x; S[e + 1] = s.y;
+        y = e ? fma2(s, make_float2(c[e], c[e + 1]), y) : mul2(s, make_float2(c[e], c[e + 1]));
+    }
+    return y.x + y.y;
+}
+template <int E>
+__device__ __forceinline__ void ss_decays(const double (&A)[E], double dt, double dx, const float* b, double (&decay)[E], double (&add)[E]) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        decay[e] = exp(dt * A[e]);
+        add[e] = dx * (double)b[e];
+    }
+}
+template <int E>
+__device__ __forceinline__ double ss_advance(double (&S)[E], const double (&decay)[E], const double (&add)[E], const float* c) {
+    double y = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        S[e] = fma(decay[e], S[e], add[e]);
+        y = fma(S[e], (double)c[e], y);
+    }
+    return y;
+}
+__device__ __forceinline__ void ss_pair(const unsigned char* p, float (&d)[2]) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    d[0] = v.x; d[1] = v.y;
+}
+__device__ __forceinline__ void ss_pair(const unsigned char* p, double (&d)[2]) {
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    d[0] = v.x; d[1] = v.y;
+}
+
+__device__ __forceinline__ void ss_put2(unsigned char* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void ss_put2(unsigned char* p, double a, double b) { *reinterpret_cast<double2*>(p) = make_double2(a, b); }
+// A lane's sums of a run's tokens, and the sums of them over the G lanes of a channel, in the order of ss_reduce.
+__device__ __forceinline__ void ss_put(unsigned char* p, const float (&v)[SS_RUN]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void ss_put(unsigned char* p, const double (&v)[SS_RUN]) {
+    ss_put2(p, v[0], v[1]);
+    ss_put2(p + 16, v[2], v[3]);
+}
+__device__ __forceinline__ void ss_get(const unsigned char* p, float (&v)[SS_RUN]) {
+    const float4 u = *reinterpret_cast<const float4*>(p);
+    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+}
+__device__ __forceinline__ void ss_get(const unsigned char* p, double (&v)[SS_RUN]) {
+    const double2 u = *reinterpret_cast<const double2*>(p), w = *reinterpret_cast<const double2*>(p + 16);
+    v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
+}
+template <int G, typename ACC> __device__ __forceinline__ void ss_gather(const unsigned char* p, ACC (&y)[SS_RUN]) {
+    constexpr int PITCH = SS_RUN * sizeof(ACC);
+    ACC v[G / 2][SS_RUN];
+#pragma unroll
+    for (int i = 0; i < G / 2; ++i) {
+        ACC u[SS_RUN];
+        ss_get(p + i * PITCH, v[i]);
+        ss_get(p + (i + G / 2) * PITCH, u);
+#pragma unroll
+        for (int t = 0; t < SS_RUN; ++t) v[i][t] += u[t];
+    }
+#pragma unroll
+    for (int w = G / 4; w > 0; w >>= 1)
+#pragma unroll
+        for (int i = 0; i < w; ++i)
+#pragma unroll
+            for (int t = 0; t < SS_RUN; ++t) v[i][t] += v[i + w][t];
+#pragma unroll
+    for (int t = 0; t < SS_RUN; ++t) y[t] = v[0][t];
+}
+template <int G, typename ACC> __device__ __forceinline__ ACC ss_reduce(ACC y) {
+#pragma unroll
+    for (int w = G >> 1; w > 0; w >>= 1) y += __shfl_xor_sync(0xffffffffu, y, w);
+    return y;
+}
+
+// Entry e of a lane's E neighbours at `p`; `have` of them exist, the others read 0.
+template <int E, typename ACC>
+__device__ __forceinline__ void ss_load(ACC (&v)[E], const float* p, int have) {
+    if (have >= E && (uintptr_t)p % (E < 4 ? 8 : 16) == 0) {
+        if (E == 2) {
+            const float2 u = *reinterpret_cast<const float2*>(p);
+            v[0] = u.x; v[1] = u.y;
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; e += 4) {
+                const float4 u = *reinterpret_cast<const float4*>(p + e);
+                v[e] = u.x; v[(e + 1) % E] = u.y; v[(e + 2) % E] = u.z; v[(e + 3) % E] = u.w;
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = e < have ? p[e] : 0.f;
+}
+template <int E, typename ACC>
+__device__ __forceinline__ void ss_store(const ACC (&v)[E], float* p, int have) {
+    if (have >= E && (uintptr_t)p % (E < 4 ? 8 : 16) == 0) {
+        if (E == 2) {
+            *reinterpret_cast<float2*>(p) = make_float2((float)v[0], (float)v[1]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; e += 4)
+                *reinterpret_cast<float4*>(p + e) = make_float4((float)v[e], (float)v[(e + 1) % E], (float)v[(e + 2) % E], (float)v[(e + 3) % E]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+        if (e < have) p[e] = (float)v[e];
+}
+
+
+// A request's single token.
+template <typename T, typename ACC, int G, int E>
+__global__ void __launch_bounds__(SS_WALKERS<G>) selective_step_kernel(const ScanArgs a) {
+    constexpr int CH = SS_WALKERS<G> / G;
+    const int r = blockIdx.x, l = threadIdx.x % G;
+    const int c = blockIdx.y * CH + threadIdx.x / G;
     const bool ok = c < a.inner;
-    const int begin = a.q_start[r], end = a.q_start[r + 1];
-    if (end <= begin) return;
-    const int p0 = a.positions[begin];
-    float* slot = a.state + (size_t)a.slots[r] * a.state_slot;
-    const float* rd = slot + ((p0 + 1) & 1) * a.state_half;
-    float* wr = slot + ((p0 + end - begin - 1) & 1) * a.state_half;
-    ACC S[NS];
-    float A[NS];
+    const int cc = ok ? c : 0, have = ok ? a.states - l * E : 0;
+    float rate[E];
+    ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);           // weights: nothing of the step writes them
+    const float bias = a.dt_bias[cc], Dc = a.D[cc];
+    pdl_wait();
+    pdl_trigger();
+    const int t = a.q_start[r];
+    if (a.q_start[r + 1] - t != 1) return;
+    const int p0 = a.positions[t];
+    float* slot = a.state + (size_t)a.slots[r] * a.state_slot + (size_t)cc * a.states + l * E;
+    ACC S[E], A[E];
+    ss_load<E>(S, slot + ((p0 + 1) & 1) * a.state_half, have);
+    float b[E], k[E];
+    ss_load<E>(b, a.B + (size_t)t * a.bc_t + l * E, a.states - l * E);
+    ss_load<E>(k, a.C + (size_t)t * a.bc_t + l * E, a.states - l * E);
+    const float x = a.x[(size_t)t * a.x_t + cc], raw = a.dt[(size_t)t * a.dt_t + cc];
+    const float z = a.z ? a.z[(size_t)t * a.z_t + cc] : 0.f;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        const int n = k * L + l;
-        const bool have = ok && n < Nst;
-        S[k] = have ? (ACC)rd[(size_t)c * Nst + n] : (ACC)0;
-        A[k] = have ? a.A[(size_t)c * Nst + n] : 0.f;
+    for (int e = 0; e < E; ++e) A[e] = ss_rate(rate[e], ACC());
+    const ACC dt = ss_softplus((ACC)(raw + bias));
+    ACC decay[E], add[E];
+    ss_decays<E>(A, dt, dt * (ACC)x, b, decay, add);
+    const ACC y = ss_reduce<G>(ss_advance<E>(S, decay, add, k));
+    ss_store<E>(S, slot + (p0 & 1) * a.state_half, have);
+    if (ok && l == 0) {
+        float o = (float)fma((ACC)Dc, (ACC)x, y);
+        if (a.z) o *= ss_gate(z, ACC());
+        reinterpret_cast<T*>(a.out)[(size_t)t * a.out_t + c] = from_float<T>(o);
     }
-    const float dt_b = ok ? a.dt_bias[c] : 0.f;
-    const float Dc = ok ? a.D[c] : 0.f;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void ss_copy(float* dst, const float* src, bool have) {      // not there: zeros
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int n = have ? BYTES : 0;
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;\n" ::"r"(d), "l"(src), "r"(n), "n"(BYTES) : "memory");
+}
+
+// Shared memory of a walk: a ring of stages, each the x, dt and z rows of STAGE tokens [token][channel] and their B and C in the
+// order of a channel's lanes ([token][lane][E of B | E of C]); three buffers of step sizes [channel][token] (step size, step size
+// times x); two of the lanes' sums [run][channel][lane][SS_RUN tokens]. The pitches spread a warp's channels over the banks.
+template <typename ACC, int G, int E> struct ScanSmem {
+    static constexpr int CH = SS_WALKERS<G> / G, P = G * E;
+    static constexpr int STAGE = P > 64 || CH > 16 ? 16 : 32;  // tokens; two blocks an SM where that can be
+    static constexpr int STAGES = 5;                           // one walked, one behind it, two before it, one under way
+    static constexpr int ROWS = STAGE * CH;
+    static constexpr int STAGE_FLOATS = 3 * ROWS + STAGE * 2 * P;
+    static constexpr int STEP_PITCH = STAGE * 2 * (int)sizeof(ACC) + 16;          // bytes
+    static constexpr int SUM_PITCH = G * SS_RUN * (int)sizeof(ACC) + 16, SUM_BYTES = STAGE / SS_RUN * CH * SUM_PITCH;
+    static constexpr size_t BYTES = (size_t)STAGES * STAGE_FLOATS * 4 + 3 * CH * STEP_PITCH + 2 * SUM_BYTES;
+};
+
+// WIDE: x, dt and z rows may be copied by 16 bytes (alignment, and `inner` a multiple of the block's channels), B and C by E floats.
+// Requests of a single token are left to the step kernel where `singles` says that it runs too.
+template <typename T, typename ACC, int G, int E, bool WIDE>
+__global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 4 ? 2 : 1) selective_walk_kernel(const ScanArgs a) {
+    typedef ScanSmem<ACC, G, E> L;
+    constexpr int CH = L::CH, P = L::P, STAGE = L::STAGE;
+    extern __shared__ __align__(16) float ss_smem[];
+    unsigned char* const steps = reinterpret_cast<unsigned char*>(ss_smem + L::STAGES * L::STAGE_FLOATS);
+    unsigned char* const sums = steps + 3 * CH * L::STEP_PITCH;
+    const int r = blockIdx.x, tid = threadIdx.x, c0 = blockIdx.y * CH;
+    pdl_wait();                                                // what the kernels before wrote is complete
+    pdl_trigger();
+    const int begin = a.q_start[r], n = a.q_start[r + 1] - begin;
+    if (n <= a.singles) return;
+    const int stages = (n + STAGE - 1) / STAGE;
+
+    if (tid < SS_WALKERS<G>) {
+        const int l = tid % G, lc = tid / G, c = c0 + lc;      // lane of its channel, channel of the block
+        const bool ok = c < a.inner;
+        const int cc = ok ? c : 0, have = ok ? a.states - l * E : 0;
+        const int p0 = a.positions[begin];
+        float* slot = a.state + (size_t)a.slots[r] * a.state_slot + (size_t)cc * a.states + l * E;
+        ACC S[E], A[E];
+        {
+            float rate[E];
+            ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);
+#pragma unroll
+            for (int e = 0; e < E; ++e) A[e] = ss_rate(rate[e], ACC());
+        }
+        ss_load<E>(S, slot + ((p0 + 1) & 1) * a.state_half, have);
+        // In turn j: decays of run j + 1, the chain over run j, the rows of run j + 2 from shared memory. Nothing in a turn waits for
+        // another part of it. Two sets of registers take turns.
+        ACC decay[2][SS_RUN][E], add[2][SS_RUN][E], step[2][SS_RUN][2];
+        float rows[2][SS_RUN][2 * E];                          // B | C
+        const float* const bc0 = ss_smem + 3 * L::ROWS + l * 2 * E;
+        const unsigned char* const step0 = steps + lc * L::STEP_PITCH;
+        unsigned char* const sum0 = sums + lc * L::SUM_PITCH + l * SS_RUN * sizeof(ACC);
+        constexpr int RUN_BC = SS_RUN * 2 * P, RUN_STEP = SS_RUN * 2 * (int)sizeof(ACC), RUN_SUM = CH * L::SUM_PITCH;
+        auto fetch = [&](int set, const float* bc, const unsigned char* st) {
+#pragma unroll
+            for (int t = 0; t < SS_RUN; ++t) {
+                ss_pair(st + t * 2 * sizeof(ACC), step[set][t]);
+                const float4* at = reinterpret_cast<const float4*>(bc + t * 2 * P);
+#pragma unroll
+                for (int i = 0; i < E / 2; ++i) {
+                    const float4 w = at[i];
+                    rows[set][t][4 * i] = w.x; rows[set][t][4 * i + 1] = w.y; rows[set][t][4 * i + 2] = w.z; rows[set][t][4 * i + 3] = w.w;
+                }
+            }
+        };
+        auto decays = [&](int set) {
+#pragma unroll
+            for (int t = 0; t < SS_RUN; ++t) ss_decays<E>(A, step[set][t][0], step[set][t][1], rows[set][t], decay[set][t], add[set][t]);
+        };
+        __syncthreads();                                       // the first stages are in
+        __syncthreads();                                       // and the first two's step sizes there
+        fetch(0, bc0, step0);
+        fetch(1, bc0 + RUN_BC, step0 + RUN_STEP);
+        decays(0);
+        int ring = 0, buffer = 0;                              // of this stage
+        for (int s = 0; s < stages; ++s) {
+            const int ring1 = ring + 1 == L::STAGES ? 0 : ring + 1, buffer1 = buffer == 2 ? 0 : buffer + 1;
+            const float* bc = bc0 + ring * L::STAGE_FLOATS;
+            const unsigned char* st = step0 + buffer * CH * L::STEP_PITCH;
+            unsigned char* to = sum0 + (s & 1) * L::SUM_BYTES;
+#pragma unroll 1
+            for (int t0 = 0; t0 < min(STAGE, n - s * STAGE); t0 += 2 * SS_RUN) {
+                const bool last = t0 + 2 * SS_RUN == STAGE;    // then the runs to fetch are the next stage's first two
+                bc = last ? bc0 + ring1 * L::STAGE_FLOATS : bc + 2 * RUN_BC;
+                st = last ? step0 + buffer1 * CH * L::STEP_PITCH : st + 2 * RUN_STEP;
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    ACC part[SS_RUN];
+                    decays(u ^ 1);
+#pragma unroll
+                    for (int t = 0; t < SS_RUN; ++t) part[t] = ss_advance<E>(S, decay[u][t], add[u][t], rows[u][t] + E);
+                    fetch(u, bc + u * RUN_BC, st + u * RUN_STEP);
+                    ss_put(to, part);
+                    to += RUN_SUM;
+                }
+            }
+            ring = ring1;
+            buffer = buffer1;
+            __syncthreads();
+        }
+        ss_store<E>(S, slot + ((p0 + n - 1) & 1) * a.state_half, have);
+        return;
+    }
+
     const bool gated = a.z != nullptr;
-    T* out = reinterpret_cast<T*>(a.out);
-    constexpr int CPW = SS_THREADS / L;                        // channels of the block
-    const int stage_floats = SS_CHUNK * 2 * Nst;               // a chunk's rows [B | C]
+    if (tid < SS_WALKERS<G> + 32) {
+        // Stage s of the ring <- its STAGE tokens; zeros past the end. A lane copies the same places of every stage: of the rows of x,
+        // dt and z the floats at xq of every xt-th token, of the rows B | C likewise.
+        const int h = tid % 32;
+        constexpr int XU = WIDE ? 4 : 1, XCOLS = CH / XU, XT = 32 / XCOLS, BU = WIDE ? (E < 4 ? E : 4) : 1, BCOLS = 2 * P / BU;
+        constexpr int BT = 32 >= BCOLS ? 32 / BCOLS : 1, BJ = BCOLS >= 32 ? BCOLS / 32 : 1;
+        const int xq = h % XCOLS * XU, x0 = h / XCOLS, b0 = h / BCOLS;
+        const bool in_x = c0 + xq < a.inner;
+        const float* px = a.x + (size_t)begin * a.x_t + (in_x ? c0 + xq : 0);
+        const float* pd = a.dt + (size_t)begin * a.dt_t + (in_x ? c0 + xq : 0);
+        const float* pz = gated ? a.z + (size_t)begin * a.z_t + (in_x ? c0 + xq : 0) : a.x;
+        const int x_t = (int)a.x_t, d_t = (int)a.dt_t, z_t = (int)a.z_t, bc_t = (int)a.bc_t;
+        auto copy_stage = [&](int s) {
+            if (s < stages) {
+                float* st = ss_smem + (s % L::STAGES) * L::STAGE_FLOATS;
+                const int t0 = s * STAGE, nt = n - t0;
+                const float* sx = px + (size_t)t0 * a.x_t;
+                const float* sd = pd + (size_t)t0 * a.dt_t;
+                const float* sz = gated ? pz + (size_t)t0 * a.z_t : pz;
+#pragma unroll
+                for (int i = 0; i < (STAGE + XT - 1) / XT; ++i) {
+                    const int t = x0 + i * XT;
+                    if (XT > STAGE && t >= STAGE) break;
+                    const bool in = t < nt && in_x;
+                    const int row = in ? t : 0;
+                    float* d = st + t * CH + xq;
+                    ss_copy<XU * 4>(d, sx + (long)row * x_t, in);
+                    ss_copy<XU * 4>(d + L::ROWS, sd + (long)row * d_t, in);
+                    if (gated) ss_copy<XU * 4>(d + 2 * L::ROWS, sz + (long)row * z_t, in);
+                }
+#pragma unroll
+                for (int i = 0; i < BJ; ++i) {
+                    const int j = h % BCOLS + i * 32, e = j % (BCOLS / 2) * BU;
+                    const bool is_c = j >= BCOLS / 2, in_e = e < a.states;
+                    const float* src = (is_c ? a.C : a.B) + (size_t)(begin + t0) * a.bc_t + (in_e ? e : 0);
+                    float* d = st + 3 * L::ROWS + e / E * 2 * E + (is_c ? E : 0) + e % E;
+#pragma unroll
+                    for (int k = 0; k < STAGE / BT; ++k) {
+                        const int t = (BCOLS <= 32 ? b0 : 0) + k * BT;
+                        const bool in = t < nt && in_e;
+                        ss_copy<BU * 4>(d + t * 2 * P, src + (long)(in ? t : 0) * bc_t, in);
+                    }
+                }
+            }
+        };
+        for (int s = 0; s < 3; ++s) copy_stage(s);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();                                       // stages 0, 1 and 2 are in
+        __syncthreads();
+        for (int s = 0; s < stages; ++s) {
+            copy_stage(s + 3);                                 // into the place of stage s - 2, whose outputs are made
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncthreads();
+        }
+        return;
+    }
 
-    // a chunk's B and C rows go to a stage of the ring by 4-byte asynchronous copies, SS_AHEAD chunks before their turn
-    auto copy_stage = [&](int t0, int nt, float* dst) {
-        for (int tt = 0; tt < nt; ++tt) {
-            for (int j = threadIdx.x; j < 2 * Nst; j += SS_THREADS)
-                ss_cp_async_4(dst + tt * 2 * Nst + j, j < Nst ? a.B + (size_t)(t0 + tt) * a.bc_t + j : a.C + (size_t)(t0 + tt) * a.bc_t + j - Nst);
+    if (tid < SS_WALKERS<G> + 160) {
+        // the step sizes of a stage, and its gates in the place of z; a token past the end has step size 0: decay 1 and nothing added
+        constexpr int PER = 128 / CH, OWN = (STAGE + PER - 1) / PER;
+        const int h = tid - SS_WALKERS<G> - 32, lc = h % CH, own = h / CH, c = c0 + lc;
+        const float bias = a.dt_bias[c < a.inner ? c : 0];
+        auto prepare = [&](int s) {
+            float* st = ss_smem + (s % L::STAGES) * L::STAGE_FLOATS + lc;
+            unsigned char* to = steps + (s % 3 * CH + lc) * L::STEP_PITCH;
+#pragma unroll
+            for (int o = 0; o < OWN; ++o) {
+                const int t = o * PER + own;
+                if (STAGE % PER && t >= STAGE) break;
+                const ACC dt = ss_softplus((ACC)(st[t * CH + L::ROWS] + bias));
+                const ACC mine = s * STAGE + t < n ? dt : (ACC)0;
+                ss_put2(to + t * 2 * sizeof(ACC), mine, mine * (ACC)st[t * CH]);
+                if (gated) st[t * CH + 2 * L::ROWS] = ss_gate(st[t * CH + 2 * L::ROWS], ACC());
+            }
+        };
+        __syncthreads();
+        prepare(0);
+        prepare(1);
+        __syncthreads();
+        for (int s = 0; s < stages; ++s) {
+            prepare(s + 2);                                    // past the last stage: of stale rows, and nobody uses it
+            __syncthreads();
         }
-        // rows past the portion's end take part in the chunk's arithmetic with step size 0: they must hold numbers
-        for (int j = nt * 2 * Nst + threadIdx.x; j < SS_CHUNK * 2 * Nst; j += SS_THREADS) dst[j] = 0.f;
+        return;
+    }
+
+    // the outputs of the stage behind: a thread takes a channel's run and adds up its lanes' sums
+    constexpr int ITEMS = CH * (STAGE / SS_RUN), OWN = (ITEMS + 63) / 64;
+    const int h = tid - SS_WALKERS<G> - 160, lc = h % CH, c = c0 + lc;
+    const bool ok = c < a.inner;
+    const float Dc = a.D[ok ? c : 0];
+    T* out = reinterpret_cast<T*>(a.out) + (size_t)begin * a.out_t + (ok ? c : 0);
+    auto finish = [&](int s) {
+        const float* st = ss_smem + (s % L::STAGES) * L::STAGE_FLOATS + lc;
+#pragma unroll
+        for (int o = 0; o < OWN; ++o) {
+            const int run = h / CH + o * (64 / CH);
+            if (ITEMS % 64 && run >= STAGE / SS_RUN) break;
+            ACC y[SS_RUN];
+            ss_gather<G>(sums + (s & 1) * L::SUM_BYTES + (run * CH + lc) * L::SUM_PITCH, y);
+            const int t0 = run * SS_RUN, at = s * STAGE + t0;
+            T* to = out + (size_t)at * a.out_t;
+#pragma unroll
+            for (int t = 0; t < SS_RUN; ++t) {
+                float v = (float)fma((ACC)Dc, (ACC)st[(t0 + t) * CH], y[t]);
+                if (gated) v *= st[(t0 + t) * CH + 2 * L::ROWS];
+                if (ok && at + t < n) to[t * a.out_t] = from_float<T>(v);
+            }
+        }
     };
-    // a lane looks after the tokens l, l + L, .. of a chunk: it loads their x, step size and gate (a chunk ahead, into
-    // registers that nothing reads before the chunk's turn), takes the softplus, and at the chunk's end gates and stores
-    // their outputs; the walk gets a token's step size from its lane by a shuffle
-    float xr[OWN], dr[OWN], zr[OWN];
-    auto load_rows = [&](int t0, int nt, float (&xv)[OWN], float (&dv)[OWN], float (&zv)[OWN]) {
-#pragma unroll
-        for (int o = 0; o < OWN; ++o) {
-            const int tt = o * L + l;
-            const bool have = ok && tt < nt;
-            xv[o] = have ? a.x[(size_t)(t0 + tt) * a.x_t + c] : 0.f;
-            dv[o] = have ? a.dt[(size_t)(t0 + tt) * a.dt_t + c] : 0.f;
-            zv[o] = have && gated ? a.z[(size_t)(t0 + tt) * a.z_t + c] : 0.f;
-        }
-    };
-    load_rows(begin, min(SS_CHUNK, end - begin), xr, dr, zr);
-    const int chunks = (end - begin + SS_CHUNK - 1) / SS_CHUNK;
-#pragma unroll
-    for (int i = 0; i < SS_AHEAD; ++i) {
-        if (i < chunks) copy_stage(begin + i * SS_CHUNK, min(SS_CHUNK, end - begin - i * SS_CHUNK), bc_s + i * stage_floats);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    __syncthreads();
+    __syncthreads();
+    for (int s = 0; s < stages; ++s) {
+        if (s > 0) finish(s - 1);
+        __syncthreads();
     }
-    for (int i = 0; i < chunks; ++i) {
-        const int t0 = begin + i * SS_CHUNK;
-        const int nt = min(SS_CHUNK, end - t0);
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(SS_AHEAD - 1) : "memory");
-        __syncthreads();                                       // this chunk's stage is in; the stage read a round ago is free
-        if (i + SS_AHEAD < chunks) {
-            const int t1 = t0 + SS_AHEAD * SS_CHUNK;
-            copy_stage(t1, min(SS_CHUNK, end - t1), bc_s + ((i + SS_AHEAD) % SS_STAGES) * stage_floats);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        const float* rows = bc_s + (i % SS_STAGES) * stage_floats;
-        float xn[OWN], dn[OWN], zn[OWN];
-        const bool more = i + 1 < chunks;
-        if (more) load_rows(t0 + SS_CHUNK, min(SS_CHUNK, end - t0 - SS_CHUNK), xn, dn, zn);
-        // straight-line code for the chunk, so that the tokens' independent parts (shuffles, decays, the sums over the
-        // lanes) overlap and only the multiply-adds on S form a chain. A token past the portion's end has step size 0:
-        // decay 1 and nothing added.
-        ACC dts[OWN], dxs[OWN], ys[OWN];
-#pragma unroll
-        for (int o = 0; o < OWN; ++o) {
-            dts[o] = o * L + l < nt ? ss_softplus((ACC)(dr[o] + dt_b)) : (ACC)0;
-            dxs[o] = dts[o] * (ACC)xr[o];
-            ys[o] = 0;
-        }
-        ACC dtv[SS_CHUNK], dxv[SS_CHUNK], yv[SS_CHUNK];
-#pragma unroll
-        for (int tt = 0; tt < SS_CHUNK; ++tt) {
-            dtv[tt] = L > 1 ? __shfl_sync(0xffffffffu, dts[tt / L], tt % L, L) : dts[tt / L];
-            dxv[tt] = L > 1 ? __shfl_sync(0xffffffffu, dxs[tt / L], tt % L, L) : dxs[tt / L];
-            yv[tt] = 0;
-        }
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            const int n = k * L + l;
-            const bool have = n < Nst;
-            float Bv[SS_CHUNK], Cv[SS_CHUNK];
-            ACC dA[SS_CHUNK];
-#pragma unroll
-            for (int tt = 0; tt < SS_CHUNK; ++tt) {
-                Bv[tt] = have ? rows[tt * 2 * Nst + n] : 0.f;
-                Cv[tt] = have ? rows[tt * 2 * Nst + Nst + n] : 0.f;
-                dA[tt] = ss_exp(dtv[tt] * (ACC)A[k]);
-            }
-#pragma unroll
-            for (int tt = 0; tt < SS_CHUNK; ++tt) {
-                S[k] = fma(dA[tt], S[k], dxv[tt] * (ACC)Bv[tt]);
-                yv[tt] = fma(S[k], (ACC)Cv[tt], yv[tt]);
-            }
-        }
-#pragma unroll
-        for (int w = L >> 1; w > 0; w >>= 1) {
-#pragma unroll
-            for (int tt = 0; tt < SS_CHUNK; ++tt) yv[tt] += __shfl_xor_sync(0xffffffffu, yv[tt], w);
-        }
-#pragma unroll
-        for (int tt = 0; tt < SS_CHUNK; ++tt)
-            if (tt % L == l) ys[tt / L] = yv[tt];
-#pragma unroll
-        for (int o = 0; o < OWN; ++o) {
-            const int tt = o * L + l;
-            if (ok && tt < nt) {
-                float yf = (float)fma((ACC)Dc, (ACC)xr[o], ys[o]);
-                if (gated) yf *= sizeof(ACC) == 8 ? zr[o] / (1.f + expf(-zr[o])) : __fdividef(zr[o], 1.f + __expf(-zr[o]));
-                out[(size_t)(t0 + tt) * a.out_t + c] = from_float<T>(yf);
-            }
-        }
-        if (more) {
-#pragma unroll
-            for (int o = 0; o < OWN; ++o) { xr[o] = xn[o]; dr[o] = dn[o]; zr[o] = zn[o]; }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        const int n = k * L + l;
-        if (ok && n < Nst) wr[(size_t)c * Nst + n] = (float)S[k];
-    }
+    finish(stages - 1);
 }
 
-template <int L, int NS>
-void launch_scan(const ScanArgs& a, int out_dtype, int R, cudaStream_t stream) {
-    constexpr int per_block = SS_THREADS / L;
-    dim3 grid(R, (unsigned)((a.inner + per_block - 1) / per_block));
-    const size_t smem = (size_t)SS_STAGES * SS_CHUNK * 2 * a.states * sizeof(float);
-    if (out_dtype == LLMP_BF16) {
-        LLMP_ALLOW_SMEM((selective_scan_kernel<bf16, float, L, NS>), smem);
-        llmp_launch_dependent(selective_scan_kernel<bf16, float, L, NS>, grid, dim3(SS_THREADS), smem, stream, a);
+template <typename T, typename ACC, int G, int E>
+void launch_scan(const ScanArgs& a, int R, int max_q_len, cudaStream_t stream) {
+    constexpr int CH = SS_WALKERS<G> / G, U = E < 4 ? E : 4;      // channels of a block, in both forms
+    const dim3 grid(R, (unsigned)((a.inner + CH - 1) / CH));
+    if (max_q_len == 1 || R > 1) llmp_launch_dependent(selective_step_kernel<T, ACC, G, E>, grid, dim3(SS_WALKERS<G>), 0, stream, a);
+    if (max_q_len == 1) return;
+    const bool wide = a.inner % CH == 0 && ((uintptr_t)a.x | (uintptr_t)a.dt | (uintptr_t)a.z) % 16 == 0 && (a.x_t | a.dt_t | a.z_t) % 4 == 0 &&
+                      a.states == G * E && ((uintptr_t)a.B | (uintptr_t)a.C) % (4 * U) == 0 && a.bc_t % U == 0;
+    constexpr size_t smem = ScanSmem<ACC, G, E>::BYTES;
+    auto launch = [&](auto kernel) { llmp_launch_dependent(kernel, grid, dim3(SS_WALKERS<G> + 224), smem, stream, a); };
+    if (wide) {
+        LLMP_ALLOW_SMEM((selective_walk_kernel<T, ACC, G, E, true>), smem);
+        launch(selective_walk_kernel<T, ACC, G, E, true>);
     } else {
-        LLMP_ALLOW_SMEM((selective_scan_kernel<float, double, L, NS>), smem);
-        llmp_launch_dependent(selective_scan_kernel<float, double, L, NS>, grid, dim3(SS_THREADS), smem, stream, a);
+        LLMP_ALLOW_SMEM((selective_walk_kernel<T, ACC, G, E, false>), smem);
+        launch(selective_walk_kernel<T, ACC, G, E, false>);
     }
 }
 
-// ---- many tokens: segments side by side --------------------------------------------------------------------------------
+template <int G, int E> void launch_scan(ScanArgs& a, int out_dtype, int R, int max_q_len, cudaStream_t stream) {
+    a.singles = max_q_len != 1 && R > 1;
+    if (out_dtype == LLMP_BF16) launch_scan<bf16, float, G, E>(a, R, max_q_len, stream);
+    else launch_scan<float, double, G, E>(a, R, max_q_len, stream);
+}
+
+// ---- few channels and many tokens: segments side by side ---------------------------------------------------------------
 // The recurrence is linear in S, and over a run of tokens every entry decays by exp(A times the sum of the step sizes). So a
 // request's tokens are cut into segments of SEG_TOKENS, counted from the portion's first token, and three launches take them:
 //   1. every segment but a request's last, from a zero state: its own sum and the sum of its step sizes, to scratch;
 //   2. along a request's segments: scratch becomes the state before each (requests of one segment have nothing to do);
 //   3. every segment from the state before it: the outputs; the last segment leaves the state in the slot.
-// Token by token, a prompt was one chain of 2,048 steps with 110 instructions a token and warp of two channels, most of them
-// spent on what 16 lanes share. Here a thread holds a whole channel, so a token's step size, gate and sum over the entries
-// cost once and the entries' multiply-adds go two at a time; the bound is then the special-function unit (an exponential per
-// token and entry, in 1 and in 3: busy for 72 and 59 % of these launches). 2,048 tokens of 4,096 channels with 16 entries: 641 us
-// token by token, 126 so (51, 18 and 68 with cold caches). Tried: three pairs of eight exponentials as polynomials on the
-// multiply-add pipe (137 us), segments of 96 tokens (128), loads two tokens ahead (133), seven blocks an SM (126).
+// This takes every exponential twice, but nothing waits for a chain of all tokens: where the channels are too few to fill the chip
+// and the tokens many, it ends first. 8,192 tokens of 16 entries, walk against segments: 512 channels 199 and 107 us, 1,024 260 and 142;
+// 2,048 tokens of 1,024, 2,048, 4,096 channels 53 and 67, 54 and 84, 94 and 117.
 constexpr int SEG_TOKENS = 64;
 constexpr int SEG_CHANNELS = 128;         // threads of a block, a channel each
 constexpr int SEG_AHEAD = 4;              // tokens whose loads are under way while as many are worked on
@@ -273,25 +555,6 @@ __device__ __forceinline__ Segment find_segment(const int* q_start, int requests
     }
     return g;
 }
-
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(reinterpret_cast<unsigned long long&>(d))
-        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
-    return d;
-}
-__device__ __forceinline__ float ex2(float v) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(v));
-    return r;
-}
-constexpr float LOG2_E = 1.4426950408889634f;
 
 // OUT false: launch 1; true: launch 3. NS: state entries a thread holds, `states` rounded up (the others decay by 1 and stay 0).
 template <int NS, bool OUT>
@@ -495,7 +758,7 @@ LLMP_API int llmp_selective_scan_segments(const float* x, long x_t, const float*
     ScanArgs& a = g.s;
     a.x = x; a.x_t = x_t; a.dt = dt; a.dt_t = dt_t; a.dt_bias = dt_bias; a.B = B; a.C = C; a.bc_t = bc_t; a.A = A; a.D = D;
     a.z = z; a.z_t = z_t; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
-    a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states; a.L = 0;
+    a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states;
     g.sums = entries ? scratch : nullptr; g.steps = scratch + entries * inner * padded; g.requests = R;
     const int segments = more + R;
     if (padded == 8) launch_segments<8>(g, segments, stream);
@@ -504,36 +767,27 @@ LLMP_API int llmp_selective_scan_segments(const float* x, long x_t, const float*
     return llmp_check_launch("selective_scan_segments");
 }
 
+// max_q_len: the most tokens a request brings, or more.
 LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long dt_t, const float* dt_bias, const float* B,
                                  const float* C, long bc_t, const float* A, const float* D, const float* z, long z_t, float* state,
                                  long state_slot, long state_half, const int* q_start, const int* slots, const int* positions,
-                                 void* out, int out_dtype, long out_t, int R, int inner, int states, cudaStream_t stream) {
+                                 void* out, int out_dtype, long out_t, int R, int inner, int states, int max_q_len, cudaStream_t stream) {
     if (R <= 0) return 0;
     LLMP_REQUIRE(inner > 0 && states > 0 && states <= 256, "selective_scan: %d channels with %d state entries (up to 256 are served)",
                  inner, states);
     LLMP_REQUIRE(state_half >= (long)inner * states, "selective_scan: the state piece is shorter than the state");
-    // a lane per state entry up to 32 entries, then 32 lanes with more each: a long prompt is a chain of dependent steps
-    // per warp, and what hides their latency is the number of warps (measured: 0.59 ms for 2,048 tokens of 4,096 channels
-    // with 16 entries so; 1.08 ms with 8 entries a lane, a sixth of the instructions but an eighth of the warps)
-    int L = 1;
-    while (L < 32 && L < states) L *= 2;
-    const int NS = (states + L - 1) / L;
+    for (long stride : {x_t, dt_t, bc_t, z ? z_t : 0l})
+        LLMP_REQUIRE(stride >= 0 && stride < (1l << 31), "selective_scan: a row stride of %ld entries", stride);
+    LLMP_REQUIRE((inner + 3) / 4 <= 65535, "selective_scan: too many channels %d", inner);
     ScanArgs a;
     a.x = x; a.x_t = x_t; a.dt = dt; a.dt_t = dt_t; a.dt_bias = dt_bias; a.B = B; a.C = C; a.bc_t = bc_t; a.A = A; a.D = D;
-    a.z = z; a.z_t = z_t; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
-    a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states; a.L = L;
-    LLMP_REQUIRE(((long)inner * L + SS_THREADS - 1) / SS_THREADS <= 65535, "selective_scan: too many channels %d", inner);
-    switch (L) {
-        case 1: launch_scan<1, 1>(a, out_dtype, R, stream); break;
-        case 2: launch_scan<2, 1>(a, out_dtype, R, stream); break;
-        case 4: launch_scan<4, 1>(a, out_dtype, R, stream); break;
-        case 8: launch_scan<8, 1>(a, out_dtype, R, stream); break;
-        case 16: launch_scan<16, 1>(a, out_dtype, R, stream); break;
-        default:
-            if (NS <= 1) launch_scan<32, 1>(a, out_dtype, R, stream);
-            else if (NS <= 2) launch_scan<32, 2>(a, out_dtype, R, stream);
-            else if (NS <= 4) launch_scan<32, 4>(a, out_dtype, R, stream);
-            else launch_scan<32, 8>(a, out_dtype, R, stream);
-    }
+    a.z = z; a.z_t = z ? z_t : 0; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
+    a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states;
+    if (states <= 8) launch_scan<4, 2>(a, out_dtype, R, max_q_len, stream);
+    else if (states <= 16) launch_scan<8, 2>(a, out_dtype, R, max_q_len, stream);
+    else if (states <= 32) launch_scan<16, 2>(a, out_dtype, R, max_q_len, stream);
+    else if (states <= 64) launch_scan<32, 2>(a, out_dtype, R, max_q_len, stream);
+    else if (states <= 128) launch_scan<32, 4>(a, out_dtype, R, max_q_len, stream);
+    else launch_scan<32, 8>(a, out_dtype, R, max_q_len, stream);
     return llmp_check_launch("selective_scan");
 }

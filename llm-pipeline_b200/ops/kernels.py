@@ -77,8 +77,8 @@ _SIGNATURES = {
     "llmp_capped_attention": [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _L, _I, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "llmp_capped_attention_mma": [_P, _L, _P, _L, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F,
                                   _I, _I, _I, _P, _P, _I, _P],
-    "llmp_selective_scan": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _I, _L, _I, _I, _I, _P],
     "llmp_selective_scan_segments": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _P],
+    "llmp_selective_scan": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _I, _L, _I, _I, _I, _I, _P],
     "llmp_add_rmsnorm_multi": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _I, _L, _L, _P, _I, _I, _P],
     "llmp_gated_act": [_P, _I, _L, _P, _I, _L, _I, _I, _P],
     "llmp_sigmoid_gate": [_P, _P, _L, _P, _I, _L, _I, _P],
@@ -2010,8 +2010,8 @@ def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Ten
 SELECTIVE_SCAN_MAX_STATES = 256
 
 
-SCAN_SEGMENT_TOKENS, SCAN_SEGMENTS_MAX_STATES = 64, 32       # csrc/selective_scan.cu
-SCAN_SEGMENTS_MIN_TOKENS = 288
+SCAN_SEGMENT_TOKENS, SCAN_SEGMENTS_MAX_STATES, SCAN_SEGMENTS_MAX_CHANNELS = 64, 32, 1024       # csrc/selective_scan.cu
+SCAN_SEGMENTS_MIN_TOKENS = 4096
 
 
 def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: torch.Tensor, c: torch.Tensor, a: torch.Tensor,
@@ -2037,12 +2037,11 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: 
     ptr, slot_stride, half = _state_views(state, state_offset, inner * states, "selective_scan")
     requests = slots.numel()
     if max_q_len is None:
-        max_q_len = N - requests + 1
-    # Long portions: their segments side by side (2,048 tokens of 4,096 channels with 16 entries 126 us, token by token 641). Up
-    # to SCAN_SEGMENTS_MIN_TOKENS the walk token by token (0.31 us a token) ends before the host has launched the layer's other
-    # kernels, and the two launches more and their scratch cost it 8 us (a layer of 2,048 channels: 257 tokens 139 us so and 147
-    # in segments, 300 tokens 150 and 147). float32 output: the state is float64 in between.
-    if (max_q_len > SCAN_SEGMENTS_MIN_TOKENS and states <= SCAN_SEGMENTS_MAX_STATES and out.dtype == torch.bfloat16 and
+        max_q_len = N
+    # Few channels leave a walk over many tokens alone on the chip: then the tokens go in segments side by side, which take every
+    # exponential twice (8,192 tokens of 1,024 channels 142 us, walked 260; of 2,048 tokens 67 and 53). float32 output: the state is
+    # float64 in between.
+    if (max_q_len > SCAN_SEGMENTS_MIN_TOKENS and states <= SCAN_SEGMENTS_MAX_STATES and inner <= SCAN_SEGMENTS_MAX_CHANNELS and out.dtype == torch.bfloat16 and
             max(x.stride(0), dt.stride(0), out.stride(0), z.stride(0) if z is not None else 0) < 1 << 24):
         more = (N - 1) // SCAN_SEGMENT_TOKENS
         padded = 8 if states <= 8 else 16 if states <= 16 else 32
@@ -2053,7 +2052,7 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: 
         return out
     _call("llmp_selective_scan", _ptr(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(b), _ptr(c), b.stride(0), _ptr(a),
           _ptr(d_skip), _ptr(z), z.stride(0) if z is not None else 0, ptr, slot_stride, half, _ptr(q_start), _ptr(slots),
-          _ptr(positions), _ptr(out), dtype_code(out.dtype), out.stride(0), slots.numel(), inner, states, _stream())
+          _ptr(positions), _ptr(out), dtype_code(out.dtype), out.stride(0), requests, inner, states, int(max_q_len), _stream())
     return out
 
 

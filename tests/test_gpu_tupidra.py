@@ -125,6 +125,45 @@ def test_selective_scan_alone(dtype, sizes):
         assert _rel(kept, last) < 2e-5, cuts
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("sizes", [(64, 8), (128, 16), (100, 16), (48, 32), (24, 64), (16, 100), (10, 200)], ids=str)
+def test_selective_scan_stages(dtype, sizes):
+    """Portions around a stage's end (16 and 32 tokens), a turn's (4 and 8) and single tokens side by side, rows that are aligned (and
+    copied by 16 bytes where a block's channels are whole) and not: each request has the bits it has alone, and matches float64. bfloat16
+    rounds an output to 2^-9 of itself."""
+    from llm_pipeline_b200.ops import kernels
+    inner, states = sizes
+    lengths = [1, 7, 8, 9, 16, 31, 32, 33, 64, 1, 97, 130]
+    starts = [0] + list(itertools.accumulate(lengths))
+    R, n = len(lengths), starts[-1]
+    gen = torch.Generator().manual_seed(inner * states)
+    dt_bias, skip = torch.randn(inner, generator=gen) * 0.5 - 1.0, torch.randn(inner, generator=gen)
+    A = -torch.exp(torch.rand(inner, states, generator=gen) * 5.0 - 4.5)
+    for pad in (0, 3):
+        x, raw, z = (torch.randn(n, inner + pad, generator=gen).to(DEV)[:, pad:] for _ in range(3))
+        bc = torch.randn(n, 2 * states + pad, generator=gen).to(DEV)[:, pad:]
+
+        def step(requests):
+            own = [lengths[r] for r in requests]
+            part = [torch.cat([y[starts[r]:starts[r + 1]] for r in requests]) if len(requests) < R else y for y in (x, raw, z, bc)]
+            out, state = torch.empty(sum(own), inner, device=DEV, dtype=dtype), torch.zeros(R + 1, 2 * inner * states, device=DEV)
+            kernels.selective_scan(part[0], part[1], dt_bias.to(DEV), part[3][:, :states], part[3][:, states:], A.to(DEV), skip.to(DEV), part[2], state,
+                                   0, _i32([0] + list(itertools.accumulate(own))), _i32([R - r for r in requests]),
+                                   _i32([p for m in own for p in range(m)]), out, max(own))
+            return out, state
+
+        out, state = step(list(range(R)))
+        assert (state[0] == 0.0).all()
+        for r, m in enumerate(lengths):
+            mine = slice(starts[r], starts[r + 1])
+            alone, kept = step([r])
+            assert torch.equal(out[mine], alone) and torch.equal(state[R - r], kept[R - r]), (pad, r)
+            dt = torch.nn.functional.softplus(raw[mine].cpu().double() + dt_bias.double())
+            y, S = plain.scan(x[mine].cpu().double(), dt, A.double(), bc[mine, :states].cpu().double(), bc[mine, states:].cpu().double(), skip.double())
+            assert _rel(out[mine], y * plain.silu(z[mine].cpu().double())) < (2e-5 if dtype == torch.float32 else 4e-3), (pad, r)
+            assert _rel(state[R - r].view(2, inner, states)[(m - 1) & 1], S) < 2e-5, (pad, r)
+
+
 @pytest.mark.parametrize("lengths", [(1, 64, 65), (128, 2, 1, 129, 31), (200,)], ids=str)
 @pytest.mark.parametrize("sizes", [(130, 16), (37, 5), (129, 32)], ids=str)
 def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
