@@ -523,11 +523,11 @@ template <int KS> void launch_chunks(const DeltaChunkArgs& a, int chunks, cudaSt
 
 // delta_rule.cu
 LLMP_API int llmp_delta_prep(float* q, long q_t, float* k, long k_t, float* decay, long decay_t, float* beta, long beta_t, const float* a_log,
-                             const float* dt_bias, const int* token_request, const int* q_start, int max_tokens, int tokens, int H, int G, int d,
+                             const float* dt_bias, const int* token_request, const int* q_start, int least, int max_tokens, int tokens, int H, int G, int d,
                              cudaStream_t stream);
 LLMP_API int llmp_delta_scan(const float* q, long q_t, const float* k, long k_t, const float* v, long v_t, const float* decay, long decay_t,
                              const float* beta, long beta_t, float* state, long state_slot, long state_half, const int* q_start, const int* slots,
-                             const int* positions, float* o, long o_t, int max_tokens, int R, int H, int G, int d, int dv, cudaStream_t stream);
+                             const int* positions, float* o, long o_t, int least, int max_tokens, int R, int H, int G, int d, int dv, cudaStream_t stream);
 
 // Bytes of scratch for `rows` tokens of R requests; 0: these sizes are not served.
 LLMP_API long llmp_delta_chunks_scratch(int rows, int R, int H, int d, int dv) {
@@ -537,11 +537,11 @@ LLMP_API long llmp_delta_chunks_scratch(int rows, int R, int H, int d, int dv) {
 
 // q, k, v: the convolved rows; decay, beta: pre-activations (delta_prep and delta_scan in one). list: `count` of the R requests, in
 // ascending order, which have `rows` of the step's tokens together; the others, which have up to max_tokens each, go token by token
-// (their rows are prepared in place). null: all requests in chunks.
+// (their rows are prepared in place), those of fewer than `least` are left alone. null: all requests in chunks.
 LLMP_API int llmp_delta_chunks(float* q, long q_t, float* k, long k_t, const float* v, long v_t, float* decay, long decay_t,
                                float* beta, long beta_t, const float* a_log, const float* dt_bias, float* state, long state_slot,
                                long state_half, const int* q_start, const int* slots, const int* positions, float* o, long o_t, void* scratch,
-                               long scratch_bytes, const int* list, int count, int rows, const int* token_request, int max_tokens, int tokens,
+                               long scratch_bytes, const int* list, int count, int rows, const int* token_request, int least, int max_tokens, int tokens,
                                int R, int H, int G, int d, int dv, int* error_flag, cudaStream_t stream) {
     if (R <= 0 || tokens <= 0) return 0;
     LLMP_REQUIRE(rows > 0 && rows <= tokens && count > 0 && count <= R && (list ? token_request != nullptr : count == R && rows == tokens),
@@ -559,12 +559,12 @@ LLMP_API int llmp_delta_chunks(float* q, long q_t, float* k, long k_t, const flo
     const int chunks = (rows - 1) / DC_TOKENS + count;
     if (d == 64) launch_chunks<1>(a, chunks, stream);
     else launch_chunks<2>(a, chunks, stream);
-    if (list) {
-        const int failed = llmp_delta_prep(q, q_t, k, k_t, decay, decay_t, beta, beta_t, a_log, dt_bias, token_request, q_start, max_tokens, tokens,
+    if (list && least <= max_tokens) {
+        const int failed = llmp_delta_prep(q, q_t, k, k_t, decay, decay_t, beta, beta_t, a_log, dt_bias, token_request, q_start, least, max_tokens, tokens,
                                            H, G, d, stream);
         if (failed) return failed;
         return llmp_delta_scan(q, q_t, k, k_t, v, v_t, decay, decay_t, beta, beta_t, state, state_slot, state_half, q_start, slots, positions, o, o_t,
-                               max_tokens, R, H, G, d, dv, stream);
+                               least, max_tokens, R, H, G, d, dv, stream);
     }
     return llmp_check_launch("delta_chunks");
 }

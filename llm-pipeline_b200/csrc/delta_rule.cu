@@ -23,7 +23,7 @@ struct PrepArgs {
     float* beta; long beta_t;                     // [tokens, H]
     const float* a_log; const float* dt_bias;     // [H], [H d]
     const int* token_request; const int* q_start; // null: all tokens
-    int max_tokens;                               // requests that bring more are left alone
+    int least, max_tokens;                        // requests that bring fewer or more are left alone
     int H, G, d;
 };
 
@@ -33,7 +33,8 @@ __global__ void delta_prep_kernel(const PrepArgs a) {
     const int t = blockIdx.x;
     if (a.token_request) {
         const int r = a.token_request[t];
-        if (a.q_start[r + 1] - a.q_start[r] > a.max_tokens) return;
+        const int n = a.q_start[r + 1] - a.q_start[r];
+        if (n < a.least || n > a.max_tokens) return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const float q_scale = 1.f / sqrtf((float)a.d);
@@ -59,7 +60,7 @@ struct DeltaArgs {
     float* state; long state_slot; long state_half;      // copy: [H][d][dv]
     const int* q_start; const int* slots; const int* positions;
     float* o; long o_t;                                  // [tokens, H dv]
-    int max_tokens;                                      // requests that bring more are left to delta_chunks.cu
+    int least, max_tokens;                               // requests that bring fewer are left to delta_step.cu, more to delta_chunks.cu
     int H, G, d, dv;
 };
 
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(DS_THREADS + 32 * DS_COPY_WARPS) delta_scan_ke
     pdl_wait();                                    // what the kernels before wrote is complete
     pdl_trigger();
     const int begin = a.q_start[r], end = a.q_start[r + 1];
-    if (end <= begin || end - begin > a.max_tokens) return;
+    if (end <= begin || end - begin < a.least || end - begin > a.max_tokens) return;
     const int d = a.d, dv = a.dv;
     const bool loader = threadIdx.x >= DS_THREADS;
     const int copy_warp = ((int)threadIdx.x - DS_THREADS) >> 5;      // which of the copying warps (negative for the others)
@@ -207,14 +208,14 @@ __global__ void __launch_bounds__(DS_THREADS + 32 * DS_COPY_WARPS) delta_scan_ke
 }  // namespace
 
 LLMP_API int llmp_delta_prep(float* q, long q_t, float* k, long k_t, float* decay, long decay_t, float* beta, long beta_t,
-                             const float* a_log, const float* dt_bias, const int* token_request, const int* q_start, int max_tokens,
+                             const float* a_log, const float* dt_bias, const int* token_request, const int* q_start, int least, int max_tokens,
                              int tokens, int H, int G, int d, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && d > 0, "delta_prep: bad sizes heads=%d qk_heads=%d dim=%d", H, G, d);
     PrepArgs a;
     a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.decay = decay; a.decay_t = decay_t; a.beta = beta; a.beta_t = beta_t;
     LLMP_REQUIRE(!token_request || q_start, "delta_prep: the tokens' requests need their starts");
-    a.a_log = a_log; a.dt_bias = dt_bias; a.token_request = token_request; a.q_start = q_start; a.max_tokens = max_tokens;
+    a.a_log = a_log; a.dt_bias = dt_bias; a.token_request = token_request; a.q_start = q_start; a.least = least; a.max_tokens = max_tokens;
     a.H = H; a.G = G; a.d = d;
     llmp_launch_dependent(delta_prep_kernel, dim3(tokens), dim3(256), 0, stream, a);
     return llmp_check_launch("delta_prep");
@@ -222,7 +223,7 @@ LLMP_API int llmp_delta_prep(float* q, long q_t, float* k, long k_t, float* deca
 
 LLMP_API int llmp_delta_scan(const float* q, long q_t, const float* k, long k_t, const float* v, long v_t, const float* decay,
                              long decay_t, const float* beta, long beta_t, float* state, long state_slot, long state_half,
-                             const int* q_start, const int* slots, const int* positions, float* o, long o_t, int max_tokens, int R, int H,
+                             const int* q_start, const int* slots, const int* positions, float* o, long o_t, int least, int max_tokens, int R, int H,
                              int G, int d, int dv, cudaStream_t stream) {
     if (R <= 0) return 0;
     LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && d > 0 && dv > 0 && dv <= 1024 && H <= 65535,
@@ -231,7 +232,7 @@ LLMP_API int llmp_delta_scan(const float* q, long q_t, const float* k, long k_t,
     DeltaArgs a;
     a.q = q; a.q_t = q_t; a.k = k; a.k_t = k_t; a.v = v; a.v_t = v_t; a.decay = decay; a.decay_t = decay_t;
     a.beta = beta; a.beta_t = beta_t; a.state = state; a.state_slot = state_slot; a.state_half = state_half;
-    a.q_start = q_start; a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.max_tokens = max_tokens; a.H = H; a.G = G; a.d = d; a.dv = dv;
+    a.q_start = q_start; a.slots = slots; a.positions = positions; a.o = o; a.o_t = o_t; a.least = least; a.max_tokens = max_tokens; a.H = H; a.G = G; a.d = d; a.dv = dv;
     // lanes that share a column: the fewest (a power of two up to 32) that leave a lane at most 16 rows (32 past 512 rows)
     int rows = 1;
     while (rows < 32 && (d + rows - 1) / rows > 16) rows *= 2;

@@ -103,9 +103,10 @@ _SIGNATURES = {
     "llmp_chunked_scan": [_P, _P, _P, _L, _P, _L, _P, _P, _P, _P, _P, _L, _L, _P, _P, _P, _P, _I, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _P],
     "llmp_stream_step": [_P, _L, _L, _P, _P, _I, _P, _F, _F, _P, _I, _P, _F, _F, _P, _P, _P, _P, _P, _I, _F, _P, _I, _P, _I, _I, _I, _P],
     "llmp_gated_group_norm": [_P, _L, _P, _L, _P, _P, _I, _L, _I, _I, _I, _I, _F, _P],
-    "llmp_delta_prep": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
-    "llmp_delta_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _P],
-    "llmp_delta_chunks": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I,
+    "llmp_delta_prep": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],
+    "llmp_delta_scan": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P],
+    "llmp_delta_step": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _L, _L, _P, _P, _P, _P, _I, _L, _I, _I, _I, _I, _I, _I, _F, _P],
+    "llmp_delta_chunks": [_P, _L, _P, _L, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I,
                           _I, _P, _P],
     "llmp_sig_qkv_post": [_P, _L, _P, _I, _P, _P, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "llmp_sigmoid_attention": [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
@@ -1633,8 +1634,10 @@ def gated_group_norm(y: torch.Tensor, gate: torch.Tensor, weight: Optional[torch
 
 
 def delta_prep(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
-               heads: int, qk_heads: int, dim: int) -> None:
-    """In place, per token (csrc/delta_rule.cu): ``q`` and ``k`` float32 [tokens, qk_heads dim] become unit vectors per head (q also
+               heads: int, qk_heads: int, dim: int, token_request: Optional[torch.Tensor] = None, q_start: Optional[torch.Tensor] = None,
+               least: int = 1) -> None:
+    """In place, per token (csrc/delta_rule.cu), of the requests that bring at least ``least`` tokens (above 1 it needs ``token_request``
+    and ``q_start``): ``q`` and ``k`` float32 [tokens, qk_heads dim] become unit vectors per head (q also
     times dim^(-1/2)); ``decay`` float32 [tokens, heads dim] goes from its pre-activation to exp(-exp(a_log[head]) softplus(. +
     dt_bias)); ``beta`` float32 [tokens, heads] to its sigmoid. All four may be views with a dense last axis."""
     N = q.shape[0]
@@ -1643,13 +1646,14 @@ def delta_prep(q: torch.Tensor, k: torch.Tensor, decay: torch.Tensor, beta: torc
     _need(a_log.dtype == torch.float32 and a_log.numel() == heads and a_log.is_contiguous() and dt_bias.dtype == torch.float32 and
           dt_bias.numel() == heads * dim and dt_bias.is_contiguous(), "delta_prep takes float32 A_log [heads] and dt_bias [heads dim]")
     _call("llmp_delta_prep", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(decay), decay.stride(0), _ptr(beta), beta.stride(0),
-          _ptr(a_log), _ptr(dt_bias), None, None, 0, N, heads, qk_heads, dim, _stream())
+          _ptr(a_log), _ptr(dt_bias), _ptr(token_request) if least > 1 else None, _ptr(q_start) if least > 1 else None, int(least), (1 << 31) - 1, N,
+          heads, qk_heads, dim, _stream())
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,
                state_offset: int, q_start: torch.Tensor, slots: torch.Tensor, positions: torch.Tensor, out: torch.Tensor,
-               heads: int, qk_heads: int, dim: int, vdim: int) -> torch.Tensor:
-    """The gated delta rule over the step's tokens, request by request (csrc/delta_rule.cu); inputs as ``delta_prep`` leaves
+               heads: int, qk_heads: int, dim: int, vdim: int, least: int = 1) -> torch.Tensor:
+    """The gated delta rule over the tokens of the step's requests that bring at least ``least``, request by request (csrc/delta_rule.cu); inputs as ``delta_prep`` leaves
     them, ``v`` float32 [tokens, heads vdim], ``out`` float32 [tokens, heads vdim]. The state piece holds two copies of
     [heads, dim, vdim]."""
     N = q.shape[0]
@@ -1661,7 +1665,39 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     ptr, slot_stride, half = _state_views(state, state_offset, heads * dim * vdim, "delta_scan")
     _call("llmp_delta_scan", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0),
           _ptr(beta), beta.stride(0), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
-          (1 << 31) - 1, slots.numel(), heads, qk_heads, dim, vdim, _stream())
+          int(least), (1 << 31) - 1, slots.numel(), heads, qk_heads, dim, vdim, _stream())
+    return out
+
+
+def delta_step_serves(channels: int, dim: int, vdim: int, taps: int, state: torch.Tensor, state_offset: int) -> bool:
+    """Whether ``delta_step`` takes single tokens through a layer of these sizes: it follows from the layer and its state alone."""
+    fn = library().llmp_delta_step_serves
+    fn.argtypes, fn.restype = [_I, _I, _I, _I], _I
+    return bool(fn(channels, dim, vdim, taps)) and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0 and state_offset % 4 == 0
+
+
+def delta_step(proj: torch.Tensor, decay: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
+               norm: torch.Tensor, state: torch.Tensor, scan_offset: int, q_start: torch.Tensor, slots: torch.Tensor, positions: torch.Tensor,
+               out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, eps: float) -> torch.Tensor:
+    """The convolution, ``delta_prep``, ``delta_scan`` and the gated norm for the step's requests that bring one token, in one kernel
+    (csrc/delta_step.cu); the others are left alone. ``proj`` float32 [tokens, >= C + heads] = q | k | v | beta as projected (C = 2 qk_heads dim +
+    heads vdim), ``decay`` [tokens, heads dim] and ``gate`` [tokens, heads vdim] before their functions, ``taps`` [C, K], ``out`` [tokens, heads
+    vdim] in the compute type. The convolution's inputs lie at the front of the slot, the rule's state at ``scan_offset``."""
+    H, G, d, dv = int(heads), int(qk_heads), int(dim), int(vdim)
+    N, C = proj.shape[0], 2 * int(qk_heads) * int(dim) + int(heads) * int(vdim)
+    for t, width, name in ((proj, C + H, "proj"), (decay, H * d, "decay"), (gate, H * dv, "gate")):
+        _need(t.dtype == torch.float32 and t.stride(1) == 1 and t.shape[0] == N and t.shape[1] >= width, f"delta_step: {name} must be float32 rows of {width} entries")
+    for t, n in ((a_log, H), (dt_bias, H * d), (norm, dv)):
+        _need(t.dtype == torch.float32 and t.is_contiguous() and t.numel() == n, "delta_step: the layer's vectors must be float32 and of its sizes")
+    _need(taps.dtype == torch.float32 and taps.is_contiguous() and taps.dim() == 2 and taps.shape[0] == C, "delta_step takes float32 taps [channels, taps]")
+    _need(out.shape == (N, H * dv) and out.stride(1) == 1, "delta_step: the output has the wrong shape")
+    for t, name in ((q_start, "q_start"), (slots, "slots"), (positions, "positions")):
+        _i32(t, name)
+    ptr, slot_stride, _half = _state_views(state, 0, (K := taps.shape[1]) * C - C, "delta_step")
+    _need(scan_offset + 2 * H * d * dv <= state.shape[1], "delta_step: the state piece does not fit the slot")
+    _call("llmp_delta_step", _ptr(proj), proj.stride(0), _ptr(decay), decay.stride(0), _ptr(gate), gate.stride(0), _ptr(taps), _ptr(a_log), _ptr(dt_bias),
+          _ptr(norm), ptr, slot_stride, int(scan_offset), _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), dtype_code(out.dtype), out.stride(0),
+          slots.numel(), H, G, d, dv, K, float(eps), _stream())
     return out
 
 
@@ -1690,11 +1726,11 @@ def delta_chunks_scratch(dtype: torch.dtype, rows: int, requests: int, max_q_len
 def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, a_log: torch.Tensor,
                  dt_bias: torch.Tensor, state: torch.Tensor, state_offset: int, q_start: torch.Tensor, slots: torch.Tensor,
                  positions: torch.Tensor, out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, scratch: int,
-                 long: Optional[Tuple[torch.Tensor, int]] = None, token_request: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 long: Optional[Tuple[torch.Tensor, int]] = None, token_request: Optional[torch.Tensor] = None, least: int = 1) -> torch.Tensor:
     """``delta_prep`` and ``delta_scan`` in chunks on the tensor cores (csrc/delta_chunks.cu): the same rows before ``delta_prep``,
     which stay as they are. ``long``: which of the step's requests (int32 on the device, ascending: those of at least
     ``DELTA_CHUNKS_MIN_TOKENS`` tokens) and their tokens together; the others, whose rows ``token_request`` tells, are prepared in place
-    and walked token by token in the same call. None: all requests in chunks. ``scratch``: what ``delta_chunks_scratch`` gave for the
+    and walked token by token in the same call, those of fewer than ``least`` tokens left alone. None: all requests in chunks. ``scratch``: what ``delta_chunks_scratch`` gave for the
     tokens and the number of the requests in chunks."""
     H, G, d, dv = int(heads), int(qk_heads), int(dim), int(vdim)
     N = q.shape[0]
@@ -1713,8 +1749,8 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch
     room = torch.empty(scratch, dtype=torch.uint8, device=q.device)
     _call("llmp_delta_chunks", _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), decay.stride(0), _ptr(beta),
           beta.stride(0), _ptr(a_log), _ptr(dt_bias), ptr, slot_stride, half, _ptr(q_start), _ptr(slots), _ptr(positions), _ptr(out), out.stride(0),
-          _ptr(room), scratch, *((None, R, N, None, 0) if long is None else (_ptr(long[0]), long[0].numel(), long[1], _ptr(token_request),
-                                                                             DELTA_CHUNKS_MIN_TOKENS - 1)),
+          _ptr(room), scratch, *((None, R, N, None, 1, 0) if long is None else (_ptr(long[0]), long[0].numel(), long[1], _ptr(token_request),
+                                                                                int(least), DELTA_CHUNKS_MIN_TOKENS - 1)),
           N, R, H, G, d, dv, error_flag().data_ptr(), _stream())
     return out
 

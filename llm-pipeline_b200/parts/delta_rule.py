@@ -15,7 +15,7 @@ The six products that read h are one product against [Wq; Wk; Wv; Wb; Wa1; Wg1] 
 the two-step projections are whatever the tensors have. Convolutions, unit norms, step sizes, decays, state and read-out
 are float32 (``csrc/short_conv.cu``, ``csrc/delta_rule.cu``; long portions in bfloat16 in chunks on the tensor cores with factors of
 three bfloat16 pieces, ``csrc/delta_chunks.cu``); the gated rows are rounded once to the compute type for the
-output product.
+output product. Single tokens take one kernel for all that lies between the products (``csrc/delta_step.cu``).
 
 State of a request: one float32 vector ``[conv piece | state piece]``, each piece two copies that take turns by the parity
 of the last position written (see ``state_space.py``)."""
@@ -120,27 +120,40 @@ class GatedDeltaRule(Mixer):
             raise RuntimeError("the delta-rule mixer needs its state slots")
         N, C, H = ctx.num_tokens, self.channels, self.heads
         proj = linear(x, self.w_in, out_dtype=torch.float32)
-        beta = proj[:, C:C + H]
-        low_a = proj[:, C + H:C + H + self.decay_rank]
-        low_g = proj[:, C + H + self.decay_rank:]
+        low = proj[:, C + H:]
         if x.dtype != torch.float32:
-            low_a, low_g = low_a.to(x.dtype), low_g.to(x.dtype)
-        decay = linear(low_a, self.w_a2, out_dtype=torch.float32)
-        gate = linear(low_g, self.w_g2, out_dtype=torch.float32)
-        mixed = torch.empty((N, C), dtype=torch.float32, device=x.device)
+            low = kernels.convert_rows(low, torch.empty(low.shape, dtype=x.dtype, device=x.device))
+        decay = linear(low[:, :self.decay_rank], self.w_a2, out_dtype=torch.float32)
+        gate = linear(low[:, self.decay_rank:], self.w_g2, out_dtype=torch.float32)
+        normed = torch.empty((N, self.v_size), dtype=x.dtype, device=x.device)
+        # single tokens take a kernel of their own in any company (their rows and state have the same bits there)
+        singles = (ctx.max_q_len == 1 or 1 in ctx.q_lens) and kernels.delta_step_serves(C, self.dim, self.vdim, self.taps, cache.state, 0)
+        if not singles or ctx.max_q_len > 1:
+            self._portions(ctx, cache, proj, decay, gate, normed, 2 if singles else 1)
+        if singles:
+            kernels.delta_step(proj, decay, gate, self.conv_w, self.a_log, self.dt_bias, self.norm_w, cache.state, self.conv_entries, ctx.q_start,
+                               ctx.slots, ctx.positions, normed, H, self.qk_heads, self.dim, self.vdim, self.eps)
+        return linear(normed, self.w_out, out_dtype=torch.float32), None
+
+    def _portions(self, ctx, cache, proj, decay, gate, normed, least):
+        """The convolution, the rule and the gated norm over the requests that bring at least ``least`` tokens (the others' rows of
+        ``normed`` hold nothing, their rows of ``proj`` and ``decay`` and their state of the rule stay as they are)."""
+        N, C, H = ctx.num_tokens, self.channels, self.heads
+        beta = proj[:, C:C + H]
+        mixed = torch.empty((N, C), dtype=torch.float32, device=proj.device)
         kernels.short_conv(proj[:, :C], self.conv_w, None, cache.state, 0, ctx.q_start, ctx.slots, ctx.positions, ctx.token_request,
                            mixed, ctx.max_q_len, silu=True)
         q, k, v = mixed[:, :self.qk_size], mixed[:, self.qk_size:2 * self.qk_size], mixed[:, 2 * self.qk_size:]
-        o = torch.empty((N, self.v_size), dtype=torch.float32, device=x.device)
+        o = torch.empty((N, self.v_size), dtype=torch.float32, device=proj.device)
         some, rows, count = _long_requests(ctx)
-        scratch = kernels.delta_chunks_scratch(x.dtype, rows, count, ctx.max_q_len, H, self.dim, self.vdim) if count else 0
+        scratch = kernels.delta_chunks_scratch(normed.dtype, rows, count, ctx.max_q_len, H, self.dim, self.vdim) if count else 0
         if scratch:
+            if least > 1 and not any(1 < n < kernels.DELTA_CHUNKS_MIN_TOKENS for n in ctx.q_lens):
+                least = kernels.DELTA_CHUNKS_MIN_TOKENS                          # nobody is left to walk
             kernels.delta_chunks(q, k, v, decay, beta, self.a_log, self.dt_bias, cache.state, self.conv_entries, ctx.q_start, ctx.slots,
-                                 ctx.positions, o, H, self.qk_heads, self.dim, self.vdim, scratch, some, ctx.token_request)
+                                 ctx.positions, o, H, self.qk_heads, self.dim, self.vdim, scratch, some, ctx.token_request, least)
         else:
-            kernels.delta_prep(q, k, decay, beta, self.a_log, self.dt_bias, H, self.qk_heads, self.dim)
+            kernels.delta_prep(q, k, decay, beta, self.a_log, self.dt_bias, H, self.qk_heads, self.dim, ctx.token_request, ctx.q_start, least)
             kernels.delta_scan(q, k, v, decay, beta, cache.state, self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, o,
-                               H, self.qk_heads, self.dim, self.vdim)
-        normed = torch.empty((N, self.v_size), dtype=x.dtype, device=x.device)
+                               H, self.qk_heads, self.dim, self.vdim, least)
         kernels.gated_group_norm(o, gate, self.norm_w, normed, self.vdim, self.eps, gate_first=False)
-        return linear(normed, self.w_out, out_dtype=torch.float32), None

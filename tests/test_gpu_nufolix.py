@@ -322,6 +322,45 @@ def test_gated_delta_rule_in_chunks_is_causal_for_what_is_no_number(what, t, bad
         assert torch.equal(got[:, others], want[:, others])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("sizes", [(2, 1, 64, 16, 4), (2, 2, 128, 128, 4), (1, 1, 192, 128, 2), (3, 1, 20, 12, 1), (4, 2, 36, 100, 8)], ids=str)
+def test_gated_delta_rule_single_tokens_in_one_kernel(sizes, dtype):
+    """Requests of one token among others, at positions of both parities, against the convolution, the preparation, the walk and the norm as
+    kernels of their own: the same float32 operations but for the order of the sums over up to 192 channels (192 roundings of 2^-24, within
+    1.2e-5), an output in bfloat16 then within a rounding of 2^-8. Rows, state and slots of the others stay as they are."""
+    from llm_pipeline_b200.ops import kernels
+    heads, qk_heads, dim, vdim, taps = sizes
+    gen, dev = torch.Generator().manual_seed(dim + vdim), "cuda"
+    C, piece = 2 * qk_heads * dim + heads * vdim, heads * dim * vdim
+    lengths, where = [1, 3, 1, 1, 2, 1], [6, 2, 9, 4, 0, 1]
+    singles, N, scan = [0, 2, 3, 5], sum(lengths), 2 * (taps - 1) * C
+    starts = [sum(lengths[:r]) for r in range(len(lengths) + 1)]
+    rand = lambda *shape: torch.randn(*shape, generator=gen).to(dev)   # noqa: E731
+    proj, decay, gate, conv_w, norm = rand(N, C + heads + 5), rand(N, heads * dim), rand(N, heads * vdim), rand(C, taps), rand(vdim)
+    a_log, dt_bias, state = rand(heads), rand(heads * dim), rand(len(lengths) + 1, scan + 2 * piece)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=dev)   # noqa: E731
+    slots, positions = i32(range(len(lengths), 0, -1)), i32([where[r] + i for r, n in enumerate(lengths) for i in range(n)])
+    assert kernels.delta_step_serves(C, dim, vdim, taps, state, 0)
+    got, left = torch.full((N, heads * vdim), 7.0, dtype=dtype, device=dev), state.clone()
+    before = proj.clone(), decay.clone()
+    kernels.delta_step(proj, decay, gate, conv_w, a_log, dt_bias, norm, left, scan, i32(starts), slots, positions, got, heads, qk_heads, dim, vdim, 1e-5)
+    assert torch.equal(proj, before[0]) and torch.equal(decay, before[1])
+    rows = [starts[r] for r in singles]
+    mixed, o, want, kept = torch.empty(4, C, device=dev), torch.empty(4, heads * vdim, device=dev), torch.empty(4, heads * vdim, device=dev), state.clone()
+    at = i32(range(5)), slots[singles].contiguous(), positions[rows].contiguous()
+    kernels.short_conv(proj[rows][:, :C], conv_w, None, kept, 0, *at, i32(range(4)), mixed, 1, silu=True)
+    q, k, v = (t.contiguous() for t in mixed.split([qk_heads * dim, qk_heads * dim, heads * vdim], dim=1))
+    g, beta = decay[rows], proj[rows][:, C:C + heads].contiguous()
+    kernels.delta_prep(q, k, g, beta, a_log, dt_bias, heads, qk_heads, dim)
+    kernels.delta_scan(q, k, v, g, beta, kept, scan, *at, o, heads, qk_heads, dim, vdim)
+    kernels.gated_group_norm(o, gate[rows], norm, want, vdim, 1e-5, gate_first=False)
+    assert float((got[rows].double() - want.double()).norm() / want.double().norm()) < (1.2e-5 if dtype == torch.float32 else 4e-3)
+    assert float((left.double() - kept.double()).norm() / kept.double().norm()) < 1.2e-5
+    assert torch.equal(left[:, :scan], kept[:, :scan])
+    others = [t for r, n in enumerate(lengths) if n > 1 for t in range(starts[r], starts[r + 1])]
+    assert (got[others] == 7.0).all() and torch.equal(left[[0, 2, 5]], state[[0, 2, 5]])
+
+
 @pytest.mark.parametrize("sizes", [(2, 1, 64, 16), (1, 1, 128, 48)], ids=str)
 def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
     """Forty portions in chunks and as many short ones token by token in one step, more than a warp looks at in one go, in an order
