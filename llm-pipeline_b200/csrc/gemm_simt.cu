@@ -181,7 +181,7 @@ LLMP_API int llmp_gemm_simt(const void* A, const void* W, const void* bias, int 
     return llmp_check_launch("gemm_simt");
 }
 
-// The same batch for at most 16 rows a product (a decode step): a warp per output column reads the column's weight
+// A batch of products of at most 16 rows each (a decode step), float32 or without 16-byte rows (else gemm_few_batched.cu): a warp per output column reads the column's weight
 // row once and keeps one sum per row of A; the K products of a sum are added lane by lane in ascending k, then across
 // the lanes in a fixed order.
 #define GR_MAX_ROWS 16
@@ -246,6 +246,11 @@ gemm_rows_kernel(const TI* __restrict__ A, const TI* __restrict__ W, TO* __restr
     }
 }
 
+// gemm_few_batched.cu
+LLMP_API int llmp_gemm_few_batched_supports(const void* A, const void* W, int M, int K, long lda, long ldw, long batch_a, long batch_w);
+LLMP_API int llmp_gemm_few_batched(const void* A, const void* W, void* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
+                                   long batch_a, long batch_w, long batch_c, cudaStream_t stream);
+
 // A batch of such products in one launch: product b reads A + b * batch_a and W + b * batch_w and writes C + b * batch_c
 // (strides in elements; rows of any of them may lie further apart than they are long, so one product per head
 // can read and write the heads of a [tokens, heads, size] tensor in place).
@@ -255,19 +260,21 @@ LLMP_API int llmp_gemm_simt_batched(const void* A, const void* W, void* C, int i
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     LLMP_REQUIRE(K > 0, "batched gemm: bad K %d", K);
     LLMP_REQUIRE(M <= GT_MAX_ROWS && batch <= 65535, "batched gemm: too many rows %d or products %d", M, batch);
+    if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16 && llmp_gemm_few_batched_supports(A, W, M, K, lda, ldw, batch_a, batch_w))
+        return llmp_gemm_few_batched(A, W, C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream);
     if (M <= GR_MAX_ROWS && (N + 7) / 8 <= 65535) {
         dim3 rows_grid((N + 7) / 8, batch);
         const size_t esize = in_dtype == LLMP_F32 ? 4 : 2;
         const bool vec = K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && batch_a % 8 == 0 && batch_w % 8 == 0 &&
                          ((size_t)A | (size_t)W) % 16 == 0 && esize > 0;
-#define LLMP_ROWS(TI, TO)                                                                                                         \
+#define LLMP_ROWS(TI, TO, WIDE)                                                                                                   \
     do {                                                                                                                          \
-        llmp_launch_dependent(vec ? gemm_rows_kernel<TI, TO, true> : gemm_rows_kernel<TI, TO, false>, rows_grid, dim3(256), 0, stream,  \
+        llmp_launch_dependent(vec && WIDE ? gemm_rows_kernel<TI, TO, WIDE> : gemm_rows_kernel<TI, TO, false>, rows_grid, dim3(256), 0, stream,  \
                               (const TI*)A, (const TI*)W, (TO*)C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c);            \
     } while (0)
-        if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32) LLMP_ROWS(float, float);
-        else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16) LLMP_ROWS(bf16, bf16);
-        else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_F32) LLMP_ROWS(bf16, float);
+        if (in_dtype == LLMP_F32 && out_dtype == LLMP_F32) LLMP_ROWS(float, float, true);
+        else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16) LLMP_ROWS(bf16, bf16, false);
+        else if (in_dtype == LLMP_BF16 && out_dtype == LLMP_F32) LLMP_ROWS(bf16, float, true);
         else {
             llmp_set_error("batched gemm: unsupported type combination in=%d out=%d", in_dtype, out_dtype);
             return 1;

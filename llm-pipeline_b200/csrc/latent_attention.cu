@@ -26,6 +26,17 @@ __global__ void latent_kv_post_kernel(T* __restrict__ qd, long ld, int H, int d,
     const int half = rot_dims / 2;
     const float* cs = cos_t + (size_t)n * half;
     const float* sn = sin_t + (size_t)n * half;
+    if (blockIdx.y) {
+        // every head's rotated query part, in place (a pair is read and written by one thread)
+        for (int e = threadIdx.x; e < H * half; e += blockDim.x) {
+            const int h = e / half, i = e % half;
+            T* qr = q + (size_t)h * (d + r) + d;
+            const float a = to_float(qr[i]), b = to_float(qr[i + half]);
+            qr[i] = from_float<T>(a * cs[i] - b * sn[i]);
+            qr[i + half] = from_float<T>(b * cs[i] + a * sn[i]);
+        }
+        return;
+    }
     const int slot = slots ? slots[n] : -1;
     float ss = 0.f;
     for (int c = threadIdx.x; c < rank; c += blockDim.x) {
@@ -46,14 +57,6 @@ __global__ void latent_kv_post_kernel(T* __restrict__ qd, long ld, int H, int d,
             row[rank + i] = from_float<T>(v);
         }
     }
-    // every head's rotated query part, in place (a pair is read and written by one thread)
-    for (int e = threadIdx.x; e < H * half; e += blockDim.x) {
-        const int h = e / half, i = e % half;
-        T* qr = q + (size_t)h * (d + r) + d;
-        const float a = to_float(qr[i]), b = to_float(qr[i + half]);
-        qr[i] = from_float<T>(a * cs[i] - b * sn[i]);
-        qr[i + half] = from_float<T>(b * cs[i] + a * sn[i]);
-    }
 }
 
 LLMP_API int llmp_latent_kv_post(void* qd, int dtype, long ld, int H, int d, int r, int rank, const void* norm_w, int norm_w_dtype,
@@ -63,11 +66,12 @@ LLMP_API int llmp_latent_kv_post(void* qd, int dtype, long ld, int H, int d, int
     LLMP_REQUIRE(H > 0 && d >= 0 && r >= 0 && rank > 0 && rot_dims >= 0 && rot_dims <= r && rot_dims % 2 == 0,
                  "latent_kv_post: bad sizes heads=%d dim=%d rot=%d rank=%d rotated=%d", H, d, r, rank, rot_dims);
     LLMP_REQUIRE(rot_dims == 0 || (cos_t && sin_t), "latent_kv_post: a rotation needs its tables");
+    const bool half = rot_dims > 0;                // a block for a token's cached row and one for its queries' rotation
     if (dtype == LLMP_F32)
-        llmp_launch_dependent(latent_kv_post_kernel<float>, dim3(N), dim3(128), 0, stream, (float*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
+        llmp_launch_dependent(latent_kv_post_kernel<float>, dim3(N, half ? 2 : 1), dim3(128), 0, stream, (float*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
                                                             sin_t, rot_dims, slots, (float*)pages);
     else
-        llmp_launch_dependent(latent_kv_post_kernel<bf16>, dim3(N), dim3(128), 0, stream, (bf16*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
+        llmp_launch_dependent(latent_kv_post_kernel<bf16>, dim3(N, half ? 2 : 1), dim3(128), 0, stream, (bf16*)qd, ld, H, d, r, rank, norm_w, norm_w_dtype == LLMP_BF16, eps, cos_t,
                                                            sin_t, rot_dims, slots, (bf16*)pages);
     return llmp_check_launch("latent_kv_post");
 }

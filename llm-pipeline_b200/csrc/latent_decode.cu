@@ -228,8 +228,9 @@ __global__ void __launch_bounds__(LD_THREADS, 1) latent_decode_kernel(const Late
 }
 
 // out = sum_s 2^(m_s - m) o_s / sum_s 2^(m_s - m) l_s over the ranges that hold keys the token sees, in ascending order. A block per
-// (token, head); the ranges' weights are made once, four columns a thread.
-constexpr int LD_MAX_RANGES = 1024;
+// (token, head), four columns a thread. The first LD_MERGE_AHEAD ranges' sums are asked for beside the maxima and the sums of weights
+// (one load after another took 6.0 us of a decoding layer's 53).
+constexpr int LD_MAX_RANGES = 1024, LD_MERGE_AHEAD = 16;
 __global__ void __launch_bounds__(128) latent_decode_merge_kernel(const LatentDecodeArgs a, int rank) {
     __shared__ float weight[LD_MAX_RANGES], part[8];
     const int n = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
@@ -237,30 +238,50 @@ __global__ void __launch_bounds__(128) latent_decode_merge_kernel(const LatentDe
     pdl_wait();
     const int ranges = (a.ctx_len[n] - 1) / a.range_keys + 1;
     const size_t step = (size_t)a.N * a.H, first = (size_t)n * a.H + h;
+    const float* from = a.part_o + first * rank + tid * 4;
+    float4 v[LD_MERGE_AHEAD];
+#pragma unroll
+    for (int s = 0; s < LD_MERGE_AHEAD; ++s)
+        v[s] = s < ranges && tid * 4 < rank ? *reinterpret_cast<const float4*>(from + s * step * rank) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float sk = a.sink ? a.sink[h] * 1.4426950408889634f : -INFINITY;
-    float m = sk;
-    for (int s = tid; s < ranges; s += 128) m = fmaxf(m, a.part_ml[(s * step + first) * 2]);
+    float m = sk, l = 0.f;
+    const float2 own = tid < ranges ? *reinterpret_cast<const float2*>(a.part_ml + (tid * step + first) * 2) : make_float2(-INFINITY, 0.f);
+    m = fmaxf(m, own.x);
+    for (int s = tid + 128; s < ranges; s += 128) m = fmaxf(m, a.part_ml[(s * step + first) * 2]);
     m = warp_max(m);
     if ((tid & 31) == 0) part[tid >> 5] = m;
     __syncthreads();
     m = fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3]));
-    for (int s = tid; s < ranges; s += 128) weight[s] = m > -INFINITY ? ld_ex2(a.part_ml[(s * step + first) * 2] - m) : 0.f;
-    __syncthreads();
-    float l = a.sink ? ld_ex2(sk - m) : 0.f;
-    for (int s = 0; s < ranges; ++s) l = fmaf(weight[s], a.part_ml[(s * step + first) * 2 + 1], l);
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    for (int c = tid * 4; c < rank; c += 512) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int s = 0; s < ranges; ++s) {
-            const float4 v = *reinterpret_cast<const float4*>(a.part_o + (s * step + first) * rank + c);
-            const float w = weight[s];
-            acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
-        }
-        unsigned* o = reinterpret_cast<unsigned*>(a.out + (size_t)n * a.o_t + (size_t)h * a.o_h + c);
-        o[0] = ld_pack(acc.x * inv, acc.y * inv);
-        o[1] = ld_pack(acc.z * inv, acc.w * inv);
+    if (tid < ranges) {
+        weight[tid] = m > -INFINITY ? ld_ex2(own.x - m) : 0.f;
+        l = weight[tid] * own.y;
     }
+    for (int s = tid + 128; s < ranges; s += 128) {
+        const float2 other = *reinterpret_cast<const float2*>(a.part_ml + (s * step + first) * 2);
+        weight[s] = m > -INFINITY ? ld_ex2(other.x - m) : 0.f;
+        l = fmaf(weight[s], other.y, l);
+    }
+    l = warp_sum(l);
+    if ((tid & 31) == 0) part[4 + (tid >> 5)] = l;
+    __syncthreads();
+    l = ((part[4] + part[5]) + (part[6] + part[7])) + (a.sink ? ld_ex2(sk - m) : 0.f);
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    if (tid * 4 >= rank) return;                                 // (the latent has up to 512 columns: four a thread)
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int s = 0; s < LD_MERGE_AHEAD; ++s) {
+        const float w = s < ranges ? weight[s] : 0.f;
+        acc.x = fmaf(w, v[s].x, acc.x); acc.y = fmaf(w, v[s].y, acc.y); acc.z = fmaf(w, v[s].z, acc.z); acc.w = fmaf(w, v[s].w, acc.w);
+    }
+#pragma unroll 8
+    for (int s = LD_MERGE_AHEAD; s < ranges; ++s) {
+        const float4 u = *reinterpret_cast<const float4*>(from + s * step * rank);
+        const float w = weight[s];
+        acc.x = fmaf(w, u.x, acc.x); acc.y = fmaf(w, u.y, acc.y); acc.z = fmaf(w, u.z, acc.z); acc.w = fmaf(w, u.w, acc.w);
+    }
+    unsigned* o = reinterpret_cast<unsigned*>(a.out + (size_t)n * a.o_t + (size_t)h * a.o_h + tid * 4);
+    o[0] = ld_pack(acc.x * inv, acc.y * inv);
+    o[1] = ld_pack(acc.z * inv, acc.w * inv);
 }
 
 size_t ld_smem(int rank, int rot) { return sizeof(bf16) * ((size_t)(LD_ROWS + LD_KEYS) * (rank + rot + 8) + 2 * LD_ROWS * LD_PS); }

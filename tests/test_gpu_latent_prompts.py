@@ -185,3 +185,24 @@ def test_single_tokens(ctx, heads, rank, rot, sink):
             p = torch.softmax(score, dim=1)[:, :ctx[r]]
             v = rows[r][:, :rank].double()
             assert ((out[r].double().cpu() - p @ v).abs() <= 2.0 ** -7 * (1 + 1 / 8) * (p @ v.abs())).all(), (r, longest)
+
+
+@pytest.mark.parametrize("batch,rows,n,k", [(3, 1, 16, 8), (2, 8, 64, 128), (2, 9, 65, 136), (4, 16, 512, 256), (3, 7, 130, 264), (2, 16, 15, 512), (1, 3, 17, 1048)], ids=str)
+def test_few_rows_of_several_heads(batch, rows, n, k):
+    """The heads' maps of a decode step's rows around the tiles of 16 weight rows and 8 rows, runs of 32 of K and the split of a long K, on
+    transposed views with other entries between; float64 within bfloat16's rounding of the result (half of the last of 7 stored bits: 2^-8) and float32 sums. A row has the bits
+    that it has alone."""
+    from llm_pipeline_b200.ops import kernels
+    gen = torch.Generator().manual_seed(rows * n + k)
+    x = torch.randn(rows, batch, k + 8, generator=gen).to(torch.bfloat16).to(DEV)
+    w = torch.randn(batch, n, k, generator=gen).to(torch.bfloat16).to(DEV)
+    out = torch.full((rows, batch, n + 3), 7.0, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_batched(x[:, :, :k].transpose(0, 1), w, out[:, :, :n].transpose(0, 1))
+    want = torch.einsum("mbk,bnk->mbn", x[:, :, :k].double(), w.double())
+    scale = torch.einsum("mbk,bnk->mbn", x[:, :, :k].double().abs(), w.double().abs())
+    assert ((out[:, :, :n].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * scale).all()
+    assert (out[:, :, n:] == 7.0).all()
+    for m in {0, rows - 1}:
+        alone = torch.empty(1, batch, n, dtype=torch.bfloat16, device=DEV)
+        kernels.gemm_batched(x[m:m + 1, :, :k].transpose(0, 1), w, alone.transpose(0, 1))
+        assert torch.equal(alone[0], out[m, :, :n])
