@@ -97,6 +97,7 @@ __device__ __forceinline__ unsigned cm_pack(float lo, float hi) {
     return *reinterpret_cast<const unsigned*>(&v);
 }
 
+constexpr int CM_MERGE_AHEAD = 8;
 constexpr float CM_LOG2E = 1.4426950408889634f;
 
 // the lowest key (kept first tokens aside) that the token at `pos` sees
@@ -114,8 +115,9 @@ __global__ void __launch_bounds__(CM_THREADS, 2) capped_attention_mma_kernel(con
     constexpr int D = D16 * 16, DV = V16 * 16;
     constexpr int RS = D + DV;                                   // a cached row
     constexpr int QSTRIDE = D + 8, KSTRIDE = RS + 8;             // padded rows: conflict-free ldmatrix
-    bf16* Qs = reinterpret_cast<bf16*>(cm_smem);                 // [CM_ROWS][QSTRIDE]
-    bf16* ring = Qs + CM_ROWS * QSTRIDE;                         // [stages][CM_KEYS][KSTRIDE]
+    bf16* Qs = reinterpret_cast<bf16*>(cm_smem);                 // [q_rows][QSTRIDE]
+    const int q_rows = p.split ? 16 : CM_ROWS;
+    bf16* ring = Qs + q_rows * QSTRIDE;                          // [stages][CM_KEYS][KSTRIDE]
     constexpr int STAGE_ELEMS = CM_KEYS * KSTRIDE;
     __shared__ long long key_off[4][CM_KEYS];
     const bool split = p.split != 0;                             // four warps on the 16 rows of a one-token tile
@@ -126,8 +128,8 @@ __global__ void __launch_bounds__(CM_THREADS, 2) capped_attention_mma_kernel(con
     const int per_tile = p.nkv * p.head_chunks;
     const int tile = p.num_tiles - 1 - (int)(blockIdx.x / (unsigned)per_tile);      // long tiles first
     const int in_tile = (int)(blockIdx.x % (unsigned)per_tile);
-    const int r = p.tile_req[tile];
-    const int tok0 = p.tile_tok0[tile];
+    const int r = p.tile_req ? p.tile_req[tile] : tile;          // null: one token a request, tile i is request i's
+    const int tok0 = p.tile_req ? p.tile_tok0[tile] : 0;
     const int kvh = in_tile / p.head_chunks, chunk = in_tile % p.head_chunks;
     const int G = p.nq / p.nkv;
     const int hpc = p.heads_per_cta;
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(CM_THREADS, 2) capped_attention_mma_kernel(con
 
     // query rows: row = token * hpc + head
     constexpr int QVEC = D / 8;
-    for (int e = tid; e < CM_ROWS * QVEC; e += CM_THREADS) {
+    for (int e = tid; e < q_rows * QVEC; e += CM_THREADS) {
         const int row = e / QVEC, c = (e % QVEC) * 8;
         const int tl = row / hpc, h = row % hpc;
         const bool ok = tl < ntok && h < heads;
@@ -456,14 +458,25 @@ __global__ void __launch_bounds__(CM_THREADS, 2) capped_attention_mma_kernel(con
                 const int head = kvh * G + head0 + h;
                 const float* src = p.scratch + (n * p.nq + head) * (DV + 2);
                 const size_t step = (size_t)p.total_tokens * p.nq * (DV + 2);
-                float m = -INFINITY;
-                for (int s0 = 0; s0 < seg_needed; ++s0) m = fmaxf(m, __ldcg(src + s0 * step + DV));
-                float l = 0.f, a = 0.f, b = 0.f;
-                for (int s0 = 0; s0 < seg_needed; ++s0) {
-                    const float2 ml = __ldcg(reinterpret_cast<const float2*>(src + s0 * step + DV));
-                    const float2 v = __ldcg(reinterpret_cast<const float2*>(src + s0 * step + c));
-                    const float w = ml.x > -INFINITY ? cm_ex2(ml.x - m) : 0.f;
-                    l = fmaf(ml.y, w, l); a = fmaf(v.x, w, a); b = fmaf(v.y, w, b);
+                float m = -INFINITY, l = 0.f, a = 0.f, b = 0.f;
+                for (int s0 = 0; s0 < seg_needed; s0 += CM_MERGE_AHEAD) {      // so many segments' sums asked for at once
+                    float2 ml[CM_MERGE_AHEAD], v[CM_MERGE_AHEAD];
+#pragma unroll
+                    for (int i = 0; i < CM_MERGE_AHEAD; ++i) {
+                        const bool have = s0 + i < seg_needed;
+                        ml[i] = have ? __ldcg(reinterpret_cast<const float2*>(src + (s0 + i) * step + DV)) : make_float2(-INFINITY, 0.f);
+                        v[i] = have ? __ldcg(reinterpret_cast<const float2*>(src + (s0 + i) * step + c)) : make_float2(0.f, 0.f);
+                    }
+                    float top = m;
+#pragma unroll
+                    for (int i = 0; i < CM_MERGE_AHEAD; ++i) top = fmaxf(top, ml[i].x);
+                    const float kept = m > -INFINITY ? cm_ex2(m - top) : 0.f;
+                    m = top; l *= kept; a *= kept; b *= kept;
+#pragma unroll
+                    for (int i = 0; i < CM_MERGE_AHEAD; ++i) {
+                        const float w = ml[i].x > -INFINITY ? cm_ex2(ml[i].x - m) : 0.f;
+                        l = fmaf(ml[i].y, w, l); a = fmaf(v[i].x, w, a); b = fmaf(v[i].y, w, b);
+                    }
                 }
                 const float inv = l > 0.f ? 1.f / l : 0.f;
                 a *= inv; b *= inv;
@@ -509,7 +522,7 @@ bool cm_size_served(int d, int dv) {
 
 template <int D16, int V16>
 int launch_capped_mma(const CappedMmaParams& p, unsigned grid, cudaStream_t stream) {
-    const size_t q_bytes = sizeof(bf16) * (size_t)CM_ROWS * (D16 * 16 + 8);
+    const size_t q_bytes = sizeof(bf16) * (size_t)(p.split ? 16 : CM_ROWS) * (D16 * 16 + 8);
     const size_t stage = sizeof(bf16) * (size_t)CM_KEYS * (D16 * 16 + V16 * 16 + 8);
     // two buffers for prompts, so that two blocks share an SM; four for steps of single tokens, whose few blocks are each a
     // chain of copies that should be under way early

@@ -110,6 +110,7 @@ _SIGNATURES = {
                           _I, _P, _P],
     "llmp_sig_qkv_post": [_P, _L, _P, _I, _P, _P, _I, _P, _I, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
     "llmp_sigmoid_attention": [_P, _L, _P, _I, _P, _I, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
+    "llmp_sigmoid_decode": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "llmp_sigmoid_attention_mma": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "llmp_wkv_shift": [_P, _P, _P, _L, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "llmp_wkv_decay": [_P, _L, _P, _P, _P, _I, _I, _I, _P],
@@ -1853,6 +1854,37 @@ def sigmoid_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Te
     return out
 
 
+SIGMOID_DECODE_BLOCKS_PER_SM = 1     # key ranges grow once the blocks would be more (a block fills an SM)
+
+
+def sigmoid_decode_keys(dtype: torch.dtype, heads: int, kv_heads: int, dim: int, vdim: int) -> int:
+    """Keys that ``sigmoid_decode`` takes at a time (its ranges are multiples), or 0 where it does not serve the sizes."""
+    return int(library().llmp_sigmoid_decode_keys(heads, kv_heads, dim, vdim)) if dtype == torch.bfloat16 else 0
+
+
+def sigmoid_decode(q: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor, ctx_len: torch.Tensor, talk: torch.Tensor, head_bias: torch.Tensor,
+                   out: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, scale: float, softcap: float, segments: int,
+                   segment_keys: int) -> torch.Tensor:
+    """``sigmoid_attention`` for steps of one token a request (csrc/sigmoid_decode.cu): row n of the bfloat16 queries is request n's.
+    ``segments`` > 1: ranges of ``segment_keys`` keys (a multiple of ``sigmoid_decode_keys``) go to blocks of their own; together they must
+    cover the most keys a request sees."""
+    N = q.shape[0]
+    _need(q.dtype == out.dtype == pages.dtype == torch.bfloat16 and q.shape == (N, heads * dim) and q.stride(1) == 1 and
+          out.shape == (N, heads * vdim) and out.stride(1) == 1, "sigmoid_decode takes bfloat16 queries, pages and output of matching shapes")
+    _need(pages.dim() == 4 and pages.is_contiguous() and pages.shape[1] == kv_heads and pages.shape[3] == dim + vdim,
+          "sigmoid_decode: pages must be [pages, kv_heads, page_size, dim + vdim]")
+    _need(talk.dtype == torch.float32 and talk.is_contiguous() and talk.shape == (heads, heads) and head_bias.dtype == torch.float32 and
+          head_bias.is_contiguous() and head_bias.numel() == heads, "sigmoid_decode takes a float32 head mix [heads, heads] and bias [heads]")
+    _need(tables.dtype == torch.int32 and tables.dim() == 2 and tables.is_contiguous() and tables.shape[0] == N, "block tables must be dense int32 [requests, width]")
+    _i32(ctx_len, "ctx_len")
+    _need(ctx_len.numel() == N, "sigmoid_decode takes one token a request")
+    partial = torch.empty((N, segments, heads * vdim), dtype=torch.float32, device=q.device) if segments > 1 else None
+    _call("llmp_sigmoid_decode", _ptr(q), q.stride(0), _ptr(pages), _ptr(tables), tables.shape[1], _ptr(ctx_len), _ptr(talk), _ptr(head_bias),
+          _ptr(out), out.stride(0), _ptr(partial), int(segments), int(segment_keys), N, heads, kv_heads, dim, vdim, pages.shape[2], float(scale),
+          float(softcap or 0.0), _stream())
+    return out
+
+
 def xielu(z: torch.Tensor, bias: Optional[torch.Tensor], a_pos: float, a_neg: float, out: torch.Tensor) -> torch.Tensor:
     """out = f(z + bias) with f(v) = a_pos v^2 + v / 2 for v > 0 and a_neg (exp(v) - 1 - v) + v / 2 otherwise; ``z`` float32."""
     N, F = z.shape
@@ -1986,7 +2018,7 @@ def capped_attention(q: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor,
 
 
 CAPPED_TILE_KEYS = 64                # csrc/capped_attention_mma.cu: keys of a tile
-CAPPED_SEGMENT_KEYS = 256            # keys of a segment (a multiple of the tile)
+CAPPED_SEGMENT_KEYS = 256            # keys of a segment (a multiple of the tile) where the caller names none
 
 
 def capped_mma_supports(dtype: torch.dtype, dim: int, vdim: int) -> bool:
@@ -2007,14 +2039,14 @@ def capped_mma_tokens_per_tile(num_heads: int, num_kv_heads: int) -> int:
 
 
 def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor, q_start: torch.Tensor, ctx_len: torch.Tensor,
-                         tile_req: torch.Tensor, tile_tok0: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_heads: int, dim: int,
+                         tile_req: Optional[torch.Tensor], tile_tok0: Optional[torch.Tensor], out: torch.Tensor, num_heads: int, num_kv_heads: int, dim: int,
                          vdim: int, window: int, keep_first: int, scale: float, softcap: float, slopes: Optional[torch.Tensor] = None,
                          sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, split: bool = False, chunk: int = 0,
-                         segments: int = 0) -> torch.Tensor:
+                         segments: int = 0, segment_keys: int = 0) -> torch.Tensor:
     """``capped_attention`` on the tensor cores for bfloat16 (csrc/capped_attention_mma.cu). ``tile_req``/``tile_tok0``: the work
-    list (request and first token of every tile of ``capped_mma_tokens_per_tile`` tokens). ``split``: every tile is one token,
+    list (request and first token of every tile of ``capped_mma_tokens_per_tile`` tokens; None with ``split``: tile i is request i's). ``split``: every tile is one token,
     and the four warps of a block share its keys; ``segments`` > 0 then cuts the keys of a row into that many runs of
-    ``CAPPED_SEGMENT_KEYS`` with blocks of their own, whose sums the block that ends last adds up (it must cover the most keys a
+    ``segment_keys`` (a multiple of the tile; ``CAPPED_SEGMENT_KEYS`` when 0) with blocks of their own, whose sums the block that ends last adds up (it must cover the most keys a
     token sees, rounded up to whole tiles at both ends)."""
     N = q.shape[0]
     _need(q.dtype == torch.bfloat16 and pages.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "capped_attention_mma takes bfloat16")
@@ -2024,22 +2056,24 @@ def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Ten
           "capped attention pages have the wrong layout")
     _sink(sink, num_heads); _sink(slopes, num_heads)
     gate_heads = _capped_gate(gate, N, num_heads, vdim)
-    for t, name in ((tables, "tables"), (q_start, "q_start"), (ctx_len, "ctx_len"), (tile_req, "tile_req"), (tile_tok0, "tile_tok0")):
+    for t, name in ((tables, "tables"), (q_start, "q_start"), (ctx_len, "ctx_len")) + ((() if tile_req is None else ((tile_req, "tile_req"), (tile_tok0, "tile_tok0")))):
         _i32(t, name)
-    _need(not split or tile_req.numel() == N, "warps share a tile's keys only in steps of one token a request")
+    tiles = N if tile_req is None else tile_req.numel()
+    _need(split or tile_req is not None, "capped_attention_mma: portions need a work list")
+    _need(not split or tiles == N, "warps share a tile's keys only in steps of one token a request")
     scratch = counters = None
     if split:
         # at most one counter per (tile, kv head, chunk of heads); asked for in every such step, so that they exist before a step
         # is captured whose eager run needed no segments
-        counters = attention_counters(q.device, tile_req.numel() * num_heads)
+        counters = attention_counters(q.device, tiles * num_heads)
     if segments > 0:
         _need(split, "capped_attention_mma: segments are for steps of one token a request")
         scratch = torch.empty(segments * N * num_heads * (vdim + 2), dtype=torch.float32, device=q.device)
     _call("llmp_capped_attention_mma", _ptr(q), q.stride(0), _ptr(out), out.stride(0), _ptr(pages), _ptr(tables), tables.shape[1],
-          _ptr(q_start), _ptr(ctx_len), _ptr(tile_req), _ptr(tile_tok0), tile_req.numel(), _ptr(slopes), _ptr(sink), _ptr(gate),
+          _ptr(q_start), _ptr(ctx_len), _ptr(tile_req), _ptr(tile_tok0), tiles, _ptr(slopes), _ptr(sink), _ptr(gate),
           gate.stride(0) if gate is not None else 0, 1 if gate_heads else 0, num_heads, num_kv_heads, dim, vdim, pages.shape[2],
           int(window), int(keep_first), int(chunk), float(scale), float(softcap), 1 if split else 0, int(segments),
-          CAPPED_SEGMENT_KEYS if segments > 0 else 0, _ptr(scratch), _ptr(counters), N, _stream())
+          (int(segment_keys) or CAPPED_SEGMENT_KEYS) if segments > 0 else 0, _ptr(scratch), _ptr(counters), N, _stream())
     return out
 
 

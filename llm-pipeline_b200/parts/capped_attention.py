@@ -109,35 +109,37 @@ class CappedAttention(Mixer):
             return ("q",)
         return ("q", "k") if self.values_are_keys else ("q", "k", "v")
 
-    def _segments(self, ctx) -> int:
-        """Into how many segments a step of single tokens cuts its keys (0: not at all)."""
+    def _segments(self, ctx):
+        """(segments, keys of a segment) into which a step of single tokens cuts its keys (0, 0: not at all): as many as fill the places of
+        the blocks, of which an SM holds two, once (16 requests of 4 heads over 1,088 keys: 4 of 320 keys in one round of 256 blocks, where
+        5 of 256 keys are 320), of two tiles or more."""
         if ctx.max_q_len != 1:
-            return 0
+            return 0, 0
         longest = ctx.decode_ctx_bound or ctx.max_ctx_len
         tile = kernels.CAPPED_TILE_KEYS
         bounds = [n for n in (self.window, self.chunk) if n]
         reach = min([longest] + [n + tile for n in bounds])            # from the tile a row's keys begin in
         blocks = ctx.num_requests * self.num_kv_heads * -(-(self.num_heads // self.num_kv_heads) // 16)
         if reach < self.SEGMENTS_MIN_KEYS or blocks >= self.SEGMENTS_BELOW_BLOCKS_PER_SM * kernels.sm_count():
-            return 0
-        return -(-reach // kernels.CAPPED_SEGMENT_KEYS)
+            return 0, 0
+        most = max(1, 2 * kernels.sm_count() // blocks)
+        keys = tile * max(2, -(-reach // (tile * most)))
+        return -(-reach // keys), keys
 
     def _name(self, key: str) -> str:
         return f"{self.prefix}.{self.names[key]}"
 
     def _tiles(self, ctx, per_tile: int):
+        """(request, first token) of every tile; None: a step of single tokens, whose tile r is request r."""
+        if ctx.max_q_len == 1:
+            return None, None
         key = ("capped_attention_tiles", per_tile)
         tiles = ctx.memo.get(key)
         if tiles is None:
-            if ctx.max_q_len == 1:
-                # one token a request: tile r is request r (made on the device, so that a captured step holds no copy from the host)
-                tiles = (torch.arange(ctx.num_requests, dtype=torch.int32, device=ctx.device),
-                         torch.zeros(ctx.num_requests, dtype=torch.int32, device=ctx.device))
-            else:
-                req, tok0, _seg, _slot, _places = AttentionPolicy.plan_items(ctx.starts, ctx.q_lens, per_tile, 0, 1, 1, kernels.sm_count())
-                host = torch.tensor([req, tok0], dtype=torch.int32).pin_memory()
-                dev = host.to(ctx.device, non_blocking=True)
-                tiles = (dev[0].contiguous(), dev[1].contiguous())
+            req, tok0, _seg, _slot, _places = AttentionPolicy.plan_items(ctx.starts, ctx.q_lens, per_tile, 0, 1, 1, kernels.sm_count())
+            host = torch.tensor([req, tok0], dtype=torch.int32).pin_memory()
+            dev = host.to(ctx.device, non_blocking=True)
+            tiles = (dev[0].contiguous(), dev[1].contiguous())
             ctx.memo[key] = tiles
         return tiles
 
@@ -209,9 +211,10 @@ class CappedAttention(Mixer):
             # bfloat16 and sizes the tensor-core kernel has instances of: prompts in tiles of 64 rows (token, head of a group),
             # single tokens with the four warps of a block sharing the keys
             tile_req, tile_tok0 = self._tiles(ctx, kernels.capped_mma_tokens_per_tile(self.num_heads, self.num_kv_heads))
+            segments, segment_keys = self._segments(ctx)
             kernels.capped_attention_mma(q, cache.pages, tables, ctx.q_start, ctx.ctx_len, tile_req, tile_tok0, out, *sizes, slopes=self.slopes,
                                          sink=self.sinks, gate=gate, split=ctx.max_q_len == 1, chunk=self.chunk or 0,
-                                         segments=self._segments(ctx))
+                                         segments=segments, segment_keys=segment_keys)
         else:
             kernels.capped_attention(q, cache.pages, tables, ctx.token_request, ctx.positions, out, *sizes, slopes=self.slopes, sink=self.sinks,
                                      gate=gate, chunk=self.chunk or 0)

@@ -66,6 +66,7 @@ class SigmoidAttention(Mixer):
         self.names.update(names or {})
         self.w_qkv = self.b_qkv = self.w_o = self.talk = self.pb = None
         self.compute_dtype = None      # the type of the queries and pages, known once the weights are loaded
+        self._single = None            # keys of a tile of the kernel for single tokens, 0: none serves these sizes
         self._mma = None               # whether the tensor-core kernel takes this mixer's sizes in that type
 
     def cache_spec(self) -> HeadRowPagesSpec:
@@ -77,8 +78,25 @@ class SigmoidAttention(Mixer):
     def graph_key(self, shape) -> int:
         """The key ranges a step of single tokens takes (their number and size): a captured step holds the grid it was
         captured with."""
+        if self._decode_keys():
+            return 0                           # its ranges follow from the bound on the context, which the block tables' width gives
         segments, keys = self._segments(shape.num_requests, shape.longest)
         return segments | keys << 20
+
+    def _decode_keys(self) -> int:
+        """Keys of a tile of the kernel for single tokens, 0 where that does not serve this mixer's sizes in its type."""
+        if self._single is None:
+            self._single = kernels.sigmoid_decode_keys(self.compute_dtype, self.num_heads, self.num_kv_heads, self.dim, self.vdim)
+        return self._single
+
+    def _decode_ranges(self, tokens: int, longest: int):
+        """(number of key ranges, keys of a range) of a step of single tokens: one tile a range until the blocks are many."""
+        tile = self._decode_keys()
+        most = max(1, min(self.SEGMENTS_MAX_BYTES // (4 * tokens * self.num_heads * self.vdim),
+                          kernels.SIGMOID_DECODE_BLOCKS_PER_SM * kernels.sm_count() // tokens))
+        tiles = -(-longest // tile)
+        keys = tile * -(-tiles // most)
+        return -(-longest // keys), keys
 
     def _segments(self, tokens: int, longest: int):
         """(number of key ranges, keys of a range) for a step of ``tokens`` new tokens whose longest context is ``longest``."""
@@ -144,7 +162,7 @@ class SigmoidAttention(Mixer):
         self.w_qkv = torch.cat([get(self._name(n), "matrix") for n in ("q", "k", "v")], dim=0).contiguous()
         self.w_o = get(self._name("o"), "matrix").contiguous()
         device = self.w_o.device
-        self.compute_dtype, self._mma = self.w_o.dtype, None
+        self.compute_dtype, self._mma, self._single = self.w_o.dtype, None, None
         if self.bias:
             self.b_qkv = torch.cat([get(self._name(n) + ".b", "vector").float() for n in ("q", "k", "v")]).contiguous()
         self.talk = (get(self._name("talk"), "vector").float().contiguous() if self.head_mix
@@ -164,7 +182,12 @@ class SigmoidAttention(Mixer):
         kernels.sig_qkv_post(qkv, self.b_qkv, cos, sin, self.rotary_dim, q, ctx.slot_mapping[cache.group] if cache.writes else None,
                              cache.pages if cache.writes else None, self.num_heads, self.num_kv_heads, self.dim, self.vdim)
         out = torch.empty((N, self.num_heads * self.vdim), dtype=x.dtype, device=x.device)
-        segments, segment_keys = self._segments(N, ctx.decode_ctx_bound or ctx.max_ctx_len)
+        longest = ctx.decode_ctx_bound or ctx.max_ctx_len
+        if ctx.max_q_len == 1 and self._decode_keys():
+            kernels.sigmoid_decode(q, cache.pages, ctx.block_tables[cache.group], ctx.ctx_len, self.talk, self.pb, out, self.num_heads,
+                                   self.num_kv_heads, self.dim, self.vdim, self.scale, self.softcap, *self._decode_ranges(N, longest))
+            return linear(out, self.w_o, out_dtype=torch.float32), None
+        segments, segment_keys = self._segments(N, longest)
         sizes = (self.num_heads, self.num_kv_heads, self.dim, self.vdim, self.scale, self.softcap, segments)
         if self._mma and q.dtype == torch.bfloat16:
             tile_req, tile_tok0 = self._tiles(ctx)

@@ -462,6 +462,44 @@ def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, ca
     return results, want
 
 
+@pytest.mark.parametrize("sizes", [(4, 2, 16, 32, 0.0), (16, 4, 128, 128, 3.0), (12, 12, 32, 64, 0.0), (16, 1, 64, 64, 30.0), (8, 8, 128, 128, 0.0), (6, 3, 96, 64, 5.0), (1, 1, 48, 128, 1.0)], ids=str)
+def test_sigmoid_attention_of_single_tokens(sizes):
+    """The kernel for single tokens: contexts around a tile's and a range's end in one step, over shuffled pages with garbage in the
+    others, keys in one block and in ranges of one, two and three tiles. The mixed weights are rounded to bfloat16 and so is the result: 2^-8
+    of the sizes of its terms each."""
+    from llm_pipeline_b200.ops import kernels
+    heads, kv_heads, dim, vdim, cap = sizes
+    tile = kernels.sigmoid_decode_keys(torch.bfloat16, heads, kv_heads, dim, vdim)
+    assert tile in (32, 64)
+    gen, dev, page, scale = torch.Generator().manual_seed(sum(sizes[:4])), "cuda", 16, dim ** -0.5
+    ctx = [1, tile - 1, tile, tile + 1, 2 * tile, 3 * tile + 5, 7 * tile - 3]
+    need = [-(-c // page) for c in ctx]
+    order = torch.randperm(sum(need) + 3, generator=gen).tolist()
+    pages = torch.full((sum(need) + 3, kv_heads, page, dim + vdim), 7.0)
+    tables = torch.full((len(ctx), max(need)), -1, dtype=torch.int32)
+    q = torch.randn(len(ctx), heads, dim, generator=gen).to(torch.bfloat16)
+    talk, pb = torch.eye(heads) * 0.6 + torch.randn(heads, heads, generator=gen) * 0.4, torch.randn(heads, generator=gen) * 0.5 - 1.0
+    kv_of, want, size = torch.arange(heads) // (heads // kv_heads), [], []
+    for r, c in enumerate(ctx):
+        rows = torch.randn(c, kv_heads, dim + vdim, generator=gen).to(torch.bfloat16).float()
+        for i in range(need[r]):
+            tables[r, i] = order.pop()
+            part = rows[i * page:(i + 1) * page]
+            pages[tables[r, i], :, :part.shape[0]] = part.transpose(0, 1)
+        s = torch.einsum("hd,jhd->hj", q[r].double(), rows[:, kv_of, :dim].double()) * scale
+        w = torch.sigmoid((cap * torch.tanh(s / cap) if cap else s) + pb.double()[:, None])
+        m, v = talk.double() @ w, rows[:, kv_of, dim:].double()
+        want.append(torch.einsum("hj,jhv->hv", m, v).reshape(-1))
+        size.append(torch.einsum("hj,jhv->hv", m.abs(), v.abs()).reshape(-1))
+    want, size = torch.stack(want), torch.stack(size)
+    args = (q.reshape(len(ctx), -1).to(dev), pages.to(torch.bfloat16).to(dev), tables.to(dev), torch.tensor(ctx, dtype=torch.int32, device=dev), talk.to(dev),
+            pb.to(dev))
+    for keys in (8 * tile, tile, 2 * tile, 3 * tile):
+        out = torch.empty(len(ctx), heads * vdim, dtype=torch.bfloat16, device=dev)
+        kernels.sigmoid_decode(*args, out, heads, kv_heads, dim, vdim, scale, cap, -(-max(ctx) // keys), keys)
+        assert ((out.cpu().double() - want).abs() <= 2.0 ** -8 * (size + want.abs())).all(), keys
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("sizes", [(4, 2, 16, 24, 0.0), (3, 3, 12, 20, 2.0), (6, 1, 48, 48, 8.0), (2, 2, 128, 64, 0.0), (32, 2, 16, 16, 30.0), (4, 2, 16, 32, 0.0), (6, 3, 96, 64, 5.0),
                                    (16, 4, 128, 128, 3.0), (12, 12, 32, 96, 0.0),
