@@ -311,12 +311,19 @@ int launch_capped(const CappedArgs& a, int N, cudaStream_t stream) {
 
 }  // namespace
 
+// qkv_rows_post.cu
+LLMP_API int llmp_qkv_rows_post(const float* qkv, long qkv_t, const void* bias, int bias_bf16, const float* cos_t, const float* sin_t, int rot,
+                                float v_eps, int v_norm, void* q_out, int dtype, long q_out_t, const int* slots, void* pages, int page_size, int N,
+                                int H, int G, int d, int dv, cudaStream_t stream);
+
 LLMP_API int llmp_capped_qkv_post(const float* qkv, long qkv_t, const void* bias, int bias_dtype, float v_eps, int v_norm, void* q_out,
                                   int dtype, long q_out_t, const int* slots, void* pages, int page_size, int N, int H, int G, int d,
                                   int dv, cudaStream_t stream) {
     if (N <= 0) return 0;
     LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && d > 0 && dv > 0, "capped_qkv_post: bad sizes heads=%d kv=%d dim=%d vdim=%d", H, G, d, dv);
     LLMP_REQUIRE(pages == nullptr || page_size > 0, "capped_qkv_post: pages without a page size");
+    if (!llmp_qkv_rows_post(qkv, qkv_t, bias, bias_dtype == LLMP_BF16, nullptr, nullptr, 0, v_eps, v_norm, q_out, dtype, q_out_t, slots, pages,
+                            page_size, N, H, G, d, dv, stream)) return llmp_check_launch("capped_qkv_post");
     if (dtype == LLMP_F32)
         llmp_launch_dependent(capped_qkv_post_kernel<float>, dim3(N), dim3(256), 0, stream, qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), v_eps, v_norm, (float*)q_out,
                                                              q_out_t, slots, (float*)pages, page_size, H, G, d, dv);

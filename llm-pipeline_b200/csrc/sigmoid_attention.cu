@@ -182,6 +182,11 @@ __global__ void sigmoid_segments_kernel(const float* __restrict__ partial, const
 
 }  // namespace
 
+// qkv_rows_post.cu
+LLMP_API int llmp_qkv_rows_post(const float* qkv, long qkv_t, const void* bias, int bias_bf16, const float* cos_t, const float* sin_t, int rot,
+                                float v_eps, int v_norm, void* q_out, int dtype, long q_out_t, const int* slots, void* pages, int page_size, int N,
+                                int H, int G, int d, int dv, cudaStream_t stream);
+
 LLMP_API int llmp_sig_qkv_post(const float* qkv, long qkv_t, const void* bias, int bias_dtype, const float* cos_t,
                                const float* sin_t, int rot, void* q_out, int dtype, long q_out_t, const int* slots, void* pages,
                                int page_size, int N, int H, int G, int d, int dv, cudaStream_t stream) {
@@ -190,6 +195,8 @@ LLMP_API int llmp_sig_qkv_post(const float* qkv, long qkv_t, const void* bias, i
                  H, G, d, dv, rot);
     LLMP_REQUIRE(!rot || (cos_t && sin_t), "sig_qkv_post: a rotation needs its tables");
     LLMP_REQUIRE(!pages || (slots && page_size > 0), "sig_qkv_post: pages need slots and a page size");
+    if (!llmp_qkv_rows_post(qkv, qkv_t, bias, bias_dtype == LLMP_BF16, cos_t, sin_t, rot, 0.f, 0, q_out, dtype, q_out_t, slots, pages, page_size, N,
+                            H, G, d, dv, stream)) return llmp_check_launch("sig_qkv_post");
     if (dtype == LLMP_BF16)
         llmp_launch_dependent(sig_qkv_post_kernel<bf16>, dim3(N), dim3(256), 0, stream, qkv, qkv_t, bias, (int)(bias_dtype == LLMP_BF16), cos_t, sin_t, rot, (bf16*)q_out,
                                                          q_out_t, slots, (bf16*)pages, page_size, H, G, d, dv);

@@ -462,6 +462,36 @@ def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, ca
     return results, want
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("sizes", [(4, 2, 128, 128, 64), (3, 1, 20, 12, 8), (16, 4, 64, 512, 0), (2, 2, 36, 260, 32), (1, 1, 4, 4, 0)], ids=str)
+@pytest.mark.parametrize("bias", [None, torch.float32, torch.bfloat16], ids=str)
+def test_rows_in_pieces_of_sixteen_bytes(sizes, bias, dtype):
+    """The row steps of sigmoid and of windowed attention on aligned rows against the same on rows that are not (the kernels an entry a
+    thread): one token has no slot, the others' are on several pages. The same float32 operations but for the order of a value norm's sum of up to
+    512 squares: 2^-20 of the row's largest entry, and a rounding to bfloat16 that falls the other way, 2^-7 of the entry."""
+    from llm_pipeline_b200.ops import kernels
+    heads, kv_heads, dim, vdim, rot = sizes
+    gen, dev, n, page = torch.Generator().manual_seed(dim + vdim), "cuda", 5, 4
+    width = (heads + kv_heads) * dim + kv_heads * vdim
+    wide = torch.randn(n, width + 3, generator=gen).to(dev)
+    rows = wide[:, 3:].contiguous()
+    slots = torch.tensor([9, 0, -1, 6, 3], dtype=torch.int32, device=dev)
+    cos, sin = (torch.randn(n, rot // 2, generator=gen).to(dev) for _ in range(2)) if rot else (None, None)
+    b = None if bias is None else torch.randn(width, generator=gen).to(bias).to(dev)
+    for which in ("sigmoid", "capped", "capped without a norm"):
+        got = []
+        for x in (rows, wide[:, 3:]):
+            q, pages = torch.full((n, heads * dim), 7.0, dtype=dtype, device=dev), torch.full((3, kv_heads, page, dim + vdim), 7.0, dtype=dtype, device=dev)
+            if which == "sigmoid":
+                kernels.sig_qkv_post(x, b, cos, sin, rot, q, slots, pages, heads, kv_heads, dim, vdim)
+            else:
+                kernels.capped_qkv_post(x, b, 1e-5 if which == "capped" else None, q, slots, pages, heads, kv_heads, dim, vdim)
+            got += [q.float(), pages.float()]
+        for mine, plain_ in zip(got[:2], got[2:]):
+            step = 2.0 ** -20 * plain_.abs().amax(-1, keepdim=True) + (2.0 ** -7 * plain_.abs() if dtype == torch.bfloat16 else 0.0)
+            assert ((mine - plain_).abs() <= step).all(), which
+
+
 @pytest.mark.parametrize("sizes", [(4, 2, 16, 32, 0.0), (16, 4, 128, 128, 3.0), (12, 12, 32, 64, 0.0), (16, 1, 64, 64, 30.0), (8, 8, 128, 128, 0.0), (6, 3, 96, 64, 5.0), (1, 1, 48, 128, 1.0)], ids=str)
 def test_sigmoid_attention_of_single_tokens(sizes):
     """The kernel for single tokens: contexts around a tile's and a range's end in one step, over shuffled pages with garbage in the
