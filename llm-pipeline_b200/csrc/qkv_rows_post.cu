@@ -5,7 +5,7 @@
 //
 // A warp takes 128 neighbouring entries of a token's queries and keys, or one value head, a lane four entries, so that the few rows of a
 // decode step are one load deep: with a block a token and an entry a thread 16 rows of 3,072 entries took 6.5 us of a decoding layer,
-// POST_US so, and 2,048 rows with rotation 20 us, PROMPT_US so (37.7 MB: 5.8 us at the copy rate).
+// 2.2 so, and 2,048 rows with rotation 20 us, 17 so (37.7 MB, 5.8 us at the copy rate; four tokens a warp, all asked for at once: 17).
 #include "common.cuh"
 
 namespace {
