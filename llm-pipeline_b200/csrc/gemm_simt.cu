@@ -1,7 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the CUDA cores with float32 accumulation.
 // This is the matrix product of the true 32-bit path (no tensor core, no reduced-precision
-// mode) and accepts every size. Each output element adds its K products in ascending k, so a
-// row's result does not depend on how many other rows are in the call.
+// mode) and accepts every size. Each output element adds its K products in ascending k (of a narrow matrix with a long K: those of
+// each segment of K, and the segments' sums in their order; which it is follows from the matrix alone), so a row's result does not
+// depend on how many other rows are in the call.
 #include "common.cuh"
 
 int llmp_sm_count();
@@ -27,18 +28,29 @@ template <bool VEC> __device__ __forceinline__ float4 gt_load4(const bf16* row, 
 // A block makes BM x BN outputs with TM x TN of them a thread. BK entries of K at a time lie in shared memory as rows padded by 4
 // (a quarter-warp's 16-byte reads of consecutive rows meet no bank twice), in two buffers, one barrier for each; those of the next
 // AHEAD are on their way in registers. A thread reads 4 entries of K of its TM + TN rows as 16-byte words for 4 TM TN multiply-adds.
-template <typename TI, typename TO, int BM, int BN, int BK, int TM, int TN, int AHEAD, bool VEC>
+// CLUSTER: K is cut into segments, a block of a cluster for each. They leave their sums in shared memory, and each adds up a share of the
+// tile from all of them.
+template <typename TI, typename TO, int BM, int BN, int BK, int TM, int TN, int AHEAD, bool VEC, bool CLUSTER>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* __restrict__ bias, int bias_bf16,
-               TO* __restrict__ C, int M, int N, int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c) {
+               TO* __restrict__ C, int M, int N, int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c, int segment) {
     constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY, QUADS = BK / 4, LD = BK + 4;
     constexpr int LA = BM * QUADS / THREADS, LW = BN * QUADS / THREADS;      // 4-entry pieces of each operand a thread brings
     static_assert(LA * THREADS == BM * QUADS && LW * THREADS == BN * QUADS, "the pieces of a tile are shared out evenly");
     // blockIdx.z counts the products of a batch: each has its own A, W and C, the given strides apart
-    A += (size_t)blockIdx.z * batch_a;
-    W += (size_t)blockIdx.z * batch_w;
-    C += (size_t)blockIdx.z * batch_c;
-    __shared__ __align__(16) float As[2][BM * LD], Ws[2][BN * LD];
+    const int segments = CLUSTER ? (K + segment - 1) / segment : 1, rank = CLUSTER ? (int)blockIdx.z % segments : 0;
+    const int product = CLUSTER ? (int)blockIdx.z / segments : (int)blockIdx.z;
+    A += (size_t)product * batch_a;
+    W += (size_t)product * batch_w;
+    C += (size_t)product * batch_c;
+    if (CLUSTER) {                                 // this block's part of K
+        A += (size_t)rank * segment;
+        W += (size_t)rank * segment;
+        K = min(segment, K - rank * segment);
+    }
+    __shared__ __align__(16) float operands[2 * (BM + BN) * LD];
+    float (*const As)[BM * LD] = reinterpret_cast<float (*)[BM * LD]>(operands);
+    float (*const Ws)[BN * LD] = reinterpret_cast<float (*)[BN * LD]>(operands + 2 * BM * LD);
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     float acc[TM][TN] = {};
@@ -107,6 +119,36 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
             multiply(i & 1);
         }
     }
+    if (CLUSTER) {
+        constexpr int PITCH = BN + 1;
+        static_assert(BM * PITCH <= 2 * (BM + BN) * LD, "a tile's sums take the operands' place");
+        float* sums = operands;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) sums[(ty + i * TY) * PITCH + tx + j * TX] = acc[i][j];
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        const unsigned own = (unsigned)__cvta_generic_to_shared(sums);
+        for (int e = rank * THREADS + tid; e < BM * BN; e += segments * THREADS) {
+            const int m = m0 + e / BN, n = n0 + e % BN;
+            if (m >= M || n >= N) continue;
+            const unsigned at = own + (unsigned)(e / BN * PITCH + e % BN) * 4u;
+            float v = 0.f;
+            for (int q = 0; q < segments; ++q) {
+                unsigned there;
+                float s;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(there) : "r"(at), "r"(q));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(s) : "r"(there) : "memory");
+                v = q ? v + s : s;
+            }
+            if (bias) v += load_as_float(bias, bias_bf16, n);
+            C[(size_t)m * ldc + n] = from_float<TO>(v);
+        }
+        // nobody leaves while another block reads its sums
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int m = m0 + ty + i * TY;
@@ -122,24 +164,54 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
     }
 }
 
+// Few weight rows with a long K leave SMs idle up to thousands of rows, so K is cut into up to as many segments as a cluster may have
+// blocks. 96 x 2,048, microseconds with a whole K in a block and in segments: 1 row 35 and 8, 203 rows 35 and 12. Not for wider
+// matrices: there many rows fill the chip, where segments are slower (4,096 x 4,096 by 2,048 rows 1,710 us, side by side 2,062, walked by one
+// block 2,324; 96 x 2,048 by 2,048 rows 53 and 42, by 40,000 646 and 695), and whether K is cut may not depend on the rows.
+constexpr int GT_SEGMENT = 256, GT_MAX_SEGMENTS = 8, GT_NARROW = 128;
+int gt_segment(int N, int K, bool float32) {
+    const int most = (K + GT_SEGMENT - 1) / GT_SEGMENT, count = most < GT_MAX_SEGMENTS ? most : GT_MAX_SEGMENTS;
+    return N > GT_NARROW || !float32 ? K : ((K + count - 1) / count + 31) / 32 * 32;
+}
+
 // Shared memory delivers a thread's words at 128 bytes a clock and SM whether lanes ask for the same or not, so a tile's speed is
 // its multiply-adds per word read: 8 x 8 outputs a thread make 42 TFLOP/s (700 x 6,144 x 2,048; 4 x 4 made 31, and 4-byte reads
 // of a single buffer 21), but their blocks of two warps need three an SM. Fewer blocks, smaller tiles, so that every SM has
 // one; and where even the smallest leave SMs idle, more threads a tile for the latency. 203 rows, microseconds before and now:
-// 4,096 x 1,024 114 -> 77, 1,024 x 2,048 148 -> 53, 96 x 2,048 148 -> 35; 1 row, 1,024 x 1,024 74 -> 18; 2,048 rows, 4,096 x
-// 4,096 2,951 -> 1,708. An output's sum runs in ascending k whatever the tile: the same bits.
+// 4,096 x 1,024 114 -> 77, 1,024 x 2,048 148 -> 53; 1 row, 1,024 x 1,024 74 -> 18; 2,048 rows, 4,096 x 4,096 2,951 -> 1,708.
 template <typename TI, typename TO, bool VEC>
 void launch_nt(const TI* A, const TI* W, const void* bias, int bias_bf16, TO* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
                long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
     const long sms = llmp_sm_count();
+    const int segment = gt_segment(N, K, sizeof(TI) == 4), segments = (K + segment - 1) / segment;
     auto blocks = [&](int bm, int bn) { return (long)((N + bn - 1) / bn) * ((M + bm - 1) / bm) * batch; };
-#define LLMP_NT(BM, BN, BK, TM, TN, AHEAD)                                                                                              \
-    gemm_nt_kernel<TI, TO, BM, BN, BK, TM, TN, AHEAD, VEC><<<dim3((N + BN - 1) / BN, (M + BM - 1) / BM, batch), (BM / TM) * (BN / TN), 0, stream>>>( \
-        A, W, bias, bias_bf16, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c)
-    if (blocks(64, 64) >= 3 * sms) LLMP_NT(64, 64, 32, 8, 8, 1);
-    else if (blocks(64, 64) >= sms) LLMP_NT(64, 64, 16, 8, 4, 1);
-    else if (blocks(32, 32) >= sms) LLMP_NT(32, 32, 32, 4, 4, 1);
-    else LLMP_NT(32, 32, 32, 2, 2, 2);
+    auto launch = [&](auto kernel, int bm, int bn, int threads, bool cluster) {
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3((N + bn - 1) / bn, (M + bm - 1) / bm, (unsigned)(batch * (cluster ? segments : 1)));
+        config.blockDim = dim3(threads);
+        config.stream = stream;
+        cudaLaunchAttribute attr[1];                           // (not a dependent launch: blocks that begin before the last kernel's have
+        attr[0].id = cudaLaunchAttributeClusterDimension;      // ended crowd on the SMs that are free first, 250 -> 302 us a layer)
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = segments;
+        config.attrs = attr;
+        config.numAttrs = cluster ? 1 : 0;
+        cudaLaunchKernelEx(&config, kernel, A, W, bias, bias_bf16, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, segment);
+    };
+#define LLMP_NT(BM, BN, BK, TM, TN, AHEAD, SEG) \
+    launch(gemm_nt_kernel<TI, TO, BM, BN, BK, TM, TN, AHEAD, VEC, SEG>, BM, BN, (BM / TM) * (BN / TN), SEG)
+    if constexpr (sizeof(TI) == 4) {
+        if (segments > 1) {
+            if (blocks(64, 64) * segments >= 2 * sms) LLMP_NT(64, 64, 32, 8, 8, 1, true);
+            else if (blocks(32, 32) * segments >= sms) LLMP_NT(32, 32, 32, 4, 4, 1, true);
+            else LLMP_NT(32, 32, 32, 2, 2, 2, true);
+            return;
+        }
+    }
+    if (blocks(64, 64) >= 3 * sms) LLMP_NT(64, 64, 32, 8, 8, 1, false);
+    else if (blocks(64, 64) >= sms) LLMP_NT(64, 64, 16, 8, 4, 1, false);
+    else if (blocks(32, 32) >= sms) LLMP_NT(32, 32, 32, 4, 4, 1, false);
+    else LLMP_NT(32, 32, 32, 2, 2, 2, false);
 #undef LLMP_NT
 }
 

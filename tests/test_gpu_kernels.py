@@ -166,6 +166,25 @@ def test_gemm_simt_gives_one_sum_whatever_the_tile(dtype, M, N, Kd):
         assert torch.equal(single[0], out[m]), m
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("M,N,Kd", [(203, 96, 2048), (33, 128, 1027), (203, 33, 257), (1, 64, 9001), (9000, 100, 600), (700, 127, 1056), (5, 129, 1000)])
+def test_gemm_simt_in_segments(dtype, M, N, Kd):
+    """A narrow matrix with K in two to eight segments, in each of the three tiles, and the first width that goes in one: every row has the bits
+    it has alone, within K 2^-24 of the sum of the products' sizes of the float64 product (2^-8 more in bfloat16)."""
+    gen = torch.Generator().manual_seed(M + N + Kd)
+    a, w = (torch.randn(n, Kd, generator=gen).to(dtype).to(DEV) for n in (M, N))
+    bias = torch.randn(N, generator=gen).to(DEV)
+    out = torch.empty(M, N, dtype=dtype, device=DEV)
+    K().gemm_simt(a, w, out, bias)
+    want, sizes = a.double() @ w.double().T + bias.double(), a.double().abs() @ w.double().abs().T + bias.double().abs()
+    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+    assert ((out.double() - want).abs() <= bound).all()
+    for m in {0, M // 2, M - 1}:
+        single = torch.empty(1, N, dtype=dtype, device=DEV)
+        K().gemm_simt(a[m:m + 1], w, single, bias)
+        assert torch.equal(single[0], out[m]), m
+
+
 def test_gemm_simt_takes_as_many_rows_as_its_largest_tiles_hold():
     """More rows than a grid of the smallest tiles could hold: the last rows, and one of each grid row, have the bits they have alone;
     a row too many is an error."""
