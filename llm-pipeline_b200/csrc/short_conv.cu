@@ -20,6 +20,8 @@
 // Inputs and outputs are float32 (what follows is a recurrence in 32-bit); taps and bias have the type they were stored in.
 #include "common.cuh"
 
+int llmp_sm_count();
+
 namespace {
 
 constexpr int CONV_MAX_TAPS = 8;
@@ -152,27 +154,30 @@ __global__ void short_conv_parallel_kernel(const ConvArgs a, const int N) {
 
 // The same with four channels a thread in 16-byte accesses, for K = 2, 3 or 4 taps. A tile of one request, which most are, is walked
 // CONV_AHEAD tokens at a time: their inputs are all asked for before the first of them is used or anything stored, and nothing looks
-// at the requests between (2,048 tokens of 6,144 channels: 49 us with a look and a load per token, 41 to 44 so; what is left is mostly the
-// exact exponential and division of SiLU).
-constexpr int CONV_AHEAD = 4;
+// at the requests between. `tile` tokens: as many as let all blocks have their places at once (CONV_BLOCKS an SM), for a last round of few
+// blocks costs a whole one, and a tile's first inputs are read twice: 2,048 tokens of 6,144 channels in tiles of 16 (2.07 rounds) 36 us,
+// 31 so, of 4,096 channels 27 and 24 (12.8 at the copy rate; 17 without SiLU, whose exact exponential and division are the rest); 203 of
+// 2,048 10.6 and 6.5.
+constexpr int CONV_AHEAD = 4, CONV_BLOCKS = 5, CONV_MOST_TOKENS = 64;
 
 template <int K>
-__global__ void __launch_bounds__(128) short_conv_by_4_kernel(const ConvArgs a, const int N) {
+__global__ void __launch_bounds__(128, CONV_BLOCKS) short_conv_by_4_kernel(const ConvArgs a, const int N, const int tile) {
     pdl_wait();
     pdl_trigger();
-    const int t0 = blockIdx.x * CONV_TILE_TOKENS;
+    const int t0 = blockIdx.x * tile;
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (c >= a.C) return;
     auto load = [&](const float* p) { return *reinterpret_cast<const float4*>(p); };
-    const int t1 = min(t0 + CONV_TILE_TOKENS, N);
+    const int t1 = min(t0 + tile, N);
     const int first = a.token_request[t0];
-    const bool whole = t1 - t0 == CONV_TILE_TOKENS && first == a.token_request[t1 - 1];
+    const bool whole = first == a.token_request[t1 - 1];
     const float* xp = a.x + (size_t)t0 * a.x_t + c;
     float4 next[CONV_AHEAD];
-    if (whole) {
+    auto ask = [&](int i) {                                        // of the tile's tokens from i on; past its end the last one's again
 #pragma unroll
-        for (int u = 0; u < CONV_AHEAD; ++u) next[u] = load(xp + (size_t)u * a.x_t);
-    }
+        for (int u = 0; u < CONV_AHEAD; ++u) next[u] = load(xp + (size_t)min(i + u, t1 - t0 - 1) * a.x_t);
+    };
+    if (whole) ask(0);
     float4 tap[K], w[K - 1];
 #pragma unroll
     for (int j = 0; j < K; ++j)
@@ -217,17 +222,14 @@ __global__ void __launch_bounds__(128) short_conv_by_4_kernel(const ConvArgs a, 
     };
     if (whole) {
         begin_request(first, t0);
-#pragma unroll
-        for (int i = 0; i < CONV_TILE_TOKENS; i += CONV_AHEAD) {
+        for (int t = t0; t < t1; t += CONV_AHEAD) {
             float4 cur[CONV_AHEAD];
 #pragma unroll
             for (int u = 0; u < CONV_AHEAD; ++u) cur[u] = next[u];
-            if (i + CONV_AHEAD < CONV_TILE_TOKENS) {
+            if (t + CONV_AHEAD < t1) ask(t + CONV_AHEAD - t0);
 #pragma unroll
-                for (int u = 0; u < CONV_AHEAD; ++u) next[u] = load(xp + (size_t)(i + CONV_AHEAD + u) * a.x_t);
-            }
-#pragma unroll
-            for (int u = 0; u < CONV_AHEAD; ++u) step(t0 + i + u, cur[u]);
+            for (int u = 0; u < CONV_AHEAD; ++u)
+                if (t + u < t1) step(t + u, cur[u]);
         }
         return;
     }
@@ -301,10 +303,14 @@ LLMP_API int llmp_short_conv(const float* x, long x_t, const void* taps, int tap
     const bool by4 = C % 4 == 0 && x_t % 4 == 0 && state_slot % 4 == 0 && state_half % 4 == 0 && ((uintptr_t)x | (uintptr_t)state) % 16 == 0 &&
                      (!out || (out_t % 4 == 0 && (uintptr_t)out % 16 == 0)) &&
                      (!out2 || (a.out2_split % 4 == 0 && out2_t % 4 == 0 && out2_block % 4 == 0 && (uintptr_t)out2 % (a.out2_bf16 ? 8 : 16) == 0));
-    const dim3 grid4((N + CONV_TILE_TOKENS - 1) / CONV_TILE_TOKENS, (C / 4 + threads - 1) / threads);
-    if (by4 && K == 2) llmp_launch_dependent(short_conv_by_4_kernel<2>, grid4, dim3(threads), 0, stream, a, N);
-    else if (by4 && K == 3) llmp_launch_dependent(short_conv_by_4_kernel<3>, grid4, dim3(threads), 0, stream, a, N);
-    else if (by4 && K == 4) llmp_launch_dependent(short_conv_by_4_kernel<4>, grid4, dim3(threads), 0, stream, a, N);
+    const int columns4 = (C / 4 + threads - 1) / threads;
+    int tiles = CONV_BLOCKS * llmp_sm_count() / columns4;          // at once
+    int tile = tiles > 0 ? ((N + tiles - 1) / tiles + CONV_AHEAD - 1) / CONV_AHEAD * CONV_AHEAD : CONV_MOST_TOKENS;
+    if (tile > CONV_MOST_TOKENS) tile = CONV_MOST_TOKENS;
+    const dim3 grid4((N + tile - 1) / tile, columns4);
+    if (by4 && K == 2) llmp_launch_dependent(short_conv_by_4_kernel<2>, grid4, dim3(threads), 0, stream, a, N, tile);
+    else if (by4 && K == 3) llmp_launch_dependent(short_conv_by_4_kernel<3>, grid4, dim3(threads), 0, stream, a, N, tile);
+    else if (by4 && K == 4) llmp_launch_dependent(short_conv_by_4_kernel<4>, grid4, dim3(threads), 0, stream, a, N, tile);
     else short_conv_parallel_kernel<<<dim3((N + CONV_TILE_TOKENS - 1) / CONV_TILE_TOKENS, col_blocks), threads, 0, stream>>>(a, N);
     if (K > 1) llmp_launch_dependent(short_conv_state_kernel, dim3(R, col_blocks), dim3(threads), 0, stream, a);
     return llmp_check_launch("short_conv (parallel)");
