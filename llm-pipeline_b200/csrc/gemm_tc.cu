@@ -326,6 +326,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem_base = tmem_slot;
+    pdl_wait();                                                // what the kernels before wrote is complete
+    pdl_trigger();                                             // (after the allocation: nobody else's may come between)
 
     if (warp == 0) {
         if (lane == 0) {
@@ -559,8 +561,164 @@ static int launch_tc_persistent(const void* A, long rows_a, long lda, const void
     const int sms = llmp_sm_count();
     const long tiles = ((rows_a + TC_BM - 1) / TC_BM) * ((rows_b + BN - 1) / BN);
     const int grid = (int)(tiles < sms ? tiles : sms);
-    kernel<<<grid, TC_THREADS, smem, stream>>>(map_a, map_b, Y, (int)rows_a, (int)rows_b, K, ldy, error_flag);
+    llmp_launch_dependent(kernel, dim3(grid), dim3(TC_THREADS), smem, stream, map_a, map_b, Y, (int)rows_a, (int)rows_b, K, ldy, error_flag);
     return llmp_check_launch("gemm_tc_persistent");
+}
+
+// ---- a narrow output of many rows with a long K --------------------------------------------------------
+// 2,048 rows by 160 columns are 16 tiles, and tiles of 32 columns, 80 of them, read the rows five times and each walk the whole K (22 us
+// at K 4,096). Here the NARROW_SPLITS blocks of a cluster share a tile of 128 rows and all columns, each with a share of K: the rows
+// are read once, and a block's ring asks for a good part of its share at once. The accumulators are put into the blocks' shared
+// memory, and each block adds a share of the tile's rows from all of them, in their order. 12.6 us; 300 rows 22.1 and 11.9; 96 columns,
+// K 2,048 12.8 and 7.9. Eight blocks: 9.0 for 300 rows, but 18.1 for 2,048, whose 16 clusters do not fit the SMs' groups at once; two: 19.6.
+// The shares follow from K alone. smem: the ring, then the same place for the accumulator, rows padded by 4 floats.
+constexpr int NARROW_SPLITS = 4, NARROW_MAX_COLS = 256, NARROW_MAX_STAGES = 8;
+template <typename TO>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+gemm_tc_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TO* __restrict__ Y, int M, int N,
+                      int K, long ldy, int bn, int stages, int* __restrict__ error_flag) {
+    extern __shared__ unsigned char tc_raw[];
+    __shared__ __align__(8) uint64_t full_bar[NARROW_MAX_STAGES], empty_bar[NARROW_MAX_STAGES], acc_full;
+    __shared__ uint32_t tmem_slot;
+    const uint32_t raw_addr = tc_smem_u32(tc_raw);
+    unsigned char* tiles = tc_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+    const uint32_t a_bytes = TC_BM * 128, stage_bytes = a_bytes + (uint32_t)bn * 128;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_ctarank(), m0 = blockIdx.x * TC_BM;
+    const int kblocks = (K + TC_BK - 1) / TC_BK, per = (kblocks + NARROW_SPLITS - 1) / NARROW_SPLITS;
+    const int kb0 = rank * per, count = max(0, min(kblocks, kb0 + per) - kb0);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        mbar_init(&acc_full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem_u32(&tmem_slot)), "r"((uint32_t)NARROW_MAX_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem_base = tmem_slot;
+    pdl_wait();                                                // what the kernels before wrote is complete
+    pdl_trigger();
+    if (warp == 0) {
+        if (lane == 0) {
+            int it = 0;
+            for (; it < count; ++it) {
+                const int s = it % stages;
+                if (it >= stages && !mbar_wait(&empty_bar[s], ((it / stages) - 1) & 1, error_flag)) break;
+                mbar_expect_tx(&full_bar[s], stage_bytes);
+                unsigned char* stage = tiles + (size_t)s * stage_bytes;
+                tma_load_2d(stage, &map_a, (kb0 + it) * TC_BK, m0, &full_bar[s]);
+                tma_load_2d(stage + a_bytes, &map_b, (kb0 + it) * TC_BK, 0, &full_bar[s]);
+            }
+            // the copies of the last stages are over before the block may end
+            for (int k = it > stages ? it - stages : 0; k < it; ++k) mbar_wait(&full_bar[k % stages], (k / stages) & 1, error_flag);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0 && count > 0) {
+            const uint32_t idesc = umma_idesc(TC_BM, bn);
+            bool ok = true;
+            for (int it = 0; it < count; ++it) {
+                const int s = it % stages;
+                if (!mbar_wait(&full_bar[s], (it / stages) & 1, error_flag)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint32_t a_addr = tc_smem_u32(tiles + (size_t)s * stage_bytes);
+                const uint64_t desc_a = umma_desc(a_addr), desc_b = umma_desc(a_addr + a_bytes);
+#pragma unroll
+                for (int k = 0; k < TC_BK / 16; ++k) umma_f16(tmem_base, desc_a + 2 * k, desc_b + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+                umma_commit(&empty_bar[s]);
+            }
+            if (ok) umma_commit(&acc_full);
+        }
+        __syncwarp();
+    }
+    const int pitch = bn + 4;
+    float* sums = reinterpret_cast<float*>(tiles);
+    bool made = count > 0;
+    if (warp >= 2 && made) {                                   // the products are done with the ring before it is written
+        made = mbar_wait(&acc_full, 0, error_flag);
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (warp >= 2) {
+        const int quarter = warp & 3;
+        float* row = sums + (size_t)(quarter * 32 + lane) * pitch;
+        made = __all_sync(0xffffffffu, made);
+        for (int c = 0; c < bn; c += 16) {
+            float v[16] = {};
+            if (made) tmem_ld_16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c, v);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(row + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    const int quads = bn / 4;
+    for (int e = threadIdx.x; e < (TC_BM / NARROW_SPLITS) * quads; e += TC_THREADS) {
+        const int r = rank * (TC_BM / NARROW_SPLITS) + e / quads, c = e % quads * 4, m = m0 + r;
+        if (m >= M || c >= N) continue;
+        const uint32_t at = tc_smem_u32(sums + (size_t)r * pitch + c);
+        float4 part[NARROW_SPLITS];
+#pragma unroll
+        for (int q = 0; q < NARROW_SPLITS; ++q) {
+            uint32_t there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(there) : "r"(at), "r"(q));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(part[q].x), "=f"(part[q].y), "=f"(part[q].z), "=f"(part[q].w) : "r"(there) : "memory");
+        }
+        float4 s = part[0];
+#pragma unroll
+        for (int q = 1; q < NARROW_SPLITS; ++q) { s.x += part[q].x; s.y += part[q].y; s.z += part[q].z; s.w += part[q].w; }
+        TO* to = Y + (size_t)m * ldy + c;
+        to[0] = from_float<TO>(s.x);
+        if (c + 1 < N) to[1] = from_float<TO>(s.y);
+        if (c + 2 < N) to[2] = from_float<TO>(s.z);
+        if (c + 3 < N) to[3] = from_float<TO>(s.w);
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    cluster_sync_all();                                        // nobody leaves while another block reads its sums
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)NARROW_MAX_COLS) : "memory");
+    }
+}
+
+template <typename TO>
+static int launch_tc_narrow(const void* A, int M, long lda, const void* B, int N, long ldb, TO* Y, int K, long ldy, int* error_flag, cudaStream_t stream) {
+    const int bn = (N + 15) / 16 * 16;
+    CUtensorMap map_a, map_b;
+    if (llmp_matrix_tensor_map(A, M, K, lda, TC_BM, &map_a) || llmp_matrix_tensor_map(B, N, K, ldb, bn, &map_b)) return 1;
+    const size_t stage = TC_BM * 128 + (size_t)bn * 128, room = 200 * 1024;      // one block an SM: tensor memory is not shared with another's
+    const int stages = room / stage < NARROW_MAX_STAGES ? (int)(room / stage) : NARROW_MAX_STAGES;
+    const size_t sums = (size_t)TC_BM * (bn + 4) * sizeof(float), smem = room + 1024;
+    LLMP_REQUIRE(sums <= room, "gemm_tc: %d columns do not fit", N);
+    auto kernel = gemm_tc_narrow_kernel<TO>;
+    LLMP_ALLOW_SMEM(kernel, smem);
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((M + TC_BM - 1) / TC_BM, NARROW_SPLITS);
+    config.blockDim = dim3(TC_THREADS);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = NARROW_SPLITS;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attr;
+    config.numAttrs = llmp_pdl_enabled() ? 2 : 1;
+    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, map_a, map_b, Y, M, N, K, ldy, bn, stages, error_flag);
+    if (err != cudaSuccess) {
+        llmp_set_error("gemm_tc: cluster launch failed: %s", cudaGetErrorString(err));
+        return 2;
+    }
+    return llmp_check_launch("gemm_tc_narrow");
 }
 
 template <typename TO>
@@ -569,9 +727,12 @@ static int dispatch_tc(const void* X, const void* W, TO* Y, int M, int N, int K,
     if (M <= 16) return launch_tc_splitk<16, 10, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 32) return launch_tc_splitk<32, 9, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 64) return launch_tc_splitk<64, 8, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
+    // Up to 256 columns with a long K, while the clusters are one round of blocks (16 tiles of 128 rows of 148 SMs).
+    if (N <= NARROW_MAX_COLS && K >= 1024 && (long)((M + TC_BM - 1) / TC_BM) * NARROW_SPLITS <= llmp_sm_count())
+        return launch_tc_narrow(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs, and 128 x 32 where the SMs
     // take even those in one go: 2,048 rows, 160 columns, K 4,096 26.2 us -> 22.2; 96 columns, K 2,048 15.8 -> 12.6. (Sharing K among
-    // the blocks of a cluster, 64 rows by 128 columns each, lost: 31 and 25 us.)
+    // the blocks of a cluster, 64 rows by 128 columns each, lost: 31 and 25 us; for a long K the kernel above.)
     if (N < 256 && (long)((M + TC_BM - 1) / TC_BM) * ((N + 31) / 32) <= llmp_sm_count())
         return launch_tc_persistent<32, 8, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     if (N >= 256) return launch_tc_persistent<256, 4, TO>(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);

@@ -244,6 +244,23 @@ def test_gemm_tcgen05(out_dtype, M, N, Kd):
 
 
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
+@pytest.mark.parametrize("M,N,Kd", [(300, 160, 4096), (129, 96, 1032), (2048, 256, 1024), (70, 17, 2048), (1000, 250, 1096), (65, 3, 1600)])
+def test_gemm_tcgen05_narrow_outputs(out_dtype, M, N, Kd):
+    """Narrow outputs with a long K, whose shares meet in shared memory: rows and columns that fill no tile, shares of K that are not
+    alike, entries beside the output untouched. Within K 2^-24 of the sum of the products' sizes (2^-8 more in
+    bfloat16) of the float64 product."""
+    gen = torch.Generator().manual_seed(M + N + Kd)
+    x, w = (torch.randn(n, Kd, generator=gen).to(torch.bfloat16).to(DEV) for n in (M, N))
+    room = torch.full((M, N + 5), 7.0, dtype=out_dtype, device=DEV)
+    K().gemm_tc(x, w, room[:, 2:2 + N])
+    want, sizes = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0)
+    assert ((room[:, 2:2 + N].double() - want).abs() <= bound).all()
+    assert (room[:, :2] == 7.0).all() and (room[:, 2 + N:] == 7.0).all()
+    K().check_error_flag()
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
 @pytest.mark.parametrize("stride,offset", [(0, 0), (1, 0), (4, 0), (8, 3)], ids=["whole", "odd", "half", "off"])
 @pytest.mark.parametrize("M,N,Kd", [(2500, 250, 72), (2500, 200, 64), (300, 200, 72), (300, 24, 72), (200, 264, 128), (129, 300, 64)])
 def test_gemm_tcgen05_stores(out_dtype, M, N, Kd, stride, offset):
