@@ -153,13 +153,15 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
-    """The current CUDA stream of the current device as a raw handle (the fast accessor where torch has it:
-    ``torch.cuda.current_stream()`` costs about 15 microseconds a call, several milliseconds per eager step)."""
+    """The current CUDA stream of the current device as a raw handle (the fast accessors where torch has them:
+    ``torch.cuda.current_stream()`` costs about 15 microseconds a call, several milliseconds per eager step, and
+    ``torch.cuda.current_device()``, which looks first whether CUDA is set up, 1.7; a kernel's tensors exist by then)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -169,7 +171,8 @@ def _need(cond: bool, message: str) -> None:
 
 
 def _i32(t: torch.Tensor, name: str) -> None:
-    _need(t.dtype == torch.int32 and t.is_contiguous(), f"{name} must be a contiguous int32 tensor")
+    if t.dtype != torch.int32 or not t.is_contiguous():        # (on every launch: the message is made only where it is needed)
+        raise KernelError(f"{name} must be a contiguous int32 tensor")
 
 
 def tokens_per_attention_tile(num_heads: int, num_kv_heads: int, dtype: torch.dtype = torch.float32,

@@ -202,10 +202,10 @@ class PagedAttention(Mixer):
             req, tok0, seg, slot, places = AttentionPolicy.plan_items(ctx.starts, ctx.q_lens, self.tokens_per_tile, first_request,
                                                                       self.max_key_segments, self.num_kv_heads, kernels.sm_count())
             rows = [req, tok0] + ([seg, slot] if places else [])
-            host = torch.tensor(rows, dtype=torch.int32).pin_memory()
+            host = torch.empty((len(rows), len(req)), dtype=torch.int32, pin_memory=True)          # (pinned as it is made: no copy between)
+            host.numpy()[:] = rows
             dev = host.to(ctx.device, non_blocking=True)
-            tiles = (dev[0].contiguous(), dev[1].contiguous(), dev[2].contiguous() if places else None,
-                     dev[3].contiguous() if places else None, places)
+            tiles = (*dev.unbind(0), *((None, None) if not places else ()), places)
             ctx.memo[key] = tiles
         return tiles
 
