@@ -802,7 +802,8 @@ def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, out_u:
 
 # ---- parts beyond the dense pre-norm decoder: norms around a sublayer, depth mixing, recurrent and latent mixers, experts ----
 def gemm_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[b, m, :] = a[b, m, :] @ w[b]^T for a [B, M, K], w [B, N, K], out [B, M, N] on the CUDA cores with float32 sums.
+    """out[b, m, :] = a[b, m, :] @ w[b]^T for a [B, M, K], w [B, N, K], out [B, M, N] with float32 sums: on the CUDA cores, or
+    (bfloat16, at most 16 rows that start on 16 bytes) with mma.sync.
     Any of the three may be a view whose batches and rows lie apart (the heads of a [tokens, heads, size] tensor
     transposed to [heads, tokens, size]); only the last axis must be dense."""
     B, M, K = a.shape

@@ -420,8 +420,8 @@ def batched_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
     """out[b] = x[b] @ weight[b]^T for x [B, M, K], weight [B, N, K], out [B, M, N]: one product per head. ``x`` and
     ``out`` may be transposed views of [M, B, .] tensors (the heads of a step's rows), so nothing is copied. float32
     operands: the CUDA-core kernel (a true 32-bit product). bfloat16 operands: the library's batched product for many
-    rows, the CUDA-core kernel (float32 sums) for the few rows of a decode step, where the product is a few
-    microseconds either way and the own kernel costs the host a plain call."""
+    rows, an own kernel (float32 sums) for the few rows of a decode step, where the product is a few microseconds
+    either way and the own kernel costs the host a plain call."""
     B, M, K = x.shape
     if M == 0 or B == 0:
         return out
