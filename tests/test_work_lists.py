@@ -1,8 +1,13 @@
 """The host-side decisions about attention work (no GPU): which decode kernel a step takes and how the work list of
 the general kernel shares a tile's keys among items, for a GPU of 148 SMs."""
 
-from llm_pipeline_b200.parts.attention import AttentionPolicy
+from types import SimpleNamespace
+
+import pytest
+
 from llm_pipeline_b200.ops import kernels
+from llm_pipeline_b200.parts.attention import AttentionPolicy
+from llm_pipeline_b200.parts.capped_attention import CappedAttention
 
 SMS = 148
 
@@ -96,3 +101,22 @@ def test_decode_graph_shape_at_the_kernels_limit():
     # a cache made for longer requests than the decode kernels take: eager steps, which refuse only what really is too long
     assert shape(limit - 5, 48, 2 * limit) == (2752, None)
     assert shape(1000, 16, 2 * limit) == (64, 1024)
+
+
+def single_tokens(requests, longest, bound=0):
+    return SimpleNamespace(max_q_len=1, num_requests=requests, decode_ctx_bound=bound, max_ctx_len=longest)
+
+
+@pytest.mark.parametrize("reach", [{}, {"window": 1024, "keep_first": 8}, {"chunk": 2048}], ids=str)
+def test_a_token_of_capped_attention_cuts_its_keys_alike_in_any_company(monkeypatch, reach):
+    """Segments of one size that cover what a token sees, whatever the number of requests and however long the longest is, so that a
+    long request beside short ones is spread over as many blocks as alone; none once the blocks are four an SM."""
+    monkeypatch.setattr(kernels, "sm_count", lambda: SMS)
+    part = CappedAttention("p", 64, 16, 4, 16, 16, 0.25, **reach)
+    for requests in (1, 8, 16, 37, 38, 59, 74, 147, 148, 300):
+        for longest in (100, 511, 512, 700, 4096, 32768):
+            sees = min([longest] + [n + kernels.CAPPED_TILE_KEYS for n in reach.values() if n > 8])
+            want = -(-sees // kernels.CAPPED_SEGMENT_KEYS) if sees >= 512 and requests * 4 < 4 * SMS else 0
+            assert part._segments(single_tokens(requests, longest)) == want
+            assert part._segments(single_tokens(requests, 1, bound=longest)) == want
+    assert part._segments(SimpleNamespace(max_q_len=2)) == 0
