@@ -283,9 +283,13 @@ template <int KT> void launch_decode(const SigDecodeArgs& a, int N, cudaStream_t
 
 }  // namespace
 
-// Keys of a tile for these sizes (ranges are multiples of it), or 0: they are not served.
+// sigmoid_attention_mma.cu
+LLMP_API int llmp_sigmoid_attention_mma_supports(int H, int G, int d, int dv);
+
+// Keys of a tile for these sizes (ranges are multiples of it), or 0: they are not served. The mixed weights are rounded to bfloat16 for
+// the product with the values, so only sizes whose prompts have theirs rounded too; the general kernel keeps float32 for the others.
 LLMP_API int llmp_sigmoid_decode_keys(int H, int G, int d, int dv) {
-    if (H <= 0 || G <= 0 || H % G || H > SD_MAX_HEADS || d <= 0 || d % 16 || d > 256 || dv <= 0 || dv % 16 || G * (dv / 16) > SD_PIECES * SD_WARPS) return 0;
+    if (!llmp_sigmoid_attention_mma_supports(H, G, d, dv) || H > SD_MAX_HEADS || G * (dv / 16) > SD_PIECES * SD_WARPS) return 0;
     for (int keys : {64, 32})
         if (sd_smem(H, G, d, dv, keys) <= SD_MOST_BYTES) return keys;
     return 0;

@@ -492,7 +492,7 @@ def test_rows_in_pieces_of_sixteen_bytes(sizes, bias, dtype):
             assert ((mine - plain_).abs() <= step).all(), which
 
 
-@pytest.mark.parametrize("sizes", [(4, 2, 16, 32, 0.0), (16, 4, 128, 128, 3.0), (12, 12, 32, 64, 0.0), (16, 1, 64, 64, 30.0), (8, 8, 128, 128, 0.0), (6, 3, 96, 64, 5.0), (1, 1, 48, 128, 1.0)], ids=str)
+@pytest.mark.parametrize("sizes", [(4, 2, 16, 32, 0.0), (16, 4, 128, 128, 3.0), (12, 12, 32, 64, 0.0), (16, 1, 64, 64, 30.0), (8, 8, 128, 128, 0.0), (6, 3, 96, 64, 5.0), (1, 1, 32, 128, 1.0)], ids=str)
 def test_sigmoid_attention_of_single_tokens(sizes):
     """The kernel for single tokens: contexts around a tile's and a range's end in one step, over shuffled pages with garbage in the
     others, keys in one block and in ranges of one, two and three tiles. The mixed weights are rounded to bfloat16 and so is the result: 2^-8
@@ -738,6 +738,28 @@ def test_far_keys_page_borders_and_first_tokens_under_sparse_weights(tmp_path, n
     N.assert_matches(H.replay(runner, H.cut_tail_one_by_one(requests, tail=3 * page + 2)), want, dtype, "sparse: decoding across borders", share)
     N.assert_matches(H.replay(runner, H.cut_portions(requests, (page - 1, 2, page + 1, 2 * page, 3))), want, dtype, "sparse: portions", share)
     N.assert_matches(H.replay(runner, H.cut_mixed(requests, (page, 2, page + 1), max_live=3, decode_tail=page + 3)), want, dtype, "sparse: mixed", share)
+
+
+@pytest.mark.parametrize("sizes", [(1, 1, 48, 128, 1.0), (4, 2, 80, 80, 0.0), (6, 3, 112, 64, 30.0), (2, 1, 64, 144, 0.0), (2, 2, 256, 256, 5.0)], ids=str)
+def test_sigmoid_attention_keeps_mixed_weights_whole_where_prompts_do(sizes):
+    """bfloat16 heads that the tensor-core kernel for prompts does not serve: single tokens take the general kernel as well, whose mixed
+    weights are float32. Scores, weights and sums over 150 keys in float32 stay within 2^-16 of a sum without cancellation, so the
+    result is the rounding of a number that near to it (weights rounded to bfloat16 first move every fortieth to another)."""
+    from llm_pipeline_b200.ops import kernels
+    from llm_pipeline_b200.parts import lookup
+    heads, kv_heads, dim, vdim, cap = sizes
+    part = lookup("mixer", "sigmoid_attention")("p", hidden_size=8, num_heads=heads, num_kv_heads=kv_heads, dim=dim, vdim=vdim, scale=1.0, softcap=cap)
+    part.compute_dtype = torch.bfloat16
+    assert not kernels.sigmoid_attention_mma_supports(torch.bfloat16, heads, kv_heads, dim, vdim) and part._decode_keys() == 0
+
+    def planted(q, k, v):                                       # one sign: no terms cancel, so the result has their size
+        v.abs_()
+
+    got, want = _sigmoid_attention_case(torch.bfloat16, heads, kv_heads, dim, vdim, 150, 16, 7, cap, plant=planted, segments=(1, 2),
+                                        mixed=lambda talk, pb: talk.abs_())
+    for name, rows in got.items():
+        low, high = ((want * (1.0 + e)).to(torch.bfloat16).float() for e in (-2.0 ** -16, 2.0 ** -16))
+        assert ((rows >= low) & (rows <= high)).all(), name
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
