@@ -38,11 +38,11 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
     constexpr int LA = BM * QUADS / THREADS, LW = BN * QUADS / THREADS;      // 4-entry pieces of each operand a thread brings
     static_assert(LA * THREADS == BM * QUADS && LW * THREADS == BN * QUADS, "the pieces of a tile are shared out evenly");
     // blockIdx.z counts the products of a batch: each has its own A, W and C, the given strides apart
-    const int segments = CLUSTER ? (K + segment - 1) / segment : 1, rank = CLUSTER ? (int)blockIdx.z % segments : 0;
-    const int product = CLUSTER ? (int)blockIdx.z / segments : (int)blockIdx.z;
-    A += (size_t)product * batch_a;
-    W += (size_t)product * batch_w;
-    C += (size_t)product * batch_c;
+    // (of a cluster the blocks are neighbours along x, where a grid may be long: a batch with its segments may be more than 65,535)
+    const int segments = CLUSTER ? (K + segment - 1) / segment : 1, rank = CLUSTER ? (int)blockIdx.x % segments : 0;
+    A += (size_t)blockIdx.z * batch_a;
+    W += (size_t)blockIdx.z * batch_w;
+    C += (size_t)blockIdx.z * batch_c;
     if (CLUSTER) {                                 // this block's part of K
         A += (size_t)rank * segment;
         W += (size_t)rank * segment;
@@ -52,7 +52,7 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
     float (*const As)[BM * LD] = reinterpret_cast<float (*)[BM * LD]>(operands);
     float (*const Ws)[BN * LD] = reinterpret_cast<float (*)[BN * LD]>(operands + 2 * BM * LD);
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * BM, n0 = (int)blockIdx.x / segments * BN;
     float acc[TM][TN] = {};
     float4 ra[AHEAD][LA], rw[AHEAD][LW];
     auto fetch = [&](int k0, float4 (&pa)[LA], float4 (&pw)[LW]) {           // past the end of K: zeros, without a read
@@ -187,13 +187,13 @@ void launch_nt(const TI* A, const TI* W, const void* bias, int bias_bf16, TO* C,
     auto blocks = [&](int bm, int bn) { return (long)((N + bn - 1) / bn) * ((M + bm - 1) / bm) * batch; };
     auto launch = [&](auto kernel, int bm, int bn, int threads, bool cluster) {
         cudaLaunchConfig_t config = {};
-        config.gridDim = dim3((N + bn - 1) / bn, (M + bm - 1) / bm, (unsigned)(batch * (cluster ? segments : 1)));
+        config.gridDim = dim3((unsigned)((N + bn - 1) / bn * (cluster ? segments : 1)), (M + bm - 1) / bm, batch);
         config.blockDim = dim3(threads);
         config.stream = stream;
         cudaLaunchAttribute attr[1];                           // (not a dependent launch: blocks that begin before the last kernel's have
         attr[0].id = cudaLaunchAttributeClusterDimension;      // ended crowd on the SMs that are free first, 250 -> 302 us a layer)
-        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = segments;
+        attr[0].val.clusterDim.x = segments;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         config.attrs = attr;
         config.numAttrs = cluster ? 1 : 0;
         cudaLaunchKernelEx(&config, kernel, A, W, bias, bias_bf16, C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, segment);

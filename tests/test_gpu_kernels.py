@@ -185,6 +185,17 @@ def test_gemm_simt_in_segments(dtype, M, N, Kd):
         assert torch.equal(single[0], out[m]), m
 
 
+def test_gemm_simt_batches_in_segments_as_long_as_a_grid_holds():
+    """40,000 products whose K goes in two segments are 80,000 of them, more than a grid's shorter sides hold: within 16 roundings of 2^-24
+    of the sizes (half of 288 products of random signs) of float64."""
+    gen = torch.Generator().manual_seed(5)
+    a, w = torch.randn(1, 17, 288, generator=gen).to(DEV), torch.randn(40000, 1, 288, generator=gen).to(DEV)
+    out = torch.empty(40000, 17, 1, device=DEV)
+    K().gemm_batched(a.expand(40000, 17, 288), w, out)
+    want, sizes = a.double() @ w.double().transpose(1, 2), a.double().abs() @ w.double().abs().transpose(1, 2)
+    assert ((out.double() - want).abs() <= 16 * 2.0 ** -24 * sizes).all()
+
+
 def test_gemm_simt_takes_as_many_rows_as_its_largest_tiles_hold():
     """More rows than a grid of the smallest tiles could hold: the last rows, and one of each grid row, have the bits they have alone;
     a row too many is an error."""
