@@ -145,7 +145,8 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
             if (bias) v += load_as_float(bias, bias_bf16, n);
             C[(size_t)m * ldc + n] = from_float<TO>(v);
         }
-        // nobody leaves while another block reads its sums
+        // nobody leaves while another block reads its sums (a warp's lanes, which have shares of different lengths, arrive as one)
+        __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         return;
     }
