@@ -4,8 +4,8 @@
 // The weights are read once and the rest is latency, so everything a warp needs is asked for at once: a warp takes 16 weight rows
 // (the m side of the MMA; the rows of A are its n side) and up to 128 of K at a time, in 16-byte words straight into registers. An
 // MMA's 16 places along K may be any 16 of K as long as both operands agree: lane t of a quad holds entries 8 t .. 8 t + 7 of a run of 32,
-// whose first four are its places of one MMA and the others of a second. The weights are asked for before the kernel waits for the one
-// before it. Up to 256 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are
+// whose first four are its places of one MMA and the others of a second. Weights that the caller holds are asked for before the kernel
+// waits for the one before it, which may be what writes others. Up to 256 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are
 // added in the order of the quarters. The split follows from K alone and a row's sums from its own entries, so its bits do not depend on
 // the other rows. A decoding layer of 16 heads (8 requests of 2,048 keys), whose maps
 // are 128 x 512 and 512 x 128: 53.3 us with a warp per output column and sums by shuffles (gemm_simt.cu, which keeps float32 and operands
@@ -20,6 +20,7 @@ struct FewArgs {
     const bf16* A; const bf16* W; bf16* C;
     int M, N, K;
     long lda, ldw, ldc, batch_a, batch_w, batch_c;
+    int held;                                  // 1: no kernel in flight writes W
 };
 
 __device__ __forceinline__ void gf_mma(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
@@ -49,9 +50,10 @@ __global__ void __launch_bounds__(32 * GF_WARPS) gemm_few_batched_kernel(const F
             }
     };
     float acc[MT][4] = {};
-    load_w(first);
+    if (a.held) load_w(first);
     pdl_wait();
     pdl_trigger();
+    if (!a.held) load_w(first);
     for (int run0 = first; run0 < last; run0 += GF_RUNS) {
 #pragma unroll
         for (int i = 0; i < GF_RUNS; ++i)
@@ -101,11 +103,11 @@ LLMP_API int llmp_gemm_few_batched_supports(const void* A, const void* W, int M,
 }
 
 LLMP_API int llmp_gemm_few_batched(const void* A, const void* W, void* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
-                                   long batch_a, long batch_w, long batch_c, cudaStream_t stream) {
+                                   long batch_a, long batch_w, long batch_c, int held, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     LLMP_REQUIRE(llmp_gemm_few_batched_supports(A, W, M, K, lda, ldw, batch_a, batch_w) && batch <= 65535,
                  "gemm_few_batched: %d products of %d rows, K %d, or operands without 16-byte rows", batch, M, K);
-    const FewArgs a = {(const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c};
+    const FewArgs a = {(const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, held};
     const bool quarters = K > 256;
     const int rows = quarters ? 16 : 16 * GF_WARPS;
     const dim3 grid((unsigned)((N + rows - 1) / rows), batch);

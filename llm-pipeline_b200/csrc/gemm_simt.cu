@@ -322,19 +322,20 @@ gemm_rows_kernel(const TI* __restrict__ A, const TI* __restrict__ W, TO* __restr
 // gemm_few_batched.cu
 LLMP_API int llmp_gemm_few_batched_supports(const void* A, const void* W, int M, int K, long lda, long ldw, long batch_a, long batch_w);
 LLMP_API int llmp_gemm_few_batched(const void* A, const void* W, void* C, int batch, int M, int N, int K, long lda, long ldw, long ldc,
-                                   long batch_a, long batch_w, long batch_c, cudaStream_t stream);
+                                   long batch_a, long batch_w, long batch_c, int held, cudaStream_t stream);
 
 // A batch of such products in one launch: product b reads A + b * batch_a and W + b * batch_w and writes C + b * batch_c
 // (strides in elements; rows of any of them may lie further apart than they are long, so one product per head
-// can read and write the heads of a [tokens, heads, size] tensor in place).
+// can read and write the heads of a [tokens, heads, size] tensor in place). held: 1 where W is the caller's for good, so that it may be
+// read while the kernel before is still at work.
 LLMP_API int llmp_gemm_simt_batched(const void* A, const void* W, void* C, int in_dtype, int out_dtype, int batch, int M, int N,
-                                    int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c,
+                                    int K, long lda, long ldw, long ldc, long batch_a, long batch_w, long batch_c, int held,
                                     cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return 0;
     LLMP_REQUIRE(K > 0, "batched gemm: bad K %d", K);
     LLMP_REQUIRE(M <= GT_MAX_ROWS && batch <= 65535, "batched gemm: too many rows %d or products %d", M, batch);
     if (in_dtype == LLMP_BF16 && out_dtype == LLMP_BF16 && llmp_gemm_few_batched_supports(A, W, M, K, lda, ldw, batch_a, batch_w))
-        return llmp_gemm_few_batched(A, W, C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, stream);
+        return llmp_gemm_few_batched(A, W, C, batch, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, held, stream);
     if (M <= GR_MAX_ROWS && (N + 7) / 8 <= 65535) {
         dim3 rows_grid((N + 7) / 8, batch);
         const size_t esize = in_dtype == LLMP_F32 ? 4 : 2;

@@ -58,7 +58,7 @@ _SIGNATURES = {
     "llmp_entropy": [_P, _L, _I, _I, _F, _P, _P],
     "llmp_bounded_wait_check": [_P, _I, _P, _P],
     "llmp_gemm_stream_chain": [_P, _I, _I, _P, _P, _P],
-    "llmp_gemm_simt_batched": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _L, _L, _L, _L, _L, _P],
+    "llmp_gemm_simt_batched": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _L, _L, _L, _L, _L, _I, _P],
     "llmp_embedding_norm": [_P, _P, _I, _P, _I, _F, _F, _P, _I, _I, _I, _P],
     "llmp_add_norm_mix": [_P, _P, _I, _P, _I, _F, _F, _P, _L, _P, _I, _P, _I, _F, _F, _P, _I, _P, _I, _I, _P],
     "llmp_poly_norm": [_P, _I, _L, _P, _F, _P, _I, _I, _I, _P],
@@ -801,18 +801,19 @@ def sample(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor, out_u:
 
 
 # ---- parts beyond the dense pre-norm decoder: norms around a sublayer, depth mixing, recurrent and latent mixers, experts ----
-def gemm_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def gemm_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, held: bool = False) -> torch.Tensor:
     """out[b, m, :] = a[b, m, :] @ w[b]^T for a [B, M, K], w [B, N, K], out [B, M, N] with float32 sums: on the CUDA cores, or
     (bfloat16, at most 16 rows that start on 16 bytes) with mma.sync.
     Any of the three may be a view whose batches and rows lie apart (the heads of a [tokens, heads, size] tensor
-    transposed to [heads, tokens, size]); only the last axis must be dense."""
+    transposed to [heads, tokens, size]); only the last axis must be dense. ``held``: ``w`` is a weight that was there before
+    this step's kernels were launched; it may then be read while the kernel before is still at work."""
     B, M, K = a.shape
     N = w.shape[1]
     _need(w.shape == (B, N, K) and out.shape == (B, M, N), "batched gemm shapes do not match")
     _need(a.dtype == w.dtype and a.stride(2) == 1 and w.stride(2) == 1 and out.stride(2) == 1,
           "batched gemm operands must have one type and a dense last axis")
     _call("llmp_gemm_simt_batched", _ptr(a), _ptr(w), _ptr(out), dtype_code(a.dtype), dtype_code(out.dtype), B, M, N, K,
-          a.stride(1), w.stride(1), out.stride(1), a.stride(0), w.stride(0), out.stride(0), _stream())
+          a.stride(1), w.stride(1), out.stride(1), a.stride(0), w.stride(0), out.stride(0), int(held), _stream())
     return out
 
 

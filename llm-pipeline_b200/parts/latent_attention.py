@@ -45,12 +45,13 @@ from .registry import register_mixer
 
 
 def _by_run(runs, rows, weights, out) -> None:
-    """Per head ``out`` = ``rows`` x ``weights``^T, both [tokens, heads, ..], for the runs of rows (first, end); None: for all of them."""
+    """Per head ``out`` = ``rows`` x ``weights``^T (the layer's own), both [tokens, heads, ..], for the runs of rows (first, end); None: for
+    all of them."""
     if runs is None:
-        batched_linear(rows.transpose(0, 1), weights, out.transpose(0, 1))
+        batched_linear(rows.transpose(0, 1), weights, out.transpose(0, 1), held=True)
         return
     for first, end in runs:
-        batched_linear(rows[first:end].transpose(0, 1), weights, out[first:end].transpose(0, 1))
+        batched_linear(rows[first:end].transpose(0, 1), weights, out[first:end].transpose(0, 1), held=True)
 
 
 @register_mixer("latent_attention")

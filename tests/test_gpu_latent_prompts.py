@@ -206,3 +206,26 @@ def test_few_rows_of_several_heads(batch, rows, n, k):
         alone = torch.empty(1, batch, n, dtype=torch.bfloat16, device=DEV)
         kernels.gemm_batched(x[m:m + 1, :, :k].transpose(0, 1), w, alone.transpose(0, 1))
         assert torch.equal(alone[0], out[m, :, :n])
+
+
+@pytest.mark.parametrize("k", [128, 512])
+def test_few_rows_of_several_heads_by_weights_just_made(k):
+    """Weights that the kernel launched before writes, other ones every time: the product is of those, as after a pause. A layer's own
+    weights, which may be read sooner, give the same bits."""
+    from llm_pipeline_b200.ops import kernels
+    gen = torch.Generator().manual_seed(k)
+    x = torch.randn(4, 8, k, generator=gen).to(torch.bfloat16).to(DEV)
+    made = [torch.randn(4 * 512, k, generator=gen).to(DEV) for _ in range(8)]
+    w = torch.zeros(4, 512, k, dtype=torch.bfloat16, device=DEV)
+    outs = torch.empty(8, 4, 8, 512, dtype=torch.bfloat16, device=DEV)
+    for rows, out in zip(made, outs):
+        kernels.convert_rows(rows, w.view(4 * 512, k))
+        kernels.gemm_batched(x, w, out)
+    for rows, out in zip(made, outs):
+        paused, held = torch.empty_like(out), torch.empty_like(out)
+        whole = rows.to(torch.bfloat16).view(4, 512, k)
+        torch.cuda.synchronize()
+        kernels.gemm_batched(x, whole, paused)
+        torch.cuda.synchronize()
+        kernels.gemm_batched(x, whole, held, held=True)
+        assert torch.equal(out, paused) and torch.equal(held, paused)
