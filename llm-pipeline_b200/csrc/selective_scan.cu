@@ -30,7 +30,9 @@
 
 namespace {
 
-constexpr int SS_RUN = 4;                  // tokens of a turn of the walk
+// Tokens of a turn of the walk, by the entries a lane holds: a turn's two sets of registers are twelve a token and entry in float64,
+// eight in float32. Four tokens of four or eight entries spilled up to 3,816 bytes a thread.
+template <typename ACC, int E> constexpr int SS_RUN = (int)sizeof(ACC) * E <= 16 ? 4 : (int)sizeof(ACC) * E <= 32 ? 2 : 1;
 // threads of a block that walk; then come a warp that copies, four for step sizes and gates, two for the outputs
 template <int G> constexpr int SS_WALKERS = G < 8 ? 64 : 128;
 
@@ -129,38 +131,47 @@ __device__ __forceinline__ void ss_pair(const unsigned char* p, double (&d)[2]) 
 __device__ __forceinline__ void ss_put2(unsigned char* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 __device__ __forceinline__ void ss_put2(unsigned char* p, double a, double b) { *reinterpret_cast<double2*>(p) = make_double2(a, b); }
 // A lane's sums of a run's tokens, and the sums of them over the G lanes of a channel, in the order of ss_reduce.
-__device__ __forceinline__ void ss_put(unsigned char* p, const float (&v)[SS_RUN]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
-__device__ __forceinline__ void ss_put(unsigned char* p, const double (&v)[SS_RUN]) {
-    ss_put2(p, v[0], v[1]);
-    ss_put2(p + 16, v[2], v[3]);
+template <int RUN, typename ACC> __device__ __forceinline__ void ss_put(unsigned char* p, const ACC (&v)[RUN]) {
+    if constexpr (RUN == 1) *reinterpret_cast<ACC*>(p) = v[0];
+    else if constexpr (RUN == 4 && sizeof(ACC) == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else {
+#pragma unroll
+        for (int t = 0; t < RUN; t += 2) ss_put2(p + t * sizeof(ACC), v[t], v[t + 1]);
+    }
 }
-__device__ __forceinline__ void ss_get(const unsigned char* p, float (&v)[SS_RUN]) {
-    const float4 u = *reinterpret_cast<const float4*>(p);
-    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+template <int RUN, typename ACC> __device__ __forceinline__ void ss_get(const unsigned char* p, ACC (&v)[RUN]) {
+    if constexpr (RUN == 1) v[0] = *reinterpret_cast<const ACC*>(p);
+    else if constexpr (RUN == 4 && sizeof(ACC) == 4) {
+        const float4 u = *reinterpret_cast<const float4*>(p);
+        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    } else {
+#pragma unroll
+        for (int t = 0; t < RUN; t += 2) {
+            ACC u[2];
+            ss_pair(p + t * sizeof(ACC), u);
+            v[t] = u[0]; v[t + 1] = u[1];
+        }
+    }
 }
-__device__ __forceinline__ void ss_get(const unsigned char* p, double (&v)[SS_RUN]) {
-    const double2 u = *reinterpret_cast<const double2*>(p), w = *reinterpret_cast<const double2*>(p + 16);
-    v[0] = u.x; v[1] = u.y; v[2] = w.x; v[3] = w.y;
-}
-template <int G, typename ACC> __device__ __forceinline__ void ss_gather(const unsigned char* p, ACC (&y)[SS_RUN]) {
-    constexpr int PITCH = SS_RUN * sizeof(ACC);
-    ACC v[G / 2][SS_RUN];
+template <int G, int RUN, typename ACC> __device__ __forceinline__ void ss_gather(const unsigned char* p, ACC (&y)[RUN]) {
+    constexpr int PITCH = RUN * sizeof(ACC);
+    ACC v[G / 2][RUN];
 #pragma unroll
     for (int i = 0; i < G / 2; ++i) {
-        ACC u[SS_RUN];
+        ACC u[RUN];
         ss_get(p + i * PITCH, v[i]);
         ss_get(p + (i + G / 2) * PITCH, u);
 #pragma unroll
-        for (int t = 0; t < SS_RUN; ++t) v[i][t] += u[t];
+        for (int t = 0; t < RUN; ++t) v[i][t] += u[t];
     }
 #pragma unroll
     for (int w = G / 4; w > 0; w >>= 1)
 #pragma unroll
         for (int i = 0; i < w; ++i)
 #pragma unroll
-            for (int t = 0; t < SS_RUN; ++t) v[i][t] += v[i + w][t];
+            for (int t = 0; t < RUN; ++t) v[i][t] += v[i + w][t];
 #pragma unroll
-    for (int t = 0; t < SS_RUN; ++t) y[t] = v[0][t];
+    for (int t = 0; t < RUN; ++t) y[t] = v[0][t];
 }
 template <int G, typename ACC> __device__ __forceinline__ ACC ss_reduce(ACC y) {
 #pragma unroll
@@ -253,16 +264,17 @@ __device__ __forceinline__ void ss_copy(float* dst, const float* src, bool have)
 
 // Shared memory of a walk: a ring of stages, each the x, dt and z rows of STAGE tokens [token][channel] and their B and C in the
 // order of a channel's lanes ([token][lane][E of B | E of C]); three buffers of step sizes [channel][token] (step size, step size
-// times x); two of the lanes' sums [run][channel][lane][SS_RUN tokens]. The pitches spread a warp's channels over the banks.
+// times x); two of the lanes' sums [run][channel][lane][RUN tokens]. The pitches spread a warp's channels over the banks.
 template <typename ACC, int G, int E> struct ScanSmem {
-    static constexpr int CH = SS_WALKERS<G> / G, P = G * E;
+    static constexpr int CH = SS_WALKERS<G> / G, P = G * E, RUN = SS_RUN<ACC, E>;
     static constexpr int STAGE = P > 64 || CH > 16 ? 16 : 32;  // tokens; two blocks an SM where that can be
     static constexpr int STAGES = 5;                           // one walked, one behind it, two before it, one under way
     static constexpr int ROWS = STAGE * CH;
     static constexpr int STAGE_FLOATS = 3 * ROWS + STAGE * 2 * P;
     static constexpr int STEP_PITCH = STAGE * 2 * (int)sizeof(ACC) + 16;          // bytes
-    static constexpr int SUM_PITCH = G * SS_RUN * (int)sizeof(ACC) + 16, SUM_BYTES = STAGE / SS_RUN * CH * SUM_PITCH;
+    static constexpr int SUM_PITCH = G * RUN * (int)sizeof(ACC) + 16, SUM_BYTES = STAGE / RUN * CH * SUM_PITCH;
     static constexpr size_t BYTES = (size_t)STAGES * STAGE_FLOATS * 4 + 3 * CH * STEP_PITCH + 2 * SUM_BYTES;
+    static_assert(BYTES <= 227 * 1024 && STAGE % (2 * RUN) == 0, "a block's shared memory; a stage is whole turns");
 };
 
 // WIDE: x, dt and z rows may be copied by 16 bytes (alignment, and `inner` a multiple of the block's channels), B and C by E floats.
@@ -270,7 +282,7 @@ template <typename ACC, int G, int E> struct ScanSmem {
 template <typename T, typename ACC, int G, int E, bool WIDE>
 __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 4 ? 2 : 1) selective_walk_kernel(const ScanArgs a) {
     typedef ScanSmem<ACC, G, E> L;
-    constexpr int CH = L::CH, P = L::P, STAGE = L::STAGE;
+    constexpr int CH = L::CH, P = L::P, STAGE = L::STAGE, RUN = L::RUN;
     extern __shared__ __align__(16) float ss_smem[];
     unsigned char* const steps = reinterpret_cast<unsigned char*>(ss_smem + L::STAGES * L::STAGE_FLOATS);
     unsigned char* const sums = steps + 3 * CH * L::STEP_PITCH;
@@ -297,15 +309,15 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
         ss_load<E>(S, slot + ((p0 + 1) & 1) * a.state_half, have);
         // In turn j: decays of run j + 1, the chain over run j, the rows of run j + 2 from shared memory. Nothing in a turn waits for
         // another part of it. Two sets of registers take turns.
-        ACC decay[2][SS_RUN][E], add[2][SS_RUN][E], step[2][SS_RUN][2];
-        float rows[2][SS_RUN][2 * E];                          // B | C
+        ACC decay[2][RUN][E], add[2][RUN][E], step[2][RUN][2];
+        float rows[2][RUN][2 * E];                          // B | C
         const float* const bc0 = ss_smem + 3 * L::ROWS + l * 2 * E;
         const unsigned char* const step0 = steps + lc * L::STEP_PITCH;
-        unsigned char* const sum0 = sums + lc * L::SUM_PITCH + l * SS_RUN * sizeof(ACC);
-        constexpr int RUN_BC = SS_RUN * 2 * P, RUN_STEP = SS_RUN * 2 * (int)sizeof(ACC), RUN_SUM = CH * L::SUM_PITCH;
+        unsigned char* const sum0 = sums + lc * L::SUM_PITCH + l * RUN * sizeof(ACC);
+        constexpr int RUN_BC = RUN * 2 * P, RUN_STEP = RUN * 2 * (int)sizeof(ACC), RUN_SUM = CH * L::SUM_PITCH;
         auto fetch = [&](int set, const float* bc, const unsigned char* st) {
 #pragma unroll
-            for (int t = 0; t < SS_RUN; ++t) {
+            for (int t = 0; t < RUN; ++t) {
                 ss_pair(st + t * 2 * sizeof(ACC), step[set][t]);
                 const float4* at = reinterpret_cast<const float4*>(bc + t * 2 * P);
 #pragma unroll
@@ -317,7 +329,7 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
         };
         auto decays = [&](int set) {
 #pragma unroll
-            for (int t = 0; t < SS_RUN; ++t) ss_decays<E>(A, step[set][t][0], step[set][t][1], rows[set][t], decay[set][t], add[set][t]);
+            for (int t = 0; t < RUN; ++t) ss_decays<E>(A, step[set][t][0], step[set][t][1], rows[set][t], decay[set][t], add[set][t]);
         };
         __syncthreads();                                       // the first stages are in
         __syncthreads();                                       // and the first two's step sizes there
@@ -331,16 +343,16 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
             const unsigned char* st = step0 + buffer * CH * L::STEP_PITCH;
             unsigned char* to = sum0 + (s & 1) * L::SUM_BYTES;
 #pragma unroll 1
-            for (int t0 = 0; t0 < min(STAGE, n - s * STAGE); t0 += 2 * SS_RUN) {
-                const bool last = t0 + 2 * SS_RUN == STAGE;    // then the runs to fetch are the next stage's first two
+            for (int t0 = 0; t0 < min(STAGE, n - s * STAGE); t0 += 2 * RUN) {
+                const bool last = t0 + 2 * RUN == STAGE;    // then the runs to fetch are the next stage's first two
                 bc = last ? bc0 + ring1 * L::STAGE_FLOATS : bc + 2 * RUN_BC;
                 st = last ? step0 + buffer1 * CH * L::STEP_PITCH : st + 2 * RUN_STEP;
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
-                    ACC part[SS_RUN];
+                    ACC part[RUN];
                     decays(u ^ 1);
 #pragma unroll
-                    for (int t = 0; t < SS_RUN; ++t) part[t] = ss_advance<E>(S, decay[u][t], add[u][t], rows[u][t] + E);
+                    for (int t = 0; t < RUN; ++t) part[t] = ss_advance<E>(S, decay[u][t], add[u][t], rows[u][t] + E);
                     fetch(u, bc + u * RUN_BC, st + u * RUN_STEP);
                     ss_put(to, part);
                     to += RUN_SUM;
@@ -385,7 +397,7 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
                     ss_copy<XU * 4>(d + L::ROWS, sd + (long)row * d_t, in);
                     if (gated) ss_copy<XU * 4>(d + 2 * L::ROWS, sz + (long)row * z_t, in);
                 }
-#pragma unroll
+#pragma unroll 1
                 for (int i = 0; i < BJ; ++i) {
                     const int j = h % BCOLS + i * 32, e = j % (BCOLS / 2) * BU;
                     const bool is_c = j >= BCOLS / 2, in_e = e < a.states;
@@ -442,7 +454,7 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
     }
 
     // the outputs of the stage behind: a thread takes a channel's run and adds up its lanes' sums
-    constexpr int ITEMS = CH * (STAGE / SS_RUN), OWN = (ITEMS + 63) / 64;
+    constexpr int ITEMS = CH * (STAGE / RUN), OWN = (ITEMS + 63) / 64;
     const int h = tid - SS_WALKERS<G> - 160, lc = h % CH, c = c0 + lc;
     const bool ok = c < a.inner;
     const float Dc = a.D[ok ? c : 0];
@@ -452,13 +464,13 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
 #pragma unroll
         for (int o = 0; o < OWN; ++o) {
             const int run = h / CH + o * (64 / CH);
-            if (ITEMS % 64 && run >= STAGE / SS_RUN) break;
-            ACC y[SS_RUN];
-            ss_gather<G>(sums + (s & 1) * L::SUM_BYTES + (run * CH + lc) * L::SUM_PITCH, y);
-            const int t0 = run * SS_RUN, at = s * STAGE + t0;
+            if (ITEMS % 64 && run >= STAGE / RUN) break;
+            ACC y[RUN];
+            ss_gather<G, RUN>(sums + (s & 1) * L::SUM_BYTES + (run * CH + lc) * L::SUM_PITCH, y);
+            const int t0 = run * RUN, at = s * STAGE + t0;
             T* to = out + (size_t)at * a.out_t;
 #pragma unroll
-            for (int t = 0; t < SS_RUN; ++t) {
+            for (int t = 0; t < RUN; ++t) {
                 float v = (float)fma((ACC)Dc, (ACC)st[(t0 + t) * CH], y[t]);
                 if (gated) v *= st[(t0 + t) * CH + 2 * L::ROWS];
                 if (ok && at + t < n) to[t * a.out_t] = from_float<T>(v);
