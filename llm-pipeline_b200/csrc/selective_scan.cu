@@ -26,6 +26,8 @@
 //         64 single tokens beside 300 102 and 57. On the way: all of it in one warp 209 and 149, sums by shuffles among the walkers 155
 //         and 106, stages of 16 tokens 109 and 84, two warps for step sizes and gates 104 and 74.
 //   segments: few channels and many tokens in bfloat16 (below).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -47,7 +49,7 @@ struct ScanArgs {
     float* state; long state_slot; long state_half;
     const int* q_start; const int* slots; const int* positions;
     void* out; long out_t;
-    int inner, states;
+    int inner, states, requests;
     int singles;                          // 1: the walk leaves requests of one token to the step kernel
 };
 
@@ -220,8 +222,8 @@ __device__ __forceinline__ void ss_store(const ACC (&v)[E], float* p, int have) 
 template <typename T, typename ACC, int G, int E>
 __global__ void __launch_bounds__(SS_WALKERS<G>) selective_step_kernel(const ScanArgs a) {
     constexpr int CH = SS_WALKERS<G> / G;
-    const int r = blockIdx.x, l = threadIdx.x % G;
-    const int c = blockIdx.y * CH + threadIdx.x / G;
+    const int r = blockIdx.x % a.requests, l = threadIdx.x % G;
+    const int c = blockIdx.x / a.requests * CH + threadIdx.x / G;
     const bool ok = c < a.inner;
     const int cc = ok ? c : 0, have = ok ? a.states - l * E : 0;
     float rate[E];
@@ -277,7 +279,8 @@ template <typename ACC, int G, int E> struct ScanSmem {
     static_assert(BYTES <= 227 * 1024 && STAGE % (2 * RUN) == 0, "a block's shared memory; a stage is whole turns");
 };
 
-// WIDE: x, dt and z rows may be copied by 16 bytes (alignment, and `inner` a multiple of the block's channels), B and C by E floats.
+// WIDE: x, dt and z rows may be copied by 16 bytes (alignment, and `inner` a multiple of the block's channels), B and C by E floats, and
+// rows lie less than 2^31 entries apart. The blocks are along x, which holds them for any number of channels and requests.
 // Requests of a single token are left to the step kernel where `singles` says that it runs too.
 template <typename T, typename ACC, int G, int E, bool WIDE>
 __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 4 ? 2 : 1) selective_walk_kernel(const ScanArgs a) {
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
     extern __shared__ __align__(16) float ss_smem[];
     unsigned char* const steps = reinterpret_cast<unsigned char*>(ss_smem + L::STAGES * L::STAGE_FLOATS);
     unsigned char* const sums = steps + 3 * CH * L::STEP_PITCH;
-    const int r = blockIdx.x, tid = threadIdx.x, c0 = blockIdx.y * CH;
+    const int r = blockIdx.x % a.requests, tid = threadIdx.x, c0 = blockIdx.x / a.requests * CH;
     pdl_wait();                                                // what the kernels before wrote is complete
     pdl_trigger();
     const int begin = a.q_start[r], n = a.q_start[r + 1] - begin;
@@ -378,7 +381,8 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
         const float* px = a.x + (size_t)begin * a.x_t + (in_x ? c0 + xq : 0);
         const float* pd = a.dt + (size_t)begin * a.dt_t + (in_x ? c0 + xq : 0);
         const float* pz = gated ? a.z + (size_t)begin * a.z_t + (in_x ? c0 + xq : 0) : a.x;
-        const int x_t = (int)a.x_t, d_t = (int)a.dt_t, z_t = (int)a.z_t, bc_t = (int)a.bc_t;
+        typedef std::conditional_t<WIDE, int, long> Stride;
+        const Stride x_t = (Stride)a.x_t, d_t = (Stride)a.dt_t, z_t = (Stride)a.z_t, bc_t = (Stride)a.bc_t;
         auto copy_stage = [&](int s) {
             if (s < stages) {
                 float* st = ss_smem + (s % L::STAGES) * L::STAGE_FLOATS;
@@ -487,13 +491,14 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
 }
 
 template <typename T, typename ACC, int G, int E>
-void launch_scan(const ScanArgs& a, int R, int max_q_len, cudaStream_t stream) {
+void launch_scan(const ScanArgs& a, int max_q_len, cudaStream_t stream) {
     constexpr int CH = SS_WALKERS<G> / G, U = E < 4 ? E : 4;      // channels of a block, in both forms
-    const dim3 grid(R, (unsigned)((a.inner + CH - 1) / CH));
+    const int R = a.requests;
+    const dim3 grid((unsigned)((a.inner + CH - 1) / CH * R));
     if (max_q_len == 1 || R > 1) llmp_launch_dependent(selective_step_kernel<T, ACC, G, E>, grid, dim3(SS_WALKERS<G>), 0, stream, a);
     if (max_q_len == 1) return;
     const bool wide = a.inner % CH == 0 && ((uintptr_t)a.x | (uintptr_t)a.dt | (uintptr_t)a.z) % 16 == 0 && (a.x_t | a.dt_t | a.z_t) % 4 == 0 &&
-                      a.states == G * E && ((uintptr_t)a.B | (uintptr_t)a.C) % (4 * U) == 0 && a.bc_t % U == 0;
+                      a.states == G * E && ((uintptr_t)a.B | (uintptr_t)a.C) % (4 * U) == 0 && a.bc_t % U == 0 && (a.x_t | a.dt_t | a.z_t | a.bc_t) < (1l << 31);
     constexpr size_t smem = ScanSmem<ACC, G, E>::BYTES;
     auto launch = [&](auto kernel) { llmp_launch_dependent(kernel, grid, dim3(SS_WALKERS<G> + 224), smem, stream, a); };
     if (wide) {
@@ -505,10 +510,13 @@ void launch_scan(const ScanArgs& a, int R, int max_q_len, cudaStream_t stream) {
     }
 }
 
-template <int G, int E> void launch_scan(ScanArgs& a, int out_dtype, int R, int max_q_len, cudaStream_t stream) {
-    a.singles = max_q_len != 1 && R > 1;
-    if (out_dtype == LLMP_BF16) launch_scan<bf16, float, G, E>(a, R, max_q_len, stream);
-    else launch_scan<float, double, G, E>(a, R, max_q_len, stream);
+template <int G, int E> int launch_scan(ScanArgs& a, int out_dtype, int max_q_len, cudaStream_t stream) {
+    constexpr int CH = SS_WALKERS<G> / G;
+    LLMP_REQUIRE(((long)a.inner + CH - 1) / CH * a.requests < (1l << 31), "selective_scan: too many channels %d of %d requests", a.inner, a.requests);
+    a.singles = max_q_len != 1 && a.requests > 1;
+    if (out_dtype == LLMP_BF16) launch_scan<bf16, float, G, E>(a, max_q_len, stream);
+    else launch_scan<float, double, G, E>(a, max_q_len, stream);
+    return llmp_check_launch("selective_scan");
 }
 
 // ---- few channels and many tokens: segments side by side ---------------------------------------------------------------
@@ -788,18 +796,15 @@ LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long
     LLMP_REQUIRE(inner > 0 && states > 0 && states <= 256, "selective_scan: %d channels with %d state entries (up to 256 are served)",
                  inner, states);
     LLMP_REQUIRE(state_half >= (long)inner * states, "selective_scan: the state piece is shorter than the state");
-    for (long stride : {x_t, dt_t, bc_t, z ? z_t : 0l})
-        LLMP_REQUIRE(stride >= 0 && stride < (1l << 31), "selective_scan: a row stride of %ld entries", stride);
-    LLMP_REQUIRE((inner + 3) / 4 <= 65535, "selective_scan: too many channels %d", inner);
     ScanArgs a;
     a.x = x; a.x_t = x_t; a.dt = dt; a.dt_t = dt_t; a.dt_bias = dt_bias; a.B = B; a.C = C; a.bc_t = bc_t; a.A = A; a.D = D;
     a.z = z; a.z_t = z ? z_t : 0; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
     a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states;
-    if (states <= 8) launch_scan<4, 2>(a, out_dtype, R, max_q_len, stream);
-    else if (states <= 16) launch_scan<8, 2>(a, out_dtype, R, max_q_len, stream);
-    else if (states <= 32) launch_scan<16, 2>(a, out_dtype, R, max_q_len, stream);
-    else if (states <= 64) launch_scan<32, 2>(a, out_dtype, R, max_q_len, stream);
-    else if (states <= 128) launch_scan<32, 4>(a, out_dtype, R, max_q_len, stream);
-    else launch_scan<32, 8>(a, out_dtype, R, max_q_len, stream);
-    return llmp_check_launch("selective_scan");
+    a.requests = R;
+    if (states <= 8) return launch_scan<4, 2>(a, out_dtype, max_q_len, stream);
+    if (states <= 16) return launch_scan<8, 2>(a, out_dtype, max_q_len, stream);
+    if (states <= 32) return launch_scan<16, 2>(a, out_dtype, max_q_len, stream);
+    if (states <= 64) return launch_scan<32, 2>(a, out_dtype, max_q_len, stream);
+    if (states <= 128) return launch_scan<32, 4>(a, out_dtype, max_q_len, stream);
+    return launch_scan<32, 8>(a, out_dtype, max_q_len, stream);
 }

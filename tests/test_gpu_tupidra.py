@@ -164,6 +164,31 @@ def test_selective_scan_stages(dtype, sizes):
             assert _rel(state[R - r].view(2, inner, states)[(m - 1) & 1], S) < 2e-5, (pad, r)
 
 
+@pytest.mark.parametrize("tokens,inner,apart", [(1, 1 << 20, 0), (2, (1 << 20) + 1, 0), (2, 64, 1 << 31)], ids=str)
+def test_selective_scan_of_as_many_channels_and_strides_as_there_are(tokens, inner, apart):
+    """More blocks of channels than a grid's shorter sides hold, and rows 2^31 entries apart: two tokens of one state entry, in float64 as
+    by hand."""
+    from llm_pipeline_b200.ops import kernels
+    gen = torch.Generator().manual_seed(inner)
+    x, raw, z = (torch.randn(tokens, inner, generator=gen).to(DEV) for _ in range(3))
+    bias, skip, A = (torch.randn(inner, generator=gen).to(DEV) for _ in range(3))
+    A = -A.abs().view(inner, 1)
+    bc = torch.randn(tokens, 2, generator=gen).to(DEV)
+    given = x
+    if apart:
+        given = torch.empty(apart + inner, device=DEV).as_strided((tokens, inner), (apart, 1))
+        given.copy_(x)
+    state, out = torch.zeros(1, 2 * inner, device=DEV), torch.empty(tokens, inner, device=DEV)
+    kernels.selective_scan(given, raw, bias, bc[:, :1], bc[:, 1:], A, skip, z, state, 0, _i32([0, tokens]), _i32([0]), _i32(list(range(tokens))), out, tokens)
+    S = torch.zeros(inner, dtype=torch.float64, device=DEV)
+    for t in range(tokens):
+        dt = torch.nn.functional.softplus(raw[t].double() + bias.double())
+        S = torch.exp(dt * A[:, 0].double()) * S + dt * x[t].double() * bc[t, 0].double()
+        want = (S * bc[t, 1].double() + skip.double() * x[t].double()) * z[t].double() * torch.sigmoid(z[t].double())
+        assert _rel(out[t], want.cpu()) < 1e-6, t
+    assert _rel(state[0].view(2, inner)[(tokens - 1) & 1], S.cpu()) < 1e-6
+
+
 @pytest.mark.parametrize("lengths", [(1, 64, 65), (128, 2, 1, 129, 31), (200,)], ids=str)
 @pytest.mark.parametrize("sizes", [(130, 16), (37, 5), (129, 32)], ids=str)
 def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
