@@ -495,7 +495,7 @@ void launch_scan(const ScanArgs& a, int max_q_len, cudaStream_t stream) {
     constexpr int CH = SS_WALKERS<G> / G, U = E < 4 ? E : 4;      // channels of a block, in both forms
     const int R = a.requests;
     const dim3 grid((unsigned)((a.inner + CH - 1) / CH * R));
-    if (max_q_len == 1 || R > 1) llmp_launch_dependent(selective_step_kernel<T, ACC, G, E>, grid, dim3(SS_WALKERS<G>), 0, stream, a);
+    if (max_q_len == 1 || a.singles) llmp_launch_dependent(selective_step_kernel<T, ACC, G, E>, grid, dim3(SS_WALKERS<G>), 0, stream, a);
     if (max_q_len == 1) return;
     const bool wide = a.inner % CH == 0 && ((uintptr_t)a.x | (uintptr_t)a.dt | (uintptr_t)a.z) % 16 == 0 && (a.x_t | a.dt_t | a.z_t) % 4 == 0 &&
                       a.states == G * E && ((uintptr_t)a.B | (uintptr_t)a.C) % (4 * U) == 0 && a.bc_t % U == 0 && (a.x_t | a.dt_t | a.z_t | a.bc_t) < (1l << 31);
@@ -510,10 +510,9 @@ void launch_scan(const ScanArgs& a, int max_q_len, cudaStream_t stream) {
     }
 }
 
-template <int G, int E> int launch_scan(ScanArgs& a, int out_dtype, int max_q_len, cudaStream_t stream) {
+template <int G, int E> int launch_scan(const ScanArgs& a, int out_dtype, int max_q_len, cudaStream_t stream) {
     constexpr int CH = SS_WALKERS<G> / G;
     LLMP_REQUIRE(((long)a.inner + CH - 1) / CH * a.requests < (1l << 31), "selective_scan: too many channels %d of %d requests", a.inner, a.requests);
-    a.singles = max_q_len != 1 && a.requests > 1;
     if (out_dtype == LLMP_BF16) launch_scan<bf16, float, G, E>(a, max_q_len, stream);
     else launch_scan<float, double, G, E>(a, max_q_len, stream);
     return llmp_check_launch("selective_scan");
@@ -787,11 +786,12 @@ LLMP_API int llmp_selective_scan_segments(const float* x, long x_t, const float*
     return llmp_check_launch("selective_scan_segments");
 }
 
-// max_q_len: the most tokens a request brings, or more.
+// max_q_len: the most tokens a request brings, or more. singles: 1 where a request of this step may bring a single token beside longer ones
+// (0 costs such a request the walk, with the same bits, and saves the others a launch).
 LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long dt_t, const float* dt_bias, const float* B,
                                  const float* C, long bc_t, const float* A, const float* D, const float* z, long z_t, float* state,
                                  long state_slot, long state_half, const int* q_start, const int* slots, const int* positions,
-                                 void* out, int out_dtype, long out_t, int R, int inner, int states, int max_q_len, cudaStream_t stream) {
+                                 void* out, int out_dtype, long out_t, int R, int inner, int states, int max_q_len, int singles, cudaStream_t stream) {
     if (R <= 0) return 0;
     LLMP_REQUIRE(inner > 0 && states > 0 && states <= 256, "selective_scan: %d channels with %d state entries (up to 256 are served)",
                  inner, states);
@@ -800,7 +800,7 @@ LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long
     a.x = x; a.x_t = x_t; a.dt = dt; a.dt_t = dt_t; a.dt_bias = dt_bias; a.B = B; a.C = C; a.bc_t = bc_t; a.A = A; a.D = D;
     a.z = z; a.z_t = z ? z_t : 0; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
     a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states;
-    a.requests = R;
+    a.requests = R; a.singles = singles && R > 1;
     if (states <= 8) return launch_scan<4, 2>(a, out_dtype, max_q_len, stream);
     if (states <= 16) return launch_scan<8, 2>(a, out_dtype, max_q_len, stream);
     if (states <= 32) return launch_scan<16, 2>(a, out_dtype, max_q_len, stream);

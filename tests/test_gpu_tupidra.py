@@ -474,6 +474,34 @@ def test_prefill_decoding_portions_and_batches(tmp_path, name, dtype):
     assert runner.cache.pages_reused > 0 or all(layer["type"] == "mamba1" for layer in cfg["layers"])
 
 
+def test_scans_launch_the_single_tokens_kernel_where_a_request_brings_one(tmp_path, monkeypatch):
+    """Steps of portions alone, and with single tokens among them: the layer says which it is, and where it says none of a step that has
+    some, the walk takes them to the same bits."""
+    from llm_pipeline_b200.ops import kernels
+    cfg, W, folder = case(tmp_path, "mixed", 6)
+    requests = requests_for(cfg, [40, 33, 21], 80)
+    runner = H.make_runner(folder, torch.bfloat16, page_size=8, num_pages=24, max_request_tokens=64, max_requests=3)
+    scan, said = kernels.selective_scan, []
+
+    def looking(*args):
+        state, q_start, out, longest, singles = args[8], args[10], args[13], args[14], args[15]
+        if longest > 1:
+            some = bool((q_start[1:] - q_start[:-1] == 1).any())
+            said.append((some, singles))
+            before = state.clone()
+            scan(*args[:15], not singles)
+            other = out.clone(), state.clone()
+            state.copy_(before)
+            scan(*args)
+            assert torch.equal(out, other[0]) and torch.equal(state, other[1])
+            return out
+        return scan(*args)
+
+    monkeypatch.setattr(kernels, "selective_scan", looking)
+    H.replay(runner, H.cut_mixed(requests, (5, 2, 9), max_live=3, decode_tail=4))
+    assert all(some == singles for some, singles in said) and {True, False} == {singles for _some, singles in said}
+
+
 def test_the_same_logits_alone_and_in_a_batch(tmp_path):
     """float32: a request's logits beside others, or cut into portions, are those it has alone, to rounding of sums."""
     cfg, W, folder = case(tmp_path, "mixed", 4)
