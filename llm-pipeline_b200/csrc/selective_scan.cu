@@ -226,11 +226,11 @@ __global__ void __launch_bounds__(SS_WALKERS<G>) selective_step_kernel(const Sca
     const int c = blockIdx.x / a.requests * CH + threadIdx.x / G;
     const bool ok = c < a.inner;
     const int cc = ok ? c : 0, have = ok ? a.states - l * E : 0;
-    float rate[E];
-    ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);           // weights: nothing of the step writes them
-    const float bias = a.dt_bias[cc], Dc = a.D[cc];
-    pdl_wait();
+    pdl_wait();                                                 // what the kernels before wrote is complete, A, D and the bias among it
     pdl_trigger();
+    float rate[E];
+    ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);
+    const float bias = a.dt_bias[cc], Dc = a.D[cc];
     const int t = a.q_start[r];
     if (a.q_start[r + 1] - t != 1) return;
     const int p0 = a.positions[t];

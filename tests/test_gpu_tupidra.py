@@ -189,6 +189,31 @@ def test_selective_scan_of_as_many_channels_and_strides_as_there_are(tokens, inn
     assert _rel(state[0].view(2, inner)[(tokens - 1) & 1], S.cpu()) < 1e-6
 
 
+def test_selective_scan_of_single_tokens_by_rates_just_made():
+    """Rates that the kernel launched before writes, other ones every time: the step is by those, as after a pause."""
+    from llm_pipeline_b200.ops import kernels
+    gen, R, inner, states = torch.Generator().manual_seed(1), 8, 2048, 16
+    x, raw, z = (torch.randn(R, inner, generator=gen).to(DEV) for _ in range(3))
+    bias, skip, bc = torch.randn(inner, generator=gen).to(DEV), torch.randn(inner, generator=gen).to(DEV), torch.randn(R, 2 * states, generator=gen).to(DEV)
+    made = [-torch.rand(inner, states, generator=gen).to(DEV) * 9 for _ in range(8)]
+    start, A = torch.randn(R, 2 * inner * states, generator=gen).to(DEV), torch.zeros(inner, states, device=DEV)
+    where = _i32(list(range(R + 1))), _i32(list(range(R))), _i32([5] * R)
+
+    def step(rates):
+        out, state = torch.empty(R, inner, device=DEV), start.clone()
+        if rates is not A:
+            kernels.convert_rows(rates, A)
+        kernels.selective_scan(x, raw, bias, bc[:, :states], bc[:, states:], A, skip, z, state, 0, *where, out, 1)
+        return out, state
+
+    at_once = [step(rates) for rates in made]
+    for rates, (out, state) in zip(made, at_once):
+        A.copy_(rates)
+        torch.cuda.synchronize()
+        paused, left = step(A)
+        assert torch.equal(out, paused) and torch.equal(state, left)
+
+
 @pytest.mark.parametrize("lengths", [(1, 64, 65), (128, 2, 1, 129, 31), (200,)], ids=str)
 @pytest.mark.parametrize("sizes", [(130, 16), (37, 5), (129, 32)], ids=str)
 def test_selective_scan_in_segments(sizes, lengths, monkeypatch):
