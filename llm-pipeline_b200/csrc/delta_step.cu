@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(DT_THREADS) delta_step_kernel(const DeltaStepA
     float* const vs = gs + d;                              // [dv]
     float* const part = vs + dv;                           // [DT_WARPS][2 dv]: a warp's shares of S^T k | S^T q
     float* const sums = part + DT_WARPS * 2 * dv;          // [2 dv]: u | S^T q
-    const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int group = a.H / a.G, kh = h / group, C = 2 * a.G * d + a.H * dv;
     // the channel that a thread filters
     const int c = tid < d ? kh * d + tid : (tid < 2 * d ? a.G * d + kh * d + tid - d : 2 * a.G * d + h * dv + tid - 2 * d);
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(DT_THREADS) delta_step_kernel(const DeltaStepA
 
 template <typename T> void launch_step(const DeltaStepArgs& a, int R, cudaStream_t stream) {
     const size_t smem = (size_t)(3 * a.d + a.dv + (DT_WARPS + 1) * 2 * a.dv) * sizeof(float);
-    auto launch = [&](auto kernel) { llmp_launch_dependent(kernel, dim3(a.H, R), dim3(DT_THREADS), smem, stream, a); };
+    auto launch = [&](auto kernel) { llmp_launch_dependent(kernel, dim3(R, a.H), dim3(DT_THREADS), smem, stream, a); };
     if (a.d <= DT_WARPS) launch(delta_step_kernel<T, 1>);
     else if (a.d <= 2 * DT_WARPS) launch(delta_step_kernel<T, 2>);
     else if (a.d <= 4 * DT_WARPS) launch(delta_step_kernel<T, 4>);
@@ -185,7 +185,7 @@ LLMP_API int llmp_delta_step(const float* proj, long proj_t, const float* decay,
                              long scan_offset, const int* q_start, const int* slots, const int* positions, void* out, int out_dtype,
                              long out_t, int R, int H, int G, int d, int dv, int K, float eps, cudaStream_t stream) {
     if (R <= 0) return 0;
-    LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && R <= 65535, "delta_step: bad sizes heads=%d qk_heads=%d requests=%d", H, G, R);
+    LLMP_REQUIRE(H > 0 && G > 0 && H % G == 0 && H <= 65535, "delta_step: bad sizes heads=%d qk_heads=%d", H, G);
     const int C = 2 * G * d + H * dv;
     LLMP_REQUIRE(llmp_delta_step_serves(C, d, dv, K), "delta_step: heads of %d x %d with %d taps are not served", d, dv, K);
     LLMP_REQUIRE((size_t)state % 16 == 0 && state_slot % 4 == 0 && scan_offset >= (long)2 * (K - 1) * C && scan_offset % 4 == 0,

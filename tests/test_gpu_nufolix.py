@@ -361,6 +361,28 @@ def test_gated_delta_rule_single_tokens_in_one_kernel(sizes, dtype):
     assert (got[others] == 7.0).all() and torch.equal(left[[0, 2, 5]], state[[0, 2, 5]])
 
 
+def test_gated_delta_rule_takes_more_single_tokens_than_a_grid_side():
+    """More requests than a grid's shorter sides hold: each has the bits it has among fewer."""
+    from llm_pipeline_b200.ops import kernels
+    heads, dim, taps, R, cut = 2, 4, 2, 65600, 40000
+    gen, C, scan = torch.Generator().manual_seed(2), 4 * heads * dim - heads * dim, 2 * 3 * heads * dim
+    rand = lambda *shape: torch.randn(*shape, generator=gen).cuda()   # noqa: E731
+    proj, decay, gate, conv_w, norm = rand(R, C + heads), rand(R, heads * dim), rand(R, heads * dim), rand(C, taps), rand(dim)
+    a_log, dt_bias, state = rand(heads), rand(heads * dim), rand(R, scan + 2 * heads * dim * dim)
+
+    def step(first, end):
+        n = end - first
+        out, left = torch.empty(n, heads * dim, device="cuda"), state.clone()
+        kernels.delta_step(proj[first:end], decay[first:end], gate[first:end], conv_w, a_log, dt_bias, norm, left, scan, _i32(range(n + 1)),
+                           _i32(range(first, end)), _i32([7] * n), out, heads, heads, dim, dim, 1e-5)
+        return out, left[first:end]
+
+    out, left = step(0, R)
+    for first, end in ((0, cut), (cut, R)):
+        part, kept = step(first, end)
+        assert torch.equal(out[first:end], part) and torch.equal(left[first:end], kept)
+
+
 @pytest.mark.parametrize("sizes", [(2, 1, 64, 16), (1, 1, 128, 48)], ids=str)
 def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
     """Forty portions in chunks and as many short ones token by token in one step, more than a warp looks at in one go, in an order
