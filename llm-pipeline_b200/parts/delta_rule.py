@@ -120,11 +120,14 @@ class GatedDeltaRule(Mixer):
             raise RuntimeError("the delta-rule mixer needs its state slots")
         N, C, H = ctx.num_tokens, self.channels, self.heads
         proj = linear(x, self.w_in, out_dtype=torch.float32)
-        low = proj[:, C + H:]
+        low = [proj[:, C + H:]]
         if x.dtype != torch.float32:
-            low = kernels.convert_rows(low, torch.empty(low.shape, dtype=x.dtype, device=x.device))
-        decay = linear(low[:, :self.decay_rank], self.w_a2, out_dtype=torch.float32)
-        gate = linear(low[:, self.decay_rank:], self.w_g2, out_dtype=torch.float32)
+            if self.decay_rank % 8 or self.gate_rank % 8:                  # each in rows of its own, which start on 16 bytes where they can
+                low = [low[0][:, :self.decay_rank], low[0][:, self.decay_rank:]]
+            low = [kernels.convert_rows(part, torch.empty(part.shape, dtype=x.dtype, device=x.device)) for part in low]
+        low_a, low_g = low if len(low) == 2 else (low[0][:, :self.decay_rank], low[0][:, self.decay_rank:])
+        decay = linear(low_a, self.w_a2, out_dtype=torch.float32)
+        gate = linear(low_g, self.w_g2, out_dtype=torch.float32)
         normed = torch.empty((N, self.v_size), dtype=x.dtype, device=x.device)
         # single tokens take a kernel of their own in any company (their rows and state have the same bits there)
         singles = (ctx.max_q_len == 1 or 1 in ctx.q_lens) and kernels.delta_step_serves(C, self.dim, self.vdim, self.taps, cache.state, 0)

@@ -365,7 +365,7 @@ def test_gated_delta_rule_takes_more_single_tokens_than_a_grid_side():
     """More requests than a grid's shorter sides hold: each has the bits it has among fewer."""
     from llm_pipeline_b200.ops import kernels
     heads, dim, taps, R, cut = 2, 4, 2, 65600, 40000
-    gen, C, scan = torch.Generator().manual_seed(2), 4 * heads * dim - heads * dim, 2 * 3 * heads * dim
+    gen, C, scan = torch.Generator().manual_seed(2), 3 * heads * dim, 6 * heads * dim
     rand = lambda *shape: torch.randn(*shape, generator=gen).cuda()   # noqa: E731
     proj, decay, gate, conv_w, norm = rand(R, C + heads), rand(R, heads * dim), rand(R, heads * dim), rand(C, taps), rand(dim)
     a_log, dt_bias, state = rand(heads), rand(heads * dim), rand(R, scan + 2 * heads * dim * dim)
@@ -381,6 +381,50 @@ def test_gated_delta_rule_takes_more_single_tokens_than_a_grid_side():
     for first, end in ((0, cut), (cut, R)):
         part, kept = step(first, end)
         assert torch.equal(out[first:end], part) and torch.equal(left[first:end], kept)
+
+
+def _delta_layer(sizes, ranks, gen, width=64):
+    """A layer in bfloat16 with random weights, and a function that runs it over portions: (requests' rows, their starts, the state
+    tensor) to the outputs; request r has slot r."""
+    from llm_pipeline_b200.engine.context import StepContext
+    from llm_pipeline_b200.parts import LayerCache, lookup
+    heads, qk_heads, dim, vdim = sizes
+    part = lookup("mixer", "gated_delta_rule")("p", hidden_size=width, heads=heads, qk_heads=qk_heads, dim=dim, vdim=vdim, decay_rank=ranks[0], gate_rank=ranks[1])
+    # (the shapes of the two-step projections are known before the tensors are here: the ranks are given)
+    part.load(lambda name, role: (torch.randn(part.param_specs()[name].shape, generator=gen) * (0.2 if role == "matrix" else 0.5)).to("cuda").to(
+        torch.bfloat16 if role == "matrix" else torch.float32))
+
+    def run(rows, starts, state):
+        lens = [x.shape[0] for x in rows]
+        ctx = StepContext(torch.device("cuda"), torch.bfloat16)
+        ctx.num_tokens, ctx.num_requests, ctx.q_lens, ctx.starts, ctx.max_q_len = sum(lens), len(lens), lens, list(starts), max(lens)
+        ctx.q_start = _i32([0] + list(itertools.accumulate(lens)))
+        ctx.positions = _i32([s + i for n, s in zip(lens, starts) for i in range(n)])
+        ctx.token_request = _i32([r for r, n in enumerate(lens) for _ in range(n)])
+        ctx.slots = _i32(range(len(lens)))
+        return part.forward(torch.cat(rows), ctx, LayerCache(state=state))[0]
+
+    return part, run
+
+
+def test_delta_rule_products_of_odd_ranks_have_rows_on_sixteen_bytes(monkeypatch):
+    """Inner sizes of the two-step projections of which one is a multiple of 8 and the other is not: the products' rows start on 16 bytes
+    as a tensor of their own would, so that they take the kernels that they take beside any other size."""
+    from llm_pipeline_b200.parts import delta_rule
+    seen, linear = [], delta_rule.linear
+
+    def looking(x, weight, **more):
+        seen.append(x.shape[1])
+        assert x.shape[1] % 8 or (x.data_ptr() % 16 == 0 and x.stride(0) % 8 == 0), (x.shape, x.stride())
+        return linear(x, weight, **more)
+
+    monkeypatch.setattr(delta_rule, "linear", looking)
+    for ranks in ((16, 12), (12, 16), (24, 8)):
+        gen = torch.Generator().manual_seed(ranks[0])
+        part, run = _delta_layer((2, 1, 64, 16), ranks, gen)
+        rows = [torch.randn(n, 64, generator=gen).to(torch.bfloat16).cuda() for n in (1, 3, 1)]
+        assert torch.isfinite(run(rows, (0, 2, 5), torch.zeros(3, part.state_entries(), device="cuda"))).all()
+        assert seen[-4:] == [64, *ranks, 32]
 
 
 @pytest.mark.parametrize("sizes", [(2, 1, 64, 16), (1, 1, 128, 48)], ids=str)
