@@ -1677,16 +1677,15 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
 
 def delta_step_serves(channels: int, dim: int, vdim: int, taps: int, state: torch.Tensor, state_offset: int) -> bool:
     """Whether ``delta_step`` takes single tokens through a layer of these sizes: it follows from the layer and its state alone."""
-    fn = library().llmp_delta_step_serves
-    fn.argtypes, fn.restype = [_I, _I, _I, _I], _I
-    return bool(fn(channels, dim, vdim, taps)) and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0 and state_offset % 4 == 0
+    return bool(library().llmp_delta_step_serves(channels, dim, vdim, taps)) and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0 and state_offset % 4 == 0
 
 
 def delta_step(proj: torch.Tensor, decay: torch.Tensor, gate: torch.Tensor, taps: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                norm: torch.Tensor, state: torch.Tensor, scan_offset: int, q_start: torch.Tensor, slots: torch.Tensor, positions: torch.Tensor,
                out: torch.Tensor, heads: int, qk_heads: int, dim: int, vdim: int, eps: float) -> torch.Tensor:
     """The convolution, ``delta_prep``, ``delta_scan`` and the gated norm for the step's requests that bring one token, in one kernel
-    (csrc/delta_step.cu); the others are left alone. ``proj`` float32 [tokens, >= C + heads] = q | k | v | beta as projected (C = 2 qk_heads dim +
+    (csrc/delta_step.cu); the others are left alone. The layer's vectors (``taps``, ``a_log``, ``dt_bias``) may be read while the kernel before is still at
+    work. ``proj`` float32 [tokens, >= C + heads] = q | k | v | beta as projected (C = 2 qk_heads dim +
     heads vdim), ``decay`` [tokens, heads dim] and ``gate`` [tokens, heads vdim] before their functions, ``taps`` [C, K], ``out`` [tokens, heads
     vdim] in the compute type. The convolution's inputs lie at the front of the slot, the rule's state at ``scan_offset``."""
     H, G, d, dv = int(heads), int(qk_heads), int(dim), int(vdim)
@@ -1871,7 +1870,7 @@ def sigmoid_decode(q: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor, c
                    out: torch.Tensor, heads: int, kv_heads: int, dim: int, vdim: int, scale: float, softcap: float, segments: int,
                    segment_keys: int) -> torch.Tensor:
     """``sigmoid_attention`` for steps of one token a request (csrc/sigmoid_decode.cu): row n of the bfloat16 queries is request n's.
-    ``segments`` > 1: ranges of ``segment_keys`` keys (a multiple of ``sigmoid_decode_keys``) go to blocks of their own; together they must
+    ``talk`` and ``head_bias`` are the layer's: they may be read while the kernel before is still at work. ``segments`` > 1: ranges of ``segment_keys`` keys (a multiple of ``sigmoid_decode_keys``) go to blocks of their own; together they must
     cover the most keys a request sees."""
     N = q.shape[0]
     _need(q.dtype == out.dtype == pages.dtype == torch.bfloat16 and q.shape == (N, heads * dim) and q.stride(1) == 1 and

@@ -473,6 +473,74 @@ def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
     kernels.check_error_flag()
 
 
+@pytest.mark.parametrize("ranks", [(8, 8), (16, 12)], ids=str)
+def test_delta_rule_layer_single_tokens_in_any_company(ranks, monkeypatch):
+    """The whole layer over two steps of single tokens, alone, beside short portions and beside portions in chunks: a request's outputs and
+    state have the same bits, and the portions have theirs without single tokens beside them. (The layer's products go through a
+    kernel whose rows do not depend on one another; the library's may.)"""
+    from llm_pipeline_b200.ops import kernels
+    from llm_pipeline_b200.parts import delta_rule
+    monkeypatch.setattr(delta_rule, "linear", lambda x, w, out_dtype: kernels.gemm_simt(x, w, torch.empty(x.shape[0], w.shape[0], dtype=out_dtype, device="cuda")))
+    monkeypatch.setattr(kernels, "DELTA_CHUNKS_MIN_TOKENS", 17)
+    gen = torch.Generator().manual_seed(ranks[1])
+    part, run = _delta_layer((2, 1, 64, 16), ranks, gen)
+    lengths, starts = [1, 5, 1, 40, 16, 1, 17, 2], [3, 0, 8, 5, 0, 2, 1, 0]
+    rows = [torch.randn(2 * n, 64, generator=gen).to(torch.bfloat16).cuda() for n in lengths]
+    state = torch.randn(len(lengths), part.state_entries(), generator=gen).cuda() * 0.1
+
+    def steps(requests):
+        left, outs = state[requests].clone(), []
+        for k in range(2):
+            own = [rows[r][k * lengths[r]:(k + 1) * lengths[r]] for r in requests]
+            out = run(own, [starts[r] + k * lengths[r] for r in requests], left)
+            outs.append(torch.split(out, [x.shape[0] for x in own]))
+        return {r: (outs[0][i], outs[1][i], left[i]) for i, r in enumerate(requests)}
+
+    alone = {r: steps([r])[r] for r in range(len(lengths))}
+    for company in ([0, 2, 5], [0, 1, 2, 4, 7], [0, 3, 6], [3, 0, 5, 6], list(range(8)), [1, 3, 4, 6, 7]):
+        for r, got in steps(company).items():
+            assert all(torch.equal(a, b) for a, b in zip(got, alone[r])), (company, r)
+    kernels.check_error_flag()
+
+
+def test_delta_rule_leaves_the_requests_below_its_least_alone(monkeypatch):
+    """``least`` of the preparation, the walk and the chunks: rows and state of requests with fewer tokens stay as they are, the others'
+    have the bits they have without it."""
+    from llm_pipeline_b200.ops import kernels
+    monkeypatch.setattr(kernels, "DELTA_CHUNKS_MIN_TOKENS", 17)
+    heads, qk_heads, dim, vdim = 2, 1, 64, 16
+    gen, dev, piece = torch.Generator().manual_seed(3), "cuda", heads * dim * vdim
+    lengths = [1, 4, 1, 24, 2, 1]
+    starts, N, R = [0] + list(itertools.accumulate(lengths)), sum(lengths), len(lengths)
+    a_log, dt_bias = torch.rand(heads, generator=gen).to(dev), torch.randn(heads * dim, generator=gen).to(dev)
+    rows = [x.to(dev) for x in _delta_rule_rows(gen, N, heads, qk_heads, dim, vdim)]
+    state = torch.randn(R, 2 * piece, generator=gen).to(dev)
+    where = _i32(starts), _i32(range(R)), _i32([5 + p for n in lengths for p in range(n)])
+    request = _i32([r for r, n in enumerate(lengths) for _ in range(n)])
+    need = kernels.delta_chunks_scratch(torch.bfloat16, 24, 1, 24, heads, dim, vdim)
+    got = {}
+    for way in ("walk", "chunks"):
+        for least in (1, 2):
+            x, left, o = [y.clone() for y in rows], state.clone(), torch.full((N, heads * vdim), 7.0, device=dev)
+            q, k, v, decay, beta = x
+            if way == "walk":
+                kernels.delta_prep(q, k, decay, beta, a_log, dt_bias, heads, qk_heads, dim, request, where[0], least)
+                kernels.delta_scan(q, k, v, decay, beta, left, 0, *where, o, heads, qk_heads, dim, vdim, least)
+            else:
+                kernels.delta_chunks(q, k, v, decay, beta, a_log, dt_bias, left, 0, *where, o, heads, qk_heads, dim, vdim, need, (_i32([3]), 24), request,
+                                     least)
+            got[way, least] = x, left, o
+    single = [0, 2, 5]
+    mine = torch.tensor([starts[r] for r in single], device=dev)
+    rest = torch.tensor([t for t in range(N) if t not in mine.tolist()], device=dev)
+    for way in ("walk", "chunks"):
+        (x1, left1, o1), (x2, left2, o2) = got[way, 1], got[way, 2]
+        assert all(torch.equal(a[mine], b[mine]) for a, b in zip(x2, rows)) and (o2[mine] == 7.0).all() and torch.equal(left2[single], state[single])
+        assert all(torch.equal(a[rest], b[rest]) for a, b in zip(x2, x1)) and torch.equal(o2[rest], o1[rest])
+        assert torch.equal(left2[[1, 3, 4]], left1[[1, 3, 4]]) and not torch.equal(left1[single], state[single])
+    kernels.check_error_flag()
+
+
 def _sigmoid_attention_case(dtype, heads, kv_heads, dim, vdim, n, page, seed, cap=0.0, plant=None, segments=(1,), bias=-1.0,
                             mixed=None):
     """Queries, keys and values as they enter the scores, written into shuffled pages; (engine outputs, plain output). ``mixed``
