@@ -1858,7 +1858,7 @@ def sigmoid_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Te
     return out
 
 
-SIGMOID_DECODE_BLOCKS_PER_SM = 1     # key ranges grow once the blocks would be more (a block fills an SM)
+SIGMOID_DECODE_RANGE_KEYS = 512      # the most keys of a range, unless there would be too many sums
 
 
 def sigmoid_decode_keys(dtype: torch.dtype, heads: int, kv_heads: int, dim: int, vdim: int) -> int:

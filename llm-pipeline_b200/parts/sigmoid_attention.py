@@ -90,13 +90,18 @@ class SigmoidAttention(Mixer):
         return self._single
 
     def _decode_ranges(self, tokens: int, longest: int):
-        """(number of key ranges, keys of a range) of a step of single tokens: one tile a range until the blocks are many."""
+        """(number of key ranges, keys of a range) of a step of single tokens: of ranges of up to ``SIGMOID_DECODE_RANGE_KEYS`` those that cost
+        least, rounds of blocks (each fills an SM) times a range's tiles and half a tile for a block's start. Longer ones would spare short
+        requests a little, but a long one beside them would be walked by a few blocks: 16 requests of 512 keys with one of 32,768 52 us,
+        in ranges as long as give one round of blocks 287; 16 of 4,096 49 and 48 us, 200 of 2,000 248 and 329."""
         tile = self._decode_keys()
-        most = max(1, min(self.SEGMENTS_MAX_BYTES // (4 * tokens * self.num_heads * self.vdim),
-                          kernels.SIGMOID_DECODE_BLOCKS_PER_SM * kernels.sm_count() // tokens))
         tiles = -(-longest // tile)
-        keys = tile * -(-tiles // most)
-        return -(-longest // keys), keys
+        fits = max(1, self.SEGMENTS_MAX_BYTES // (4 * tokens * self.num_heads * self.vdim))      # ranges whose sums take no more than that
+        least = -(-tiles // fits)
+        most = max(least, min(tiles, kernels.SIGMOID_DECODE_RANGE_KEYS // tile))
+        sms = kernels.sm_count()
+        per = min(range(least, most + 1), key=lambda n: -(-tokens * -(-tiles // n) // sms) * (2 * n + 1))
+        return -(-tiles // per), tile * per
 
     def _segments(self, tokens: int, longest: int):
         """(number of key ranges, keys of a range) for a step of ``tokens`` new tokens whose longest context is ``longest``."""

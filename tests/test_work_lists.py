@@ -8,6 +8,7 @@ import pytest
 from llm_pipeline_b200.ops import kernels
 from llm_pipeline_b200.parts.attention import AttentionPolicy
 from llm_pipeline_b200.parts.capped_attention import CappedAttention
+from llm_pipeline_b200.parts.sigmoid_attention import SigmoidAttention
 
 SMS = 148
 
@@ -120,3 +121,21 @@ def test_a_token_of_capped_attention_cuts_its_keys_alike_in_any_company(monkeypa
             assert part._segments(single_tokens(requests, longest)) == want
             assert part._segments(single_tokens(requests, 1, bound=longest)) == want
     assert part._segments(SimpleNamespace(max_q_len=2)) == 0
+
+
+@pytest.mark.parametrize("tile", [64, 32])
+def test_single_tokens_of_sigmoid_attention_take_ranges_of_bounded_length(monkeypatch, tile):
+    """Ranges of whole tiles that cover the longest context, none longer than 512 keys however many requests there are, so that a long
+    one beside short ones is spread over the SMs; longer only where the sums of all ranges would take more memory than they may."""
+    monkeypatch.setattr(kernels, "sm_count", lambda: SMS)
+    part = SigmoidAttention("p", 64, 16, 4, 128, 128, 0.1)
+    part._single = tile
+    for tokens in (1, 2, 8, 16, 37, 64, 200, 1000):
+        for longest in (1, 63, 64, 65, 300, 2000, 4096, 32768, 131072):
+            ranges, keys = part._decode_ranges(tokens, longest)
+            assert keys % tile == 0 and (ranges - 1) * keys < longest <= ranges * keys
+            taken = 4 * tokens * 16 * 128 * ranges
+            assert taken <= part.SEGMENTS_MAX_BYTES
+            assert keys <= 512 or 2 * taken > part.SEGMENTS_MAX_BYTES - 4 * tokens * 16 * 128
+    assert part._decode_ranges(8, 2000) == (-(-2000 // 128), 128)             # one round of 128 blocks
+    assert part._decode_ranges(1, tile) == (1, tile)
