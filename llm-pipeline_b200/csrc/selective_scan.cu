@@ -401,8 +401,8 @@ __global__ void __launch_bounds__(SS_WALKERS<G> + 224, E == 2 && sizeof(ACC) == 
                     ss_copy<XU * 4>(d + L::ROWS, sd + (long)row * d_t, in);
                     if (gated) ss_copy<XU * 4>(d + 2 * L::ROWS, sz + (long)row * z_t, in);
                 }
-#pragma unroll 1
-                for (int i = 0; i < BJ; ++i) {
+#pragma unroll (WIDE && BJ == 2 ? 2 : 1)
+                for (int i = 0; i < BJ; ++i) {                 // (unrolled, 256 entries are 64 copies a lane and stage, by 4 bytes 256)
                     const int j = h % BCOLS + i * 32, e = j % (BCOLS / 2) * BU;
                     const bool is_c = j >= BCOLS / 2, in_e = e < a.states;
                     const float* src = (is_c ? a.C : a.B) + (size_t)(begin + t0) * a.bc_t + (in_e ? e : 0);
