@@ -16,6 +16,7 @@
 // leaves its loops, frees its tensor memory and returns; the host reads the flag.
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -571,7 +572,7 @@ static int launch_tc_persistent(const void* A, long rows_a, long lda, const void
 // are read once, and a block's ring asks for a good part of its share at once. The accumulators are put into the blocks' shared
 // memory, and each block adds a share of the tile's rows from all of them, in their order. 12.6 us; 300 rows 22.1 and 11.9; 96 columns,
 // K 2,048 12.8 and 7.9. Eight blocks: 9.0 for 300 rows, but 18.1 for 2,048, whose 16 clusters do not fit the SMs' groups at once; two: 19.6.
-// The shares follow from K alone. smem: the ring, then the same place for the accumulator, rows padded by 4 floats.
+// The shares follow from K alone, so a row has the same bits among any number of rows that go this way (another number takes tiles). smem: the ring, then the same place for the accumulator, rows padded by 4 floats.
 constexpr int NARROW_SPLITS = 4, NARROW_MAX_COLS = 256, NARROW_MAX_STAGES = 8;
 template <typename TO>
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -688,23 +689,15 @@ gemm_tc_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
 }
 
-template <typename TO>
-static int launch_tc_narrow(const void* A, int M, long lda, const void* B, int N, long ldb, TO* Y, int K, long ldy, int* error_flag, cudaStream_t stream) {
-    const int bn = (N + 15) / 16 * 16;
-    CUtensorMap map_a, map_b;
-    if (llmp_matrix_tensor_map(A, M, K, lda, TC_BM, &map_a) || llmp_matrix_tensor_map(B, N, K, ldb, bn, &map_b)) return 1;
-    const size_t stage = TC_BM * 128 + (size_t)bn * 128, room = 200 * 1024;      // one block an SM: tensor memory is not shared with another's
-    const int stages = room / stage < NARROW_MAX_STAGES ? (int)(room / stage) : NARROW_MAX_STAGES;
-    const size_t sums = (size_t)TC_BM * (bn + 4) * sizeof(float), smem = room + 1024;
-    LLMP_REQUIRE(sums <= room, "gemm_tc: %d columns do not fit", N);
+constexpr size_t NARROW_ROOM = 200 * 1024;                     // one block an SM: tensor memory is not shared with another's
+
+template <typename TO> static cudaLaunchConfig_t narrow_config(int M, cudaLaunchAttribute (&attr)[2]) {
     auto kernel = gemm_tc_narrow_kernel<TO>;
-    LLMP_ALLOW_SMEM(kernel, smem);
+    LLMP_ALLOW_SMEM(kernel, NARROW_ROOM + 1024);
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((M + TC_BM - 1) / TC_BM, NARROW_SPLITS);
     config.blockDim = dim3(TC_THREADS);
-    config.dynamicSmemBytes = smem;
-    config.stream = stream;
-    cudaLaunchAttribute attr[2];
+    config.dynamicSmemBytes = NARROW_ROOM + 1024;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = NARROW_SPLITS;
@@ -712,8 +705,49 @@ static int launch_tc_narrow(const void* A, int M, long lda, const void* B, int N
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attr;
+    config.numAttrs = 1;
+    return config;
+}
+
+// Clusters that have their places at once. A cluster lies in one group of SMs, whose number is not a multiple of its blocks everywhere: 148
+// SMs hold fewer than 37 of four blocks. Asked once a device.
+template <typename TO> static int narrow_clusters() {
+    static std::atomic<int> known[64];
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device >= 64) return 0;
+    int n = known[device].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t config = narrow_config<TO>(1, attr);
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_tc_narrow_kernel<TO>, &config) != cudaSuccess || n <= 0) {
+            cudaGetLastError();
+            n = -1;
+        }
+        known[device].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Up to 256 columns and K of 1,024 or more, while the clusters are one round. Microseconds in tiles and in clusters, K 768, 1,024, 1,536: 2,048
+// rows by 96 columns 6.4 and 5.9, 7.5 and 6.6, 9.7 and 7.5; by 160 columns 6.5 and 7.3, 7.7 and 7.8, 10.2 and 8.6; 4,096 rows by
+// 256 columns of K 2,048 15.6 and 12.1, 4,736 rows, a second round of clusters, 15.8 and 21.5.
+template <typename TO> static bool narrow_serves(int M, int N, int K) {
+    return M > 64 && N <= NARROW_MAX_COLS && K >= 1024 && (M + TC_BM - 1) / TC_BM <= narrow_clusters<TO>();
+}
+
+template <typename TO>
+static int launch_tc_narrow(const void* A, int M, long lda, const void* B, int N, long ldb, TO* Y, int K, long ldy, int* error_flag, cudaStream_t stream) {
+    const int bn = (N + 15) / 16 * 16;
+    CUtensorMap map_a, map_b;
+    if (llmp_matrix_tensor_map(A, M, K, lda, TC_BM, &map_a) || llmp_matrix_tensor_map(B, N, K, ldb, bn, &map_b)) return 1;
+    const size_t stage = TC_BM * 128 + (size_t)bn * 128;
+    const int stages = NARROW_ROOM / stage < NARROW_MAX_STAGES ? (int)(NARROW_ROOM / stage) : NARROW_MAX_STAGES;
+    LLMP_REQUIRE((size_t)TC_BM * (bn + 4) * sizeof(float) <= NARROW_ROOM, "gemm_tc: %d columns do not fit", N);
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t config = narrow_config<TO>(M, attr);
+    config.stream = stream;
     config.numAttrs = llmp_pdl_enabled() ? 2 : 1;
-    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, map_a, map_b, Y, M, N, K, ldy, bn, stages, error_flag);
+    const cudaError_t err = cudaLaunchKernelEx(&config, gemm_tc_narrow_kernel<TO>, map_a, map_b, Y, M, N, K, ldy, bn, stages, error_flag);
     if (err != cudaSuccess) {
         llmp_set_error("gemm_tc: cluster launch failed: %s", cudaGetErrorString(err));
         return 2;
@@ -727,9 +761,7 @@ static int dispatch_tc(const void* X, const void* W, TO* Y, int M, int N, int K,
     if (M <= 16) return launch_tc_splitk<16, 10, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 32) return launch_tc_splitk<32, 9, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
     if (M <= 64) return launch_tc_splitk<64, 8, TO>(W, N, ldw, X, M, ldx, Y, K, ldy, error_flag, stream);
-    // Up to 256 columns with a long K, while the clusters are one round of blocks (16 tiles of 128 rows of 148 SMs).
-    if (N <= NARROW_MAX_COLS && K >= 1024 && (long)((M + TC_BM - 1) / TC_BM) * NARROW_SPLITS <= llmp_sm_count())
-        return launch_tc_narrow(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
+    if (narrow_serves<TO>(M, N, K)) return launch_tc_narrow(X, M, ldx, W, N, ldw, Y, K, ldy, error_flag, stream);
     // 128 x 256 tiles do twice the work per byte read from shared memory; 128 x 128 only for narrow outputs, and 128 x 32 where the SMs
     // take even those in one go: 2,048 rows, 160 columns, K 4,096 26.2 us -> 22.2; 96 columns, K 2,048 15.8 -> 12.6. (Sharing K among
     // the blocks of a cluster, 64 rows by 128 columns each, lost: 31 and 25 us; for a long K the kernel above.)
@@ -742,6 +774,11 @@ static int dispatch_tc(const void* X, const void* W, TO* Y, int M, int N, int K,
 // Y[M, N] = X[M, K] * W[N, K]^T, bfloat16 operands with 16-byte aligned rows (K, ldx, ldw multiples of 8),
 // Y bfloat16 or float32. error_flag: one int in device memory that the kernel sets to 1 when a wait
 // ran out (the host checks it after synchronising).
+// Whether a product of these sizes is shared in clusters.
+LLMP_API int llmp_gemm_tc_narrow_serves(int out_dtype, int M, int N, int K) {
+    return out_dtype == LLMP_F32 ? narrow_serves<float>(M, N, K) : narrow_serves<bf16>(M, N, K);
+}
+
 LLMP_API int llmp_gemm_tc(const void* X, const void* W, void* Y, int out_dtype, int M, int N, int K, long ldx, long ldw,
                           long ldy, int* error_flag, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;

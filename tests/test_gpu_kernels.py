@@ -272,6 +272,32 @@ def test_gemm_tcgen05_narrow_outputs(out_dtype, M, N, Kd):
 
 
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
+def test_gemm_tcgen05_narrow_outputs_go_in_clusters_of_one_round(out_dtype):
+    """Narrow outputs share K in clusters as long as all clusters have their places at once, which on SMs in groups is fewer than a quarter
+    of them; a row has the same bits among any number of rows that go so, and beyond the last of them it is in tiles, as near to
+    float64 (the bound of the test above)."""
+    from llm_pipeline_b200.ops.build import library
+    N, Kd, code = 96, 1536, K().dtype_code(out_dtype)
+    serves = library().llmp_gemm_tc_narrow_serves
+    tiles = max(t for t in range(1, 64) if serves(code, t * 128, N, Kd))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert sms // 8 <= tiles <= sms // 4 and not serves(code, tiles * 128 + 1, N, Kd) and not serves(code, 300, N, 1016) and not serves(code, 300, 257, Kd)
+    if sms == 148:
+        assert tiles < 37                                       # what 4,736 rows lose by a second round
+    M = (tiles + 1) * 128
+    x, w = rnd(M, Kd, dtype=torch.bfloat16, seed=21), rnd(N, Kd, dtype=torch.bfloat16, seed=22)
+    outs = {}
+    for rows in (65, 300, tiles * 128, M):
+        outs[rows] = torch.empty(rows, N, dtype=out_dtype, device=DEV)
+        K().gemm_tc(x[:rows], w, outs[rows])
+    K().check_error_flag()
+    assert torch.equal(outs[65], outs[300][:65]) and torch.equal(outs[300], outs[tiles * 128][:300])
+    want, sizes = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0)
+    assert all(((out.double() - want[:rows]).abs() <= bound[:rows]).all() for rows, out in outs.items())
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32out"])
 @pytest.mark.parametrize("stride,offset", [(0, 0), (1, 0), (4, 0), (8, 3)], ids=["whole", "odd", "half", "off"])
 @pytest.mark.parametrize("M,N,Kd", [(2500, 250, 72), (2500, 200, 64), (300, 200, 72), (300, 24, 72), (200, 264, 128), (129, 300, 64)])
 def test_gemm_tcgen05_stores(out_dtype, M, N, Kd, stride, offset):
