@@ -525,8 +525,8 @@ template <int G, int E> int launch_scan(const ScanArgs& a, int out_dtype, int ma
 //   2. along a request's segments: scratch becomes the state before each (requests of one segment have nothing to do);
 //   3. every segment from the state before it: the outputs; the last segment leaves the state in the slot.
 // This takes every exponential twice, but nothing waits for a chain of all tokens: where the channels are too few to fill the chip
-// and the tokens many, it ends first. 8,192 tokens of 16 entries, walk against segments: 512 channels 199 and 107 us, 1,024 260 and 142;
-// 2,048 tokens of 1,024, 2,048, 4,096 channels 53 and 67, 54 and 84, 94 and 117.
+// and the tokens many, it ends first. The caller draws the line (`scan_prefers_segments`): 4,096 tokens of 16 entries, walk against
+// segments, 512 channels 103 and 64 us, 1,024 104 and 92, 2,048 136 and 127, 4,096 184 and 226.
 constexpr int SEG_TOKENS = 64;
 constexpr int SEG_CHANNELS = 128;         // threads of a block, a channel each
 constexpr int SEG_AHEAD = 4;              // tokens whose loads are under way while as many are worked on

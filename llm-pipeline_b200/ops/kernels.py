@@ -2084,8 +2084,29 @@ def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Ten
 SELECTIVE_SCAN_MAX_STATES = 256
 
 
-SCAN_SEGMENT_TOKENS, SCAN_SEGMENTS_MAX_STATES, SCAN_SEGMENTS_MAX_CHANNELS = 64, 32, 1024       # csrc/selective_scan.cu
-SCAN_SEGMENTS_MIN_TOKENS = 4096
+SCAN_SEGMENT_TOKENS, SCAN_SEGMENTS_MAX_STATES = 64, 32       # csrc/selective_scan.cu
+SCAN_SEGMENTS_MIN_TOKENS, SCAN_SEGMENTS_MAX_WIDTH = 1024, 32768
+
+
+def _scan_entries(states: int) -> int:
+    return 8 if states <= 8 else 16 if states <= 16 else 32
+
+
+def scan_prefers_segments(tokens: int, longest: int, inner: int, states: int) -> bool:
+    """Whether a bfloat16 step of ``tokens``, of which one request brings ``longest``, goes in segments side by side. A walk takes as long
+    as the longest portion whatever the channels, until they fill the chip; segments take every exponential twice, but nothing waits for
+    a chain. Microseconds, walked and in segments, one request: 512 channels of 16 entries 1,408 tokens 39 and 42, 1,792 48 and 44,
+    4,096 103 and 64; 1,024 channels 1,792 49 and 56, 2,816 73 and 69, 4,096 104 and 92; 2,048 channels 2,816 78 and 102, 4,096 136 and 127;
+    4,096 channels 4,096 184 and 226, 16,384 719 and 841. 8 entries: 1,024 channels 1,792 43 and 39, 2,048 channels 2,304 54 and 66,
+    3,456 100 and 86; 32 entries: 512 channels 2,816 74 and 85, 4,096 105 and 106, 6,144 156 and 124. Over 426 such sizes the line costs
+    0.9 % beside the better of the two each time (several requests near it up to 38 %)."""
+    if states > SCAN_SEGMENTS_MAX_STATES or longest <= 0:
+        return False
+    entries = _scan_entries(states)
+    width = entries * inner * tokens / longest                  # of all requests, were they as long as the longest
+    if width > SCAN_SEGMENTS_MAX_WIDTH:
+        return longest > SCAN_SEGMENTS_MIN_TOKENS << 20         # (never)
+    return longest > SCAN_SEGMENTS_MIN_TOKENS * (1 + width / (12288 if entries < 32 else 6144))
 
 
 def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: torch.Tensor, c: torch.Tensor, a: torch.Tensor,
@@ -2113,14 +2134,11 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: 
     requests = slots.numel()
     if max_q_len is None:
         max_q_len = N
-    # Few channels leave a walk over many tokens alone on the chip: then the tokens go in segments side by side, which take every
-    # exponential twice (8,192 tokens of 1,024 channels 142 us, walked 260; of 2,048 tokens 67 and 53). float32 output: the state is
-    # float64 in between.
-    if (max_q_len > SCAN_SEGMENTS_MIN_TOKENS and states <= SCAN_SEGMENTS_MAX_STATES and inner <= SCAN_SEGMENTS_MAX_CHANNELS and out.dtype == torch.bfloat16 and
+    # (float32 output: the state is float64 in between)
+    if (out.dtype == torch.bfloat16 and scan_prefers_segments(N, max_q_len, inner, states) and
             max(x.stride(0), dt.stride(0), out.stride(0), z.stride(0) if z is not None else 0) < 1 << 24):
         more = (N - 1) // SCAN_SEGMENT_TOKENS
-        padded = 8 if states <= 8 else 16 if states <= 16 else 32
-        scratch = torch.empty((more + min(more, requests)) * inner * (padded + 1), dtype=torch.float32, device=x.device)
+        scratch = torch.empty((more + min(more, requests)) * inner * (_scan_entries(states) + 1), dtype=torch.float32, device=x.device)
         _call("llmp_selective_scan_segments", _ptr(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(b), _ptr(c), b.stride(0), _ptr(a),
               _ptr(d_skip), _ptr(z), z.stride(0) if z is not None else 0, ptr, slot_stride, half, _ptr(q_start), _ptr(slots),
               _ptr(positions), _ptr(out), out.stride(0), _ptr(scratch), scratch.numel(), N, requests, inner, states, _stream())

@@ -139,3 +139,16 @@ def test_single_tokens_of_sigmoid_attention_take_ranges_of_bounded_length(monkey
             assert keys <= 512 or 2 * taken > part.SEGMENTS_MAX_BYTES - 4 * tokens * 16 * 128
     assert part._decode_ranges(8, 2000) == (-(-2000 // 128), 128)             # one round of 128 blocks
     assert part._decode_ranges(1, tile) == (1, tile)
+
+
+def test_scans_go_in_segments_where_their_channels_leave_a_walk_alone():
+    """On both sides of the line for each number of state entries: which form the measured sizes take that differ by more than a tenth."""
+    def takes(states, requests, inner, tokens):
+        return kernels.scan_prefers_segments(requests * tokens, tokens, inner, states)
+
+    for walked in ((16, 1, 512, 1408), (16, 1, 1024, 1792), (16, 1, 2048, 2816), (16, 1, 4096, 16384), (16, 2, 2048, 4096), (8, 1, 2048, 2304), (8, 1, 512, 1024),
+                   (32, 1, 512, 2816), (32, 1, 1024, 4096), (32, 1, 2048, 16384), (33, 1, 256, 16384), (16, 4, 512, 2304)):
+        assert not takes(*walked), walked
+    for cut in ((16, 1, 512, 2816), (16, 1, 1024, 4096), (16, 2, 256, 2304), (16, 2, 1024, 4096), (16, 4, 512, 4096), (8, 1, 1024, 2304), (8, 1, 2048, 4096),
+                (8, 4, 512, 3456), (32, 1, 512, 6144), (32, 1, 256, 4096), (32, 2, 512, 8192), (1, 1, 64, 2048)):
+        assert takes(*cut), cut
