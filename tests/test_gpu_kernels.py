@@ -170,14 +170,16 @@ def test_gemm_simt_gives_one_sum_whatever_the_tile(dtype, M, N, Kd):
 @pytest.mark.parametrize("M,N,Kd", [(203, 96, 2048), (33, 128, 1027), (203, 33, 257), (1, 64, 9001), (9000, 100, 600), (700, 127, 1056), (5, 129, 1000)])
 def test_gemm_simt_in_segments(dtype, M, N, Kd):
     """A narrow matrix with K in two to eight segments, in each of the three tiles, and the first width that goes in one: every row has the bits
-    it has alone, within K 2^-24 of the sum of the products' sizes of the float64 product (2^-8 more in bfloat16)."""
+    it has alone, within 6 sqrt(K) 2^-24 of the root of the sum of the products' squares (the size of a sum of random signs; roundings
+    add up like one and reach 0.3 to 2.4 sqrt(K) 2^-24 of it) of the float64 product (2^-8 of the result more in bfloat16). Products of
+    11 bits, as tensor cores make of float32, leave some 2^-12 of it."""
     gen = torch.Generator().manual_seed(M + N + Kd)
     a, w = (torch.randn(n, Kd, generator=gen).to(dtype).to(DEV) for n in (M, N))
     bias = torch.randn(N, generator=gen).to(DEV)
     out = torch.empty(M, N, dtype=dtype, device=DEV)
     K().gemm_simt(a, w, out, bias)
-    want, sizes = a.double() @ w.double().T + bias.double(), a.double().abs() @ w.double().abs().T + bias.double().abs()
-    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
+    want, size = a.double() @ w.double().T + bias.double(), (a.double() ** 2 @ (w.double() ** 2).T + bias.double() ** 2).sqrt()
+    bound = 6 * Kd ** 0.5 * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0.0)
     assert ((out.double() - want).abs() <= bound).all()
     for m in {0, M // 2, M - 1}:
         single = torch.empty(1, N, dtype=dtype, device=DEV)
@@ -258,14 +260,14 @@ def test_gemm_tcgen05(out_dtype, M, N, Kd):
 @pytest.mark.parametrize("M,N,Kd", [(300, 160, 4096), (129, 96, 1032), (2048, 256, 1024), (70, 17, 2048), (1000, 250, 1096), (65, 3, 1600)])
 def test_gemm_tcgen05_narrow_outputs(out_dtype, M, N, Kd):
     """Narrow outputs with a long K, whose shares meet in shared memory: rows and columns that fill no tile, shares of K that are not
-    alike, entries beside the output untouched. Within K 2^-24 of the sum of the products' sizes (2^-8 more in
-    bfloat16) of the float64 product."""
+    alike, entries beside the output untouched. Within 4 sqrt(K) 2^-24 of the root of the sum of the products' squares (0.5
+    to 1.2 are reached; 2^-8 of the result more in bfloat16) of the float64 product."""
     gen = torch.Generator().manual_seed(M + N + Kd)
     x, w = (torch.randn(n, Kd, generator=gen).to(torch.bfloat16).to(DEV) for n in (M, N))
     room = torch.full((M, N + 5), 7.0, dtype=out_dtype, device=DEV)
     K().gemm_tc(x, w, room[:, 2:2 + N])
-    want, sizes = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
-    bound = Kd * 2.0 ** -24 * sizes + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0)
+    want, size = x.double() @ w.double().T, (x.double() ** 2 @ (w.double() ** 2).T).sqrt()
+    bound = 4 * Kd ** 0.5 * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if out_dtype == torch.bfloat16 else 0.0)
     assert ((room[:, 2:2 + N].double() - want).abs() <= bound).all()
     assert (room[:, :2] == 7.0).all() and (room[:, 2 + N:] == 7.0).all()
     K().check_error_flag()

@@ -430,7 +430,8 @@ def test_delta_rule_products_of_odd_ranks_have_rows_on_sixteen_bytes(monkeypatch
 @pytest.mark.parametrize("sizes", [(2, 1, 64, 16), (1, 1, 128, 48)], ids=str)
 def test_delta_rule_rows_do_not_depend_on_their_company(sizes, monkeypatch):
     """Forty portions in chunks and as many short ones token by token in one step, more than a warp looks at in one go, in an order
-    that mixes them: every request's outputs and state have the bits they have alone, and other rows and slots stay."""
+    that mixes them: every request's outputs and state have the bits they have alone, and other rows and slots stay. (Walks of single
+    tokens here; the layer's own kernel for them is below.)"""
     from llm_pipeline_b200.ops import kernels
     monkeypatch.setattr(kernels, "DELTA_CHUNKS_MIN_TOKENS", 17)
     heads, qk_heads, dim, vdim = sizes
@@ -900,15 +901,16 @@ def test_sigmoid_attention_keeps_mixed_weights_whole_where_prompts_do(sizes):
 def test_few_rows_over_long_contexts_take_key_segments(tmp_path, dtype):
     """Contexts of several key segments under sparse weights: decoding steps and short portions share a token's keys among
     blocks whose sums a second kernel adds; positions around the segment borders, and long portions that take one block.
-    In float32 the general kernel runs, in bfloat16 the tensor-core kernel with its shorter key ranges."""
+    In float32 the general kernel runs; in bfloat16 portions take the tensor-core kernel with its shorter key ranges, and steps of
+    single tokens the kernel of their own, in ranges that cover the longest request."""
     from llm_pipeline_b200.ops import kernels
     cfg, W, folder = case(tmp_path, "attention_first", 8, sharp=5.0, head_bias=-9.0)
     seg = kernels.SIGMOID_SEGMENT_KEYS
     requests = requests_for(cfg, [seg + 40, 2 * seg + 2, 70], 700)
     want = N.oracle(cfg, W, requests)
     runner = H.make_runner(folder, dtype, page_size=16, num_pages=3 * (seg // 16) + 16, max_request_tokens=2 * seg + 16, max_requests=3)
-    used = {"general": [], "tensor cores": []}
-    general, tensor = kernels.sigmoid_attention, kernels.sigmoid_attention_mma
+    used = {"general": [], "tensor cores": [], "single tokens": []}
+    general, tensor, single = kernels.sigmoid_attention, kernels.sigmoid_attention_mma, kernels.sigmoid_decode
 
     def counting_general(*args, **kwargs):
         used["general"].append(args[-1] if len(args) > 14 else kwargs.get("segments", 1))
@@ -918,19 +920,26 @@ def test_few_rows_over_long_contexts_take_key_segments(tmp_path, dtype):
         used["tensor cores"].append((args[-1] if len(args) > 17 else kwargs.get("segments", 1), kwargs.get("segment_keys", 0)))
         return tensor(*args, **kwargs)
 
-    kernels.sigmoid_attention, kernels.sigmoid_attention_mma = counting_general, counting_tensor
+    def counting_single(*args):
+        used["single tokens"].append((args[-2], args[-1]))
+        return single(*args)
+
+    kernels.sigmoid_attention, kernels.sigmoid_attention_mma, kernels.sigmoid_decode = counting_general, counting_tensor, counting_single
     try:
         N.assert_matches(H.replay(runner, H.cut_tail_one_by_one(requests, tail=50)), want, dtype, "segments: decoding")
         N.assert_matches(H.replay(runner, H.cut_portions(requests, (seg - 3, 2, 5, seg + 7, 3))), want, dtype, "segments: portions")
         N.assert_matches(H.replay(runner, H.cut_mixed(requests, (seg, 2, 9), max_live=3, decode_tail=12)), want, dtype, "segments: mixed")
     finally:
-        kernels.sigmoid_attention, kernels.sigmoid_attention_mma = general, tensor
+        kernels.sigmoid_attention, kernels.sigmoid_attention_mma, kernels.sigmoid_decode = general, tensor, single
     if dtype == torch.float32:
-        assert not used["tensor cores"] and any(n > 1 for n in used["general"]) and any(n == 1 for n in used["general"]), \
+        assert not used["tensor cores"] and not used["single tokens"] and any(n > 1 for n in used["general"]) and any(n == 1 for n in used["general"]), \
             "both forms of the general kernel should have run"
     else:
         assert not used["general"] and any(n > 1 for n, _ in used["tensor cores"]), "the tensor-core kernel should have run with key ranges"
         assert all(keys in (kernels.SIGMOID_MMA_SEGMENT_KEYS, kernels.SIGMOID_MMA_LONG_SEGMENT_KEYS) for _, keys in used["tensor cores"])
+        # decoded alone, up to 2 seg + 2 keys; replayed steps have the ranges they were captured with
+        assert max(n * keys for n, keys in used["single tokens"]) >= 2 * seg + 2
+        assert any(n > 1 for n, _ in used["single tokens"]) and all(keys <= kernels.SIGMOID_DECODE_RANGE_KEYS for _, keys in used["single tokens"])
 
 
 def test_recurrent_states_carry_what_was_written_hundreds_of_tokens_back(tmp_path):
