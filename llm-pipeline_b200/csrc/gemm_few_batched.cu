@@ -5,11 +5,14 @@
 // (the m side of the MMA; the rows of A are its n side) and up to 128 of K at a time, in 16-byte words straight into registers. An
 // MMA's 16 places along K may be any 16 of K as long as both operands agree: lane t of a quad holds entries 8 t .. 8 t + 7 of a run of 32,
 // whose first four are its places of one MMA and the others of a second. Weights that the caller holds are asked for before the kernel
-// waits for the one before it, which may be what writes others. Up to 256 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are
-// added in the order of the quarters. The split follows from K alone and a row's sums from its own entries, so its bits do not depend on
-// the other rows. A decoding layer of 16 heads (8 requests of 2,048 keys), whose maps
-// are 128 x 512 and 512 x 128: 53.3 us with a warp per output column and sums by shuffles (gemm_simt.cu, which keeps float32 and operands
-// without 16-byte rows; 10.9 and 6.0 us of the layer), 36.9 so and with the merge of latent_decode.cu.
+// waits for the one before it, which may be what writes others. A chain of MMAs on one accumulator loses a bit or two (the tensor core
+// cuts off what a float32 sum would round): each MMA starts from zero and the eight of 128 entries are added as a tree. Results that are
+// not the nearest bfloat16, 8 rows of 512 by 128: 4.5e-5 (entries of mean 1: 3.1e-6); a chain 6.3e-5 (2.1e-5), sums by shuffles 4.2e-5
+// (3.8e-6). Up to 256 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are added in
+// the order of the quarters. The split follows from K alone and a row's sums from its own entries, so its bits do not depend on the
+// other rows. Microseconds back to back, 16 maps of 8 rows: 128 x 512 9.5 with a warp per output column and sums by shuffles
+// (gemm_simt.cu, which keeps float32 and operands without 16-byte rows) and 1.7, 512 x 128 5.9 and 1.9; 16 rows 13.8 and 2.4, 7.4 and 2.0. A
+// decoding layer with these (8 requests of 2,048 keys): 53 and, with the merge of latent_decode.cu, 35.
 #include "common.cuh"
 
 namespace {
@@ -63,12 +66,22 @@ __global__ void __launch_bounds__(32 * GF_WARPS) gemm_few_batched_kernel(const F
                 x[i][m] = run0 + i < last && k < a.K && row < a.M ? *reinterpret_cast<const uint4*>(A + (size_t)row * a.lda + k) : none;
             }
 #pragma unroll
-        for (int i = 0; i < GF_RUNS; ++i)
+        for (int m = 0; m < MT; ++m) {
+            float part[2 * GF_RUNS][4] = {};
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                gf_mma(acc[m], w[i][0].x, w[i][1].x, w[i][0].y, w[i][1].y, x[i][m].x, x[i][m].y);
-                gf_mma(acc[m], w[i][0].z, w[i][1].z, w[i][0].w, w[i][1].w, x[i][m].z, x[i][m].w);
+            for (int i = 0; i < GF_RUNS; ++i) {
+                gf_mma(part[2 * i], w[i][0].x, w[i][1].x, w[i][0].y, w[i][1].y, x[i][m].x, x[i][m].y);
+                gf_mma(part[2 * i + 1], w[i][0].z, w[i][1].z, w[i][0].w, w[i][1].w, x[i][m].z, x[i][m].w);
             }
+#pragma unroll
+            for (int step = 1; step < 2 * GF_RUNS; step *= 2)
+#pragma unroll
+                for (int i = 0; i < 2 * GF_RUNS; i += 2 * step)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) part[i][c] += part[i + step][c];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[m][c] += part[0][c];
+        }
         if (run0 + GF_RUNS < last) load_w(run0 + GF_RUNS);
     }
     if (QUARTERS) {

@@ -208,6 +208,23 @@ def test_few_rows_of_several_heads(batch, rows, n, k):
         assert torch.equal(alone[0], out[m, :, :n])
 
 
+@pytest.mark.parametrize("rows,n,k", [(16, 512, 128), (8, 64, 256), (8, 64, 1048), (1, 128, 512)], ids=str)
+def test_few_rows_of_several_heads_hold_float32_sums(rows, n, k):
+    """Entries of one sign, where every rounding of a sum shows: the result is the nearest bfloat16 but for sums within 4 x 2^-24 of their
+    terms' sizes of the middle between two (float32 sums by a tree over 32 lanes reach 2.2, a chain of MMAs on one accumulator 5 to 7)."""
+    from llm_pipeline_b200.ops import kernels
+    for seed in range(60):
+        gen = torch.Generator(device=DEV).manual_seed(seed)
+        x = (torch.randn(16, rows, k, generator=gen, device=DEV) + 1).to(torch.bfloat16)
+        w = ((torch.randn(16, n, k, generator=gen, device=DEV) + 1) * k ** -0.5).to(torch.bfloat16)
+        out = torch.empty(16, rows, n, dtype=torch.bfloat16, device=DEV)
+        kernels.gemm_batched(x, w, out)
+        want = x.double() @ w.double().transpose(1, 2)
+        least = (want.to(torch.bfloat16).double() - want).abs()
+        sizes = x.double().abs() @ w.double().abs().transpose(1, 2)
+        assert ((out.double() - want).abs() <= least + 4 * 2.0 ** -24 * sizes).all(), seed
+
+
 @pytest.mark.parametrize("k", [128, 512])
 def test_few_rows_of_several_heads_by_weights_just_made(k):
     """Weights that the kernel launched before writes, other ones every time: the product is of those, as after a pause. A layer's own
