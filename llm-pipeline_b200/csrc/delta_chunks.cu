@@ -18,7 +18,7 @@
 // its 24 bits, and of the nine products of pieces the six larger are summed in float32, the largest apart: outputs and state are
 // as far from 64 bits as token by token (1.2e-7 to 3e-7 at decays from fast to slow, and after resets; with two pieces and three
 // products 5e-6, at 47 us less). The operands of launch 2 lie in scratch in the order of its fragments, pieces beside each other,
-// and are copied as they are. A layer of 2,048 tokens and 16 heads of 128 x 128 takes 381 us, 809 token by token. Launch 1 (96 us
+// and are copied as they are. A layer of 2,048 tokens and 16 heads of 128 x 128 takes 358 us, 809 token by token. Launch 1 (96 us
 // with cold caches) is issue-bound at 44 % with 14 warps an SM; launch 2 (148) is the chain's latency, 1.16 us a chunk (tensor pipe
 // 32 %, a warp a scheduler). On the way: 32 columns a block with fragments loaded from global memory,
 // two barriers a chunk (each slower by 15 to 45 %).

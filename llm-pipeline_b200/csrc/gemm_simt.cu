@@ -166,9 +166,10 @@ gemm_nt_kernel(const TI* __restrict__ A, const TI* __restrict__ W, const void* _
 }
 
 // Few weight rows with a long K leave SMs idle up to thousands of rows, so K is cut into up to as many segments as a cluster may have
-// blocks. 96 x 2,048, microseconds with a whole K in a block and in segments: 1 row 35 and 8, 203 rows 35 and 12. Not for wider
-// matrices: there many rows fill the chip, where segments are slower (4,096 x 4,096 by 2,048 rows 1,710 us, side by side 2,062, walked by one
-// block 2,324; 96 x 2,048 by 2,048 rows 53 and 42, by 40,000 646 and 695), and whether K is cut may not depend on the rows.
+// blocks. 96 x 2,048, microseconds with a whole K in a block and in segments: 1 row 39 and 8, 203 rows 39 and 14, 2,048 rows 54 and 39, 8,192 156
+// and 149, 40,000 646 and 695. Whether K is cut may not depend on the rows, and of wider matrices fewer rows fill the chip, where
+// segments are slower: 2,048 and 8,192 rows, K 2,048, 128 columns 54 and 40, 156 and 151; 160 columns 74 and 76, 198 and 223; 256 columns
+// 84 and 78, 219 and 297; 1,024 columns 219 and 297, 862 and 1,136.
 constexpr int GT_SEGMENT = 256, GT_MAX_SEGMENTS = 8, GT_NARROW = 128;
 int gt_segment(int N, int K, bool float32) {
     const int most = (K + GT_SEGMENT - 1) / GT_SEGMENT, count = most < GT_MAX_SEGMENTS ? most : GT_MAX_SEGMENTS;

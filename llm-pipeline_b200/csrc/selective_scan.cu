@@ -20,10 +20,11 @@
 //         twice), so the special-function unit would be done with 2,048 tokens of 4,096 channels in 37 us; what keeps a walk from that
 //         is that a scheduler has one or two warps of it, which wait for every instruction's result. So whatever the chain does not
 //         need is other warps' work (copies into a ring, step sizes and gates of the stages to come, the sums over a channel's lanes and
-//         the outputs of the stage behind; they meet the walkers at one barrier a stage), and a walker's turn of SS_RUN tokens mixes
+//         the outputs of the stage behind; they meet the walkers at one barrier a stage), and a walker's turn of up to four tokens mixes
 //         three: the chain over one run, the decays of the next, the loads of the one after. Microseconds, before and after: 2,048
 //         tokens of 4,096 channels 117 (segments) and 94, of 2,048 channels 84 and 54; 100 tokens 33 and 9; 203 in float64 68 and 31;
-//         64 single tokens beside 300 102 and 57. On the way: all of it in one warp 209 and 149, sums by shuffles among the walkers 155
+//         64 single tokens beside 300 102 and 57; with 64, 128 and 256 entries, 1,024 tokens of 2,048 channels 728, 1,772 and 5,478 and
+//         189, 310 and 623. On the way: all of it in one warp 209 and 149, sums by shuffles among the walkers 155
 //         and 106, stages of 16 tokens 109 and 84, two warps for step sizes and gates 104 and 74.
 //   segments: few channels and many tokens in bfloat16 (below).
 #include <type_traits>
@@ -50,6 +51,7 @@ struct ScanArgs {
     const int* q_start; const int* slots; const int* positions;
     void* out; long out_t;
     int inner, states, requests;
+    int held;                             // 1: no kernel in flight writes A, D or dt_bias
     int singles;                          // 1: the walk leaves requests of one token to the step kernel
 };
 
@@ -226,11 +228,16 @@ __global__ void __launch_bounds__(SS_WALKERS<G>) selective_step_kernel(const Sca
     const int c = blockIdx.x / a.requests * CH + threadIdx.x / G;
     const bool ok = c < a.inner;
     const int cc = ok ? c : 0, have = ok ? a.states - l * E : 0;
-    pdl_wait();                                                 // what the kernels before wrote is complete, A, D and the bias among it
+    float rate[E], bias, Dc;
+    auto load_layer = [&]() {
+        ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);
+        bias = a.dt_bias[cc];
+        Dc = a.D[cc];
+    };
+    if (a.held) load_layer();                                   // (a decoding layer 34.6 us without, 32.9 so)
+    pdl_wait();                                                 // what the kernels before wrote is complete
     pdl_trigger();
-    float rate[E];
-    ss_load<E>(rate, a.A + (size_t)cc * a.states + l * E, have);
-    const float bias = a.dt_bias[cc], Dc = a.D[cc];
+    if (!a.held) load_layer();
     const int t = a.q_start[r];
     if (a.q_start[r + 1] - t != 1) return;
     const int p0 = a.positions[t];
@@ -787,11 +794,12 @@ LLMP_API int llmp_selective_scan_segments(const float* x, long x_t, const float*
 }
 
 // max_q_len: the most tokens a request brings, or more. singles: 1 where a request of this step may bring a single token beside longer ones
-// (0 costs such a request the walk, with the same bits, and saves the others a launch).
+// (0 costs such a request the walk, with the same bits, and saves the others a launch). held: 1 where A, D and dt_bias are
+// the caller's for good, so that they may be read while the kernel before is still at work.
 LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long dt_t, const float* dt_bias, const float* B,
                                  const float* C, long bc_t, const float* A, const float* D, const float* z, long z_t, float* state,
                                  long state_slot, long state_half, const int* q_start, const int* slots, const int* positions,
-                                 void* out, int out_dtype, long out_t, int R, int inner, int states, int max_q_len, int singles, cudaStream_t stream) {
+                                 void* out, int out_dtype, long out_t, int R, int inner, int states, int max_q_len, int singles, int held, cudaStream_t stream) {
     if (R <= 0) return 0;
     LLMP_REQUIRE(inner > 0 && states > 0 && states <= 256, "selective_scan: %d channels with %d state entries (up to 256 are served)",
                  inner, states);
@@ -800,7 +808,7 @@ LLMP_API int llmp_selective_scan(const float* x, long x_t, const float* dt, long
     a.x = x; a.x_t = x_t; a.dt = dt; a.dt_t = dt_t; a.dt_bias = dt_bias; a.B = B; a.C = C; a.bc_t = bc_t; a.A = A; a.D = D;
     a.z = z; a.z_t = z ? z_t : 0; a.state = state; a.state_slot = state_slot; a.state_half = state_half; a.q_start = q_start;
     a.slots = slots; a.positions = positions; a.out = out; a.out_t = out_t; a.inner = inner; a.states = states;
-    a.requests = R; a.singles = singles && R > 1;
+    a.requests = R; a.singles = singles && R > 1; a.held = held;
     if (states <= 8) return launch_scan<4, 2>(a, out_dtype, max_q_len, stream);
     if (states <= 16) return launch_scan<8, 2>(a, out_dtype, max_q_len, stream);
     if (states <= 32) return launch_scan<16, 2>(a, out_dtype, max_q_len, stream);

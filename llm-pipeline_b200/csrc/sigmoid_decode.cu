@@ -9,7 +9,7 @@
 // All keys and values of the first tile are asked for at once; in a longer range the keys of the next tile are copied from the mix on,
 // its values after the products. Nothing is normalised, so ranges are sums that a second kernel adds in a fixed order, a block per 128
 // columns of a row. 8 requests of 2,000 keys, 16 heads over 4 of 128 + 128: attention and sums 28 us there, 15 here (ranges of 128
-// keys, so that the blocks, of which each fills an SM, are one round; ranges of 64 keys 16.4, of 192 18.8).
+// keys, so that the blocks, of which each fills an SM, are one round; ranges of 64 keys 17, of 192 19.5). The layer chooses the ranges.
 #include "common.cuh"
 
 namespace {

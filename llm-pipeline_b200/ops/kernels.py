@@ -78,7 +78,7 @@ _SIGNATURES = {
     "llmp_capped_attention_mma": [_P, _L, _P, _L, _P, _P, _I, _P, _P, _P, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F,
                                   _I, _I, _I, _P, _P, _I, _P],
     "llmp_selective_scan_segments": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _L, _P, _L, _I, _I, _I, _I, _P],
-    "llmp_selective_scan": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _I, _L, _I, _I, _I, _I, _I, _P],
+    "llmp_selective_scan": [_P, _L, _P, _L, _P, _P, _P, _L, _P, _P, _P, _L, _P, _L, _L, _P, _P, _P, _P, _I, _L, _I, _I, _I, _I, _I, _I, _P],
     "llmp_add_rmsnorm_multi": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _I, _F, _P, _I, _L, _L, _P, _I, _I, _P],
     "llmp_gated_act": [_P, _I, _L, _P, _I, _L, _I, _I, _P],
     "llmp_sigmoid_gate": [_P, _P, _L, _P, _I, _L, _I, _P],
@@ -2112,12 +2112,14 @@ def scan_prefers_segments(tokens: int, longest: int, inner: int, states: int) ->
 def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: torch.Tensor, c: torch.Tensor, a: torch.Tensor,
                    d_skip: torch.Tensor, z: Optional[torch.Tensor], state: torch.Tensor, state_offset: int, q_start: torch.Tensor,
                    slots: torch.Tensor, positions: torch.Tensor, out: torch.Tensor, max_q_len: Optional[int] = None,
-                   singles: bool = True) -> torch.Tensor:
+                   singles: bool = True, held: bool = False) -> torch.Tensor:
     """The selective state-space recurrence with a decay per channel and state entry (csrc/selective_scan.cu): float32 rows
     ``x``, ``dt`` [tokens, inner] (dt before bias and softplus), ``b``, ``c`` [tokens, states] (views of one matrix), ``a`` [inner,
     states] (negative), ``d_skip``, ``dt_bias`` [inner], ``z`` [tokens, inner] or None; ``out`` [tokens, inner] = y * silu(z) in the
     compute type. The state piece holds two copies of [inner, states]. ``max_q_len``: the most tokens a request brings, where
-    the caller knows it. ``singles`` False: no request of several brings a single token, which spares the launch for those."""
+    the caller knows it. ``singles`` False: no request of several brings a single token, which spares the launch for those.
+    ``held``: ``a``, ``d_skip`` and ``dt_bias`` were there before this step's kernels were launched; they may then be read while the kernel
+    before is still at work."""
     N, inner = x.shape
     states = a.shape[1]
     for t, name in ((x, "x"), (dt, "dt"), (b, "B"), (c, "C")) + (((z, "z"),) if z is not None else ()):
@@ -2145,7 +2147,7 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, b: 
         return out
     _call("llmp_selective_scan", _ptr(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(b), _ptr(c), b.stride(0), _ptr(a),
           _ptr(d_skip), _ptr(z), z.stride(0) if z is not None else 0, ptr, slot_stride, half, _ptr(q_start), _ptr(slots),
-          _ptr(positions), _ptr(out), dtype_code(out.dtype), out.stride(0), requests, inner, states, int(max_q_len), int(singles), _stream())
+          _ptr(positions), _ptr(out), dtype_code(out.dtype), out.stride(0), requests, inner, states, int(max_q_len), int(singles), int(held), _stream())
     return out
 
 

@@ -112,7 +112,9 @@ class CappedAttention(Mixer):
     def _segments(self, ctx) -> int:
         """Into how many segments of ``CAPPED_SEGMENT_KEYS`` a step of single tokens cuts its keys (0: not at all). Their size is one for all
         steps, so that a row's sums do not depend on how many other requests there are or how long they are, and a long request beside
-        short ones is not walked by a few blocks."""
+        short ones is not walked by a few blocks. Microseconds in segments of 256 keys and in as many as fill the places of the blocks
+        once, 4 key/value heads over 1,088 keys: 16 requests 17.0 and 18.6 (of 320 keys), 40 38.7 and 44.0, 74 65 and 48 (whole), 140 118
+        and 90; 8 heads, 16 requests of 4,096 keys 92 and 72, of 512 keys but one of 32,768 98 and 454."""
         if ctx.max_q_len != 1:
             return 0
         longest = ctx.decode_ctx_bound or ctx.max_ctx_len

@@ -100,5 +100,5 @@ class SelectiveScan(Mixer):
         dt = linear(d_typed, self.w_dt, out_dtype=torch.float32)                 # [N, inner], before bias and softplus
         gated = torch.empty((N, I), dtype=x.dtype, device=x.device)
         kernels.selective_scan(xc, dt, self.dt_bias, dbc[:, R:R + S], dbc[:, R + S:], self.a, self.d_skip, xz[:, I:], cache.state,
-                               self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, gated, ctx.max_q_len, 1 in ctx.q_lens)
+                               self.conv_entries, ctx.q_start, ctx.slots, ctx.positions, gated, ctx.max_q_len, 1 in ctx.q_lens, True)
         return linear(gated, self.w_out, out_dtype=torch.float32), None

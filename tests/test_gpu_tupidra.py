@@ -190,7 +190,8 @@ def test_selective_scan_of_as_many_channels_and_strides_as_there_are(tokens, inn
 
 
 def test_selective_scan_of_single_tokens_by_rates_just_made():
-    """Rates that the kernel launched before writes, other ones every time: the step is by those, as after a pause."""
+    """Rates that the kernel launched before writes, other ones every time: the step is by those, as after a pause. A layer's own, which may
+    be read sooner, give the same bits."""
     from llm_pipeline_b200.ops import kernels
     gen, R, inner, states = torch.Generator().manual_seed(1), 8, 2048, 16
     x, raw, z = (torch.randn(R, inner, generator=gen).to(DEV) for _ in range(3))
@@ -199,19 +200,21 @@ def test_selective_scan_of_single_tokens_by_rates_just_made():
     start, A = torch.randn(R, 2 * inner * states, generator=gen).to(DEV), torch.zeros(inner, states, device=DEV)
     where = _i32(list(range(R + 1))), _i32(list(range(R))), _i32([5] * R)
 
-    def step(rates):
+    def step(rates, held=False):
         out, state = torch.empty(R, inner, device=DEV), start.clone()
         if rates is not A:
             kernels.convert_rows(rates, A)
-        kernels.selective_scan(x, raw, bias, bc[:, :states], bc[:, states:], A, skip, z, state, 0, *where, out, 1)
+        kernels.selective_scan(x, raw, bias, bc[:, :states], bc[:, states:], A, skip, z, state, 0, *where, out, 1, held=held)
         return out, state
 
     at_once = [step(rates) for rates in made]
     for rates, (out, state) in zip(made, at_once):
         A.copy_(rates)
         torch.cuda.synchronize()
-        paused, left = step(A)
-        assert torch.equal(out, paused) and torch.equal(state, left)
+        for held in (False, True):
+            paused, left = step(A, held)
+            torch.cuda.synchronize()
+            assert torch.equal(out, paused) and torch.equal(state, left)
 
 
 @pytest.mark.parametrize("lengths", [(1, 64, 65), (128, 2, 1, 129, 31), (200,)], ids=str)
@@ -514,7 +517,7 @@ def test_scans_launch_the_single_tokens_kernel_where_a_request_brings_one(tmp_pa
             some = bool((q_start[1:] - q_start[:-1] == 1).any())
             said.append((some, singles))
             before = state.clone()
-            scan(*args[:15], not singles)
+            scan(*args[:15], not singles, *args[16:])
             other = out.clone(), state.clone()
             state.copy_(before)
             scan(*args)
