@@ -93,7 +93,9 @@ class SigmoidAttention(Mixer):
         """(number of key ranges, keys of a range) of a step of single tokens: of ranges of up to ``SIGMOID_DECODE_RANGE_KEYS`` those that cost
         least, rounds of blocks (each fills an SM) times a range's tiles and half a tile for a block's start. Longer ones would spare short
         requests a little, but a long one beside them would be walked by a few blocks: 16 requests of 512 keys with one of 32,768 52 us,
-        in ranges as long as give one round of blocks 287; 16 of 4,096 49 and 48 us, 200 of 2,000 248 and 329."""
+        in ranges as long as give one round of blocks 287; 16 of 4,096 47 us both, 24 of 4,096 70 and 63, 200 of 2,000 248 and 329. And a range
+        is a chain of MMAs on one accumulator, which cuts off what a float32 sum rounds: of 8,000 keys of one sign in one range 0.73 % of the
+        results are not the nearest bfloat16, in ranges of up to 512 0.39 % as in ranges of 128."""
         tile = self._decode_keys()
         tiles = -(-longest // tile)
         fits = max(1, self.SEGMENTS_MAX_BYTES // (4 * tokens * self.num_heads * self.vdim))      # ranges whose sums take no more than that
