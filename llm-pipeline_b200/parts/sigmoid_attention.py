@@ -91,8 +91,8 @@ class SigmoidAttention(Mixer):
 
     def _decode_ranges(self, tokens: int, longest: int):
         """(number of key ranges, keys of a range) of a step of single tokens: of ranges of up to ``SIGMOID_DECODE_RANGE_KEYS`` those that cost
-        least, rounds of blocks (each fills an SM) times a range's tiles and half a tile for a block's start. Longer ones would spare short
-        requests a little, but a long one beside them would be walked by a few blocks: 16 requests of 512 keys with one of 32,768 52 us,
+        least, rounds of blocks (each fills an SM) times a range's tiles and half a tile for a block's start. Longer ones are a little faster
+        for some numbers of even requests, but a long one beside short ones would be walked by a few blocks: 16 requests of 512 keys with one of 32,768 52 us,
         in ranges as long as give one round of blocks 287; 16 of 4,096 47 us both, 24 of 4,096 70 and 63, 200 of 2,000 248 and 329. And a range
         is a chain of MMAs on one accumulator, which cuts off what a float32 sum rounds: of 8,000 keys of one sign in one range 0.73 % of the
         results are not the nearest bfloat16, in ranges of up to 512 0.39 % as in ranges of 128."""
