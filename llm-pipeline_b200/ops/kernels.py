@@ -2022,7 +2022,7 @@ def capped_attention(q: torch.Tensor, pages: torch.Tensor, tables: torch.Tensor,
 
 
 CAPPED_TILE_KEYS = 64                # csrc/capped_attention_mma.cu: keys of a tile
-CAPPED_SEGMENT_KEYS = 256            # keys of a segment (a multiple of the tile)
+CAPPED_SEGMENT_KEYS = 256            # the most keys of a segment (a multiple of the tile)
 
 
 def capped_mma_supports(dtype: torch.dtype, dim: int, vdim: int) -> bool:
@@ -2046,11 +2046,11 @@ def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Ten
                          tile_req: Optional[torch.Tensor], tile_tok0: Optional[torch.Tensor], out: torch.Tensor, num_heads: int, num_kv_heads: int, dim: int,
                          vdim: int, window: int, keep_first: int, scale: float, softcap: float, slopes: Optional[torch.Tensor] = None,
                          sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, split: bool = False, chunk: int = 0,
-                         segments: int = 0) -> torch.Tensor:
+                         segments: int = 0, segment_keys: int = 0) -> torch.Tensor:
     """``capped_attention`` on the tensor cores for bfloat16 (csrc/capped_attention_mma.cu). ``tile_req``/``tile_tok0``: the work
     list (request and first token of every tile of ``capped_mma_tokens_per_tile`` tokens; None with ``split``: tile i is request i's). ``split``: every tile is one token,
     and the four warps of a block share its keys; ``segments`` > 0 then cuts the keys of a row into that many runs of
-    ``CAPPED_SEGMENT_KEYS`` with blocks of their own, whose sums the block that ends last adds up (it must cover the most keys a
+    ``segment_keys`` (``CAPPED_SEGMENT_KEYS`` when 0) with blocks of their own, whose sums the block that ends last adds up (it must cover the most keys a
     token sees, rounded up to whole tiles at both ends)."""
     N = q.shape[0]
     _need(q.dtype == torch.bfloat16 and pages.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "capped_attention_mma takes bfloat16")
@@ -2077,7 +2077,7 @@ def capped_attention_mma(q: torch.Tensor, pages: torch.Tensor, tables: torch.Ten
           _ptr(q_start), _ptr(ctx_len), _ptr(tile_req), _ptr(tile_tok0), tiles, _ptr(slopes), _ptr(sink), _ptr(gate),
           gate.stride(0) if gate is not None else 0, 1 if gate_heads else 0, num_heads, num_kv_heads, dim, vdim, pages.shape[2],
           int(window), int(keep_first), int(chunk), float(scale), float(softcap), 1 if split else 0, int(segments),
-          CAPPED_SEGMENT_KEYS if segments > 0 else 0, _ptr(scratch), _ptr(counters), N, _stream())
+          (int(segment_keys) or CAPPED_SEGMENT_KEYS) if segments > 0 else 0, _ptr(scratch), _ptr(counters), N, _stream())
     return out
 
 

@@ -109,22 +109,25 @@ class CappedAttention(Mixer):
             return ("q",)
         return ("q", "k") if self.values_are_keys else ("q", "k", "v")
 
-    def _segments(self, ctx) -> int:
-        """Into how many segments of ``CAPPED_SEGMENT_KEYS`` a step of single tokens cuts its keys (0: not at all). Their size is one for all
-        steps, so that a row's sums do not depend on how many other requests there are or how long they are, and a long request beside
-        short ones is not walked by a few blocks. Microseconds in segments of 256 keys and in as many as fill the places of the blocks
-        once, 4 key/value heads over 1,088 keys: 16 requests 17.0 and 18.6 (of 320 keys), 40 38.7 and 44.0, 74 65 and 48 (whole), 140 118
+    def _segments(self, ctx):
+        """(segments, keys of a segment) into which a step of single tokens cuts its keys (0, 0: not at all): the shortest from two
+        tiles on that have their places all at once (an SM holds two blocks), up to ``CAPPED_SEGMENT_KEYS``. Never longer: a long request beside short ones would be
+        walked by a few blocks. Microseconds in segments of 128 keys, of 256 and in as many as fill the places once, 4 key/value heads over
+        1,088 keys: 1 request 12.9 and 14.9, 8 13.9 and 16.4; 16 requests 17.0 (of 256) and 18.6 (of 320), 40 38.7 and 44.0, 74 65 and 48 (whole), 140 118
         and 90; 8 heads, 16 requests of 4,096 keys 92 and 72, of 512 keys but one of 32,768 98 and 454."""
         if ctx.max_q_len != 1:
-            return 0
+            return 0, 0
         longest = ctx.decode_ctx_bound or ctx.max_ctx_len
         tile = kernels.CAPPED_TILE_KEYS
         bounds = [n for n in (self.window, self.chunk) if n]
         reach = min([longest] + [n + tile for n in bounds])            # from the tile a row's keys begin in
         blocks = ctx.num_requests * self.num_kv_heads * -(-(self.num_heads // self.num_kv_heads) // 16)
         if reach < self.SEGMENTS_MIN_KEYS or blocks >= self.SEGMENTS_BELOW_BLOCKS_PER_SM * kernels.sm_count():
-            return 0
-        return -(-reach // kernels.CAPPED_SEGMENT_KEYS)
+            return 0, 0
+        keys = 2 * tile
+        while keys < kernels.CAPPED_SEGMENT_KEYS and blocks * -(-reach // keys) > 2 * kernels.sm_count():
+            keys += tile
+        return -(-reach // keys), keys
 
     def _name(self, key: str) -> str:
         return f"{self.prefix}.{self.names[key]}"
@@ -211,9 +214,10 @@ class CappedAttention(Mixer):
             # bfloat16 and sizes the tensor-core kernel has instances of: prompts in tiles of 64 rows (token, head of a group),
             # single tokens with the four warps of a block sharing the keys
             tile_req, tile_tok0 = self._tiles(ctx, kernels.capped_mma_tokens_per_tile(self.num_heads, self.num_kv_heads))
+            segments, segment_keys = self._segments(ctx)
             kernels.capped_attention_mma(q, cache.pages, tables, ctx.q_start, ctx.ctx_len, tile_req, tile_tok0, out, *sizes, slopes=self.slopes,
                                          sink=self.sinks, gate=gate, split=ctx.max_q_len == 1, chunk=self.chunk or 0,
-                                         segments=self._segments(ctx))
+                                         segments=segments, segment_keys=segment_keys)
         else:
             kernels.capped_attention(q, cache.pages, tables, ctx.token_request, ctx.positions, out, *sizes, slopes=self.slopes, sink=self.sinks,
                                      gate=gate, chunk=self.chunk or 0)

@@ -109,18 +109,19 @@ def single_tokens(requests, longest, bound=0):
 
 
 @pytest.mark.parametrize("reach", [{}, {"window": 1024, "keep_first": 8}, {"chunk": 2048}], ids=str)
-def test_a_token_of_capped_attention_cuts_its_keys_alike_in_any_company(monkeypatch, reach):
-    """Segments of one size that cover what a token sees, whatever the number of requests and however long the longest is, so that a
-    long request beside short ones is spread over as many blocks as alone; none once the blocks are four an SM."""
+def test_a_token_of_capped_attention_cuts_its_keys_into_segments_of_bounded_length(monkeypatch, reach):
+    """Segments that cover what a token sees, of 256 keys however long the longest request is, so that a long one beside short ones is
+    spread over the SMs; of 128 or 192 where two blocks an SM hold them all at once; none once the blocks are four an SM."""
     monkeypatch.setattr(kernels, "sm_count", lambda: SMS)
     part = CappedAttention("p", 64, 16, 4, 16, 16, 0.25, **reach)
     for requests in (1, 8, 16, 37, 38, 59, 74, 147, 148, 300):
         for longest in (100, 511, 512, 700, 4096, 32768):
             sees = min([longest] + [n + kernels.CAPPED_TILE_KEYS for n in reach.values() if n > 8])
-            want = -(-sees // kernels.CAPPED_SEGMENT_KEYS) if sees >= 512 and requests * 4 < 4 * SMS else 0
+            keys = next((k for k in (128, 192) if requests * 4 * -(-sees // k) <= 2 * SMS), 256)
+            want = (-(-sees // keys), keys) if sees >= 512 and requests * 4 < 4 * SMS else (0, 0)
             assert part._segments(single_tokens(requests, longest)) == want
             assert part._segments(single_tokens(requests, 1, bound=longest)) == want
-    assert part._segments(SimpleNamespace(max_q_len=2)) == 0
+    assert part._segments(SimpleNamespace(max_q_len=2)) == (0, 0)
 
 
 @pytest.mark.parametrize("tile", [64, 32])
