@@ -8,8 +8,8 @@
 // waits for the one before it, which may be what writes others. A chain of MMAs on one accumulator loses a bit or two (the tensor core
 // cuts off what a float32 sum would round): each MMA starts from zero and the eight of 128 entries are added as a tree. Results that are
 // not the nearest bfloat16, 8 rows of 512 by 128: 4.5e-5 (entries of mean 1: 3.1e-6); a chain 6.3e-5 (2.1e-5), sums by shuffles 4.2e-5
-// (3.8e-6). Up to 256 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are added in
-// the order of the quarters. The split follows from K alone and a row's sums from its own entries, so its bits do not depend on the
+// (3.8e-6). Up to 128 of K a warp walks alone; of a longer K each of the block's four warps takes a quarter, and their sums are added in
+// the order of the quarters (16 rows of 64 by 256 3.6 us by warps alone, 1.7 so). The split follows from K alone and a row's sums from its own entries, so its bits do not depend on the
 // other rows. Microseconds back to back, 16 maps of 8 rows: 128 x 512 9.5 with a warp per output column and sums by shuffles
 // (gemm_simt.cu, which keeps float32 and operands without 16-byte rows) and 1.7, 512 x 128 5.9 and 1.9; 16 rows 13.8 and 2.4, 7.4 and 2.0. A
 // decoding layer with these (8 requests of 2,048 keys): 53 and, with the merge of latent_decode.cu, 35.
@@ -121,7 +121,7 @@ LLMP_API int llmp_gemm_few_batched(const void* A, const void* W, void* C, int ba
     LLMP_REQUIRE(llmp_gemm_few_batched_supports(A, W, M, K, lda, ldw, batch_a, batch_w) && batch <= 65535,
                  "gemm_few_batched: %d products of %d rows, K %d, or operands without 16-byte rows", batch, M, K);
     const FewArgs a = {(const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc, batch_a, batch_w, batch_c, held};
-    const bool quarters = K > 256;
+    const bool quarters = K > 128;
     const int rows = quarters ? 16 : 16 * GF_WARPS;
     const dim3 grid((unsigned)((N + rows - 1) / rows), batch);
     auto launch = [&](auto kernel) { llmp_launch_dependent(kernel, grid, dim3(32 * GF_WARPS), 0, stream, a); };
